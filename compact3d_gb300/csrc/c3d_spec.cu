@@ -282,11 +282,13 @@ __global__ void k_ptables(Geo g, const double *ak1, const double *ak3, const dou
 
 constexpr int TWZ_MAX = 16;   // widest z-FFT tile the autotuner tries
 
+constexpr size_t SMEM_MAX = 227 * 1024;
+
 template <typename R>
 void set_spec_smem(c3d_channel *ch) {
     typedef typename Cx<R>::T C2;
     const size_t smz = 2 * (size_t)ch->g.n3m * TWZ_MAX * sizeof(C2);
-    cudaFuncSetAttribute(k_fftz<R>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smz);
+    cudaFuncSetAttribute(k_fftz<R>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(smz < SMEM_MAX ? smz : SMEM_MAX));
 }
 
 // The four-step z FFT for N3M = 32 N1; false when N3M is not of that form.
@@ -394,7 +396,8 @@ int launch_spec(c3d_channel *ch, StepArgs<R> &a, int which, int *nl) {
             return 0;
         }
     }
-    const int tw = ch->tune.twz == 0 ? 8 : ch->tune.twz;
+    int tw = ch->tune.twz == 0 ? 8 : ch->tune.twz;
+    while (tw > 1 && 2 * (size_t)ch->g.n3m * tw * sizeof(C2) > SMEM_MAX) tw /= 2;   // long FP64 lines
     const int ntile = (ch->g.n1h + tw - 1) / tw;
     const size_t smz = 2 * (size_t)ch->g.n3m * tw * sizeof(C2);
     switch (which) {
