@@ -460,112 +460,91 @@ __device__ __forceinline__ void zsweep(R (&out)[NR][L], int k0, int n, const R (
     }
 }
 
-// Cyclic carries of the segments of the block's z lines (zblock): for every recurrence q
-// and line l, a warp takes the nseg segment values v[p] = sh[(q*32 + l)*(nseg+1) + p] in
-// its lanes and replaces them by the state entering each segment.  Forward (BACK false):
-// Y(p) = v(p-1) + rL Y(p-1) cyclically, i.e. Y(p) = E(p-1) + rL^p Y(0) with the prefix
-// E(p) = v(p) + rL E(p-1) and Y(0) = E(nseg-1) / (1 - rL^nseg).  Backward: the mirror
-// image, Z(p) = v(p+1) + rL Z(p+1) from the right.  Warp-shuffle scans, log2(32) steps.
-template <typename R, int L, int NR, bool BACK>
-__device__ __forceinline__ void zcarry(const R (&r)[NR], R *sh) {
-    const int lane = threadIdx.x, w = threadIdx.y, nw = blockDim.y, nseg = blockDim.y;
-    const int pitch = nseg + 1;
-    for (int sidx = w; sidx < 32 * NR; sidx += nw) {
-        const int q = sidx >> 5, l = sidx & 31;
-        R rq = R(0);
-#pragma unroll
-        for (int t = 0; t < NR; ++t)
-            if (t == q) rq = r[t];
-        R rL = R(1);
-#pragma unroll
-        for (int t = 0; t < L; ++t) rL *= rq;
-        R *v = sh + (q * 32 + l) * pitch;
-        const int p = BACK ? nseg - 1 - lane : lane;   // position along the scan direction
-        const bool act = lane < nseg;
-        R e = act ? v[p] : R(0);
-        R pw = rL;   // rL^off
-#pragma unroll
-        for (int off = 1; off < 32; off <<= 1) {
-            const R ep = shfl_up(e, off);
-            if (lane >= off) e = e + pw * ep;
-            pw = pw * pw;
-        }
-        // rL^lane and rL^nseg by repeated squaring
-        R pl = R(1), pn = R(1), b = rL;
-#pragma unroll
-        for (int bit = 0; bit < 6; ++bit) {
-            if ((lane >> bit) & 1) pl = pl * b;
-            if ((nseg >> bit) & 1) pn = pn * b;
-            b = b * b;
-        }
-        const R tot = shfl_idx(e, nseg - 1);
-        const R y0 = tot / (R(1) - pn);
-        const R eprev = shfl_up(e, 1);
-        const R yin = (lane == 0 ? R(0) : eprev) + pl * y0;
-        if (act) v[p] = yin;
-    }
+// x^L for a compile-time L by repeated squaring.
+template <int L, typename R>
+__device__ __forceinline__ R rpow(R x) {
+    if constexpr (L == 1) return x;
+    else if constexpr (L % 2 == 0) return rpow<L / 2>(x * x);
+    else return x * rpow<L / 2>(x * x);
 }
 
-// Exact cyclic solve of NR recurrences on z lines by one block of 32 lines (threadIdx.x,
-// consecutive i) x nseg segments of L points (threadIdx.y; nseg = blockDim.y = N / L,
-// at most 32).  Each thread walks only its own segment: a local forward recurrence from
-// zero, the carries across the segments of its line (zcarry), the correction
-// y(t) += r^(t+1) Y, and the same backward.  sh holds NR*32*(nseg+1) values.  Every
-// thread of the block calls it (it synchronises the block).
-template <typename R, int L, int NR, typename F>
-__device__ __forceinline__ void zblock(R (&out)[NR][L], int k0, const R (&r)[NR], const R (&s)[NR], F &f, R *sh) {
-    const int lx = threadIdx.x, seg = threadIdx.y, pitch = blockDim.y + 1;
+// Thread layout of a joined z pass (zjoin): the block's threads are `cols` columns
+// (consecutive threads) times the nseg = N3M / L segments of a line.
+struct ZJ {
+    int cols, lx, seg, nseg;
+};
+
+// Cyclic solve of NR recurrences on z lines whose segments of L points are all in one
+// block: each thread reads its own segment's right-hand sides once (f.next), the state
+// entering a segment is joined from the segments before it (after it, backward) through
+// shared memory, and the sweeps run with it, so a solve costs 2 L multiply-adds each way
+// and no warm-up (a warm-up of M points reads M + L + M points and evaluates their
+// right-hand sides for L results).  A segment multiplies what enters it by r^L, so only
+// the K = ceil(M / L) nearest segments reach it above the precision's rounding unit
+// (|r|^M below it, as for the warm-ups).  No scale: out is B(F(d)); the caller folds s
+// into its constants.  sh holds 2 NH blockDim.x values, NH >= NR; every thread of the
+// block calls it (it synchronises the block twice; calls with the same NH may follow each
+// other directly, because a call's two exchanges use different halves of sh).
+template <typename R, int L, int M, int NR, int NH, typename F>
+__device__ __forceinline__ void zjoin(R (&out)[NR][L], int k0, const R (&r)[NR], F &f, const ZJ &z, R *sh) {
+    constexpr int K = (M + L - 1) / L;
+    const int nt = z.cols * z.nseg;
     f.start(k0);
-    R y[NR], d[NR];
+    R y[NR], d[NR], rl[NR];
 #pragma unroll
-    for (int q = 0; q < NR; ++q) y[q] = R(0);
+    for (int q = 0; q < NR; ++q) {
+        y[q] = R(0);
+        rl[q] = rpow<L>(r[q]);
+    }
 #pragma unroll
     for (int t = 0; t < L; ++t) {
         f.next(d);
 #pragma unroll
         for (int q = 0; q < NR; ++q) {
+            out[q][t] = d[q];
             y[q] = d[q] + r[q] * y[q];
-            out[q][t] = y[q];
         }
     }
-    __syncthreads();   // a previous call's readers of sh are done
 #pragma unroll
-    for (int q = 0; q < NR; ++q) sh[(q * 32 + lx) * pitch + seg] = y[q];
+    for (int q = 0; q < NR; ++q) sh[q * nt + z.seg * z.cols + z.lx] = y[q];
     __syncthreads();
-    zcarry<R, L, NR, false>(r, sh);
-    __syncthreads();
+    int p[K];
+    p[0] = z.seg == 0 ? z.nseg - 1 : z.seg - 1;
+#pragma unroll
+    for (int k = 1; k < K; ++k) p[k] = p[k - 1] == 0 ? z.nseg - 1 : p[k - 1] - 1;
 #pragma unroll
     for (int q = 0; q < NR; ++q) {
-        const R yin = sh[(q * 32 + lx) * pitch + seg];
-        R pw = r[q];
+        const R *v = sh + q * nt + z.lx;
+        R c = v[p[K - 1] * z.cols];
+#pragma unroll
+        for (int k = K - 2; k >= 0; --k) c = v[p[k] * z.cols] + rl[q] * c;
 #pragma unroll
         for (int t = 0; t < L; ++t) {
-            out[q][t] = out[q][t] + pw * yin;
-            pw *= r[q];
+            c = out[q][t] + r[q] * c;
+            out[q][t] = c;
         }
+        R b = R(0);
+#pragma unroll
+        for (int t = L - 1; t >= 0; --t) b = out[q][t] + r[q] * b;
+        y[q] = b;
     }
-    __syncthreads();   // sh is reused
+    sh += NH * nt;
+#pragma unroll
+    for (int q = 0; q < NR; ++q) sh[q * nt + z.seg * z.cols + z.lx] = y[q];
+    __syncthreads();
+    p[0] = z.seg + 1 == z.nseg ? 0 : z.seg + 1;
+#pragma unroll
+    for (int k = 1; k < K; ++k) p[k] = p[k - 1] + 1 == z.nseg ? 0 : p[k - 1] + 1;
 #pragma unroll
     for (int q = 0; q < NR; ++q) {
-        R z = R(0);
+        const R *v = sh + q * nt + z.lx;
+        R c = v[p[K - 1] * z.cols];
+#pragma unroll
+        for (int k = K - 2; k >= 0; --k) c = v[p[k] * z.cols] + rl[q] * c;
 #pragma unroll
         for (int t = L - 1; t >= 0; --t) {
-            z = out[q][t] + r[q] * z;
-            out[q][t] = z;
-        }
-        sh[(q * 32 + lx) * pitch + seg] = z;
-    }
-    __syncthreads();
-    zcarry<R, L, NR, true>(r, sh);
-    __syncthreads();
-#pragma unroll
-    for (int q = 0; q < NR; ++q) {
-        const R zin = sh[(q * 32 + lx) * pitch + seg];
-        R pw = r[q];
-#pragma unroll
-        for (int t = L - 1; t >= 0; --t) {
-            out[q][t] = s[q] * (out[q][t] + pw * zin);
-            pw *= r[q];
+            c = out[q][t] + r[q] * c;
+            out[q][t] = c;
         }
     }
 }

@@ -21,6 +21,11 @@ __device__ __forceinline__ int zprev(int k, int n) { return (k == 0) ? n - 1 : k
 // Prefetch ring of a column: the values at the D positions after the walker's current
 // one, loaded D steps before they are used so the loads of consecutive steps overlap.
 constexpr int ZPF = 4;
+// Most threads of a joined block: 64, 85, 128 or 170 registers each.
+template <typename R, int L>
+__host__ __device__ constexpr int zjt() {
+    return sizeof(R) == 8 ? (L <= 8 ? 512 : 384) : (L <= 12 ? 1024 : L <= 16 ? 768 : 384);
+}
 template <typename T>
 struct ZRing {
     T v[ZPF];
@@ -44,44 +49,65 @@ struct ZRing {
     }
 };
 
-// Thread coordinates and the line solve of the two z-pass forms: MODE 0, one thread per
-// (i, segment of L points, plane) with warm-up recurrences (zsweep); MODE 1, one block per
-// (32 consecutive i, plane) with blockDim.y = N3M / L segments and the exact cyclic
-// solve (zblock).
+// Thread coordinates and the line solve of the two z-pass forms.  MODE 0: one thread per
+// (i, segment of L points, plane) with warm-up recurrences (zsweep).  MODE 1: a block holds
+// whole lines of consecutive columns (i fastest, then the plane), one thread per segment,
+// and joins the segments through shared memory (zjoin); threads past the last column
+// compute the last one again and store nothing (zc.act).
+struct ZCo {
+    int i, j, k0;
+    bool act;
+    ZJ z;
+};
 template <int L, int MODE>
-__device__ __forceinline__ bool zcoords(const Blk blk, const Geo &g, int jlo, int &i, int &j, int &k0) {
+__device__ __forceinline__ bool zcoords(const Blk blk, const Geo &g, int jlo, ZCo &c) {
     if constexpr (MODE == 1) {
-        i = (int)blk.x * 32 + (int)threadIdx.x;
-        j = jlo + (int)blk.y;
-        k0 = (int)threadIdx.y * L;
+        c.z.nseg = g.n3m / L;
+        c.z.cols = (int)blockDim.x / c.z.nseg;
+        const int sh = 31 - __clz(c.z.cols);   // cols is a power of 2
+        c.z.seg = (int)threadIdx.x >> sh;
+        c.z.lx = (int)threadIdx.x & (c.z.cols - 1);
+        const unsigned n1 = (unsigned)g.n1m, tot = (unsigned)(g.n2m - jlo + 1) * n1;
+        unsigned q = blk.x * (unsigned)c.z.cols + (unsigned)c.z.lx;
+        c.act = q < tot;
+        if (!c.act) q = tot - 1;
+        const unsigned jq = q / n1;
+        c.i = (int)(q - jq * n1);
+        c.j = jlo + (int)jq;
+        c.k0 = c.z.seg * L;
         return true;
     } else {
-        return zcoord<L>(blk, g, jlo, i, j, k0);
+        c.act = zcoord<L>(blk, g, jlo, c.i, c.j, c.k0);
+        return c.act;
     }
 }
-template <typename R, int L, int M, int NR, int MODE, typename F>
-__device__ __forceinline__ void zsolve(R (&out)[NR][L], int k0, int n, const R (&r)[NR], const R (&s)[NR], F &f) {
+// MODE 0: out = s B(F(d)) as the reference's solve; MODE 1: out = B(F(d)), the caller's
+// constants carry s and the right-hand side's factor (zfold).
+template <typename R, int L, int M, int NR, int MODE, int NH = NR, typename F>
+__device__ __forceinline__ void zsolve(R (&out)[NR][L], const ZCo &c, int n, const R (&r)[NR], const R (&s)[NR], F &f) {
     if constexpr (MODE == 1) {
         extern __shared__ __align__(16) unsigned char zsh_raw[];
-        zblock<R, L, NR>(out, k0, r, s, f, reinterpret_cast<R *>(zsh_raw));
+        zjoin<R, L, M, NR, NH>(out, c.k0, r, f, c.z, reinterpret_cast<R *>(zsh_raw));
     } else {
-        zsweep<R, L, M, NR>(out, k0, n, r, s, f);
+        zsweep<R, L, M, NR>(out, c.k0, n, r, s, f);
     }
 }
-// L2 prefetch margin around a thread's positions: the warm-up length (MODE 0) or one point.
-template <int MODE>
-constexpr int zmargin(int m) { return MODE == 1 ? 1 : m + 1; }
+// The factor of a walker's right-hand side (1 in MODE 1) and of a solve's result (f s in MODE 1).
+template <int MODE, typename R>
+__device__ __forceinline__ R zrhs(R f) { return MODE == 1 ? R(1) : f; }
+template <int MODE, typename R>
+__device__ __forceinline__ R zfold(R f, R s) { return MODE == 1 ? f * s : R(1); }
 
 // state column: (1,10,1) RHS f12*(u- - 2u + u+) and (1,6,1) RHS 4*(u- + u) (face k)
 template <typename R>
 struct WalkVisBack {
     typedef typename SType<R>::S S;
-    const S *col; int n, s; R f12; S um, uc; ZRing<S> ru;
+    const S *col; int n, s; R f12, four; S um, uc; ZRing<S> ru;
     __device__ void start(int k) { um = col[zprev(k, n) * s]; uc = col[k * s]; ru.fill(col, k, n, s); }
     __device__ void next(R (&d)[2]) {
         S up = ru.pop(col, n, s);
         d[0] = f12 * St<R>::d2(um, uc, up);
-        d[1] = (R)4.0 * (St<R>::hi(um) + St<R>::hi(uc));
+        d[1] = four * (St<R>::hi(um) + St<R>::hi(uc));
         um = uc; uc = up;
     }
 };
@@ -90,7 +116,7 @@ struct WalkVisBack {
 template <typename R>
 struct WalkWP {
     typedef typename SType<R>::S S;
-    const S *W, *P; int n, s; R f12, f24; S wm, wc, pm, pc; ZRing<S> rw, rp;
+    const S *W, *P; int n, s; R f12, four, f24; S wm, wc, pm, pc; ZRing<S> rw, rp;
     __device__ void start(int k) {
         wm = W[zprev(k, n) * s]; wc = W[k * s]; pm = P[zprev(k, n) * s]; pc = P[k * s];
         rw.fill(W, k, n, s);
@@ -99,7 +125,7 @@ struct WalkWP {
     __device__ void next(R (&d)[3]) {
         S wp = rw.pop(W, n, s);
         d[0] = f12 * St<R>::d2(wm, wc, wp);
-        d[1] = (R)4.0 * (St<R>::hi(wc) + St<R>::hi(wp));
+        d[1] = four * (St<R>::hi(wc) + St<R>::hi(wp));
         d[2] = f24 * St<R>::d(pc, pm);
         wm = wc; wc = wp; pm = pc; pc = rp.pop(P, n, s);
     }
@@ -174,116 +200,140 @@ __device__ __forceinline__ void b_zA(const StepArgs<R> &a, const Blk blk) {
     typedef typename SType<R>::S S;
     typedef St<R> ST;
     const Geo g = a.g;
-    int i, j, k0;
-    if (!zcoords<L, MODE>(blk, g, 1, i, j, k0)) return;
+    ZCo c;
+    // the v sweep has no face at J = 1: joined lines start at J = 2, so that a block's
+    // threads all take part in the solve
+    if (!zcoords<L, MODE>(blk, g, MODE == 1 && PART == 3 ? 2 : 1, c)) return;
+    const int i = c.i, j = c.j, k0 = c.k0;
     const int n = g.n3m, s = g.n1m;
     const R RE1 = a.re1;
     const long long o = fidx(g, i, j, 0);
     constexpr int M6 = WM<R>::M6;
-    if ((g.n1m & 31) == 0) {   // the warp's column windows (32 consecutive i), requested at once
+    constexpr int NH = PART == 0 ? 3 : 2;   // the fused form's three solves share the exchange area
+    if (MODE == 0 && (g.n1m & 31) == 0) {   // the warp's column windows (32 consecutive i), requested at once
         const int lane = threadIdx.x & 31;
         const long long o0 = fidx(g, i - lane, j, 0), sb = (long long)g.n1m;
         const int ss = 32 * (int)sizeof(S), sr = 32 * (int)sizeof(R);
         if (PART <= 1) {
-            pf_cols(a.u + o0, sb * sizeof(S), ss, k0, zmargin<MODE>(M6), L, n, lane);
+            pf_cols(a.u + o0, sb * sizeof(S), ss, k0, M6 + 1, L, n, lane);
             pf_cols(a.ww1 + o0, sb * sizeof(R), sr, k0, 0, L, n, lane);
             pf_cols(a.r[0] + o0, sb * sizeof(R), sr, k0, 0, L, n, lane);
         }
         if (PART == 0 || PART == 2) {
-            pf_cols(a.w + o0, sb * sizeof(S), ss, k0, zmargin<MODE>(M6), L, n, lane);
-            pf_cols(a.p + o0, sb * sizeof(S), ss, k0, zmargin<MODE>(M6), L, n, lane);
+            pf_cols(a.w + o0, sb * sizeof(S), ss, k0, M6 + 1, L, n, lane);
+            pf_cols(a.p + o0, sb * sizeof(S), ss, k0, M6 + 1, L, n, lane);
             pf_cols(a.r[2] + o0, sb * sizeof(R), sr, k0, 0, L, n, lane);
         }
         if ((PART == 0 || PART == 3) && j >= 2) {
-            pf_cols(a.v + o0, sb * sizeof(S), ss, k0, zmargin<MODE>(M6), L, n, lane);
+            pf_cols(a.v + o0, sb * sizeof(S), ss, k0, M6 + 1, L, n, lane);
             pf_cols(a.r[1] + o0, sb * sizeof(R), sr, k0, 0, L, n, lane);
             // w at the y face: planes J and J-1 of the segment, read after the solve
             if (PART == 3) pf_cols(a.w + o0, sb * sizeof(S), ss, k0, 0, L, n, lane);
             pf_cols(a.w + fidx(g, i - lane, j - 1, 0), sb * sizeof(S), ss, k0, 0, L, n, lane);
         }
     }
+    const R f12 = zrhs<MODE>(a.f12z), four = zrhs<MODE>((R)4.0), f24 = zrhs<MODE>(a.f24z);
+    const R kv = RE1 * zfold<MODE>(a.f12z, a.c10z.s), ki = zfold<MODE>((R)4.0, a.c6z.s), kp = zfold<MODE>(a.f24z, a.c22z.s);
     if (PART == 0 || PART == 1) {   // u: R1 += (1/RE) d2u/dz2 ; E_xz = UU3 * WW1
         R out[2][L];
         const R rr[2] = {a.c10z.r, a.c6z.r}, ss[2] = {a.c10z.s, a.c6z.s};
-        WalkVisBack<R> f{a.u + o, n, s, a.f12z};
-        zsolve<R, L, M6, 2, MODE>(out, k0, n, rr, ss, f);
+        WalkVisBack<R> f{a.u + o, n, s, f12, four};
+        zsolve<R, L, M6, 2, MODE, NH>(out, c, n, rr, ss, f);
         R *Rp = a.r[0] + o, *E = a.exz + o;
         const R *Wx = a.ww1 + o;
+        if (c.act) {
 #pragma unroll
-        for (int t = 0; t < L; ++t) {
-            const int kk = (k0 + t) * s;
-            Rp[kk] = Rp[kk] + RE1 * out[0][t];
-            E[kk] = out[1][t] * Wx[kk];
+            for (int t = 0; t < L; ++t) {
+                const int kk = (k0 + t) * s;
+                Rp[kk] = Rp[kk] + kv * out[0][t];
+                E[kk] = MODE == 1 ? out[1][t] * (ki * Wx[kk]) : out[1][t] * Wx[kk];
+            }
         }
     }
     if (PART == 0 || PART == 2) {   // w, P: R3 += (1/RE) d2w/dz2 - dP/dz - PRESG3 ; WW3^2
         R out[3][L];
         const R rr[3] = {a.c10z.r, a.c6z.r, a.c22z.r}, ss[3] = {a.c10z.s, a.c6z.s, a.c22z.s};
-        WalkWP<R> f{a.w + o, a.p + o, n, s, a.f12z, a.f24z};
-        zsolve<R, L, M6, 3, MODE>(out, k0, n, rr, ss, f);
+        WalkWP<R> f{a.w + o, a.p + o, n, s, f12, four, f24};
+        zsolve<R, L, M6, 3, MODE>(out, c, n, rr, ss, f);
         const R presg3 = (R)a.scal[SCAL_PRESG3];
         R *Rp = a.r[2] + o, *Q = a.wsq + o;
+        if (c.act) {
 #pragma unroll
-        for (int t = 0; t < L; ++t) {
-            const int kk = (k0 + t) * s;
-            Rp[kk] = Rp[kk] + RE1 * out[0][t] - out[2][t] - presg3;
-            Q[kk] = out[1][t] * out[1][t];
+            for (int t = 0; t < L; ++t) {
+                const int kk = (k0 + t) * s;
+                if constexpr (MODE == 1) {
+                    Rp[kk] = Rp[kk] + kv * out[0][t] - kp * out[2][t] - presg3;
+                    const R ww3 = ki * out[1][t];
+                    Q[kk] = ww3 * ww3;
+                } else {
+                    Rp[kk] = Rp[kk] + RE1 * out[0][t] - out[2][t] - presg3;
+                    Q[kk] = out[1][t] * out[1][t];
+                }
+            }
         }
     }
-    if ((PART == 0 || PART == 3) && j >= 2) {   // v: R2 += (1/RE) d2v/dz2 ; E_yz = VV3 * (w at y face J)
+    if (PART == 0 || PART == 3) {   // v: R2 += (1/RE) d2v/dz2 ; E_yz = VV3 * (w at y face J)
+        if (MODE == 0 && j < 2) return;
         R out[2][L];
         const R rr[2] = {a.c10z.r, a.c6z.r}, ss[2] = {a.c10z.s, a.c6z.s};
-        WalkVisBack<R> f{a.v + o, n, s, a.f12z};
-        zsolve<R, L, M6, 2, MODE>(out, k0, n, rr, ss, f);
+        WalkVisBack<R> f{a.v + o, n, s, f12, four};
+        zsolve<R, L, M6, 2, MODE, NH>(out, c, n, rr, ss, f);
         const R Hj1 = a.m.rh[j], a1 = a.m.hdy[j], a2 = a.m.hdy[j - 1];
         const S *W = a.w + o, *Wm = a.w + fidx(g, i, j - 1, 0);
         R *Rp = a.r[1] + o, *E = a.eyz + o;
+        if (c.act && j >= 2) {
+            const R b1 = ki * Hj1 * a1, b2 = ki * Hj1 * a2;
 #pragma unroll
-        for (int t = 0; t < L; ++t) {
-            const int kk = (k0 + t) * s;
-            Rp[kk] = Rp[kk] + RE1 * out[0][t];
-            R wy = Hj1 * (a1 * ST::hi(Wm[kk]) + a2 * ST::hi(W[kk]));
-            E[kk] = out[1][t] * wy;
+            for (int t = 0; t < L; ++t) {
+                const int kk = (k0 + t) * s;
+                Rp[kk] = Rp[kk] + kv * out[0][t];
+                R wy = MODE == 1 ? b1 * ST::hi(Wm[kk]) + b2 * ST::hi(W[kk])
+                                 : Hj1 * (a1 * ST::hi(Wm[kk]) + a2 * ST::hi(W[kk]));
+                E[kk] = out[1][t] * wy;
+            }
         }
     }
 }
 template <typename R, int L, int PART, int MODE>
-__global__ void __launch_bounds__(MODE == 1 ? 1024 : TPB) k_zA(StepArgs<R> a) {
+__global__ void __launch_bounds__(MODE == 1 ? zjt<R, L>() : TPB) k_zA(StepArgs<R> a) {
     b_zA<R, L, PART, MODE>(a, Blk{blockIdx.x, blockIdx.y, gridDim.x});
 }
 
 template <typename R, int L, int MODE>
 __device__ __forceinline__ void b_zB(const StepArgs<R> &a, const Blk blk) {
     const Geo g = a.g;
-    int i, j, k0;
-    if (!zcoords<L, MODE>(blk, g, 1, i, j, k0)) return;
+    ZCo c;
+    if (!zcoords<L, MODE>(blk, g, 1, c)) return;
+    const int i = c.i, j = c.j, k0 = c.k0;
     const int n = g.n3m, s = g.n1m;
     const long long o = fidx(g, i, j, 0);
-    if ((g.n1m & 31) == 0) {
+    if (MODE == 0 && (g.n1m & 31) == 0) {
         const int lane = threadIdx.x & 31;
         const long long o0 = fidx(g, i - lane, j, 0), sb = (long long)g.n1m;
-        pf_cols(a.exz + o0, sb * sizeof(R), 32 * (int)sizeof(R), k0, zmargin<MODE>(WM<R>::M22), L, n, lane);
-        pf_cols(a.wsq + o0, sb * sizeof(R), 32 * (int)sizeof(R), k0, zmargin<MODE>(WM<R>::M22), L, n, lane);
-        pf_cols(a.eyz + o0, sb * sizeof(R), 32 * (int)sizeof(R), k0, zmargin<MODE>(WM<R>::M22), L, n, lane);
+        pf_cols(a.exz + o0, sb * sizeof(R), 32 * (int)sizeof(R), k0, WM<R>::M22 + 1, L, n, lane);
+        pf_cols(a.wsq + o0, sb * sizeof(R), 32 * (int)sizeof(R), k0, WM<R>::M22 + 1, L, n, lane);
+        pf_cols(a.eyz + o0, sb * sizeof(R), 32 * (int)sizeof(R), k0, WM<R>::M22 + 1, L, n, lane);
         pf_cols(a.hh[0] + o0, sb * sizeof(R), 32 * (int)sizeof(R), k0, 0, L, n, lane);
         pf_cols(a.hh[1] + o0, sb * sizeof(R), 32 * (int)sizeof(R), k0, 0, L, n, lane);
     }
     R out[3][L];
     const R rr[3] = {a.c22z.r, a.c22z.r, a.c22z.r}, ss[3] = {a.c22z.s, a.c22z.s, a.c22z.s};
-    WalkZB<R> f{a.exz + o, a.wsq + o, a.eyz + o, n, s, a.f24z};
+    WalkZB<R> f{a.exz + o, a.wsq + o, a.eyz + o, n, s, zrhs<MODE>(a.f24z)};
     f.v = (j >= 2);
-    zsolve<R, L, WM<R>::M22, 3, MODE>(out, k0, n, rr, ss, f);
+    zsolve<R, L, WM<R>::M22, 3, MODE>(out, c, n, rr, ss, f);
     R *H1 = a.hh[0] + o, *H2 = a.hh[1] + o, *H3 = a.hh[2] + o;
+    const R ks = zfold<MODE>(a.f24z, a.c22z.s);
+    if (!c.act) return;
 #pragma unroll
     for (int t = 0; t < L; ++t) {
         const int kk = (k0 + t) * s;
-        H1[kk] = H1[kk] + out[0][t];          // d(uw)/dz
-        H3[kk] = out[1][t];                   // d(ww)/dz
-        if (j >= 2) H2[kk] = H2[kk] + out[2][t];   // d(vw)/dz
+        H1[kk] = H1[kk] + ks * out[0][t];          // d(uw)/dz
+        H3[kk] = ks * out[1][t];                   // d(ww)/dz
+        if (j >= 2) H2[kk] = H2[kk] + ks * out[2][t];   // d(vw)/dz
     }
 }
 template <typename R, int L, int MODE>
-__global__ void __launch_bounds__(MODE == 1 ? 1024 : TPB) k_zB(StepArgs<R> a) {
+__global__ void __launch_bounds__(MODE == 1 ? zjt<R, L>() : TPB) k_zB(StepArgs<R> a) {
     b_zB<R, L, MODE>(a, Blk{blockIdx.x, blockIdx.y, gridDim.x});
 }
 
@@ -292,34 +342,37 @@ __global__ void __launch_bounds__(MODE == 1 ? 1024 : TPB) k_zB(StepArgs<R> a) {
 template <typename R, int L, int MODE>
 __device__ __forceinline__ void b_zC(const StepArgs<R> &a, R *d0, R *d1, R *d2, const Blk blk) {
     const Geo g = a.g;
-    int i, j, k0;
-    if (!zcoords<L, MODE>(blk, g, 1, i, j, k0)) return;
+    ZCo c;
+    if (!zcoords<L, MODE>(blk, g, 1, c)) return;
+    const int i = c.i, j = c.j, k0 = c.k0;
     const int n = g.n3m, s = g.n1m;
     const long long o = fidx(g, i, j, 0);
-    if ((g.n1m & 31) == 0) {
+    if (MODE == 0 && (g.n1m & 31) == 0) {
         const int lane = threadIdx.x & 31;
         const long long o0 = fidx(g, i - lane, j, 0), sb = (long long)g.n1m;
-        pf_cols(a.r[0] + o0, sb * sizeof(R), 32 * (int)sizeof(R), k0, zmargin<MODE>(WM<R>::MCN), L, n, lane);
-        pf_cols(a.r[1] + o0, sb * sizeof(R), 32 * (int)sizeof(R), k0, zmargin<MODE>(WM<R>::MCN), L, n, lane);
-        pf_cols(a.r[2] + o0, sb * sizeof(R), 32 * (int)sizeof(R), k0, zmargin<MODE>(WM<R>::MCN), L, n, lane);
+        pf_cols(a.r[0] + o0, sb * sizeof(R), 32 * (int)sizeof(R), k0, WM<R>::MCN + 1, L, n, lane);
+        pf_cols(a.r[1] + o0, sb * sizeof(R), 32 * (int)sizeof(R), k0, WM<R>::MCN + 1, L, n, lane);
+        pf_cols(a.r[2] + o0, sb * sizeof(R), 32 * (int)sizeof(R), k0, WM<R>::MCN + 1, L, n, lane);
     }
     R out[3][L];
     const R rr[3] = {a.cnz.r, a.cnz.r, a.cnz.r}, ss[3] = {a.cnz.s, a.cnz.s, a.cnz.s};
     WalkCN<R> f;
     f.X[0] = a.r[0] + o; f.X[1] = a.r[1] + o; f.X[2] = a.r[2] + o;
     f.n = n; f.s = s;
-    zsolve<R, L, WM<R>::MCN, 3, MODE>(out, k0, n, rr, ss, f);
+    zsolve<R, L, WM<R>::MCN, 3, MODE>(out, c, n, rr, ss, f);
     R *D0 = d0 + o, *D1 = d1 + o, *D2 = d2 + o;
+    const R ks = zfold<MODE>(R(1), a.cnz.s);
+    if (!c.act) return;
 #pragma unroll
     for (int t = 0; t < L; ++t) {
         const int kk = (k0 + t) * s;
-        D0[kk] = out[0][t];
-        D1[kk] = out[1][t];
-        D2[kk] = out[2][t];
+        D0[kk] = ks * out[0][t];
+        D1[kk] = ks * out[1][t];
+        D2[kk] = ks * out[2][t];
     }
 }
 template <typename R, int L, int MODE>
-__global__ void __launch_bounds__(MODE == 1 ? 1024 : TPB) k_zC(StepArgs<R> a, R *d0, R *d1, R *d2) {
+__global__ void __launch_bounds__(MODE == 1 ? zjt<R, L>() : TPB) k_zC(StepArgs<R> a, R *d0, R *d1, R *d2) {
     b_zC<R, L, MODE>(a, d0, d1, d2, Blk{blockIdx.x, blockIdx.y, gridDim.x});
 }
 
@@ -327,27 +380,29 @@ __global__ void __launch_bounds__(MODE == 1 ? 1024 : TPB) k_zC(StepArgs<R> a, R 
 template <typename R, int L, int MODE>
 __device__ __forceinline__ void b_zD(const StepArgs<R> &a, const R *d2, const Blk blk) {
     const Geo g = a.g;
-    int i, j, k0;
-    if (!zcoords<L, MODE>(blk, g, 1, i, j, k0)) return;
+    ZCo c;
+    if (!zcoords<L, MODE>(blk, g, 1, c)) return;
+    const int i = c.i, j = c.j, k0 = c.k0;
     const int n = g.n3m, s = g.n1m;
     const long long o = fidx(g, i, j, 0);
-    if ((g.n1m & 31) == 0) {
+    if (MODE == 0 && (g.n1m & 31) == 0) {
         const int lane = threadIdx.x & 31;
         const long long o0 = fidx(g, i - lane, j, 0), sb = (long long)g.n1m;
-        pf_cols(a.w + o0, sb * sizeof(typename SType<R>::S), 32 * (int)sizeof(typename SType<R>::S), k0, zmargin<MODE>(WM<R>::M22), L, n, lane);
-        pf_cols(d2 + o0, sb * sizeof(R), 32 * (int)sizeof(R), k0, zmargin<MODE>(WM<R>::M22), L, n, lane);
+        pf_cols(a.w + o0, sb * sizeof(typename SType<R>::S), 32 * (int)sizeof(typename SType<R>::S), k0, WM<R>::M22 + 1, L, n, lane);
+        pf_cols(d2 + o0, sb * sizeof(R), 32 * (int)sizeof(R), k0, WM<R>::M22 + 1, L, n, lane);
     }
     R out[1][L];
     const R rr[1] = {a.c22z.r}, ss[1] = {a.c22z.s};
-    WalkDivZ<R> f{a.w + o, d2 + o, n, s, a.f24z};
-    zsolve<R, L, WM<R>::M22, 1, MODE>(out, k0, n, rr, ss, f);
-    const R rdt = a.rdt;
+    WalkDivZ<R> f{a.w + o, d2 + o, n, s, zrhs<MODE>(a.f24z)};
+    zsolve<R, L, WM<R>::M22, 1, MODE>(out, c, n, rr, ss, f);
+    const R rdt = a.rdt * zfold<MODE>(a.f24z, a.c22z.s);
     R *Q = a.rdpz + o;
+    if (!c.act) return;
 #pragma unroll
     for (int t = 0; t < L; ++t) Q[(k0 + t) * s] = out[0][t] * rdt;
 }
 template <typename R, int L, int MODE>
-__global__ void __launch_bounds__(MODE == 1 ? 1024 : TPB) k_zD(StepArgs<R> a, const R *d2) {
+__global__ void __launch_bounds__(MODE == 1 ? zjt<R, L>() : TPB) k_zD(StepArgs<R> a, const R *d2) {
     b_zD<R, L, MODE>(a, d2, Blk{blockIdx.x, blockIdx.y, gridDim.x});
 }
 
@@ -357,17 +412,18 @@ __device__ __forceinline__ void b_zE(const StepArgs<R> &a, const R *d0, const R 
     typedef typename SType<R>::S S;
     typedef St<R> ST;
     const Geo g = a.g;
-    int i, j, k0;
-    if (!zcoords<L, MODE>(blk, g, 1, i, j, k0)) return;
+    ZCo c;
+    if (!zcoords<L, MODE>(blk, g, 1, c)) return;
+    const int i = c.i, j = c.j, k0 = c.k0;
     const int n = g.n3m, s = g.n1m;
     const long long o = fidx(g, i, j, 0);
     const R dt = (R)a.dt;
     const R dtdm = dt * (R)a.scal[SCAL_DMPRESG], dtdm3 = dt * (R)a.scal[SCAL_DMPRESG3];
     const R *DP = a.dp + o;
-    if ((g.n1m & 31) == 0) {
+    if (MODE == 0 && (g.n1m & 31) == 0) {
         const int lane = threadIdx.x & 31;
         const long long o0 = fidx(g, i - lane, j, 0), sb = (long long)g.n1m;
-        pf_cols(a.dp + o0, sb * sizeof(R), 32 * (int)sizeof(R), k0, zmargin<MODE>(WM<R>::M22), L, n, lane);
+        pf_cols(a.dp + o0, sb * sizeof(R), 32 * (int)sizeof(R), k0, WM<R>::M22 + 1, L, n, lane);
         pf_cols(a.u + o0, sb * sizeof(S), 32 * (int)sizeof(S), k0, 0, L, n, lane);
         pf_cols(a.v + o0, sb * sizeof(S), 32 * (int)sizeof(S), k0, 0, L, n, lane);
         pf_cols(a.w + o0, sb * sizeof(S), 32 * (int)sizeof(S), k0, 0, L, n, lane);
@@ -379,24 +435,28 @@ __device__ __forceinline__ void b_zE(const StepArgs<R> &a, const R *d0, const R 
     }
     R out[1][L];
     const R rr[1] = {a.c22z.r}, ss[1] = {a.c22z.s};
-    WalkGradZ<R> f{DP, n, s, a.f24z};
-    zsolve<R, L, WM<R>::M22, 1, MODE>(out, k0, n, rr, ss, f);
+    WalkGradZ<R> f{DP, n, s, zrhs<MODE>(a.f24z)};
+    zsolve<R, L, WM<R>::M22, 1, MODE>(out, c, n, rr, ss, f);
     S *W = a.w + o, *U = a.u + o, *V = a.v + o, *Pp = a.p + o;
     const R *D0 = d0 + o, *D1 = d1 + o, *D2 = d2 + o, *G1 = a.g1 + o;
     const R *DPm = a.dp + fidx(g, i, j - 1, 0);
-    const R rHj = a.m.rh[j];
+    const R rHj = a.m.rh[j], dtg = dt * zfold<MODE>(a.f24z, a.c22z.s), dth = dt * rHj;
+    if (!c.act) return;
 #pragma unroll
     for (int t = 0; t < L; ++t) {
         const int kk = (k0 + t) * s;
-        W[kk] = Sten<R>::upd(W[kk], D2[kk], dt * out[0][t], dtdm3);
+        W[kk] = Sten<R>::upd(W[kk], D2[kk], dtg * out[0][t], dtdm3);
         if constexpr (sizeof(R) == 4) U[kk] = ST::add(U[kk], G1[kk] - dtdm);   // G1: delta1 - DT dDP/dx (xD)
         else U[kk] = Sten<R>::upd(U[kk], D0[kk], dt * G1[kk], dtdm);
-        if (j >= 2) V[kk] = Sten<R>::upd(V[kk], D1[kk], dt * (DP[kk] - DPm[kk]) * rHj, R(0));
+        if (j >= 2) {
+            const R dpy = MODE == 1 ? dth * (DP[kk] - DPm[kk]) : dt * (DP[kk] - DPm[kk]) * rHj;
+            V[kk] = Sten<R>::upd(V[kk], D1[kk], dpy, R(0));
+        }
         if (updp) Pp[kk] = ST::add(Pp[kk], DP[kk]);
     }
 }
 template <typename R, int L, int MODE>
-__global__ void __launch_bounds__(MODE == 1 ? 1024 : TPB) k_zE(StepArgs<R> a, const R *d0, const R *d1, const R *d2, int updp) {
+__global__ void __launch_bounds__(MODE == 1 ? zjt<R, L>() : TPB) k_zE(StepArgs<R> a, const R *d0, const R *d1, const R *d2, int updp) {
     b_zE<R, L, MODE>(a, d0, d1, d2, updp, Blk{blockIdx.x, blockIdx.y, gridDim.x});
 }
 
@@ -440,12 +500,36 @@ __global__ void __launch_bounds__(TPB) k_diag_z(StepArgs<R> a, const double *div
 template <typename R, int L, int MODE>
 static int launch_zpass_l(c3d_channel *ch, StepArgs<R> &a, int which, R *d0, R *d1, R *d2, int flag, int *nl);
 
-// Segment length of the block form (MODE 1) for N3M points: the smallest of 8, 12, 16
-// that divides N3M into at most 32 segments, or 0 when none does.
-int zblock_len(int n3m) {
-    for (int L : {8, 12, 16})
-        if (n3m % L == 0 && n3m / L <= 32) return L;
-    return 0;
+// Columns per block of a joined pass with segments of L points, or 0 when a line has too
+// many segments for a block.  FP64: the fewest of 8, 16, 32 that give 96 threads (small
+// blocks overlap one block's loads with another's FP64 arithmetic: 192 x 128 x 144 points,
+// L = 12, the seven z sweeps 0.84 ms at 8 columns, 0.89 at 16, 0.98 at 32).  FP32: the most
+// up to 32 that a block holds (whole sectors of 4-byte rows).
+template <typename R, int L>
+static int zjoin_cols(int n3m) {
+    const int nseg = n3m / L, most = zjt<R, L>();
+    if (n3m % L != 0 || 8 * nseg > most) return 0;
+    int cols = 8;
+    if (sizeof(R) == 8) while (cols < 32 && cols * nseg < 96) cols *= 2;
+    else while (cols < 32 && 2 * cols * nseg <= most) cols *= 2;
+    return cols;
+}
+
+// The segment length of a joined pass over N3M points, 0 when no length fits (the warm-up
+// form runs).  FP64, whatever the schedule: 12 where it divides N3M, else 8, else 16 (long
+// lines).  Against 12 at N3M = 144, 8 and 16 cost 12% and 9% more over the seven z sweeps;
+// at N3M = 64, 16 costs 9% more than 8.  FP32 (schedule 0): 8, 12 or 16, at most 32 segments.
+template <typename R>
+static int zjoin_len(int n3m) {
+    if constexpr (sizeof(R) == 8) {
+        if (zjoin_cols<R, 12>(n3m)) return 12;
+        if (zjoin_cols<R, 8>(n3m)) return 8;
+        return zjoin_cols<R, 16>(n3m) ? 16 : 0;
+    } else {
+        if (n3m % 8 == 0 && n3m / 8 <= 32) return 8;
+        if (n3m % 12 == 0 && n3m / 12 <= 32) return 12;
+        return n3m % 16 == 0 && n3m / 16 <= 32 ? 16 : 0;
+    }
 }
 
 // ---------------------------------------------------------------------------------
@@ -453,48 +537,59 @@ int zblock_len(int n3m) {
 // points, which divides every supported N3M); zA as its three sweeps; the work arrays
 // are the channel's exz / eyz / wsq as in the step, and zE adds DP to P.
 // ---------------------------------------------------------------------------------
-template <typename R, int PART, int L>
-__global__ void __launch_bounds__(TPB) kb_zA(const StepArgs<R> *__restrict__ A, const BMap *__restrict__ map) {
+template <typename R, int PART, int L, int MODE>
+__global__ void __launch_bounds__(MODE == 1 ? zjt<R, L>() : TPB) kb_zA(const StepArgs<R> *__restrict__ A, const BMap *__restrict__ map) {
     const BMap m = map[blockIdx.x];
-    b_zA<R, L, PART, 0>(A[m.ch], Blk{m.x, m.y, m.gx});
+    b_zA<R, L, PART, MODE>(A[m.ch], Blk{m.x, m.y, m.gx});
 }
-template <typename R, int L>
-__global__ void __launch_bounds__(TPB) kb_zB(const StepArgs<R> *__restrict__ A, const BMap *__restrict__ map) {
+template <typename R, int L, int MODE>
+__global__ void __launch_bounds__(MODE == 1 ? zjt<R, L>() : TPB) kb_zB(const StepArgs<R> *__restrict__ A, const BMap *__restrict__ map) {
     const BMap m = map[blockIdx.x];
-    b_zB<R, L, 0>(A[m.ch], Blk{m.x, m.y, m.gx});
+    b_zB<R, L, MODE>(A[m.ch], Blk{m.x, m.y, m.gx});
 }
-template <typename R, int L>
-__global__ void __launch_bounds__(TPB) kb_zC(const StepArgs<R> *__restrict__ A, const BMap *__restrict__ map) {
+template <typename R, int L, int MODE>
+__global__ void __launch_bounds__(MODE == 1 ? zjt<R, L>() : TPB) kb_zC(const StepArgs<R> *__restrict__ A, const BMap *__restrict__ map) {
     const BMap m = map[blockIdx.x];
     const StepArgs<R> &a = A[m.ch];
-    b_zC<R, L, 0>(a, a.exz, a.eyz, a.wsq, Blk{m.x, m.y, m.gx});
+    b_zC<R, L, MODE>(a, a.exz, a.eyz, a.wsq, Blk{m.x, m.y, m.gx});
 }
-template <typename R, int L>
-__global__ void __launch_bounds__(TPB) kb_zD(const StepArgs<R> *__restrict__ A, const BMap *__restrict__ map) {
+template <typename R, int L, int MODE>
+__global__ void __launch_bounds__(MODE == 1 ? zjt<R, L>() : TPB) kb_zD(const StepArgs<R> *__restrict__ A, const BMap *__restrict__ map) {
     const BMap m = map[blockIdx.x];
     const StepArgs<R> &a = A[m.ch];
-    b_zD<R, L, 0>(a, a.wsq, Blk{m.x, m.y, m.gx});
+    b_zD<R, L, MODE>(a, a.wsq, Blk{m.x, m.y, m.gx});
 }
-template <typename R, int L>
-__global__ void __launch_bounds__(TPB) kb_zE(const StepArgs<R> *__restrict__ A, const BMap *__restrict__ map) {
+template <typename R, int L, int MODE>
+__global__ void __launch_bounds__(MODE == 1 ? zjt<R, L>() : TPB) kb_zE(const StepArgs<R> *__restrict__ A, const BMap *__restrict__ map) {
     const BMap m = map[blockIdx.x];
     const StepArgs<R> &a = A[m.ch];
-    b_zE<R, L, 0>(a, a.exz, a.eyz, a.wsq, 1, Blk{m.x, m.y, m.gx});
+    b_zE<R, L, MODE>(a, a.exz, a.eyz, a.wsq, 1, Blk{m.x, m.y, m.gx});
 }
 
-template <typename R, int L>
+template <typename R, int L, int MODE>
 static int zbk(const c3d_channel *ch, int which, std::vector<BKern> &out) {
-    const unsigned nb = (unsigned)nblk((long long)ch->g.n2m * (ch->g.n3m / L) * ch->g.n1m);
+    const Geo &g = ch->g;
+    const unsigned nb = (unsigned)nblk((long long)g.n2m * (g.n3m / L) * g.n1m);
+    auto put = [&](auto *fn, int njoin, int jn, int run, int piece) {
+        if (MODE == 0) {
+            out.push_back({(const void *)fn, TPB, 0, nb, run, piece});
+            return;
+        }
+        const long long ncol = (long long)jn * g.n1m;
+        const int cols = zjoin_cols<R, L>(g.n3m);
+        const unsigned nt = (unsigned)(cols * (g.n3m / L));
+        out.push_back({(const void *)fn, nt, 2 * (size_t)njoin * nt * sizeof(R), (unsigned)nblk(ncol, cols), run, piece});
+    };
     switch (which) {
         case 0:
-            out.push_back({(const void *)kb_zA<R, 1, L>, TPB, 0, nb, 2, 0});
-            out.push_back({(const void *)kb_zA<R, 2, L>, TPB, 0, nb, 2, 1});
-            out.push_back({(const void *)kb_zA<R, 3, L>, TPB, 0, nb, 2, 2});
+            put(kb_zA<R, 1, L, MODE>, 2, g.n2m, 2, 0);
+            put(kb_zA<R, 2, L, MODE>, 3, g.n2m, 2, 1);
+            put(kb_zA<R, 3, L, MODE>, 2, g.n2m - 1, 2, 2);
             return 0;
-        case 1: out.push_back({(const void *)kb_zB<R, L>, TPB, 0, nb}); return 0;
-        case 2: out.push_back({(const void *)kb_zC<R, L>, TPB, 0, nb}); return 0;
-        case 3: out.push_back({(const void *)kb_zD<R, L>, TPB, 0, nb}); return 0;
-        case 4: out.push_back({(const void *)kb_zE<R, L>, TPB, 0, nb}); return 0;
+        case 1: put(kb_zB<R, L, MODE>, 3, g.n2m, 0, 0); return 0;
+        case 2: put(kb_zC<R, L, MODE>, 3, g.n2m, 0, 0); return 0;
+        case 3: put(kb_zD<R, L, MODE>, 1, g.n2m, 0, 0); return 0;
+        case 4: put(kb_zE<R, L, MODE>, 1, g.n2m, 0, 0); return 0;
         default: return C3D_EINVAL;
     }
 }
@@ -506,9 +601,18 @@ int zpass_bkern(const c3d_channel *ch, int which, int L, std::vector<BKern> &out
     if (ch->g.n3m % ZL != 0) return C3D_EINVAL;
     if (L != 8 && L != 32) L = 16;
     if (ch->g.n3m % L != 0) L = 16;
-    if (L == 8) return zbk<R, 8>(ch, which, out);
-    if (L == 32) return zbk<R, 32>(ch, which, out);
-    return zbk<R, 16>(ch, which, out);
+    if constexpr (sizeof(R) == 8) {   // joined segments, as for one channel
+        switch (zjoin_len<R>(ch->g.n3m)) {
+            case 8: return zbk<R, 8, 1>(ch, which, out);
+            case 12: return zbk<R, 12, 1>(ch, which, out);
+            case 16: return zbk<R, 16, 1>(ch, which, out);
+            default: return zbk<R, 16, 0>(ch, which, out);
+        }
+    } else {
+        if (L == 8) return zbk<R, 8, 0>(ch, which, out);
+        if (L == 32) return zbk<R, 32, 0>(ch, which, out);
+        return zbk<R, 16, 0>(ch, which, out);
+    }
 }
 template int zpass_bkern<double>(const c3d_channel *, int, int, std::vector<BKern> &);
 template int zpass_bkern<float>(const c3d_channel *, int, int, std::vector<BKern> &);
@@ -517,28 +621,38 @@ template <typename R>
 int launch_zpass(c3d_channel *ch, StepArgs<R> &a, int which, R *d0, R *d1, R *d2, int flag, int *nl) {
     if (which == 5) return launch_zpass_l<R, ZL, 0>(ch, a, which, d0, d1, d2, flag, nl);
     const int zl = ch->tune.zl[which];
-    if (zl == 0) {   // block form; a shape it cannot take runs the segment form with L = 16
-        switch (zblock_len(ch->g.n3m)) {
+    // FP64 always joins its segments: the FP64 pipe (2 lanes per clock and SM) bounds these
+    // passes, and with M = 23 warm-up points a segment of 16 evaluates 62 right-hand sides
+    // for 16 results.  FP32 joins them where the schedule says 0; its short warm-ups (6 to
+    // 10 points) cost less than the two block synchronisations on most shapes.
+    if (sizeof(R) == 8 || zl == 0) {
+        switch (zjoin_len<R>(ch->g.n3m)) {
             case 8: return launch_zpass_l<R, 8, 1>(ch, a, which, d0, d1, d2, flag, nl);
             case 12: return launch_zpass_l<R, 12, 1>(ch, a, which, d0, d1, d2, flag, nl);
             case 16: return launch_zpass_l<R, 16, 1>(ch, a, which, d0, d1, d2, flag, nl);
             default: return launch_zpass_l<R, 16, 0>(ch, a, which, d0, d1, d2, flag, nl);
         }
     }
-    switch (zl) {
-        case 8: return launch_zpass_l<R, 8, 0>(ch, a, which, d0, d1, d2, flag, nl);
-        case 32: return launch_zpass_l<R, 32, 0>(ch, a, which, d0, d1, d2, flag, nl);
-        default: return launch_zpass_l<R, 16, 0>(ch, a, which, d0, d1, d2, flag, nl);
+    if constexpr (sizeof(R) == 4) {
+        switch (zl) {
+            case 8: return launch_zpass_l<R, 8, 0>(ch, a, which, d0, d1, d2, flag, nl);
+            case 32: return launch_zpass_l<R, 32, 0>(ch, a, which, d0, d1, d2, flag, nl);
+            default: break;
+        }
     }
+    return launch_zpass_l<R, 16, 0>(ch, a, which, d0, d1, d2, flag, nl);
 }
 
 template <typename R, int L, int MODE>
 static int launch_zpass_l(c3d_channel *ch, StepArgs<R> &a, int which, R *d0, R *d1, R *d2, int flag, int *nl) {
-    const long long nt = (long long)ch->g.n2m * (ch->g.n3m / L) * ch->g.n1m;
-    // MODE 0: TPB-thread blocks over all threads; MODE 1: (N1M/32, N2M) blocks of 32 x N3M/L
-    const dim3 nb = MODE == 1 ? dim3(ch->g.n1m / 32, ch->g.n2m) : dim3(nblk(nt));
-    const dim3 TB = MODE == 1 ? dim3(32, ch->g.n3m / L) : dim3(TPB);
-    const size_t zsm = MODE == 1 ? 3 * 32 * (size_t)(ch->g.n3m / L + 1) * sizeof(R) : 0;
+    const Geo &g = ch->g;
+    const long long nt = (long long)g.n2m * (g.n3m / L) * g.n1m, ncol = (long long)g.n2m * g.n1m;
+    // MODE 0: TPB-thread blocks over all threads; MODE 1: blocks of `cols` whole lines
+    const int cols = MODE == 1 ? zjoin_cols<R, L>(g.n3m) : 0;
+    const dim3 nb = MODE == 1 ? dim3(nblk(ncol, cols)) : dim3(nblk(nt));
+    const dim3 TB = MODE == 1 ? dim3(cols * (g.n3m / L)) : dim3(TPB);
+    const dim3 nbv = MODE == 1 ? dim3(nblk(ncol - g.n1m, cols)) : nb;   // zA's v piece: J >= 2
+    const size_t zs1 = MODE == 1 ? 2 * (size_t)TB.x * sizeof(R) : 0, zs2 = 2 * zs1, zsm = 3 * zs1;
     cudaStream_t st = ch->stream;
     const double N = (double)ch->g.n1m * ch->g.n2m * ch->g.n3m, Rb = sizeof(R);
     switch (which) {
@@ -549,11 +663,11 @@ static int launch_zpass_l(c3d_channel *ch, StepArgs<R> &a, int which, R *d0, R *
                 const bool cc = par_on(ch);
                 int rc;
                 if (cc && (rc = par_fork(ch))) return rc;
-                k_zA<R, L, 1, MODE><<<nb, TB, zsm, cc ? ch->par[0] : st>>>(a);
+                k_zA<R, L, 1, MODE><<<nb, TB, zs2, cc ? ch->par[0] : st>>>(a);
                 mark(ch, nl, "zA_u", N * (8 + 4 * Rb));    // u; WW1, R1 -> R1, E_xz
                 k_zA<R, L, 2, MODE><<<nb, TB, zsm, cc ? ch->par[1] : st>>>(a);
                 mark(ch, nl, "zA_wp", N * (16 + 3 * Rb));  // w, P; R3 -> R3, WW3^2
-                k_zA<R, L, 3, MODE><<<nb, TB, zsm, st>>>(a);
+                k_zA<R, L, 3, MODE><<<nbv, TB, zs2, st>>>(a);
                 mark(ch, nl, "zA_v", N * (16 + 3 * Rb));   // v, w; R2 -> R2, E_yz
                 if (cc && (rc = par_join(ch))) return rc;
             } else {
@@ -563,16 +677,15 @@ static int launch_zpass_l(c3d_channel *ch, StepArgs<R> &a, int which, R *d0, R *
             break;
         case 1: k_zB<R, L, MODE><<<nb, TB, zsm, st>>>(a); mark(ch, nl, "zB", N * 8 * Rb); break;
         case 2: k_zC<R, L, MODE><<<nb, TB, zsm, st>>>(a, d0, d1, d2); mark(ch, nl, "zC", N * 6 * Rb); break;
-        case 3: k_zD<R, L, MODE><<<nb, TB, zsm, st>>>(a, d2); mark(ch, nl, "zD", N * (8 + 2 * Rb)); break;
+        case 3: k_zD<R, L, MODE><<<nb, TB, zs1, st>>>(a, d2); mark(ch, nl, "zD", N * (8 + 2 * Rb)); break;
         case 4:   // the mixed form reads delta1 - DT dDP/dx from one field (xD), FP64 both
-            k_zE<R, L, MODE><<<nb, TB, zsm, st>>>(a, d0, d1, d2, flag);
+            k_zE<R, L, MODE><<<nb, TB, zs1, st>>>(a, d0, d1, d2, flag);
             mark(ch, nl, "zE", N * (64 + (sizeof(R) == 4 ? 4 : 5) * Rb));
             break;
         case 5: {
-            if (MODE == 1) return C3D_EINVAL;   // the diagnostics run the segment form only
             const double b = 22.0, r = -2.0 / (b + sqrt(b * b - 4.0));
             Cyc<double> c22 = {r, -r, (int)ceil(log(1e-17) / log(fabs(r)))};
-            k_diag_z<R, L><<<nb, TB, zsm, st>>>(a, (const double *)d0, c22);
+            k_diag_z<R, L><<<nblk(nt), TPB, 0, st>>>(a, (const double *)d0, c22);
             mark(ch, nl, "diag_z", N * 16);
             break;
         }

@@ -374,9 +374,10 @@ int c3d_checkpoint_read(c3d_channel *ch, const char *path, int *ntime, double *t
  * (C3D_SCHEDULE_LEN):
  *   [0..4] z-line segment length (8, 16, 32) of each z pass: the points each thread
  *       solves sequentially (Thomas-like) before the parallel segments of a z line
- *       meet; or 0: one block per 32 z lines of a plane, each thread one segment of
- *       8, 12 or 16 points, the segments of a line joined exactly through shared
- *       memory (N3M / segment length <= 32; otherwise segments of 16)
+ *       meet; or 0: blocks of whole z lines, each thread one segment of 8, 12 or 16
+ *       points, the segments of a line joined through shared memory (N3M / segment
+ *       length <= 32; otherwise segments of 16).  The FP64 form always joins its
+ *       segments (12 points where 12 divides N3M, else 8, else 16), whatever these say
  *   [5] rows per block of the x passes (2, 4, 8)
  *   [6] kx columns per block of the z FFT (4, 8, 16), or 0: one warp per kx column,
  *       four-step form (N3M / 32 points per lane in registers, then a 32-point
