@@ -17,6 +17,8 @@ CSRC = os.path.join(HERE, "csrc")
 OBJ = os.path.join(HERE, "_build")
 LIB = os.path.join(HERE, "libc3d.so")
 SOURCES = ["c3d_capi.cu", "c3d_step.cu", "c3d_xpass.cu", "c3d_xbatch.cu", "c3d_zpass.cu", "c3d_spec.cu", "c3d_noalloc.cu", "c3d_les.cu", "c3d_ops.cu", "c3d_refine.cu", "c3d_ckpt.cu", "c3d_stats.cu", "c3d_iwm.cu"]
+# the kernels of both precisions, compiled once for each (C3D_BITS), which halves the build
+SPLIT = {"c3d_xpass.cu", "c3d_xbatch.cu", "c3d_zpass.cu"}
 ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]
 
 
@@ -48,11 +50,12 @@ def build(force: bool = False, verbose: bool = False, ptxas_v: bool = False) -> 
     objs = []
     for src in SOURCES:
         s = os.path.join(CSRC, src)
-        o = os.path.join(OBJ, src.replace(".cu", ".o"))
-        objs.append(o)
-        if force or _stale(o, [s] + headers):
-            extra = ["-Xptxas", "-v"] if ptxas_v else []
-            jobs.append([nv] + flags(extra) + ["-c", s, "-o", o])
+        for bits in ((32, 64) if src in SPLIT else (None,)):
+            o = os.path.join(OBJ, src.replace(".cu", f"_{bits}.o" if bits else ".o"))
+            objs.append(o)
+            if force or _stale(o, [s] + headers):
+                extra = (["-Xptxas", "-v"] if ptxas_v else []) + ([f"-DC3D_BITS={bits}"] if bits else [])
+                jobs.append([nv] + flags(extra) + ["-c", s, "-o", o])
     if jobs:
         with cf.ThreadPoolExecutor(max_workers=len(jobs)) as ex:
             futs = [ex.submit(subprocess.run, j, capture_output=True, text=True) for j in jobs]

@@ -23,6 +23,7 @@
 #pragma once
 #include <cuda_runtime.h>
 #include <stdint.h>
+#include <type_traits>
 
 namespace c3d {
 
@@ -134,6 +135,14 @@ __device__ __forceinline__ bool below_half_ulp(double x) { return fabs(x) < 0x1p
 template <typename R>
 __device__ __forceinline__ bool below_half_ulp(R) { return false; }
 
+// x^L for a compile-time L by repeated squaring.
+template <int L, typename R>
+__device__ __forceinline__ R rpow(R x) {
+    if constexpr (L == 1) return x;
+    else if constexpr (L % 2 == 0) return rpow<L / 2>(x * x);
+    else return x * rpow<L / 2>(x * x);
+}
+
 // xsolve for a row whose every lane holds a chunk (P = W): every lane's chunk multiplier is
 // r^C, so the scans combine with the constant powers r^(C 2^b) (one shuffle and one
 // multiply-add per level), the chunk sweeps carry no multiplier, and the cyclic closure
@@ -205,19 +214,63 @@ __device__ __forceinline__ void xsolve_full(R (&x)[C], int lane, const Cyc<R> &c
     }
 }
 
-// Cyclic solve on a row held as lane chunks x[0..C) by a segment of W lanes (lane =
-// the lane within the segment; W = 32: one row per warp, W < 32: 32/W rows per warp,
-// every segment of the warp calling together); in place, returns s*B(F(x)).  P = W takes
-// the constant-multiplier form above; P < W (idle lanes) the general one.
-template <int W = 32, typename R, int C>
-__device__ __forceinline__ void xsolve(R (&x)[C], int lane, int P, const Cyc<R> &c) {
-    static_assert(W == 4 || W == 8 || W == 16 || W == 32, "row segments of 4, 8, 16 or 32 lanes");
-    if (P == W) {
-        xsolve_full<W>(x, lane, c);
-        return;
+// |x| < 2^-56 by its exponent (an integer test: FP64 instructions are what bounds the FP64 form).
+__device__ __forceinline__ bool negligible(double x) { return (__double2hiint(x) & 0x7ff00000) < (1023 - 56) << 20; }
+
+// What enters each lane's chunk in the FP64 recurrences of one direction: e = the chunk's own
+// sum, m = r^C.  The sums of the lanes before it (DIR -1) or after it (DIR +1) are added over
+// a ring of P lanes by doubling, each level covering twice the lanes, and the levels stop
+// where the next factor r^(C 2^b) is below the rounding unit: after one or two for the
+// compact operators and chunks of 4 points or more (a scan over 32 lanes has five).  A level
+// that runs round the ring adds the next period of the periodic sum, so there is no closure.
+template <int W, int DIR>
+__device__ __forceinline__ double ring_carry(double e, double m, int lane, int P) {
+    int off = 1;
+    for (int b = 0; b < 12 && !negligible(m); ++b) {
+        int src = DIR < 0 ? lane - off : lane + off;
+        if (DIR < 0 && src < 0) src += P;
+        if (DIR > 0 && src >= P) src -= P;
+        e = e + m * shfl_idx(e, src, W);
+        m *= m;
+        off *= 2;
+        if (off >= P) off -= P;
     }
+    return shfl_idx(e, DIR < 0 ? (lane == 0 ? P - 1 : lane - 1) : (lane + 1 >= P ? 0 : lane + 1), W);
+}
+
+// FP64 solve on lane chunks without the scale s (B(F(d)); callers fold s into their
+// constants): two sweeps of C multiply-adds each way and the ring carries.  Against scans
+// over all lanes with per-lane multipliers and a closure it executes about half the FP64
+// instructions, and the FP64 pipe bounds the FP64 x passes (192 x 128 x 144 points: xA's
+// pieces 409, 312, 222 -> 264, 240, 152 us, xB 529 -> 353, xC 337 -> 303, xD 279 -> 244).
+template <int W, int C>
+__device__ __forceinline__ void xsolve_ring(double (&x)[C], int lane, int P, const Cyc<double> &c) {
+    const double r = c.r, m = rpow<C>(r);
+    double y = x[0];
+#pragma unroll
+    for (int t = 1; t < C; ++t) y = x[t] + r * y;
+    y = ring_carry<W, -1>(y, m, lane, P);
+#pragma unroll
+    for (int t = 0; t < C; ++t) {
+        y = x[t] + r * y;
+        x[t] = y;
+    }
+    double z = x[C - 1];
+#pragma unroll
+    for (int t = C - 2; t >= 0; --t) z = x[t] + r * z;
+    z = ring_carry<W, +1>(z, m, lane, P);
+#pragma unroll
+    for (int t = C - 1; t >= 0; --t) {
+        z = x[t] + r * z;
+        x[t] = z;
+    }
+}
+
+// The general form of a segment with idle lanes (P < W).
+template <int W, typename R, int C>
+__device__ __forceinline__ void xsolve_general(R (&x)[C], int lane, int P, const Cyc<R> &c) {
     const bool act = lane < P;
-    const R r = c.r;
+    const R r = c.r, s = c.s;
     R y = R(0), m = R(1);
 #pragma unroll
     for (int t = 0; t < C; ++t) {
@@ -268,13 +321,42 @@ __device__ __forceinline__ void xsolve(R (&x)[C], int lane, int P, const Cyc<R> 
         R en1 = shfl_down(e, 1, W), mn1 = shfl_down(m, 1, W);
         z = (lane == W - 1) ? z0 : en1 + mn1 * z0;
     }
-    const R s = c.s;
 #pragma unroll
     for (int t = C - 1; t >= 0; --t) {
         z = x[t] + r * z;
         x[t] = s * z;
     }
 }
+
+// Cyclic solve on a row held as lane chunks x[0..C) by a segment of W lanes (lane =
+// the lane within the segment; W = 32: one row per warp, W < 32: 32/W rows per warp,
+// every segment of the warp calling together); in place, returns s*B(F(x)).  FP64 takes the
+// ring form; otherwise P = W takes the constant-multiplier form above and P < W (idle lanes)
+// the general one.
+template <int W = 32, typename R, int C>
+__device__ __forceinline__ void xsolve(R (&x)[C], int lane, int P, const Cyc<R> &c) {
+    static_assert(W == 4 || W == 8 || W == 16 || W == 32, "row segments of 4, 8, 16 or 32 lanes");
+    if constexpr (std::is_same<R, double>::value) {
+        xsolve_ring<W>(x, lane, P, c);
+#pragma unroll
+        for (int t = 0; t < C; ++t) x[t] *= c.s;
+        return;
+    } else if (P == W) {
+        xsolve_full<W>(x, lane, c);
+        return;
+    }
+    if constexpr (!std::is_same<R, double>::value) xsolve_general<W>(x, lane, P, c);
+}
+
+// The same with the FP64 scale left to the caller: xfold(f, c) is the factor f of a
+// right-hand side with the operator's scale folded in (FP64) or f itself.
+template <int W = 32, typename R, int C>
+__device__ __forceinline__ void xsolve_f(R (&x)[C], int lane, int P, const Cyc<R> &c) {
+    if constexpr (std::is_same<R, double>::value) xsolve_ring<W>(x, lane, P, c);
+    else xsolve<W>(x, lane, P, c);
+}
+__device__ __forceinline__ double xfold(double f, const Cyc<double> &c) { return f * c.s; }
+__device__ __forceinline__ float xfold(float f, const Cyc<float> &) { return f; }
 
 // Lane-chunk load/store of one row (row pointer + lane*C).  Inactive lanes are skipped.
 template <int C>
@@ -458,14 +540,6 @@ __device__ __forceinline__ void zsweep(R (&out)[NR][L], int k0, int n, const R (
             out[q][t] = s[q] * z;
         }
     }
-}
-
-// x^L for a compile-time L by repeated squaring.
-template <int L, typename R>
-__device__ __forceinline__ R rpow(R x) {
-    if constexpr (L == 1) return x;
-    else if constexpr (L % 2 == 0) return rpow<L / 2>(x * x);
-    else return x * rpow<L / 2>(x * x);
 }
 
 // Thread layout of a joined z pass (zjoin): the block's threads are `cols` columns

@@ -355,8 +355,11 @@ __device__ __forceinline__ bool mbar_wait(uint64_t *b, uint32_t parity, unsigned
     return true;
 }
 
-// Bytes of the per-warp staging buffer for rows of n1m points.
-__host__ __device__ inline size_t stage_bytes(int n1m, int C) { return (size_t)(n1m + n1m / C + 2) * 8; }
+// Bytes of the per-warp staging buffer for rows of n1m points (none when rows move directly:
+// reserved shared memory would only shrink the L1 cache).
+__host__ __device__ inline size_t stage_bytes(int n1m, int C) {
+    return C3D_STAGED_ROWS ? (size_t)(n1m + n1m / C + 2) * 8 : 0;
+}
 
 // ---------------------------------------------------------------------------------
 // Complex helpers and the shared-memory Stockham FFT (radices 4, 2, 3)

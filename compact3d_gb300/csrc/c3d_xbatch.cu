@@ -1,5 +1,6 @@
 // c3d_xbatch.cu -- batch kernels of the x-row passes (kernel bodies in c3d_xrows.cuh):
-// one launch per pass and kernel instance over the blocks of many channels.
+// one launch per pass and kernel instance over the blocks of many channels.  Compiled once
+// per precision (C3D_BITS).
 #include <vector>
 #include "c3d_xrows.cuh"
 
@@ -87,11 +88,13 @@ static int xbk_seg(const c3d_channel *ch, int which, int xw, std::vector<BKern> 
     }
 }
 
+#if C3D_BITS == 32
 // The row segment of the x passes for N1M (lanes W, chunk C = N1M/W), or 0 for a whole warp.
 int x_segment_lanes(int n1m, int n3m) {
     const int w = (n1m == 48 || n1m == 64 || n1m == 96) ? 8 : (n1m == 128) ? 16 : 32;
     return (w < 32 && n3m % (32 / w) == 0) ? w : 0;
 }
+#endif
 
 template <typename R>
 int xpass_bkern(const c3d_channel *ch, int which, int xw, std::vector<BKern> &out) {
@@ -116,7 +119,10 @@ int xpass_bkern(const c3d_channel *ch, int which, int xw, std::vector<BKern> &ou
         default: return C3D_EINVAL;
     }
 }
+#if C3D_BITS == 64
 template int xpass_bkern<double>(const c3d_channel *, int, int, std::vector<BKern> &);
+#else
 template int xpass_bkern<float>(const c3d_channel *, int, int, std::vector<BKern> &);
+#endif
 
 }  // namespace c3d

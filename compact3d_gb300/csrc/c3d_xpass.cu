@@ -1,5 +1,6 @@
 // c3d_xpass.cu -- launchers of the x-row passes for one channel (kernel bodies in
-// c3d_xrows.cuh) and the self-test of the staged passes' bounded wait.
+// c3d_xrows.cuh) and the self-test of the staged passes' bounded wait.  Compiled once per
+// precision (C3D_BITS).
 #include <algorithm>
 #include <map>
 #include <mutex>
@@ -7,6 +8,7 @@
 #include "c3d_xrows.cuh"
 
 namespace c3d {
+#if C3D_BITS == 32
 // The bounded stage wait of the staged x passes, run on a barrier that nothing arrives on
 // and no copy targets, so the wait runs out after limit_ns and sets SCAL_PIPEERR exactly
 // as a stalled stage would (c3d_pipe_wait_selftest).
@@ -25,6 +27,7 @@ int launch_pipe_selftest(c3d_channel *ch, double limit_ms) {
     k_pipe_selftest<<<1, 32, 0, ch->stream>>>(ch->scal, (unsigned long long)(limit_ms * 1e6));
     return cudaGetLastError() == cudaSuccess ? 0 : C3D_ECUDA;
 }
+#endif
 
 // ---------------------------------------------------------------------------------
 // launcher
@@ -245,7 +248,10 @@ int launch_xpass(c3d_channel *ch, StepArgs<R> &a, int which, const R *p0, const 
     }
 }
 
+#if C3D_BITS == 64
 template int launch_xpass<double>(c3d_channel *, StepArgs<double> &, int, const double *, const double *, int *);
+#else
 template int launch_xpass<float>(c3d_channel *, StepArgs<float> &, int, const float *, const float *, int *);
+#endif
 
 }  // namespace c3d

@@ -67,7 +67,7 @@ __device__ __forceinline__ void xa_piece(const StepArgs<R> &a, int j, long long 
     typedef typename SType<R>::S S;
     typedef St<R> ST;
     const int n = a.g.n1m;
-    const R RE1 = a.re1, f12 = a.f12x, f24 = a.f24x, four = (R)4.0;
+    const R RE1 = a.re1, f12 = xfold(a.f12x, a.c10x), f24 = xfold(a.f24x, a.c22x), four = xfold((R)4.0, a.c6x);
     const R presg = (R)a.scal[SCAL_PRESG];
     if (PART == 2 && j >= 2) {
         // The v piece on its own, ordered so that few rows are live at once: the y
@@ -108,7 +108,7 @@ __device__ __forceinline__ void xa_piece(const StepArgs<R> &a, int j, long long 
             S l = (t == 0) ? pv : vc[t - 1], rr = (t == C - 1) ? nx : vc[t + 1];
             d[t] = f12 * ST::d2(l, vc[t], rr);
         }
-        xsolve<W>(d, lane, P, a.c10x);
+        xsolve_f<W>(d, lane, P, a.c10x);
 #pragma unroll
         for (int t = 0; t < C; ++t) acc[t] = acc[t] + RE1 * d[t];
         srow_store(a.r[1] + o, acc, sbR, lane, P);
@@ -117,7 +117,7 @@ __device__ __forceinline__ void xa_piece(const StepArgs<R> &a, int j, long long 
             S l = (t == 0) ? pv : vc[t - 1];
             d[t] = four * (ST::hi(l) + ST::hi(vc[t]));
         }
-        xsolve<W>(d, lane, P, a.c6x);
+        xsolve_f<W>(d, lane, P, a.c6x);
         {   // u at the y faces
             S uc[C], um[C];
             xrow<STG>(uc, xa_src<STG, PART>(a, XA_UC, o, om, op, st, n), sbS, lane, P);
@@ -150,7 +150,7 @@ __device__ __forceinline__ void xa_piece(const StepArgs<R> &a, int j, long long 
             S l = (t == 0) ? pv : uc[t - 1], rr = (t == C - 1) ? nx : uc[t + 1];
             d[t] = f12 * ST::d2(l, uc[t], rr);
         }
-        xsolve<W>(d, lane, P, a.c10x);
+        xsolve_f<W>(d, lane, P, a.c10x);
 #pragma unroll
         for (int t = 0; t < C; ++t) acc[t] = acc[t] + RE1 * d[t];
 #pragma unroll
@@ -158,7 +158,7 @@ __device__ __forceinline__ void xa_piece(const StepArgs<R> &a, int j, long long 
             S rr = (t == C - 1) ? nx : uc[t + 1];
             d[t] = four * (ST::hi(uc[t]) + ST::hi(rr));
         }
-        xsolve<W>(d, lane, P, a.c6x);
+        xsolve_f<W>(d, lane, P, a.c6x);
         R sq[C];
 #pragma unroll
         for (int t = 0; t < C; ++t) sq[t] = d[t] * d[t];
@@ -168,7 +168,7 @@ __device__ __forceinline__ void xa_piece(const StepArgs<R> &a, int j, long long 
             R l = (t == 0) ? ps : sq[t - 1];
             d[t] = f24 * (sq[t] - l);
         }
-        xsolve<W>(d, lane, P, a.c22x);
+        xsolve_f<W>(d, lane, P, a.c22x);
         srow_store(a.hh[0] + o, d, sbR, lane, P);
         {
             S pc[C];
@@ -180,7 +180,7 @@ __device__ __forceinline__ void xa_piece(const StepArgs<R> &a, int j, long long 
                 d[t] = f24 * ST::d(pc[t], l);
             }
         }
-        xsolve<W>(d, lane, P, a.c22x);
+        xsolve_f<W>(d, lane, P, a.c22x);
 #pragma unroll
         for (int t = 0; t < C; ++t) acc[t] = acc[t] - d[t] - presg;
         srow_store(a.r[0] + o, acc, sbR, lane, P);
@@ -206,7 +206,7 @@ __device__ __forceinline__ void xa_piece(const StepArgs<R> &a, int j, long long 
             S l = (t == 0) ? pv : wc[t - 1], rr = (t == C - 1) ? nx : wc[t + 1];
             d[t] = f12 * ST::d2(l, wc[t], rr);
         }
-        xsolve<W>(d, lane, P, a.c10x);
+        xsolve_f<W>(d, lane, P, a.c10x);
 #pragma unroll
         for (int t = 0; t < C; ++t) acc[t] = acc[t] + RE1 * d[t];
         srow_store(a.r[2] + o, acc, sbR, lane, P);
@@ -215,7 +215,7 @@ __device__ __forceinline__ void xa_piece(const StepArgs<R> &a, int j, long long 
             S l = (t == 0) ? pv : wc[t - 1];
             d[t] = four * (ST::hi(l) + ST::hi(wc[t]));
         }
-        xsolve<W>(d, lane, P, a.c6x);
+        xsolve_f<W>(d, lane, P, a.c6x);
         srow_store(a.ww1 + o, d, sbR, lane, P);
     }
 }
@@ -237,7 +237,7 @@ __device__ __forceinline__ void b_xA(const StepArgs<R> &a, const Blk blk) {
     S *sbS = reinterpret_cast<S *>(smem_raw + wid * stage_bytes(g.n1m, C));
     R *sbR = reinterpret_cast<R *>(sbS);
     const int nrows = g.n2m * g.n3m;
-    const R RE1 = a.re1, f12 = a.f12x, f24 = a.f24x, four = (R)4.0;
+    const R RE1 = a.re1, f12 = xfold(a.f12x, a.c10x), f24 = xfold(a.f24x, a.c22x), four = xfold((R)4.0, a.c6x);
     const R presg = (R)a.scal[SCAL_PRESG];
     for (int row = blk.x * rpb + wid; row < nrows; row += blk.gx * rpb) {
         const int j = 1 + row / g.n3m, k = row % g.n3m;
@@ -270,7 +270,7 @@ __device__ __forceinline__ void b_xA(const StepArgs<R> &a, const Blk blk) {
                 S l = (t == 0) ? pv : uc[t - 1], rr = (t == C - 1) ? nx : uc[t + 1];
                 d[t] = f12 * ST::d2(l, uc[t], rr);
             }
-            xsolve<W>(d, lane, P, a.c10x);
+            xsolve_f<W>(d, lane, P, a.c10x);
 #pragma unroll
             for (int t = 0; t < C; ++t) acc[t] = RE1 * ST::yvisc(HPj, HCj, HMj, Z0, up[t], uc[t], um[t]) + RE1 * d[t];
             {
@@ -282,7 +282,7 @@ __device__ __forceinline__ void b_xA(const StepArgs<R> &a, const Blk blk) {
                     S l = (t == 0) ? pp : pc[t - 1];
                     d[t] = f24 * ST::d(pc[t], l);
                 }
-                xsolve<W>(d, lane, P, a.c22x);
+                xsolve_f<W>(d, lane, P, a.c22x);
 #pragma unroll
                 for (int t = 0; t < C; ++t) acc[t] = acc[t] - d[t] - presg;
                 srow_store(a.r[0] + o, acc, sbR, lane, P);
@@ -292,7 +292,7 @@ __device__ __forceinline__ void b_xA(const StepArgs<R> &a, const Blk blk) {
                 S rr = (t == C - 1) ? nx : uc[t + 1];
                 d[t] = four * (ST::hi(uc[t]) + ST::hi(rr));
             }
-            xsolve<W>(d, lane, P, a.c6x);
+            xsolve_f<W>(d, lane, P, a.c6x);
             R sq[C];
 #pragma unroll
             for (int t = 0; t < C; ++t) sq[t] = d[t] * d[t];
@@ -302,7 +302,7 @@ __device__ __forceinline__ void b_xA(const StepArgs<R> &a, const Blk blk) {
                 R l = (t == 0) ? ps : sq[t - 1];
                 d[t] = f24 * (sq[t] - l);
             }
-            xsolve<W>(d, lane, P, a.c22x);
+            xsolve_f<W>(d, lane, P, a.c22x);
             srow_store(a.hh[0] + o, d, sbR, lane, P);
             if (PART == 0 && j >= 2) {
                 const R Hj1 = a.m.rh[j], a1 = a.m.hdy[j], a2 = a.m.hdy[j - 1];
@@ -323,7 +323,7 @@ __device__ __forceinline__ void b_xA(const StepArgs<R> &a, const Blk blk) {
                 S l = (t == 0) ? pv : vc[t - 1], rr = (t == C - 1) ? nx : vc[t + 1];
                 d[t] = f12 * ST::d2(l, vc[t], rr);
             }
-            xsolve<W>(d, lane, P, a.c10x);
+            xsolve_f<W>(d, lane, P, a.c10x);
             const R DYPj = a.m.dyp[j], DYCj = a.m.dyc[j], DYMj = a.m.dym[j], Z0 = a.m.dyz[j];
             const R Hj = a.m.h[j], Hj1 = a.m.rh[j];
             {
@@ -345,7 +345,7 @@ __device__ __forceinline__ void b_xA(const StepArgs<R> &a, const Blk blk) {
                 S l = (t == 0) ? pv : vc[t - 1];
                 d[t] = four * (ST::hi(l) + ST::hi(vc[t]));
             }
-            xsolve<W>(d, lane, P, a.c6x);
+            xsolve_f<W>(d, lane, P, a.c6x);
 #pragma unroll
             for (int t = 0; t < C; ++t) d[t] = d[t] * uy[t];
             srow_store(a.exy + o, d, sbR, lane, P);
@@ -363,7 +363,7 @@ __device__ __forceinline__ void b_xA(const StepArgs<R> &a, const Blk blk) {
                 S l = (t == 0) ? pv : wc[t - 1], rr = (t == C - 1) ? nx : wc[t + 1];
                 d[t] = f12 * ST::d2(l, wc[t], rr);
             }
-            xsolve<W>(d, lane, P, a.c10x);
+            xsolve_f<W>(d, lane, P, a.c10x);
             const R HPj = a.m.hp[j], HCj = a.m.hc[j], HMj = a.m.hm[j], Z0 = a.m.hz[j];
 #pragma unroll
             for (int t = 0; t < C; ++t) acc[t] = RE1 * ST::yvisc(HPj, HCj, HMj, Z0, wp[t], wc[t], wm[t]) + RE1 * d[t];
@@ -373,16 +373,17 @@ __device__ __forceinline__ void b_xA(const StepArgs<R> &a, const Blk blk) {
                 S l = (t == 0) ? pv : wc[t - 1];
                 d[t] = four * (ST::hi(l) + ST::hi(wc[t]));
             }
-            xsolve<W>(d, lane, P, a.c6x);
+            xsolve_f<W>(d, lane, P, a.c6x);
             srow_store(a.ww1 + o, d, sbR, lane, P);
         }
     }
 }
 // At least 3 blocks of XMAXT threads per SM: at most 80 registers, so more rows are in
 // flight (the pieces are latency-bound; measured on 384-point rows: 0.742 -> 0.705 ms for
-// the three pieces, with a few dozen bytes of spills).
+// the three pieces, with a few dozen bytes of spills).  FP64 holds twice the registers and is
+// bound by the FP64 pipe, which a few warps fill: two blocks.
 template <typename R, int C, int PART, int W = 32>
-__global__ void __launch_bounds__(XMAXT, 3) k_xA(StepArgs<R> a) {
+__global__ void __launch_bounds__(XMAXT, sizeof(R) == 8 ? 2 : 3) k_xA(StepArgs<R> a) {
     b_xA<R, C, PART, W>(a, Blk{blockIdx.x, blockIdx.y, gridDim.x});
 }
 
@@ -455,18 +456,19 @@ __global__ void __launch_bounds__(XMAXT) k_xAs(StepArgs<R> a) {
 template <typename R, int C, int W = 32>
 __device__ __forceinline__ void ab2_cnx(const StepArgs<R> &a, int c, long long o, const R (&hc)[C], R *sb,
                                         int lane, int P, R dt) {
+    const R dts = xfold(dt, a.cnx);
     R rr[C], ho[C], d[C];
     srow_load(rr, a.r[c] + o, sb, lane, P);
     srow_load(ho, a.ho[c] + o, sb, lane, P);
 #pragma unroll
-    for (int t = 0; t < C; ++t) rr[t] = (rr[t] - (R)1.5 * hc[t] + (R)0.5 * ho[t]) * dt;
+    for (int t = 0; t < C; ++t) rr[t] = (rr[t] - (R)1.5 * hc[t] + (R)0.5 * ho[t]) * dts;
     R pv = sprev<W>(rr[C - 1], lane, P), nx = snext<W>(rr[0], lane, P);
 #pragma unroll
     for (int t = 0; t < C; ++t) {
         R l = (t == 0) ? pv : rr[t - 1], r2 = (t == C - 1) ? nx : rr[t + 1];
         d[t] = (l + (R)10.0 * rr[t]) + r2;
     }
-    xsolve<W>(d, lane, P, a.cnx);
+    xsolve_f<W>(d, lane, P, a.cnx);
     srow_store(a.r[c] + o, d, sb, lane, P);
 }
 
@@ -479,7 +481,7 @@ __device__ __forceinline__ void b_xB(const StepArgs<R> &a, const Blk blk) {
     const int P = g.n1m / C;
     R *sb = reinterpret_cast<R *>(smem_raw + wid * stage_bytes(g.n1m, C));
     const int nrows = g.n2m * g.n3m;
-    const R f = a.f24x;
+    const R f = xfold(a.f24x, a.c22x);
     const R dt = (R)a.dt;
     for (int row = blk.x * rpb + wid; row < nrows; row += blk.gx * rpb) {
         const int j = 1 + row / g.n3m, k = row % g.n3m;
@@ -519,7 +521,7 @@ __device__ __forceinline__ void b_xB(const StepArgs<R> &a, const Blk blk) {
                 R rr = (t == C - 1) ? nx : e[t + 1];
                 d[t] = f * (rr - e[t]);
             }
-            xsolve<W>(d, lane, P, a.c22x);
+            xsolve_f<W>(d, lane, P, a.c22x);
 #pragma unroll
             for (int t = 0; t < C; ++t) h2[t] = h2[t] + d[t];                 // d(uv)/dx
             srow_store(a.hh[1] + o, h2, sb, lane, P);
@@ -535,7 +537,7 @@ __device__ __forceinline__ void b_xB(const StepArgs<R> &a, const Blk blk) {
                 d[t] = f * (rr - e[t]);
             }
         }
-        xsolve<W>(d, lane, P, a.c22x);
+        xsolve_f<W>(d, lane, P, a.c22x);
 #pragma unroll
         for (int t = 0; t < C; ++t) h3[t] = h3[t] + d[t];
         if (j >= 2) srow_load(e, a.eyz + o, sb, lane, P);
@@ -590,7 +592,7 @@ __device__ __forceinline__ void xc_row(const StepArgs<R> &a, int j, int k, const
     S *sbS = reinterpret_cast<S *>(sbuf);
     R *sbR = reinterpret_cast<R *>(sbuf);
     R *rbuf = reinterpret_cast<R *>(bufa);
-    const R rdt = a.rdt, f24 = a.f24x;
+    const R rdt = a.rdt, f24 = xfold(a.f24x, a.c22x);
     R d[C], base[C];
     {
         S uc[C];
@@ -605,7 +607,7 @@ __device__ __forceinline__ void xc_row(const StepArgs<R> &a, int j, int k, const
             R rd = (t == C - 1) ? nd : dd[t + 1];
             d[t] = f24 * Sten<R>::dd(ru, rd, uc[t], dd[t]);
         }
-        xsolve<W>(d, lane, P, a.c22x);
+        xsolve_f<W>(d, lane, P, a.c22x);
     }
     {
         const bool up = (j + 1 <= g.n2m), lo = (j >= 2);
@@ -765,7 +767,7 @@ __device__ __forceinline__ void b_xD(const StepArgs<R> &a, const R *d0, const R 
     const C2 *twx;
     if constexpr (sizeof(R) == 8) twx = reinterpret_cast<const C2 *>(a.twx64);
     else twx = reinterpret_cast<const C2 *>(a.twx32);
-    const R scale = a.xscale, f24 = a.f24x;
+    const R scale = a.xscale, f24 = xfold(a.f24x, a.c22x);
     for (int row = blk.x * rpb + wid; row < nrows; row += blk.gx * rpb) {
         const int j = 1 + row / g.n3m, k = row % g.n3m;
         const long long o = fidx(g, 0, j, k);
@@ -811,7 +813,7 @@ __device__ __forceinline__ void b_xD(const StepArgs<R> &a, const R *d0, const R 
             R l = (t == 0) ? pv : dpv[t - 1];
             d[t] = f24 * (dpv[t] - l);
         }
-        xsolve<W>(d, lane, P, a.c22x);
+        xsolve_f<W>(d, lane, P, a.c22x);
         // bulk-flow partial sums below: sum_i delta * DY(J)/DX3/DX1 for u and w
         R q1[C], q3[C];
         srow_load(q1, d0 + o, sbR, lane, P);

@@ -7,6 +7,7 @@
 //   zD  RHSDP along z (8187-8210)
 //   zE  UPCALC along z and the velocity / pressure update (1052-1238)
 //   diag_z  DIVCHECK z part and max|div| (9099-9128)
+// Compiled once per precision (C3D_BITS).
 #include "c3d_kern.cuh"
 
 namespace c3d {
@@ -670,8 +671,11 @@ int zpass_bkern(const c3d_channel *ch, int which, int L, std::vector<BKern> &out
         return zbk<R, 16, 0>(ch, which, out);
     }
 }
+#if C3D_BITS == 64
 template int zpass_bkern<double>(const c3d_channel *, int, int, std::vector<BKern> &);
+#else
 template int zpass_bkern<float>(const c3d_channel *, int, int, std::vector<BKern> &);
+#endif
 
 template <typename R>
 int launch_zpass(c3d_channel *ch, StepArgs<R> &a, int which, R *d0, R *d1, R *d2, int flag, int *nl) {
@@ -750,7 +754,10 @@ static int launch_zpass_l(c3d_channel *ch, StepArgs<R> &a, int which, R *d0, R *
     return 0;
 }
 
+#if C3D_BITS == 64
 template int launch_zpass<double>(c3d_channel *, StepArgs<double> &, int, double *, double *, double *, int, int *);
+#else
 template int launch_zpass<float>(c3d_channel *, StepArgs<float> &, int, float *, float *, float *, int, int *);
+#endif
 
 }  // namespace c3d
