@@ -108,7 +108,8 @@ enum {
     SCAL_WSMC = 12,    // 3 values: /WSMEM/ WSM as the SGS model and the wall model see it
     SCAL_WALLERR = 15, // 1 when a wall point's Newton iteration hit its cap in the last step
     SCAL_PIPEERR = 16, // 1 when a bulk-copy stage wait gave up (sticky)
-    SCAL_COUNT = 17
+    SCAL_TICKET = 17,  // blocks of k_diag_sums that have stored their sums (an integer, wraps to 0)
+    SCAL_COUNT = 18
 };
 
 // the shifted-point wall models' scratch: per wall U_ave, UTAU2, TAUW1, CC, DELTS, nfix

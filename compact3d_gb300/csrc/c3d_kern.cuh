@@ -24,6 +24,17 @@ constexpr int XMAXT = 256;   // largest block of the tunable x passes (8 rows)
 // ---------------------------------------------------------------------------------
 template <typename R> struct St;
 
+// float -> double in integer arithmetic: the conversion instruction runs at the FP64 rate (2
+// lanes per clock and SM).  Exact for normal numbers, zeros, infinities and NaN; magnitudes
+// below 2^-126 (which a low part reaches only where its value is below 2^-102) become zero.
+__device__ __forceinline__ double f2d(float x) {
+    const unsigned b = __float_as_uint(x), e = b & 0x7f800000u;
+    unsigned hi = ((b & 0x7fffffffu) >> 3) + 0x38000000u, lo = b << 29;
+    if (e == 0x7f800000u) hi += 0x38000000u;
+    if (e == 0) hi = lo = 0;
+    return __hiloint2double((int)(hi | (b & 0x80000000u)), (int)lo);
+}
+
 template <> struct St<double> {
     typedef double S;
     static __device__ __forceinline__ double hi(double a) { return a; }
@@ -55,7 +66,7 @@ template <> struct St<float> {
         float l = e - (h - s);
         return make_float2(h, l);
     }
-    static __device__ __forceinline__ double dbl(float2 a) { return (double)a.x + (double)a.y; }
+    static __device__ __forceinline__ double dbl(float2 a) { return f2d(a.x) + f2d(a.y); }
     static __device__ __forceinline__ float2 scale(float2 a, float s) { return make_float2(a.x * s, a.y * s); }
     static __host__ __device__ __forceinline__ float2 from_double(double a) {
         float h = (float)a;
@@ -656,8 +667,28 @@ __device__ __forceinline__ void pf_cols(const void *base, long long stride_bytes
     }
 }
 
-__device__ __forceinline__ void atomic_max_nonneg(double *addr, double v) {
-    atomicMax(reinterpret_cast<unsigned long long *>(addr), (unsigned long long)__double_as_longlong(v));
+// Non-negative FP64 values order like their bits: maxima are taken in integer arithmetic.
+// INF_BITS itself and everything above it (NaN) are not finite.
+constexpr unsigned long long INF_BITS = 0x7ff0000000000000ull;
+__device__ __forceinline__ unsigned long long abs_bits(double v) {
+    return (unsigned long long)__double_as_longlong(v) & 0x7fffffffffffffffull;
+}
+// The warp's maximum of m into *addr (one atomic, and none where *addr is already as large);
+// the block's last warp may be partial.  bad in any lane sets *flag.
+__device__ __forceinline__ void warp_max_to(double *addr, unsigned long long m, bool bad, double *flag) {
+    const int lane = threadIdx.x & 31, nl = min(32, (int)blockDim.x - ((int)threadIdx.x & ~31));
+    const unsigned mask = nl == 32 ? FULL : (1u << nl) - 1u;
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1) {
+        const unsigned long long o = __shfl_down_sync(mask, m, off);
+        if (lane + off < nl && o > m) m = o;
+    }
+    const bool any = __any_sync(mask, bad);
+    if (lane == 0) {
+        unsigned long long *p = reinterpret_cast<unsigned long long *>(addr);
+        if (m > *reinterpret_cast<volatile unsigned long long *>(p)) atomicMax(p, m);
+        if (any) *flag = 1.0;
+    }
 }
 
 inline int nblk(long long n, int b = TPB) { return (int)((n + b - 1) / b); }

@@ -878,7 +878,10 @@ __global__ void __launch_bounds__(XMAXT) k_xD(StepArgs<R> a, const R *d0, const 
 
 // ---------------------------------------------------------------------------------
 // Diagnostics, x part: DIVCHECK's (V(J+1)-V(J))/DY + compact dU/dx into an FP64
-// scratch field, and the CFL maximum.  Always FP64.
+// scratch field, and the CFL maximum.  Always FP64, so bound by the FP64 pipe: divisions by
+// DY are products, the mixed state converts in integer arithmetic (f2d), maxima are integer
+// (128 x 96 x 128 points, mixed: 173 us with a division, a conversion and an FP64 compare
+// per term).
 // ---------------------------------------------------------------------------------
 template <typename R, int C>
 __global__ void __launch_bounds__(TPB) k_diag_x(StepArgs<R> a, double *divx, Cyc<double> c22) {
@@ -891,8 +894,9 @@ __global__ void __launch_bounds__(TPB) k_diag_x(StepArgs<R> a, double *divx, Cyc
     S *sbS = reinterpret_cast<S *>(smem_raw + wid * stage_bytes(g.n1m, C));
     double *sbD = reinterpret_cast<double *>(sbS);
     const int nrows = g.n2m * g.n3m;
-    double cmax = 0.0;
-    int bad = 0;
+    unsigned long long cmax = 0;
+    bool bad = false;
+    const double h1 = 0.5 * g.dx1, h3 = 0.5 * g.dx3, f = 24.0 * g.dx1 * c22.s;
     for (int row = blockIdx.x * (TPB / 32) + wid; row < nrows; row += gridDim.x * (TPB / 32)) {
         const int j = 1 + row / g.n3m, k = row % g.n3m;
         const int kp = (k + 1 == g.n3m) ? 0 : k + 1;
@@ -906,37 +910,26 @@ __global__ void __launch_bounds__(TPB) k_diag_x(StepArgs<R> a, double *divx, Cyc
         double uc[C], d[C];
 #pragma unroll
         for (int t = 0; t < C; ++t) uc[t] = ST::dbl(su[t]);
-        double nx = snext(uc[0], lane, P);
+        const double nx = snext(uc[0], lane, P);
+#pragma unroll
+        for (int t = 0; t < C; ++t) d[t] = ((t == C - 1) ? nx : uc[t + 1]) - uc[t];
+        xsolve_f<32>(d, lane, P, c22);
+        const double rdy = 1.0 / g.dy[j], h2 = 0.5 * rdy;
 #pragma unroll
         for (int t = 0; t < C; ++t) {
-            double rr = (t == C - 1) ? nx : uc[t + 1];
-            d[t] = 24.0 * g.dx1 * (rr - uc[t]);
-        }
-        xsolve(d, lane, P, c22);
-        const double dyj = g.dy[j];
-#pragma unroll
-        for (int t = 0; t < C; ++t) {
-            double rr = (t == C - 1) ? nx : uc[t + 1];
-            double vc = ST::dbl(sv[t]), vp = ST::dbl(svp[t]);
-            d[t] = (vp - vc) / dyj + d[t];
-            double cf = fabs(uc[t] + rr) * 0.5 * g.dx1 + fabs(vc + vp) * 0.5 / dyj +
-                        fabs(ST::dbl(sw[t]) + ST::dbl(swk[t])) * 0.5 * g.dx3;
+            const double rr = (t == C - 1) ? nx : uc[t + 1];
+            const double vc = ST::dbl(sv[t]), vp = ST::dbl(svp[t]);
+            d[t] = (vp - vc) * rdy + f * d[t];
+            const unsigned long long cf =
+                abs_bits(fabs(uc[t] + rr) * h1 + fabs(vc + vp) * h2 + fabs(ST::dbl(sw[t]) + ST::dbl(swk[t])) * h3);
             if (lane < P) {
-                if (!isfinite(cf)) bad = 1;
-                cmax = fmax(cmax, cf);
+                bad |= cf >= INF_BITS;
+                if (cf <= INF_BITS && cf > cmax) cmax = cf;   // not a NaN
             }
         }
         srow_store(divx + o, d, sbD, lane, P);
     }
-#pragma unroll
-    for (int off = 16; off > 0; off >>= 1) {
-        cmax = fmax(cmax, __shfl_down_sync(FULL, cmax, off));
-        bad |= __shfl_down_sync(FULL, bad, off);
-    }
-    if (lane == 0) {
-        atomic_max_nonneg(&a.scal[SCAL_CFL], cmax);
-        if (bad) a.scal[SCAL_NONFIN] = 1.0;
-    }
+    warp_max_to(&a.scal[SCAL_CFL], cmax, bad, &a.scal[SCAL_NONFIN]);
 }
 
 }  // namespace c3d

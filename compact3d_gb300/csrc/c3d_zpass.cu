@@ -517,41 +517,44 @@ __global__ void __launch_bounds__(MODE == 1 ? zjt<R, L>() : TPB) k_zE(StepArgs<R
     b_zE<R, L, MODE>(a, d0, d1, d2, updp, Blk{blockIdx.x, blockIdx.y, gridDim.x});
 }
 
-// DIVCHECK z part and max |div| (FP64)
-template <typename R, int L>
-__global__ void __launch_bounds__(TPB) k_diag_z(StepArgs<R> a, const double *divx, Cyc<double> c22) {
+// DIVCHECK z part and max |div| (FP64): joined segments, or warm-ups (L = ZL) on lines too
+// long for a block.
+template <typename R>
+struct WalkDiagZ {
     typedef typename SType<R>::S S;
-    typedef St<R> ST;
+    const S *W; int n, s; double wc; int kn;
+    __device__ void start(int k) { wc = St<R>::dbl(W[k * s]); kn = znext(k, n); }
+    __device__ void next(double (&d)[1]) {
+        const double wp = St<R>::dbl(W[kn * s]);
+        d[0] = wp - wc;
+        wc = wp;
+        kn = znext(kn, n);
+    }
+};
+template <typename R, int L, int MODE>
+__global__ void __launch_bounds__(MODE == 1 ? zjt<double, L>() : TPB) k_diag_z(StepArgs<R> a, const double *divx,
+                                                                               Cyc<double> c22) {
     const Geo g = a.g;
-    int i, j, k0;
-    double m = 0.0;
-    int bad = 0;
-    if (zcoord<L>(g, 1, i, j, k0)) {
+    ZCo c;
+    unsigned long long m = 0;
+    bool bad = false;
+    if (zcoords<L, MODE>(Blk{blockIdx.x, blockIdx.y, gridDim.x}, g, 1, c)) {
         const int n = g.n3m, s = g.n1m;
-        const long long o = fidx(g, i, j, 0);
-        const S *W = a.w + o;
+        const long long o = fidx(g, c.i, c.j, 0);
         const double *DX = divx + o;
-        double out[L];
-        zseg<double, L>(out, k0, n, c22, [&](int kk) {
-            int kp = kk == n - 1 ? 0 : kk + 1;
-            return 24.0 * g.dx3 * (ST::dbl(W[kp * s]) - ST::dbl(W[kk * s]));
-        });
+        double out[1][L], dx[L];
+        const double rr[1] = {c22.r}, ss[1] = {1.0}, f = 24.0 * g.dx3 * c22.s;
+        WalkDiagZ<R> w{a.w + o, n, s};
+        zsolve<double, L, WM<double>::M22, 1, MODE>(out, c, n, rr, ss, w);
+        zload(dx, DX, c.k0, s);
 #pragma unroll
         for (int t = 0; t < L; ++t) {
-            double dv = DX[(k0 + t) * s] + out[t];
-            if (!isfinite(dv)) bad = 1;
-            m = fmax(m, fabs(dv));
+            const unsigned long long dv = abs_bits(dx[t] + f * out[0][t]);
+            bad |= c.act && dv >= INF_BITS;
+            if (c.act && dv <= INF_BITS && dv > m) m = dv;
         }
     }
-#pragma unroll
-    for (int off = 16; off > 0; off >>= 1) {
-        m = fmax(m, __shfl_down_sync(FULL, m, off));
-        bad |= __shfl_down_sync(FULL, bad, off);
-    }
-    if ((threadIdx.x & 31) == 0) {
-        atomic_max_nonneg(&a.scal[SCAL_DIVMAX], m);
-        if (bad) a.scal[SCAL_NONFIN] = 1.0;
-    }
+    warp_max_to(&a.scal[SCAL_DIVMAX], m, bad, &a.scal[SCAL_NONFIN]);
 }
 
 template <typename R, int L, int MODE>
@@ -678,8 +681,28 @@ template int zpass_bkern<float>(const c3d_channel *, int, int, std::vector<BKern
 #endif
 
 template <typename R>
+static int launch_diag_z(c3d_channel *ch, StepArgs<R> &a, const double *divx, int *nl) {
+    const Geo &g = ch->g;
+    const double b = 22.0, r = -2.0 / (b + sqrt(b * b - 4.0));
+    const Cyc<double> c22 = {r, -r, WM<double>::M22};
+    const long long ncol = (long long)g.n2m * g.n1m;
+    auto go = [&](auto *fn, int L, int cols) {
+        const int nt = cols * (g.n3m / L);
+        fn<<<nblk(ncol, cols), nt, 2 * (size_t)nt * sizeof(double), ch->stream>>>(a, divx, c22);
+    };
+    switch (zjoin_len<double>(g.n3m)) {
+        case 8: go(k_diag_z<R, 8, 1>, 8, zjoin_cols<double, 8>(g.n3m)); break;
+        case 12: go(k_diag_z<R, 12, 1>, 12, zjoin_cols<double, 12>(g.n3m)); break;
+        case 16: go(k_diag_z<R, 16, 1>, 16, zjoin_cols<double, 16>(g.n3m)); break;
+        default: k_diag_z<R, ZL, 0><<<nblk(ncol * (g.n3m / ZL)), TPB, 0, ch->stream>>>(a, divx, c22);
+    }
+    mark(ch, nl, "diag_z", (double)ncol * g.n3m * 16);
+    return 0;
+}
+
+template <typename R>
 int launch_zpass(c3d_channel *ch, StepArgs<R> &a, int which, R *d0, R *d1, R *d2, int flag, int *nl) {
-    if (which == 5) return launch_zpass_l<R, ZL, 0>(ch, a, which, d0, d1, d2, flag, nl);
+    if (which == 5) return launch_diag_z<R>(ch, a, (const double *)d0, nl);
     const int zl = ch->tune.zl[which];
     // FP64 always joins its segments: the FP64 pipe (2 lanes per clock and SM) bounds these
     // passes, and with M = 23 warm-up points a segment of 16 evaluates 62 right-hand sides
@@ -742,13 +765,6 @@ static int launch_zpass_l(c3d_channel *ch, StepArgs<R> &a, int which, R *d0, R *
             k_zE<R, L, MODE><<<nb, TB, zs1, st>>>(a, d0, d1, d2, flag);
             mark(ch, nl, "zE", N * (64 + (sizeof(R) == 4 ? 4 : 5) * Rb));
             break;
-        case 5: {
-            const double b = 22.0, r = -2.0 / (b + sqrt(b * b - 4.0));
-            Cyc<double> c22 = {r, -r, (int)ceil(log(1e-17) / log(fabs(r)))};
-            k_diag_z<R, L><<<nblk(nt), TPB, 0, st>>>(a, (const double *)d0, c22);
-            mark(ch, nl, "diag_z", N * 16);
-            break;
-        }
         default: return C3D_EINVAL;
     }
     return 0;
