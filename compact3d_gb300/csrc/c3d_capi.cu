@@ -1309,7 +1309,7 @@ int c3d_plane_spectra(c3d_channel *ch, const double *vmo, double *xspec, double 
     if (!ch->specbuf && dalloc(&ch->specbuf, nm + 3 * nx + 2 * nz)) return C3D_ENOMEM;
     double *dvmo = ch->specbuf, *dxs = dvmo + nm, *dzs = dxs + nx, *drxx = dzs + nz, *drzz = drxx + nx,
            *drxy = drzz + nz;
-    int rc = launch_stats(ch, ch->stats, ch->stats + nout);
+    int rc = launch_stats(ch, ch->stats, ch->stats + nout, 1);
     if (rc) return rc;
     if (vmo) {
         CK(cudaMemcpyAsync(dvmo, vmo, nm * sizeof(double), cudaMemcpyHostToDevice, ch->stream));
@@ -1376,7 +1376,7 @@ int c3d_corr3d(c3d_channel *ch, double *out) {
     const Geo &g = ch->g;
     const size_t n = 3 * (size_t)g.n1m * g.n2m * g.n3m, nout = (size_t)g.n2m * 29;
     if (!ch->stats && dalloc(&ch->stats, stats_scratch_doubles(g))) return C3D_ENOMEM;
-    int rc = launch_stats(ch, ch->stats, ch->stats + nout);
+    int rc = launch_stats(ch, ch->stats, ch->stats + nout, 1);
     if (rc) return rc;
     double *buf = nullptr;
     if (dalloc(&buf, n)) return C3D_ENOMEM;

@@ -321,8 +321,9 @@ int launch_poisson_tables(c3d_channel *ch);
 // what: 0 U component, 1 P, 2 HH component, 3 SGSVIS (to host), 4 operand (to device),
 // 5 operator result (to host)
 // ENERGY's plane statistics of the current state into out (N2M x 29, device), with
-// `part` as scratch (stats_scratch_doubles(g) doubles hold both)
-int launch_stats(c3d_channel *ch, double *out, double *part);
+// `part` as scratch (stats_scratch_doubles(g) doubles hold both); means: only the columns the
+// spectra and correlations read (VM, VRMS of the three components)
+int launch_stats(c3d_channel *ch, double *out, double *part, int means = 0);
 size_t stats_scratch_doubles(const c3d::Geo &g);
 // Checkpoint records (CWRITE's order) between the device state and buf; dir 0 packs,
 // what 0 U, 1 P, 2 HH (three components)

@@ -703,15 +703,15 @@ void batch_args(c3d_channel *ch, double dt, void *dst) {
 }
 
 template <typename R>
-int launch_stats_t(c3d_channel *ch, StepArgs<R> &a, double *out, double *part);
+int launch_stats_t(c3d_channel *ch, StepArgs<R> &a, double *out, double *part, int means);
 
-int launch_stats(c3d_channel *ch, double *out, double *part) {
+int launch_stats(c3d_channel *ch, double *out, double *part, int means) {
     if (ch->precision == C3D_MIXED) {
         StepArgs<float> a = make_args<float>(ch, ch->dt_cached > 0 ? ch->dt_cached : 1.0);
-        return launch_stats_t<float>(ch, a, out, part);
+        return launch_stats_t<float>(ch, a, out, part, means);
     }
     StepArgs<double> a = make_args<double>(ch, ch->dt_cached > 0 ? ch->dt_cached : 1.0);
-    return launch_stats_t<double>(ch, a, out, part);
+    return launch_stats_t<double>(ch, a, out, part, means);
 }
 
 template <typename R>
