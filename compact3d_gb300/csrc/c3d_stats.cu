@@ -8,7 +8,7 @@
 // next points share, the x neighbours come by shuffles, cell-centre values are kept doubled
 // (a sum of two, the powers of two leave in the last step), divisions by plane constants are
 // products, and the mixed state converts in integer arithmetic (f2d).  192 x 128 x 192
-// points, mixed state: plane statistics 2.95 -> 0.75 ms, spectra and correlations 8.5 -> 1.5.
+// points, mixed state: plane statistics 2.95 -> 1.07 ms, spectra and correlations 8.5 -> 2.2.
 #include "c3d_kern.cuh"
 
 namespace c3d {
