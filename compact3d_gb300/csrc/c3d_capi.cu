@@ -527,10 +527,12 @@ int c3d_create(const c3d_grid *gr, c3d_channel **out) {
         }
         if ((ch->files == 1 || ch->files == 3) && cudaMalloc(&ch->dyn, 21 * (size_t)g.n2m * g.np * rs) != cudaSuccess)
             return fail(C3D_ENOMEM);
-        if (ch->files == 3) {   // SGSSD: per-plane sums of tiles of 32 x 16 points
+        if (ch->files == 1 || ch->files == 3) {   // SGSDY, SGSSD: sums of tiles of 32 x 16 points
             ch->sdnt = ((g.n1m + 31) / 32) * (g.n3m / 16);
-            if (dalloc(&ch->sdpart, (size_t)g.n2m * ch->sdnt * 10) || dalloc(&ch->sdbeta, (size_t)g.n2 + 1))
-                return fail(C3D_ENOMEM);
+            if (dalloc(&ch->sdpart, (size_t)g.n2m * ch->sdnt * (ch->files == 1 ? 2 : 10))) return fail(C3D_ENOMEM);
+        }
+        if (ch->files == 3) {
+            if (dalloc(&ch->sdbeta, (size_t)g.n2 + 1)) return fail(C3D_ENOMEM);
             cudaMemset(ch->sdbeta, 0, ((size_t)g.n2 + 1) * 8);
             if (cudaStreamCreateWithFlags(&ch->sside, cudaStreamNonBlocking) != cudaSuccess ||
                 cudaEventCreateWithFlags(&ch->sfork, cudaEventDisableTiming) != cudaSuccess ||

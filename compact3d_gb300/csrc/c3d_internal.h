@@ -194,7 +194,7 @@ struct c3d_channel {
     // MARUSIC1 / PIOMELLI: Y(0:N2), YC(0:N2), per-wall constants and YP heights; the
     // reference plane ZS of MARUSIC1 (the Y(J) nearest 0.06) and tan(16 deg)
     double *wshift = nullptr;
-    // SGSSD: per-plane partial sums of k_sgs_sd_sums (N2M x sdnt x 10) and BETA(0:N2)
+    // SGSDY / SGSSD: the tiles' partial sums (N2M x sdnt x 2 / 10); SGSSD: BETA(0:N2)
     double *specbuf = nullptr;   // c3d_plane_spectra: means and the five output tables
     // WALLMODEL_IWMLES_SMOOTH: per-point state, whether it is set, the accumulated model
     // step, DY(1) + DY(2) + DY(3)/2, the driver's CFLMAX and the NTIME of the step

@@ -7,8 +7,8 @@
 //   sgs_cs      SGSCS: nu = max(coef |S|, -1/RE) with |S| from STRAIN (5558-5689)
 //   sgs_raw     SGSDY (1250-1400): per point S_ij, |S|, DELTA^2 |S| S_ij, the cell-centre
 //               velocities and their products
-//   sgs_dyn     SGSDY: FILTER (5190-5228) of those, M_ij, L_ij, the plane sums, SMAGC(J)
-//               and nu, one block per plane
+//   sgs_dy_*    SGSDY: FILTER (5190-5228) of those, M_ij, L_ij, the plane sums and SMAGC(J);
+//               sgs_apply: nu
 //   sgs_sd_*    SGSSD (1502-1948): both test filters, the Germano sums, the quintic's
 //               root by CHHQR (11571-11676) and SMAGC; sgs_apply: nu
 //   wall        WALLMODEL_INSTANT (2319-2493): damped Newton for u_tau per wall point
@@ -229,75 +229,108 @@ __global__ void __launch_bounds__(TPB) k_sgs_raw(StepArgs<R> a, LesArgs<R> l) {
     l.dyn[20 * fs + q0] = u3 * u3;
 }
 
-// FILTER of one raw quantity at (i, k): Simpson (1,4,1)/6 along x, then along z.
+// SGSDY's test-filter stage and the sums of L:M and M:M, one block per tile of SD_TX x SD_TZ
+// points of a plane (grid: x tiles, z tiles, N2M), one thread per point: field by field the
+// tile and its halo are staged in shared memory and filtered along x, then along z, so each
+// (1,4,1) stencil is evaluated once (a block per plane gathering nine points per field left
+// most of the device idle: 1.49 -> 0.12 ms on 96 x 48 x 64 points, FP64).  The FP64 form, bound by
+// the FP64 pipe, keeps the filtered values times 36 (M then carries 1/36, L 1/1296: the sums
+// are scaled once, in k_sgs_dy_coef); FP32 divides as FILTER does.  Block sums in FP64, fixed
+// order, to part[((j - 1) tiles + tile) 2 + q].
+constexpr int SD_TX = 32, SD_TZ = 16, SD_THREADS = SD_TX * SD_TZ;
 template <typename R>
-__device__ __forceinline__ R filt(const R *f, int n1, int n3, int i, int k) {
-    const int ip = wrapp(i, n1), im = wrapm(i, n1), kp = wrapp(k, n3), km = wrapm(k, n3);
-    const R six = (R)6.0, four = (R)4.0;
-    auto T = [&](int kk) {
-        const R *r = f + (long long)kk * n1;
-        return (r[im] + four * r[i] + r[ip]) / six;
-    };
-    return (T(km) + four * T(k) + T(kp)) / six;
+__device__ __forceinline__ R simpson(R fm, R fc, R fp) {
+    if constexpr (sizeof(R) == 8) return (fm + (R)4.0 * fc) + fp;
+    else return (fm + (R)4.0 * fc + fp) / (R)6.0;
 }
-
-// SGSDY's test-filter stage, the plane sums (FP64, fixed order) and nu, one block per plane.
 template <typename R>
-__global__ void __launch_bounds__(256) k_sgs_dyn(StepArgs<R> a, LesArgs<R> l) {
+__global__ void __launch_bounds__(SD_THREADS) k_sgs_dy_sums(StepArgs<R> a, LesArgs<R> l, double *part) {
     const Geo g = a.g;
-    const int j = 1 + blockIdx.x;
+    const int n1 = g.n1m, n3 = g.n3m;
+    const int j = 1 + blockIdx.z, i0 = blockIdx.x * SD_TX, k0 = blockIdx.y * SD_TZ;
+    const int tx = threadIdx.x % SD_TX, tz = threadIdx.x / SD_TX;
     const long long fs = (long long)g.n2m * g.np, pb = (long long)(j - 1) * g.np;
-    __shared__ double sn[256], sd[256];
-    __shared__ R coefj;
-    double snum = 0.0, sden = 0.0;
-    const R fd = (R)4.0 * l.d23r[j];
-    for (int e = threadIdx.x; e < g.np; e += blockDim.x) {
-        const int i = e % g.n1m, k = e / g.n1m;
-        R m[6], cf[6];
+    __shared__ R raw[SD_TZ + 2][SD_TX + 2];
+    __shared__ R fx[SD_TZ + 2][SD_TX];
+    R f[21];
 #pragma unroll
-        for (int c = 0; c < 6; ++c) {
-            m[c] = filt(l.dyn + c * fs + pb, g.n1m, g.n3m, i, k);
-            cf[c] = filt(l.dyn + (6 + c) * fs + pb, g.n1m, g.n3m, i, k);
-        }
-        const R fdabs = fd * sqrt((R)2.0 * sumsq6(m));
-#pragma unroll
-        for (int c = 0; c < 6; ++c) m[c] = fdabs * m[c] - cf[c];
-        R uc[3], up[6];
-#pragma unroll
-        for (int c = 0; c < 3; ++c) uc[c] = filt(l.dyn + (12 + c) * fs + pb, g.n1m, g.n3m, i, k);
-#pragma unroll
-        for (int c = 0; c < 6; ++c) up[c] = filt(l.dyn + (15 + c) * fs + pb, g.n1m, g.n3m, i, k);
-        const R L11 = up[0] - uc[0] * uc[0], L12 = up[1] - uc[0] * uc[1], L13 = up[2] - uc[0] * uc[2];
-        const R L22 = up[3] - uc[1] * uc[1], L23 = up[4] - uc[1] * uc[2], L33 = up[5] - uc[2] * uc[2];
-        const R two = (R)2.0;
-        const R sqmm = sumsq6(m);
-        const R sqlm = two * L12 * m[1] + L11 * m[0] + two * L13 * m[2] + L22 * m[3] + two * L23 * m[4] + L33 * m[5];
-        sden += (double)sqmm;
-        snum += (double)sqlm;
-    }
-    sn[threadIdx.x] = snum;
-    sd[threadIdx.x] = sden;
-    __syncthreads();
-    for (int s = blockDim.x / 2; s > 0; s >>= 1) {
-        if (threadIdx.x < s) {
-            sn[threadIdx.x] += sn[threadIdx.x + s];
-            sd[threadIdx.x] += sd[threadIdx.x + s];
+    for (int c = 0; c < 21; ++c) {
+        const R *q0 = l.dyn + c * fs + pb;
+        for (int q = threadIdx.x; q < (SD_TZ + 2) * (SD_TX + 2); q += SD_THREADS) {
+            const int rz = q / (SD_TX + 2), rx = q - rz * (SD_TX + 2);
+            int ii = i0 + rx - 1, kk = k0 + rz - 1;
+            ii = ii < 0 ? ii + n1 : (ii >= n1 ? ii - n1 : ii);
+            kk = kk < 0 ? kk + n3 : (kk >= n3 ? kk - n3 : kk);
+            ii = ii >= n1 ? ii - n1 : ii;   // tiles wider than N1M
+            raw[rz][rx] = q0[(long long)kk * n1 + ii];
         }
         __syncthreads();
+        for (int q = threadIdx.x; q < (SD_TZ + 2) * SD_TX; q += SD_THREADS) {
+            const int rz = q / SD_TX, x = q - rz * SD_TX;
+            const R *r = &raw[rz][x];
+            fx[rz][x] = simpson(r[0], r[1], r[2]);
+        }
+        __syncthreads();
+        f[c] = simpson(fx[tz][tx], fx[tz + 1][tx], fx[tz + 2][tx]);
     }
-    if (threadIdx.x == 0) {
-        const double nxz = 1.0 / (double)g.np;
-        const double sm = -0.5 * (sn[0] * nxz) / (sd[0] * nxz);
-        l.smagc[j] = sm;
-        coefj = (R)(sm * l.d23[j]);
+    double snum = 0.0, sden = 0.0;
+    if (i0 + tx < n1) {
+        constexpr bool S36 = sizeof(R) == 8;
+        const R fd = (R)4.0 * l.d23r[j] * (S36 ? (R)(1.0 / 36.0) : R(1)), two = (R)2.0;
+        R m[6], cf[6], uc[3], up[6];
+#pragma unroll
+        for (int c = 0; c < 6; ++c) { m[c] = f[c]; cf[c] = f[6 + c]; up[c] = f[15 + c]; }
+#pragma unroll
+        for (int c = 0; c < 3; ++c) uc[c] = f[12 + c];
+        const R fdabs = fd * sqrt(two * sumsq6(m));
+#pragma unroll
+        for (int c = 0; c < 6; ++c) m[c] = fdabs * m[c] - cf[c];
+        if constexpr (S36) {
+#pragma unroll
+            for (int c = 0; c < 6; ++c) up[c] *= (R)36.0;
+        }
+        const R L11 = up[0] - uc[0] * uc[0], L12 = up[1] - uc[0] * uc[1], L13 = up[2] - uc[0] * uc[2];
+        const R L22 = up[3] - uc[1] * uc[1], L23 = up[4] - uc[1] * uc[2], L33 = up[5] - uc[2] * uc[2];
+        const R sqmm = sumsq6(m);
+        const R sqlm = two * L12 * m[1] + L11 * m[0] + two * L13 * m[2] + L22 * m[3] + two * L23 * m[4] + L33 * m[5];
+        sden = (double)sqmm;
+        snum = (double)sqlm;
     }
+    __shared__ double red[SD_THREADS / 32][2];
+    for (int o = 16; o > 0; o >>= 1) {
+        snum += __shfl_down_sync(FULL, snum, o);
+        sden += __shfl_down_sync(FULL, sden, o);
+    }
+    if ((threadIdx.x & 31) == 0) { red[threadIdx.x >> 5][0] = snum; red[threadIdx.x >> 5][1] = sden; }
     __syncthreads();
-    const R c = coefj;
-    R *nup = l.nu + fidx(g, 0, j, 0);
-    for (int e = threadIdx.x; e < g.np; e += blockDim.x) {
-        const R t = c * nup[e];
-        nup[e] = t > -l.reninv ? t : -l.reninv;
+    if (threadIdx.x < 2) {
+        double v = 0.0;
+        for (int w = 0; w < SD_THREADS / 32; ++w) v += red[w][threadIdx.x];
+        const int nt = gridDim.x * gridDim.y, tile = blockIdx.y * gridDim.x + blockIdx.x;
+        part[((long long)(j - 1) * nt + tile) * 2 + threadIdx.x] = v;
     }
+}
+
+// SMAGC(J) and nu's coefficient from the tiles' sums, a warp per plane.
+template <typename R>
+__global__ void k_sgs_dy_coef(StepArgs<R> a, LesArgs<R> l, const double *part, int nt) {
+    const Geo g = a.g;
+    const int j = 1 + blockIdx.x;
+    double sn = 0.0, sd = 0.0;
+    for (int t = threadIdx.x; t < nt; t += 32) {
+        sn += part[((long long)(j - 1) * nt + t) * 2];
+        sd += part[((long long)(j - 1) * nt + t) * 2 + 1];
+    }
+    for (int o = 16; o > 0; o >>= 1) {
+        sn += __shfl_down_sync(FULL, sn, o);
+        sd += __shfl_down_sync(FULL, sd, o);
+    }
+    if (threadIdx.x != 0) return;
+    const double nxz = 1.0 / (double)g.np;
+    if (sizeof(R) == 8) { sn *= 1.0 / (36.0 * 1296.0); sd *= 1.0 / 1296.0; }
+    const double sm = -0.5 * (sn * nxz) / (sd * nxz);
+    l.smagc[j] = sm;
+    l.coef[j] = (R)(sm * l.d23[j]);
 }
 
 // ---------------------------------------------------------------------------------
@@ -349,7 +382,6 @@ __device__ __forceinline__ void sd_level(const R *f, R d23, double *acc) {
 // one thread per point.  Field by field, the tile and a halo of two is staged in shared
 // memory, filtered along x by both stencils, then along z at each point; both levels'
 // sums go to part[((j - 1) tiles + tile) SD_NS + q].
-constexpr int SD_TX = 32, SD_TZ = 16, SD_THREADS = SD_TX * SD_TZ;
 template <typename R>
 __global__ void __launch_bounds__(SD_THREADS) k_sgs_sd_sums(StepArgs<R> a, LesArgs<R> l, double *part) {
     const Geo g = a.g;
@@ -1518,7 +1550,10 @@ int launch_les(c3d_channel *ch, StepArgs<R> &a, LesArgs<R> &l, int stage, int *n
             if ((rc = wall_model())) return rc;
             k_sgs_raw<R><<<nblk((long long)g.n2m * g.np), TPB, 0, st>>>(a, l);
             mark(ch, nl, "sgs_raw", N * (6 * 8 + 22 * Rb));
-            k_sgs_dyn<R><<<g.n2m, 256, 0, st>>>(a, l);
+            k_sgs_dy_sums<R><<<dim3((g.n1m + SD_TX - 1) / SD_TX, g.n3m / SD_TZ, g.n2m), SD_THREADS, 0, st>>>(a, l, ch->sdpart);
+            k_sgs_dy_coef<R><<<g.n2m, 32, 0, st>>>(a, l, ch->sdpart, ch->sdnt);
+            k_sgs_apply<R><<<nblk((long long)g.n2m * g.np), TPB, 0, st>>>(a, l);
+            *nl += 2;
             mark(ch, nl, "sgs_dyn", N * 23 * Rb);
         } else if (ch->files == 3) {
             if ((rc = wall_model())) return rc;
