@@ -35,7 +35,7 @@
 // point's own velocity and the Leonard stress from values relative to a per-plane
 // constant (the dynamic procedure is Galilean invariant), so FP32 keeps its relative
 // accuracy; plane sums, the coefficient and the wall model run in FP64.
-#include "c3d_kern.cuh"
+#include "c3d_zcols.cuh"
 
 namespace c3d {
 
@@ -1204,7 +1204,7 @@ __global__ void __launch_bounds__(TPB) k_les_x1(StepArgs<R> a, LesArgs<R> l) {
 template <typename R>
 struct WalkLesZ1 {
     typedef typename SType<R>::S S;
-    const R *NU, *NUX; const S *U, *V, *W; int n, s; R f24; bool hv;
+    const R *NU, *NUX; const S *U, *V, *W; int n, s; R four, f24; bool hv;
     R num, nuxm; S um, vm, wc; int kn, kc;
     __device__ void start(int k) {
         const int kp = zprev(k, n);
@@ -1214,8 +1214,8 @@ struct WalkLesZ1 {
     __device__ void next(R (&d)[5]) {
         const R nuc = NU[kc * s], nuxc = NUX[kc * s];
         const S uc = U[kc * s], wp = W[kn * s];
-        d[0] = (R)4.0 * (num + nuc);
-        d[1] = (R)4.0 * (nuxm + nuxc);
+        d[0] = four * (num + nuc);
+        d[1] = four * (nuxm + nuxc);
         d[2] = f24 * St<R>::d(uc, um);
         d[3] = f24 * St<R>::d(wp, wc);
         if (hv) {
@@ -1227,29 +1227,37 @@ struct WalkLesZ1 {
         }
         num = nuc; nuxm = nuxc; um = uc; wc = wp; kc = kn; kn = znext(kn, n);
     }
-    __device__ static int zprev(int k, int n) { return k == 0 ? n - 1 : k - 1; }
-    __device__ static int znext(int k, int n) { return k + 1 == n ? 0 : k + 1; }
 };
 
-template <typename R, int L>
-__global__ void __launch_bounds__(TPB) k_les_z1(StepArgs<R> a, LesArgs<R> l) {
+// FP64 joins its segments (MODE 1), FP32 runs warm-ups (MODE 0), as the z passes of the step.
+template <typename R, int L, int MODE>
+__global__ void __launch_bounds__(MODE == 1 ? zjt<R, L>() : TPB) k_les_z1(StepArgs<R> a, LesArgs<R> l) {
     const Geo g = a.g;
-    int i, j, k0;
-    if (!zcoord<L>(g, 1, i, j, k0)) return;
-    const int n = g.n3m, s = g.n1m;
-    const long long o = fidx(g, i, j, 0);
+    ZCo c;
+    if (!zcoords<L, MODE>(Blk{blockIdx.x, blockIdx.y, gridDim.x}, g, 1, c)) return;
+    const int n = g.n3m, s = g.n1m, j = c.j, k0 = c.k0;
+    const long long o = fidx(g, c.i, j, 0);
     R out[5][L];
     const R rr[5] = {a.c6z.r, a.c6z.r, a.c22z.r, a.c22z.r, a.c22z.r};
     const R ss[5] = {a.c6z.s, a.c6z.s, a.c22z.s, a.c22z.s, a.c22z.s};
-    WalkLesZ1<R> f{l.nu + o, l.nux + o, a.u + o, a.v + o, a.w + o, n, s, a.f24z, j >= 2};
-    zsweep<R, L, WM<R>::M6, 5>(out, k0, n, rr, ss, f);
+    WalkLesZ1<R> f{l.nu + o, l.nux + o, a.u + o, a.v + o, a.w + o, n, s, zrhs<MODE>((R)4.0), zrhs<MODE>(a.f24z), j >= 2};
+    zsolve<R, L, WM<R>::M6, 5, MODE>(out, c, n, rr, ss, f);
+    if (!c.act) return;
+    const R k6 = zfold<MODE>((R)4.0, a.c6z.s), k22 = zfold<MODE>(a.f24z, a.c22z.s);
+    constexpr int B = ztb<L>();
 #pragma unroll
-    for (int t = 0; t < L; ++t) {
-        const long long kk = o + (long long)(k0 + t) * s;
-        l.nuz[kk] = out[0][t];
-        l.t13[kk] = out[1][t] * (out[2][t] + l.dwdx[kk]);
-        l.nuwz[kk] = l.nu[kk] * out[3][t];
-        if (j >= 2) l.dvdz[kk] = out[4][t];
+    for (int b = 0; b < L; b += B) {
+        R dw[B], nu[B];
+        zload(dw, l.dwdx + o, k0 + b, s);
+        zload(nu, l.nu + o, k0 + b, s);
+#pragma unroll
+        for (int t = 0; t < B; ++t) {
+            const long long kk = o + (long long)(k0 + b + t) * s;
+            l.nuz[kk] = k6 * out[0][b + t];
+            l.t13[kk] = k6 * out[1][b + t] * (k22 * out[2][b + t] + dw[t]);
+            l.nuwz[kk] = nu[t] * (k22 * out[3][b + t]);
+            if (j >= 2) l.dvdz[kk] = k22 * out[4][b + t];
+        }
     }
 }
 
@@ -1280,20 +1288,23 @@ struct WalkLesZ2 {
     }
 };
 
-template <typename R, int L>
-__global__ void __launch_bounds__(TPB) k_les_z2(StepArgs<R> a, LesArgs<R> l) {
+template <typename R, int L, int MODE>
+__global__ void __launch_bounds__(MODE == 1 ? zjt<R, L>() : TPB) k_les_z2(StepArgs<R> a, LesArgs<R> l) {
     typedef St<R> ST;
+    typedef typename SType<R>::S S;
     const Geo g = a.g;
-    int i, j, k0;
-    if (!zcoord<L>(g, 1, i, j, k0)) return;
-    const int n = g.n3m, s = g.n1m;
+    ZCo c;
+    if (!zcoords<L, MODE>(Blk{blockIdx.x, blockIdx.y, gridDim.x}, g, 1, c)) return;
+    const int n = g.n3m, s = g.n1m, i = c.i, j = c.j, k0 = c.k0;
     const long long o = fidx(g, i, j, 0), om = fidx(g, i, j - 1, 0), op = fidx(g, i, j + 1, 0);
     const bool hv = j >= 2;
     R out[3][L];
     const R rr[3] = {a.c22z.r, a.c22z.r, a.c22z.r}, ss[3] = {a.c22z.s, a.c22z.s, a.c22z.s};
     WalkLesZ2<R> f{l.t13 + o, l.nuwz + o, l.nuz + o, l.nuz + om, l.dvdz + o, a.w + o, a.w + om,
-                   n, s, a.f24z, a.m.rh[j], a.m.hdy[j], a.m.hdy[j - 1], hv};
-    zsweep<R, L, WM<R>::M22, 3>(out, k0, n, rr, ss, f);
+                   n, s, zrhs<MODE>(a.f24z), a.m.rh[j], a.m.hdy[j], a.m.hdy[j - 1], hv};
+    zsolve<R, L, WM<R>::M22, 3, MODE>(out, c, n, rr, ss, f);
+    if (!c.act) return;
+    const R ks = zfold<MODE>(a.f24z, a.c22z.s);
     const bool fjum = (j != 1), fjup = (j != g.n2m);
     const R half = (R)0.5, two = (R)2.0;
     const R f2 = (R)(1.0 - l.ifwall * (fjup ? 0.0 : 1.0) * (g.aly - 1.0));
@@ -1301,21 +1312,36 @@ __global__ void __launch_bounds__(TPB) k_les_z2(StepArgs<R> a, LesArgs<R> l) {
     const R rdy = a.m.rdy[j], rh = a.m.rh[j], rhp = a.m.rh[j + 1];
     const R hdj = a.m.hdy[j], hdjm = a.m.hdy[j - 1], hdjp = a.m.hdy[j + 1];
     const long long w0 = fidx(g, i, 0, 0), wt = fidx(g, i, g.n2, 0);
+    constexpr int B = ztb<L>() / 2;   // eleven fields are live
 #pragma unroll
-    for (int t = 0; t < L; ++t) {
-        const int k = k0 + t, km = (k == 0) ? n - 1 : k - 1;
-        const long long kk = (long long)k * s, kkm = (long long)km * s;
-        const R sj2 = fjup ? rhp * (hdj * l.nuz[op + kk] + hdjp * l.nuz[o + kk])
-                           : half * (l.nu[wt + kk] + l.nu[wt + kkm]);
-        const R sj1 = fjum ? rh * (hdjm * l.nuz[o + kk] + hdj * l.nuz[om + kk])
-                           : half * (l.nu[w0 + kk] + l.nu[w0 + kkm]);
-        const R ww22 = rhp * ST::d(a.w[op + kk], a.w[o + kk]);
-        const R ww11 = rh * ST::d(a.w[o + kk], a.w[om + kk]);
-        const R yflux = rdy * ((f2 * sj2) * (ww22 + l.dvdz[op + kk]) - (f1 * sj1) * (ww11 + l.dvdz[o + kk]));
-        R *H1 = a.hh[0] + o + kk, *H2 = a.hh[1] + o + kk, *H3 = a.hh[2] + o + kk;
-        *H1 = *H1 - out[0][t];
-        *H3 = *H3 - two * out[1][t] - yflux;
-        if (hv) *H2 = *H2 - out[2][t];
+    for (int b = 0; b < L; b += B) {
+        R zm[B], zc[B], zp[B], dc[B], dp[B], h1[B], h2[B], h3[B];
+        S wm[B], wc[B], wp[B];
+        zload(zc, l.nuz + o, k0 + b, s);
+        zload(wm, a.w + om, k0 + b, s);
+        zload(wc, a.w + o, k0 + b, s);
+        zload(wp, a.w + op, k0 + b, s);
+        zload(dc, l.dvdz + o, k0 + b, s);
+        zload(dp, l.dvdz + op, k0 + b, s);
+        if (fjup) zload(zp, l.nuz + op, k0 + b, s);
+        if (fjum) zload(zm, l.nuz + om, k0 + b, s);
+        zload(h1, a.hh[0] + o, k0 + b, s);
+        zload(h3, a.hh[2] + o, k0 + b, s);
+        if (hv) zload(h2, a.hh[1] + o, k0 + b, s);
+#pragma unroll
+        for (int t = 0; t < B; ++t) {
+            const int k = k0 + b + t, km = (k == 0) ? n - 1 : k - 1;
+            const long long kk = (long long)k * s, kkm = (long long)km * s;
+            const R sj2 = fjup ? rhp * (hdj * zp[t] + hdjp * zc[t]) : half * (l.nu[wt + kk] + l.nu[wt + kkm]);
+            const R sj1 = fjum ? rh * (hdjm * zc[t] + hdj * zm[t]) : half * (l.nu[w0 + kk] + l.nu[w0 + kkm]);
+            const R ww22 = rhp * ST::d(wp[t], wc[t]);
+            const R ww11 = rh * ST::d(wc[t], wm[t]);
+            const R yflux = rdy * ((f2 * sj2) * (ww22 + dp[t]) - (f1 * sj1) * (ww11 + dc[t]));
+            R *H1 = a.hh[0] + o + kk, *H2 = a.hh[1] + o + kk, *H3 = a.hh[2] + o + kk;
+            *H1 = h1[t] - ks * out[0][b + t];
+            *H3 = h3[t] - two * (ks * out[1][b + t]) - yflux;
+            if (hv) *H2 = h2[t] - ks * out[2][b + t];
+        }
     }
 }
 
@@ -1470,6 +1496,34 @@ void launch_wall_shift_init(c3d_channel *ch) {
 
 size_t wall_shift_doubles(const Geo &g) { return WsMesh::size(g); }
 
+// les_z1 (which 0) or les_z2: joined segments in FP64, warm-ups in FP32 and on lines too long
+// for a block.
+template <typename R>
+static int launch_les_z(c3d_channel *ch, StepArgs<R> &a, LesArgs<R> &l, int which) {
+    const Geo &g = ch->g;
+    const long long ncol = (long long)g.n2m * g.n1m;
+    auto go = [&](auto *fn, int nr, int L, int cols) {
+        const int nt = cols * (g.n3m / L);
+        fn<<<nblk(ncol, cols), nt, 2 * (size_t)nr * nt * sizeof(R), ch->stream>>>(a, l);
+    };
+    if constexpr (sizeof(R) == 8) {
+        switch (zjoin_len<R>(g.n3m)) {
+            case 8:
+                if (which == 0) go(k_les_z1<R, 8, 1>, 5, 8, zjoin_cols<R, 8>(g.n3m, ncol));
+                else go(k_les_z2<R, 8, 1>, 3, 8, zjoin_cols<R, 8>(g.n3m, ncol));
+                return 0;
+            case 12:
+                if (which == 0) go(k_les_z1<R, 12, 1>, 5, 12, zjoin_cols<R, 12>(g.n3m, ncol));
+                else go(k_les_z2<R, 12, 1>, 3, 12, zjoin_cols<R, 12>(g.n3m, ncol));
+                return 0;
+            default: break;
+        }
+    }
+    if (which == 0) k_les_z1<R, ZL, 0><<<nblk(ncol * (g.n3m / ZL)), TPB, 0, ch->stream>>>(a, l);
+    else k_les_z2<R, ZL, 0><<<nblk(ncol * (g.n3m / ZL)), TPB, 0, ch->stream>>>(a, l);
+    return 0;
+}
+
 template <typename R>
 int launch_les(c3d_channel *ch, StepArgs<R> &a, LesArgs<R> &l, int stage, int *nl) {
     cudaStream_t st = ch->stream;
@@ -1593,10 +1647,10 @@ int launch_les(c3d_channel *ch, StepArgs<R> &a, LesArgs<R> &l, int stage, int *n
         case 12: launch_les_x<R, 12>(ch, a, l, 0, nl); break;
         default: set_error("unsupported N1M"); return C3D_EINVAL;
     }
-    const long long nz = (long long)g.n2m * (g.n3m / ZL) * g.n1m;
-    k_les_z1<R, ZL><<<nblk(nz), TPB, 0, st>>>(a, l);
+    int rc;
+    if ((rc = launch_les_z<R>(ch, a, l, 0))) return rc;
     mark(ch, nl, "les_z1", N * (24 + 7 * Rb));
-    k_les_z2<R, ZL><<<nblk(nz), TPB, 0, st>>>(a, l);
+    if ((rc = launch_les_z<R>(ch, a, l, 1))) return rc;
     mark(ch, nl, "les_z2", N * (16 + 12 * Rb));
     if (ch->wjoin_pending) {   // TAUW/TAUB of this step's wall model
         CK_RC(cudaStreamWaitEvent(st, ch->wjoin, 0));

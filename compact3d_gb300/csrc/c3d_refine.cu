@@ -17,7 +17,7 @@
 //   (fftz, poisson, fftz: the spectral solve of the main pressure step)
 //   ir_d  complex-to-real FFT along x -> DP2, compact d(DP2)/dx
 //   ir_e  compact d(DP2)/dz and the update of u, v, w and P
-#include "c3d_kern.cuh"
+#include "c3d_zcols.cuh"
 
 namespace c3d {
 
@@ -192,13 +192,28 @@ __global__ void __launch_bounds__(TPB) k_ir_e(StepArgs<float> a, int updp) {
     float2 *W = a.w + o, *U = a.u + o, *V = a.v + o, *Pp = a.p + o;
     const float *DP = a.dp + o, *DPm = a.dp + fidx(g, i, j - 1, 0), *G1 = a.g1 + o;
     const float Hj = a.m.h[j];
+    constexpr int B = ztb<L>() / 2;   // loaded in batches before the first store, as in zE
 #pragma unroll
-    for (int t = 0; t < L; ++t) {
-        const int kk = (k0 + t) * s;
-        W[kk] = ST::add(W[kk], -(dt * out[0][t]));
-        U[kk] = ST::add(U[kk], -(dt * G1[kk]));
-        if (j >= 2) V[kk] = ST::add(V[kk], -(dt * (DP[kk] - DPm[kk]) / Hj));
-        if (updp) Pp[kk] = ST::add(Pp[kk], DP[kk]);
+    for (int b = 0; b < L; b += B) {
+        float2 wv[B], uv[B], vv[B], pv[B];
+        float gv[B], pc[B], pm[B];
+        zload(wv, W, k0 + b, s);
+        zload(uv, U, k0 + b, s);
+        zload(gv, G1, k0 + b, s);
+        zload(pc, DP, k0 + b, s);
+        if (j >= 2) {
+            zload(vv, V, k0 + b, s);
+            zload(pm, DPm, k0 + b, s);
+        }
+        if (updp) zload(pv, Pp, k0 + b, s);
+#pragma unroll
+        for (int t = 0; t < B; ++t) {
+            const int kk = (k0 + b + t) * s;
+            W[kk] = ST::add(wv[t], -(dt * out[0][b + t]));
+            U[kk] = ST::add(uv[t], -(dt * gv[t]));
+            if (j >= 2) V[kk] = ST::add(vv[t], -(dt * (pc[t] - pm[t]) / Hj));
+            if (updp) Pp[kk] = ST::add(pv[t], pc[t]);
+        }
     }
 }
 
