@@ -270,7 +270,7 @@ __device__ __forceinline__ void xsolve_ring(double (&x)[C], int lane, int P, con
 template <int W, typename R, int C>
 __device__ __forceinline__ void xsolve_general(R (&x)[C], int lane, int P, const Cyc<R> &c) {
     const bool act = lane < P;
-    const R r = c.r, s = c.s;
+    const R r = c.r;
     R y = R(0), m = R(1);
 #pragma unroll
     for (int t = 0; t < C; ++t) {
@@ -321,6 +321,7 @@ __device__ __forceinline__ void xsolve_general(R (&x)[C], int lane, int P, const
         R en1 = shfl_down(e, 1, W), mn1 = shfl_down(m, 1, W);
         z = (lane == W - 1) ? z0 : en1 + mn1 * z0;
     }
+    const R s = c.s;
 #pragma unroll
     for (int t = C - 1; t >= 0; --t) {
         z = x[t] + r * z;
