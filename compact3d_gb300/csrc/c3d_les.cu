@@ -229,6 +229,17 @@ __global__ void __launch_bounds__(TPB) k_sgs_raw(StepArgs<R> a, LesArgs<R> l) {
     l.dyn[20 * fs + q0] = u3 * u3;
 }
 
+// 2 a1 b1 + a0 b0 + 2 a2 b2 + a3 b3 + 2 a4 b4 + a5 b5 by multiply-adds in this order
+template <typename R>
+__device__ __forceinline__ R dot6f(const R (&a)[6], const R (&b)[6]) {
+    const R two = (R)2.0;
+    R x = fma(two * a[1], b[1], a[0] * b[0]);
+    x = fma(two * a[2], b[2], x);
+    x = fma(a[3], b[3], x);
+    x = fma(two * a[4], b[4], x);
+    return fma(a[5], b[5], x);
+}
+
 // SGSDY's test-filter stage and the sums of L:M and M:M, one block per tile of SD_TX x SD_TZ
 // points of a plane (grid: x tiles, z tiles, N2M), one thread per point: field by field the
 // tile and its halo are staged in shared memory and filtered along x, then along z, so each
@@ -282,19 +293,19 @@ __global__ void __launch_bounds__(SD_THREADS) k_sgs_dy_sums(StepArgs<R> a, LesAr
         for (int c = 0; c < 6; ++c) { m[c] = f[c]; cf[c] = f[6 + c]; up[c] = f[15 + c]; }
 #pragma unroll
         for (int c = 0; c < 3; ++c) uc[c] = f[12 + c];
-        const R fdabs = fd * sqrt(two * sumsq6(m));
+        // the products' roundings are written out (L is a small difference, so SMAGC of the
+        // FP32 form follows them): one rounding per multiply-add everywhere
+        const R fdabs = fd * sqrt(two * dot6f(m, m));
 #pragma unroll
-        for (int c = 0; c < 6; ++c) m[c] = fdabs * m[c] - cf[c];
+        for (int c = 0; c < 6; ++c) m[c] = fma(fdabs, m[c], -cf[c]);
         if constexpr (S36) {
 #pragma unroll
             for (int c = 0; c < 6; ++c) up[c] *= (R)36.0;
         }
-        const R L11 = up[0] - uc[0] * uc[0], L12 = up[1] - uc[0] * uc[1], L13 = up[2] - uc[0] * uc[2];
-        const R L22 = up[3] - uc[1] * uc[1], L23 = up[4] - uc[1] * uc[2], L33 = up[5] - uc[2] * uc[2];
-        const R sqmm = sumsq6(m);
-        const R sqlm = two * L12 * m[1] + L11 * m[0] + two * L13 * m[2] + L22 * m[3] + two * L23 * m[4] + L33 * m[5];
-        sden = (double)sqmm;
-        snum = (double)sqlm;
+        const R L[6] = {fma(-uc[0], uc[0], up[0]), fma(-uc[0], uc[1], up[1]), fma(-uc[0], uc[2], up[2]),
+                        fma(-uc[1], uc[1], up[3]), fma(-uc[1], uc[2], up[4]), fma(-uc[2], uc[2], up[5])};
+        sden = (double)dot6f(m, m);
+        snum = (double)dot6f(L, m);
     }
     __shared__ double red[SD_THREADS / 32][2];
     for (int o = 16; o > 0; o >>= 1) {
