@@ -688,6 +688,7 @@ int c3d_create(const c3d_grid *gr, c3d_channel **out) {
     ch->fz.tw32 = ch->tw32 + nx;
     ch->dt_cached = -1.0;
     ch->cur = 0;
+    ch->pdl = 1;
     cudaError_t e = cudaDeviceSynchronize();
     if (e != cudaSuccess) {
         set_error(std::string("create: ") + cudaGetErrorString(e));
@@ -1965,7 +1966,19 @@ static int batch_capture_worklist(c3d_batch *b, const double *dt, int par) {
             void *A = b->dargs[par];
             BMap *M = b->dmap[par] + gr.off;
             void *kargs[] = {&A, &M};
-            cudaError_t e = cudaLaunchKernel(gr.fn, dim3((unsigned)gr.cnt), dim3(gr.block), kargs, gr.smem, ls);
+            // the batch kernels begin with pdl_enter: a kernel right after another on the same
+            // stream takes a programmatic dependence on it (see klaunch)
+            cudaLaunchAttribute at[1];
+            at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+            at[0].val.programmaticStreamSerializationAllowed = 1;
+            cudaLaunchConfig_t lc = {};
+            lc.gridDim = dim3((unsigned)gr.cnt);
+            lc.blockDim = dim3(gr.block);
+            lc.dynamicSmemBytes = gr.smem;
+            lc.stream = ls;
+            lc.attrs = at;
+            lc.numAttrs = 1;
+            cudaError_t e = cudaLaunchKernelExC(&lc, gr.fn, kargs);
             if (e != cudaSuccess && le == cudaSuccess) le = e;
         }
         if (run) join();
@@ -2011,7 +2024,9 @@ static int batch_capture(c3d_batch *b, const double *dt, int par) {
         cudaStreamWaitEvent(c->stream, b->fork, 0);
         int keep = c->prof_on;
         c->prof_on = 0;
+        c->pdl = 0;   // plain dependences between the graph's nodes
         rc = launch_step(c, dt[i], &nl);
+        c->pdl = 1;
         c->prof_on = keep;
         cudaEventRecord(b->join[i], c->stream);
         cudaStreamWaitEvent(b->stream, b->join[i], 0);

@@ -267,6 +267,7 @@ struct c3d_channel {
     c3d::dfl *rdydf;          // 1/DY(J) as double-float pairs (refinement)
     // per-kernel profiler (CUDA events around every launch when enabled)
     int prof_on;
+    int pdl;                                 // the step's launches may overlap their successor's start (klaunch)
     int prof_n;                              // events recorded in the current step
     std::vector<cudaEvent_t> prof_ev;        // event pool
     std::vector<int> prof_iv;                // kernel index of interval i

@@ -126,6 +126,7 @@ __device__ __forceinline__ R sumsq6(const R (&s)[6]) {
 // WALLSS into WSM (the SGSCS input): one block, FP64, fixed order.
 template <typename R>
 __global__ void k_les_wallss(StepArgs<R> a) {
+    pdl_enter();
     typedef St<R> ST;
     const Geo g = a.g;
     __shared__ double sh[3][256];
@@ -163,6 +164,7 @@ __global__ void k_les_wallss(StepArgs<R> a) {
 // SGSCS's plane coefficients from WSM: SMAGC(J) = (0.1 (1 - exp(-y+/26)))^2.
 template <typename R>
 __global__ void k_sgs_coef(StepArgs<R> a, LesArgs<R> l) {
+    pdl_enter();
     const Geo g = a.g;
     const double w1 = a.scal[SCAL_WSMC], w3 = a.scal[SCAL_WSMC + 2];
     const double utau = sqrt(sqrt(w1 * w1 + w3 * w3));
@@ -177,6 +179,7 @@ __global__ void k_sgs_coef(StepArgs<R> a, LesArgs<R> l) {
 
 template <typename R>
 __global__ void __launch_bounds__(TPB) k_sgs_cs(StepArgs<R> a, LesArgs<R> l) {
+    pdl_enter();
     const Geo g = a.g;
     // 32-bit index arithmetic (a field has fewer than 2^31 points)
     const unsigned tid = blockIdx.x * blockDim.x + threadIdx.x;
@@ -194,6 +197,7 @@ __global__ void __launch_bounds__(TPB) k_sgs_cs(StepArgs<R> a, LesArgs<R> l) {
 // velocities (relative to the plane's velocity at (0, j, 0)), q[15..20] their products.
 template <typename R>
 __global__ void __launch_bounds__(TPB) k_sgs_raw(StepArgs<R> a, LesArgs<R> l) {
+    pdl_enter();
     typedef St<R> ST;
     const Geo g = a.g;
     // 32-bit index arithmetic (a field has fewer than 2^31 points)
@@ -256,6 +260,7 @@ __device__ __forceinline__ R simpson(R fm, R fc, R fp) {
 }
 template <typename R>
 __global__ void __launch_bounds__(SD_THREADS) k_sgs_dy_sums(StepArgs<R> a, LesArgs<R> l, double *part) {
+    pdl_enter();
     const Geo g = a.g;
     const int n1 = g.n1m, n3 = g.n3m;
     const int j = 1 + blockIdx.z, i0 = blockIdx.x * SD_TX, k0 = blockIdx.y * SD_TZ;
@@ -325,6 +330,7 @@ __global__ void __launch_bounds__(SD_THREADS) k_sgs_dy_sums(StepArgs<R> a, LesAr
 // SMAGC(J) and nu's coefficient from the tiles' sums, a warp per plane.
 template <typename R>
 __global__ void k_sgs_dy_coef(StepArgs<R> a, LesArgs<R> l, const double *part, int nt) {
+    pdl_enter();
     const Geo g = a.g;
     const int j = 1 + blockIdx.x;
     double sn = 0.0, sd = 0.0;
@@ -395,6 +401,7 @@ __device__ __forceinline__ void sd_level(const R *f, R d23, double *acc) {
 // sums go to part[((j - 1) tiles + tile) SD_NS + q].
 template <typename R>
 __global__ void __launch_bounds__(SD_THREADS) k_sgs_sd_sums(StepArgs<R> a, LesArgs<R> l, double *part) {
+    pdl_enter();
     const Geo g = a.g;
     const int n1 = g.n1m, n3 = g.n3m;
     const int j = 1 + blockIdx.z, i0 = blockIdx.x * SD_TX, k0 = blockIdx.y * SD_TZ;
@@ -567,6 +574,7 @@ __device__ void sd_chhqr5_warp(double *A, double *WR, double EPS) {
 template <typename R>
 __global__ void __launch_bounds__(32) k_sgs_sd_coef(StepArgs<R> a, LesArgs<R> l, const double *part, int nt,
                                                     double *beta) {
+    pdl_enter();
     const Geo g = a.g;
     const int j = 1 + blockIdx.x, lane = threadIdx.x;
     __shared__ double Am[25], WR[5], s[SD_NS];
@@ -615,6 +623,7 @@ __global__ void __launch_bounds__(32) k_sgs_sd_coef(StepArgs<R> a, LesArgs<R> l,
 // nu = max(coef(J) |S|, -1/RE) over the N2M planes (|S| left in nu by k_sgs_raw)
 template <typename R>
 __global__ void __launch_bounds__(TPB) k_sgs_apply(StepArgs<R> a, LesArgs<R> l) {
+    pdl_enter();
     const Geo g = a.g;
     const unsigned tid = blockIdx.x * blockDim.x + threadIdx.x;
     if (tid >= (unsigned)g.n2m * (unsigned)g.np) return;
@@ -631,6 +640,7 @@ __global__ void __launch_bounds__(TPB) k_sgs_apply(StepArgs<R> a, LesArgs<R> l) 
 // ---------------------------------------------------------------------------------
 template <typename R>
 __global__ void __launch_bounds__(TPB) k_wall(StepArgs<R> a, LesArgs<R> l) {
+    pdl_enter();
     typedef St<R> ST;
     const Geo g = a.g;
     __shared__ double ssum[TPB], sbad[TPB];
@@ -684,6 +694,7 @@ __global__ void __launch_bounds__(TPB) k_wall(StepArgs<R> a, LesArgs<R> l) {
 // velocity of plane 3, with per-block sums of TAUW1 for WSM(1).
 template <typename R>
 __global__ void __launch_bounds__(TPB) k_wall_rough(StepArgs<R> a, LesArgs<R> l, double klog) {
+    pdl_enter();
     typedef St<R> ST;
     const Geo g = a.g;
     __shared__ double ssum[TPB];
@@ -716,6 +727,7 @@ __global__ void __launch_bounds__(TPB) k_wall_rough(StepArgs<R> a, LesArgs<R> l,
 // the z index (IPA(K), F:4852) is kept.  VCASE uses WSM(1) of the step before.
 template <typename R>
 __global__ void __launch_bounds__(TPB) k_wall_werner(StepArgs<R> a, LesArgs<R> l, double *tw4) {
+    pdl_enter();
     typedef St<R> ST;
     const Geo g = a.g;
     __shared__ double ssum[TPB];
@@ -762,6 +774,7 @@ __global__ void __launch_bounds__(TPB) k_wall_werner(StepArgs<R> a, LesArgs<R> l
 // neighbour with the z index again, F:4924), TAUB = (TAUWE(K) + TAUWE(K-1)) / 2, both walls.
 template <typename R>
 __global__ void __launch_bounds__(TPB) k_wall_werner_avg(StepArgs<R> a, LesArgs<R> l, const double *tw4) {
+    pdl_enter();
     const Geo g = a.g;
     const int e = blockIdx.x * blockDim.x + threadIdx.x;
     if (e >= g.np) return;
@@ -855,6 +868,7 @@ __global__ void k_wall_shift_init(Geo g, double *ws) {
 // BCOND sets V(J=1) while the model may still run beside it, so the plane is copied first
 template <typename R>
 __global__ void __launch_bounds__(TPB) k_wall_shift_v1(StepArgs<R> a, double *ws) {
+    pdl_enter();
     typedef St<R> ST;
     const Geo g = a.g;
     const int e = blockIdx.x * blockDim.x + threadIdx.x;
@@ -940,6 +954,7 @@ __device__ double ws_interp(const StepArgs<R> &a, const WsMesh &m, double XP, do
 // per-block sums of u on the two reference planes (jd: bottom, ju: top)
 template <typename R>
 __global__ void __launch_bounds__(TPB) k_wall_shift_mean(StepArgs<R> a, LesArgs<R> l, int jd, int ju) {
+    pdl_enter();
     typedef St<R> ST;
     const Geo g = a.g;
     __shared__ double sd[TPB], su[TPB];
@@ -1013,6 +1028,7 @@ __device__ double ws_bisect_warp(double U_ave, double DELTAP, double RE, double 
 // plane means, u_tau, the per-wall constants and the YP heights; one block of 256
 template <typename R>
 __global__ void k_wall_shift_fin(StepArgs<R> a, LesArgs<R> l, int nb, double *ws, int zs, double tan16) {
+    pdl_enter();
     const Geo g = a.g;
     __shared__ double s[256], b[256];
     double x = 0.0, y = 0.0;
@@ -1080,6 +1096,7 @@ __global__ void k_wall_shift_fin(StepArgs<R> a, LesArgs<R> l, int nb, double *ws
 // TAUW and TAUB of one wall point per thread (2 N1M N3M threads: wall-major)
 template <typename R>
 __global__ void __launch_bounds__(TPB) k_wall_shift(StepArgs<R> a, LesArgs<R> l, const double *ws, WsMesh m) {
+    pdl_enter();
     const Geo g = a.g;
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= 2 * g.np) return;
@@ -1113,6 +1130,7 @@ __global__ void __launch_bounds__(TPB) k_wall_shift(StepArgs<R> a, LesArgs<R> l,
 
 template <typename R>
 __global__ void k_wall_sum(StepArgs<R> a, LesArgs<R> l, int nb) {
+    pdl_enter();
     __shared__ double s[256], b[256];
     double x = 0.0, y = 0.0;
     for (int q = threadIdx.x; q < nb; q += blockDim.x) {
@@ -1145,6 +1163,7 @@ __global__ void k_wall_sum(StepArgs<R> a, LesArgs<R> l, int nb) {
 // ---------------------------------------------------------------------------------
 template <typename R, int C>
 __global__ void __launch_bounds__(TPB) k_les_x1(StepArgs<R> a, LesArgs<R> l) {
+    pdl_enter();
     typedef typename SType<R>::S S;
     typedef St<R> ST;
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -1243,6 +1262,7 @@ struct WalkLesZ1 {
 // FP64 joins its segments (MODE 1), FP32 runs warm-ups (MODE 0), as the z passes of the step.
 template <typename R, int L, int MODE>
 __global__ void __launch_bounds__(MODE == 1 ? zjt<R, L>() : TPB) k_les_z1(StepArgs<R> a, LesArgs<R> l) {
+    pdl_enter();
     const Geo g = a.g;
     ZCo c;
     if (!zcoords<L, MODE>(Blk{blockIdx.x, blockIdx.y, gridDim.x}, g, 1, c)) return;
@@ -1301,6 +1321,7 @@ struct WalkLesZ2 {
 
 template <typename R, int L, int MODE>
 __global__ void __launch_bounds__(MODE == 1 ? zjt<R, L>() : TPB) k_les_z2(StepArgs<R> a, LesArgs<R> l) {
+    pdl_enter();
     typedef St<R> ST;
     typedef typename SType<R>::S S;
     const Geo g = a.g;
@@ -1362,6 +1383,7 @@ __global__ void __launch_bounds__(MODE == 1 ? zjt<R, L>() : TPB) k_les_z2(StepAr
 // ---------------------------------------------------------------------------------
 template <typename R, int C>
 __global__ void __launch_bounds__(TPB) k_les_x2(StepArgs<R> a, LesArgs<R> l) {
+    pdl_enter();
     typedef typename SType<R>::S S;
     typedef St<R> ST;
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -1492,11 +1514,11 @@ static void launch_les_x(c3d_channel *ch, StepArgs<R> &a, LesArgs<R> &l, int whi
     const double N = (double)ch->g.n1m * ch->g.n2m * ch->g.n3m, Rb = sizeof(R);
     if (which == 0) {
         cudaFuncSetAttribute(k_les_x1<R, C>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sb);
-        k_les_x1<R, C><<<grid, TPB, sb, ch->stream>>>(a, l);
+        klaunch(ch, ch->stream, k_les_x1<R, C>, grid, TPB, sb, a, l);
         mark(ch, nl, "les_x1", N * (24 + 6 * Rb));
     } else {
         cudaFuncSetAttribute(k_les_x2<R, C>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sb);
-        k_les_x2<R, C><<<grid, TPB, sb, ch->stream>>>(a, l);
+        klaunch(ch, ch->stream, k_les_x2<R, C>, grid, TPB, sb, a, l);
         mark(ch, nl, "les_x2", N * (16 + 14 * Rb));
     }
 }
@@ -1515,7 +1537,7 @@ static int launch_les_z(c3d_channel *ch, StepArgs<R> &a, LesArgs<R> &l, int whic
     const long long ncol = (long long)g.n2m * g.n1m;
     auto go = [&](auto *fn, int nr, int L, int cols) {
         const int nt = cols * (g.n3m / L);
-        fn<<<nblk(ncol, cols), nt, 2 * (size_t)nr * nt * sizeof(R), ch->stream>>>(a, l);
+        klaunch(ch, ch->stream, fn, nblk(ncol, cols), nt, 2 * (size_t)nr * nt * sizeof(R), a, l);
     };
     if constexpr (sizeof(R) == 8) {
         switch (zjoin_len<R>(g.n3m)) {
@@ -1530,8 +1552,8 @@ static int launch_les_z(c3d_channel *ch, StepArgs<R> &a, LesArgs<R> &l, int whic
             default: break;
         }
     }
-    if (which == 0) k_les_z1<R, ZL, 0><<<nblk(ncol * (g.n3m / ZL)), TPB, 0, ch->stream>>>(a, l);
-    else k_les_z2<R, ZL, 0><<<nblk(ncol * (g.n3m / ZL)), TPB, 0, ch->stream>>>(a, l);
+    if (which == 0) klaunch(ch, ch->stream, k_les_z1<R, ZL, 0>, nblk(ncol * (g.n3m / ZL)), TPB, 0, a, l);
+    else klaunch(ch, ch->stream, k_les_z2<R, ZL, 0>, nblk(ncol * (g.n3m / ZL)), TPB, 0, a, l);
     return 0;
 }
 
@@ -1551,7 +1573,7 @@ int launch_les(c3d_channel *ch, StepArgs<R> &a, LesArgs<R> &l, int stage, int *n
             ch->sjoin_pending = 0;
         }
         if (ch->files != 0 && ch->wmodel == 0) {
-            k_les_wallss<R><<<1, 256, 0, st>>>(a);
+            klaunch(ch, st, k_les_wallss<R>, 1, 256, 0, a);
             mark(ch, nl, "les_wallss", 64.0 * g.np);
         }
         // The wall model reads the state and WSM and writes TAUW, TAUB and WSM(1); the SGS
@@ -1563,7 +1585,7 @@ int launch_les(c3d_channel *ch, StepArgs<R> &a, LesArgs<R> &l, int stage, int *n
         const cudaStream_t wst = fork ? ch->wside : st;
         auto wall_model = [&]() -> int {
             if (ch->files != 0 && ch->wmodel == 5) {
-                k_wall_shift_v1<R><<<nblk(g.np), TPB, 0, st>>>(a, ch->wshift);
+                klaunch(ch, st, k_wall_shift_v1<R>, nblk(g.np), TPB, 0, a, ch->wshift);
                 *nl += 1;
             }
             if (fork) {
@@ -1572,19 +1594,19 @@ int launch_les(c3d_channel *ch, StepArgs<R> &a, LesArgs<R> &l, int stage, int *n
             }
             if (ch->files != 0 && ch->wmodel == 1 && ch->wrough) {
                 const int nb = nblk(g.np);
-                k_wall_rough<R><<<nb, TPB, 0, wst>>>(a, l, ch->wklog);
-                k_wall_sum<R><<<1, 256, 0, wst>>>(a, l, nb);
+                klaunch(ch, wst, k_wall_rough<R>, nb, TPB, 0, a, l, ch->wklog);
+                klaunch(ch, wst, k_wall_sum<R>, 1, 256, 0, a, l, nb);
                 mark(ch, nl, "wall", 24.0 * g.np);
             } else if (ch->files != 0 && ch->wmodel == 1) {
                 const int nb = nblk(g.np);
-                k_wall<R><<<nb, TPB, 0, wst>>>(a, l);
-                k_wall_sum<R><<<1, 256, 0, wst>>>(a, l, nb);
+                klaunch(ch, wst, k_wall<R>, nb, TPB, 0, a, l);
+                klaunch(ch, wst, k_wall_sum<R>, 1, 256, 0, a, l, nb);
                 mark(ch, nl, "wall", 32.0 * g.np);
             } else if (ch->files != 0 && ch->wmodel == 4) {
                 const int nb = nblk(g.np);
-                k_wall_werner<R><<<nb, TPB, 0, wst>>>(a, l, ch->wtaue);
-                k_wall_sum<R><<<1, 256, 0, wst>>>(a, l, nb);
-                k_wall_werner_avg<R><<<nb, TPB, 0, wst>>>(a, l, ch->wtaue);
+                klaunch(ch, wst, k_wall_werner<R>, nb, TPB, 0, a, l, ch->wtaue);
+                klaunch(ch, wst, k_wall_sum<R>, 1, 256, 0, a, l, nb);
+                klaunch(ch, wst, k_wall_werner_avg<R>, nb, TPB, 0, a, l, ch->wtaue);
                 *nl += 2;
                 mark(ch, nl, "wall", 96.0 * g.np);
             } else if (ch->files != 0 && ch->wmodel == 2) {
@@ -1594,9 +1616,9 @@ int launch_les(c3d_channel *ch, StepArgs<R> &a, LesArgs<R> &l, int stage, int *n
             } else if (ch->files != 0 && (ch->wmodel == 3 || ch->wmodel == 5)) {
                 const int nb = nblk(g.np);
                 const int jd = ch->wmodel == 3 ? ch->wzs : 1, ju = ch->wmodel == 3 ? g.n2m - ch->wzs + 1 : g.n2m;
-                k_wall_shift_mean<R><<<nb, TPB, 0, wst>>>(a, l, jd, ju);
-                k_wall_shift_fin<R><<<1, 256, 0, wst>>>(a, l, nb, ch->wshift, ch->wzs, ch->wtan16);
-                k_wall_shift<R><<<nblk(2LL * g.np), TPB, 0, wst>>>(a, l, ch->wshift, WsMesh::of(g, ch->wshift));
+                klaunch(ch, wst, k_wall_shift_mean<R>, nb, TPB, 0, a, l, jd, ju);
+                klaunch(ch, wst, k_wall_shift_fin<R>, 1, 256, 0, a, l, nb, ch->wshift, ch->wzs, ch->wtan16);
+                klaunch(ch, wst, k_wall_shift<R>, nblk(2LL * g.np), TPB, 0, a, l, ch->wshift, WsMesh::of(g, ch->wshift));
                 *nl += 2;
                 // per wall point: u on two planes, eight corners of two components, two stresses
                 const double Sb = sizeof(typename StepArgs<R>::S);
@@ -1607,24 +1629,24 @@ int launch_les(c3d_channel *ch, StepArgs<R> &a, LesArgs<R> &l, int stage, int *n
         };
         int rc = 0;
         if (ch->files == 2) {
-            k_sgs_coef<R><<<1, 128, 0, st>>>(a, l);
+            klaunch(ch, st, k_sgs_coef<R>, 1, 128, 0, a, l);
             if ((rc = wall_model())) return rc;
-            k_sgs_cs<R><<<nblk((long long)g.n2m * g.np), TPB, 0, st>>>(a, l);
+            klaunch(ch, st, k_sgs_cs<R>, nblk((long long)g.n2m * g.np), TPB, 0, a, l);
             mark(ch, nl, "sgs_cs", N * (6 * 8 + Rb));
         } else if (ch->files == 1) {
             if ((rc = wall_model())) return rc;
-            k_sgs_raw<R><<<nblk((long long)g.n2m * g.np), TPB, 0, st>>>(a, l);
+            klaunch(ch, st, k_sgs_raw<R>, nblk((long long)g.n2m * g.np), TPB, 0, a, l);
             mark(ch, nl, "sgs_raw", N * (6 * 8 + 22 * Rb));
-            k_sgs_dy_sums<R><<<dim3((g.n1m + SD_TX - 1) / SD_TX, g.n3m / SD_TZ, g.n2m), SD_THREADS, 0, st>>>(a, l, ch->sdpart);
-            k_sgs_dy_coef<R><<<g.n2m, 32, 0, st>>>(a, l, ch->sdpart, ch->sdnt);
-            k_sgs_apply<R><<<nblk((long long)g.n2m * g.np), TPB, 0, st>>>(a, l);
+            klaunch(ch, st, k_sgs_dy_sums<R>, dim3((g.n1m + SD_TX - 1) / SD_TX, g.n3m / SD_TZ, g.n2m), SD_THREADS, 0, a, l, ch->sdpart);
+            klaunch(ch, st, k_sgs_dy_coef<R>, g.n2m, 32, 0, a, l, ch->sdpart, ch->sdnt);
+            klaunch(ch, st, k_sgs_apply<R>, nblk((long long)g.n2m * g.np), TPB, 0, a, l);
             *nl += 2;
             mark(ch, nl, "sgs_dyn", N * 23 * Rb);
         } else if (ch->files == 3) {
             if ((rc = wall_model())) return rc;
-            k_sgs_raw<R><<<nblk((long long)g.n2m * g.np), TPB, 0, st>>>(a, l);
+            klaunch(ch, st, k_sgs_raw<R>, nblk((long long)g.n2m * g.np), TPB, 0, a, l);
             mark(ch, nl, "sgs_raw", N * (6 * 8 + 22 * Rb));
-            k_sgs_sd_sums<R><<<dim3((g.n1m + SD_TX - 1) / SD_TX, g.n3m / SD_TZ, g.n2m), SD_THREADS, 0, st>>>(a, l, ch->sdpart);
+            klaunch(ch, st, k_sgs_sd_sums<R>, dim3((g.n1m + SD_TX - 1) / SD_TX, g.n3m / SD_TZ, g.n2m), SD_THREADS, 0, a, l, ch->sdpart);
             mark(ch, nl, "sgs_sd_sums", N * 21 * Rb);
             const bool sfork = ch->sside && !ch->prof_on;
             const cudaStream_t sst = sfork ? ch->sside : st;
@@ -1632,8 +1654,8 @@ int launch_les(c3d_channel *ch, StepArgs<R> &a, LesArgs<R> &l, int stage, int *n
                 CK_RC(cudaEventRecord(ch->sfork, st));
                 CK_RC(cudaStreamWaitEvent(sst, ch->sfork, 0));
             }
-            k_sgs_sd_coef<R><<<g.n2m, 32, 0, sst>>>(a, l, ch->sdpart, ch->sdnt, ch->sdbeta);
-            k_sgs_apply<R><<<nblk((long long)g.n2m * g.np), TPB, 0, sst>>>(a, l);
+            klaunch(ch, sst, k_sgs_sd_coef<R>, g.n2m, 32, 0, a, l, ch->sdpart, ch->sdnt, ch->sdbeta);
+            klaunch(ch, sst, k_sgs_apply<R>, nblk((long long)g.n2m * g.np), TPB, 0, a, l);
             if (sfork) {
                 CK_RC(cudaEventRecord(ch->sjoin, sst));
                 ch->sjoin_pending = 1;

@@ -35,6 +35,7 @@ struct WalkIrZ {
 
 template <int L>
 __global__ void __launch_bounds__(TPB) k_ir_z(StepArgs<float> a, RefArgs r) {
+    pdl_enter();
     const Geo g = a.g;
     int i, j, k0;
     if (!zcoord<L>(g, 1, i, j, k0)) return;
@@ -54,6 +55,7 @@ __global__ void __launch_bounds__(TPB) k_ir_z(StepArgs<float> a, RefArgs r) {
 
 template <int C>
 __global__ void __launch_bounds__(TPB) k_ir_x(StepArgs<float> a, RefArgs r) {
+    pdl_enter();
     typedef float2 C2;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const Geo g = a.g;
@@ -121,6 +123,7 @@ __global__ void __launch_bounds__(TPB) k_ir_x(StepArgs<float> a, RefArgs r) {
 
 template <int C>
 __global__ void __launch_bounds__(TPB) k_ir_d(StepArgs<float> a) {
+    pdl_enter();
     typedef float2 C2;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const Geo g = a.g;
@@ -178,6 +181,7 @@ struct WalkIrGrad {
 
 template <int L>
 __global__ void __launch_bounds__(TPB) k_ir_e(StepArgs<float> a, int updp) {
+    pdl_enter();
     typedef St<float> ST;
     const Geo g = a.g;
     int i, j, k0;
@@ -224,10 +228,10 @@ static void launch_ir_x(c3d_channel *ch, StepArgs<float> &a, RefArgs &r, int whi
     const int grid = nblk((long long)ch->g.n2m * ch->g.n3m, TPB / 32);
     if (which == 0) {
         cudaFuncSetAttribute(k_ir_x<C>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fb);
-        k_ir_x<C><<<grid, TPB, fb, ch->stream>>>(a, r);
+        klaunch(ch, ch->stream, k_ir_x<C>, grid, TPB, fb, a, r);
     } else {
         cudaFuncSetAttribute(k_ir_d<C>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fb);
-        k_ir_d<C><<<grid, TPB, fb, ch->stream>>>(a);
+        klaunch(ch, ch->stream, k_ir_d<C>, grid, TPB, fb, a);
     }
 }
 
@@ -249,7 +253,7 @@ int launch_refine(c3d_channel *ch, StepArgs<float> &a, RefArgs &r, int *nl) {
     const double N = (double)g.n1m * g.n2m * g.n3m;
     const long long nz = (long long)g.n2m * (g.n3m / ZL) * g.n1m;
     int rc;
-    k_ir_z<ZL><<<nblk(nz), TPB, 0, ch->stream>>>(a, r);
+    klaunch(ch, ch->stream, k_ir_z<ZL>, nblk(nz), TPB, 0, a, r);
     mark(ch, nl, "ir_z", N * 16);
     if ((rc = ir_x(ch, a, r, 0))) return rc;
     mark(ch, nl, "ir_x", N * (24 + 8 + 8));
@@ -258,7 +262,7 @@ int launch_refine(c3d_channel *ch, StepArgs<float> &a, RefArgs &r, int *nl) {
         return rc;
     if ((rc = ir_x(ch, a, r, 1))) return rc;
     mark(ch, nl, "ir_d", N * (8 + 8));
-    k_ir_e<ZL><<<nblk(nz), TPB, 0, ch->stream>>>(a, r.updp);
+    klaunch(ch, ch->stream, k_ir_e<ZL>, nblk(nz), TPB, 0, a, r.updp);
     mark(ch, nl, "ir_e", N * (64 + 12));
     return 0;
 }

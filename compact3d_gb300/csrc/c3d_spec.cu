@@ -35,6 +35,7 @@ __device__ __forceinline__ void b_fftz(const StepArgs<R> &a, int sign, int tw, c
 }
 template <typename R>
 __global__ void __launch_bounds__(TPB) k_fftz(StepArgs<R> a, int sign, int tw) {
+    pdl_enter();
     b_fftz<R>(a, sign, tw, Blk{blockIdx.x, blockIdx.y, gridDim.x});
 }
 
@@ -116,6 +117,7 @@ __device__ __forceinline__ void b_fftz4(const StepArgs<R> &a, const Blk blk) {
 }
 template <typename R, int N1, int SIGN>
 __global__ void __launch_bounds__(FZW * 32) k_fftz4(StepArgs<R> a) {
+    pdl_enter();
     b_fftz4<R, N1, SIGN>(a, Blk{blockIdx.x, blockIdx.y, gridDim.x});
 }
 
@@ -182,6 +184,7 @@ __device__ __forceinline__ void b_poisson64(const StepArgs<double> &a, const Blk
     }
 }
 __global__ void __launch_bounds__(TPB) k_poisson64(StepArgs<double> a) {
+    pdl_enter();
     b_poisson64(a, Blk{blockIdx.x, blockIdx.y, gridDim.x});
 }
 
@@ -253,6 +256,7 @@ __device__ __forceinline__ void b_poisson32(const StepArgs<float> &a, const Blk 
     }
 }
 __global__ void __launch_bounds__(TPB) k_poisson32(StepArgs<float> a) {
+    pdl_enter();
     b_poisson32(a, Blk{blockIdx.x, blockIdx.y, gridDim.x});
 }
 
@@ -319,7 +323,7 @@ static bool launch_fftz4(c3d_channel *ch, StepArgs<R> &a) {
         cudaGetLastError();
         return false;
     }
-    fn<<<grid, blk, sm, ch->stream>>>(a);
+    klaunch(ch, ch->stream, fn, grid, blk, sm, a);
     return true;
 }
 
@@ -332,19 +336,23 @@ constexpr int TW_BATCH = 8;
 
 template <typename R, int N1, int SIGN>
 __global__ void __launch_bounds__(FZW * 32) kb_fftz4(const StepArgs<R> *__restrict__ A, const BMap *__restrict__ map) {
+    pdl_enter();
     const BMap m = map[blockIdx.x];
     b_fftz4<R, N1, SIGN>(A[m.ch], Blk{m.x, m.y, m.gx});
 }
 template <typename R, int SIGN>
 __global__ void __launch_bounds__(TPB) kb_fftz(const StepArgs<R> *__restrict__ A, const BMap *__restrict__ map) {
+    pdl_enter();
     const BMap m = map[blockIdx.x];
     b_fftz<R>(A[m.ch], SIGN, TW_BATCH, Blk{m.x, m.y, m.gx});
 }
 __global__ void __launch_bounds__(TPB) kb_poisson64(const StepArgs<double> *__restrict__ A, const BMap *__restrict__ map) {
+    pdl_enter();
     const BMap m = map[blockIdx.x];
     b_poisson64(A[m.ch], Blk{m.x, m.y, m.gx});
 }
 __global__ void __launch_bounds__(TPB) kb_poisson32(const StepArgs<float> *__restrict__ A, const BMap *__restrict__ map) {
+    pdl_enter();
     const BMap m = map[blockIdx.x];
     b_poisson32(A[m.ch], Blk{m.x, m.y, m.gx});
 }
@@ -404,13 +412,13 @@ int launch_spec(c3d_channel *ch, StepArgs<R> &a, int which, int *nl) {
     const int ntile = (ch->g.n1h + tw - 1) / tw;
     const size_t smz = 2 * (size_t)ch->g.n3m * tw * sizeof(C2);
     switch (which) {
-        case 0: k_fftz<R><<<ch->g.n2m * ntile, TPB, smz, st>>>(a, -1, tw); mark(ch, nl, "fftz_fwd", N * 2 * Rb); break;
+        case 0: klaunch(ch, st, k_fftz<R>, ch->g.n2m * ntile, TPB, smz, a, -1, tw); mark(ch, nl, "fftz_fwd", N * 2 * Rb); break;
         case 1:
-            if constexpr (sizeof(R) == 8) k_poisson64<<<nblk((long long)ch->g.n1h * ch->g.n3m), TPB, 0, st>>>(a);
-            else k_poisson32<<<nblk((long long)ch->g.n1h * ch->g.n3m), TPB, 0, st>>>(a);
+            if constexpr (sizeof(R) == 8) klaunch(ch, st, k_poisson64, nblk((long long)ch->g.n1h * ch->g.n3m), TPB, 0, a);
+            else klaunch(ch, st, k_poisson32, nblk((long long)ch->g.n1h * ch->g.n3m), TPB, 0, a);
             mark(ch, nl, "poisson", N * 2 * Rb + N * 8);
             break;
-        case 2: k_fftz<R><<<ch->g.n2m * ntile, TPB, smz, st>>>(a, +1, tw); mark(ch, nl, "fftz_inv", N * 2 * Rb); break;
+        case 2: klaunch(ch, st, k_fftz<R>, ch->g.n2m * ntile, TPB, smz, a, +1, tw); mark(ch, nl, "fftz_inv", N * 2 * Rb); break;
         default: return C3D_EINVAL;
     }
     return 0;

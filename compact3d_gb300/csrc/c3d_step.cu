@@ -44,6 +44,7 @@ __device__ __forceinline__ void b_bcond(Geo g, typename SType<R>::S *u, typename
 }
 template <typename R>
 __global__ void k_bcond(Geo g, typename SType<R>::S *u, typename SType<R>::S *v, typename SType<R>::S *w) {
+    pdl_enter();
     b_bcond<R>(g, u, v, w, Blk{blockIdx.x, blockIdx.y, gridDim.x});
 }
 
@@ -99,6 +100,7 @@ __device__ __forceinline__ void b_ycn(const StepArgs<R> &a, const R *ycn, const 
 }
 template <typename R>
 __global__ void __launch_bounds__(TPB) k_ycn(StepArgs<R> a, const R *ycn) {
+    pdl_enter();
     b_ycn<R>(a, ycn, Blk{blockIdx.x, blockIdx.y, gridDim.x});
 }
 
@@ -205,6 +207,7 @@ __device__ __forceinline__ void b_ycnt(const StepArgs<R> &a, const R *ycn, const
 }
 template <typename R, int TX>
 __global__ void __launch_bounds__(64) k_ycnt(StepArgs<R> a, const R *ycn) {
+    pdl_enter();
     b_ycnt<R, TX>(a, ycn, Blk{blockIdx.x, blockIdx.y, gridDim.x});
 }
 
@@ -222,14 +225,14 @@ static void launch_ycn(c3d_channel *ch, StepArgs<R> &a, int *nl) {
         if (tx == 32) {
             cudaFuncSetAttribute(k_ycnt<R, 32>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
             cudaFuncSetAttribute(k_ycnt<R, 32>, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
-            k_ycnt<R, 32><<<nb, 32, sm, ch->stream>>>(a, ycn);
+            klaunch(ch, ch->stream, k_ycnt<R, 32>, nb, 32, sm, a, ycn);
         } else {
             cudaFuncSetAttribute(k_ycnt<R, 64>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
             cudaFuncSetAttribute(k_ycnt<R, 64>, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
-            k_ycnt<R, 64><<<nb, 64, sm, ch->stream>>>(a, ycn);
+            klaunch(ch, ch->stream, k_ycnt<R, 64>, nb, 64, sm, a, ycn);
         }
     } else {
-        k_ycn<R><<<nblk(3LL * ch->g.np), TPB, 0, ch->stream>>>(a, ycn);
+        klaunch(ch, ch->stream, k_ycn<R>, nblk(3LL * ch->g.np), TPB, 0, a, ycn);
     }
     mark(ch, nl, "ycn", (double)ch->g.n1m * ch->g.n2m * ch->g.n3m * 6 * sizeof(R));
 }
@@ -294,6 +297,7 @@ __device__ __forceinline__ void b_reduce1(Geo g, typename A::T *part, const Blk 
 }
 template <typename A>
 __global__ void __launch_bounds__(256) k_reduce1(Geo g, typename A::T *part) {
+    pdl_enter();
     b_reduce1<A>(g, part, Blk{blockIdx.x, blockIdx.y, gridDim.x});
 }
 
@@ -316,6 +320,7 @@ __device__ __forceinline__ void b_reduce2(Geo g, const typename A::T *part, doub
 }
 template <typename A>
 __global__ void __launch_bounds__(RB) k_reduce2(Geo g, const typename A::T *part, double *scal, double dt, int bulk) {
+    pdl_enter();
     b_reduce2<A>(g, part, scal, dt, bulk, Blk{blockIdx.x, blockIdx.y, gridDim.x});
 }
 
@@ -331,6 +336,7 @@ inline int diag_blocks(const Geo &g) {
 template <typename R>
 __global__ void __launch_bounds__(DST) k_diag_sums(Geo g, const typename SType<R>::S *u, const typename SType<R>::S *v,
                                                    const typename SType<R>::S *w, double *scal, double *part) {
+    pdl_enter();
     typedef St<R> ST;
     __shared__ double sh[5][DST];
     __shared__ bool last;
@@ -533,11 +539,11 @@ static int pressure_and_update(c3d_channel *ch, StepArgs<R> &a, R *d0, R *d1, R 
     if ((rc = launch_spec<R>(ch, a, 2, nl))) return rc;                       // fftz inv
     if ((rc = launch_xpass<R>(ch, a, 3, d0, d2, nl))) return rc;              // xD
     if constexpr (sizeof(R) == 8) {
-        k_reduce1<AddF64><<<RB, 256, 0, ch->stream>>>(ch->g, ch->part);
-        k_reduce2<AddF64><<<1, RB, 0, ch->stream>>>(ch->g, ch->part, ch->scal, a.dt, a.bulk);
+        klaunch(ch, ch->stream, k_reduce1<AddF64>, RB, 256, 0, ch->g, ch->part);
+        klaunch(ch, ch->stream, k_reduce2<AddF64>, 1, RB, 0, ch->g, ch->part, ch->scal, a.dt, a.bulk);
     } else {
-        k_reduce1<AddDF><<<RB, 256, 0, ch->stream>>>(ch->g, (float2 *)ch->part);
-        k_reduce2<AddDF><<<1, RB, 0, ch->stream>>>(ch->g, (const float2 *)ch->part, ch->scal, a.dt, a.bulk);
+        klaunch(ch, ch->stream, k_reduce1<AddDF>, RB, 256, 0, ch->g, (float2 *)ch->part);
+        klaunch(ch, ch->stream, k_reduce2<AddDF>, 1, RB, 0, ch->g, (const float2 *)ch->part, ch->scal, a.dt, a.bulk);
     }
     ++*nl;   // the reduction is two launches under one profiler mark
     mark(ch, nl, "reduce", 16.0 * ch->g.n2m * ch->g.n3m);
@@ -610,7 +616,7 @@ static int step_impl(c3d_channel *ch, double dt, int *nl) {
     LesArgs<R> l = make_les_args<R>(ch);
     // GETUP order (compact3d.f:931-940): SGS model and wall model, then BCOND
     if (ch->files != 0 && (rc = launch_les<R>(ch, a, l, 0, nl))) return rc;
-    k_bcond<R><<<nblk(ch->g.np), TPB, 0, ch->stream>>>(ch->g, (S *)ch->u, (S *)ch->v, (S *)ch->w);
+    klaunch(ch, ch->stream, k_bcond<R>, nblk(ch->g.np), TPB, 0, ch->g, (S *)ch->u, (S *)ch->v, (S *)ch->w);
     mark(ch, nl, "bcond", 64.0 * ch->g.np);
     if ((rc = launch_xpass<R>(ch, a, 0, nullptr, nullptr, nl))) return rc;    // xA
     if ((rc = launch_zpass<R>(ch, a, 0, nullptr, nullptr, nullptr, 0, nl))) return rc;   // zA
@@ -635,24 +641,28 @@ static int step_impl(c3d_channel *ch, double dt, int *nl) {
 // ---------------------------------------------------------------------------------
 template <typename R>
 __global__ void __launch_bounds__(TPB) kb_bcond(const StepArgs<R> *__restrict__ A, const BMap *__restrict__ map) {
+    pdl_enter();
     const BMap m = map[blockIdx.x];
     const StepArgs<R> &a = A[m.ch];
     b_bcond<R>(a.g, a.u, a.v, a.w, Blk{m.x, m.y, m.gx});
 }
 template <typename R>
 __global__ void __launch_bounds__(TPB) kb_ycn(const StepArgs<R> *__restrict__ A, const BMap *__restrict__ map) {
+    pdl_enter();
     const BMap m = map[blockIdx.x];
     const StepArgs<R> &a = A[m.ch];
     b_ycn<R>(a, a.ycnw, Blk{m.x, m.y, m.gx});
 }
 template <typename R, typename Add>
 __global__ void __launch_bounds__(256) kb_reduce1(const StepArgs<R> *__restrict__ A, const BMap *__restrict__ map) {
+    pdl_enter();
     const BMap m = map[blockIdx.x];
     const StepArgs<R> &a = A[m.ch];
     b_reduce1<Add>(a.g, reinterpret_cast<typename Add::T *>(a.part), Blk{m.x, m.y, m.gx});
 }
 template <typename R, typename Add>
 __global__ void __launch_bounds__(RB) kb_reduce2(const StepArgs<R> *__restrict__ A, const BMap *__restrict__ map) {
+    pdl_enter();
     const BMap m = map[blockIdx.x];
     const StepArgs<R> &a = A[m.ch];
     b_reduce2<Add>(a.g, reinterpret_cast<const typename Add::T *>(a.part), a.scal, a.dt, a.bulk, Blk{m.x, m.y, m.gx});
@@ -793,7 +803,7 @@ static int project_impl(c3d_channel *ch, int *nl) {
     cudaMemsetAsync(dd0, 0, bytes, ch->stream);
     cudaMemsetAsync(dd1, 0, bytes, ch->stream);
     cudaMemsetAsync(dd2, 0, bytes, ch->stream);
-    k_bcond<R><<<nblk(ch->g.np), TPB, 0, ch->stream>>>(ch->g, (S *)ch->u, (S *)ch->v, (S *)ch->w);
+    klaunch(ch, ch->stream, k_bcond<R>, nblk(ch->g.np), TPB, 0, ch->g, (S *)ch->u, (S *)ch->v, (S *)ch->w);
     mark(ch, nl, "bcond", 64.0 * ch->g.np);
     int rc = pressure_and_update<R>(ch, a, dd0, dd1, dd2, 0, nl);
     if (rc) return rc;
@@ -815,8 +825,7 @@ static int diag_impl(c3d_channel *ch, int *nl) {
     if ((rc = launch_xpass<R>(ch, a, 4, (const R *)ch->diagbuf, nullptr, nl))) return rc;
     if ((rc = launch_zpass<R>(ch, a, 5, (R *)ch->diagbuf, nullptr, nullptr, 0, nl))) return rc;
     // its partial sums go to the scratch field, which diag_z has finished reading
-    k_diag_sums<R><<<diag_blocks(ch->g), DST, 0, ch->stream>>>(ch->g, (const S *)ch->u, (const S *)ch->v, (const S *)ch->w,
-                                                              ch->scal, ch->diagbuf);
+    klaunch(ch, ch->stream, k_diag_sums<R>, diag_blocks(ch->g), DST, 0, ch->g, (const S *)ch->u, (const S *)ch->v, (const S *)ch->w, ch->scal, ch->diagbuf);
     mark(ch, nl, "diag_sums", 64.0 * ch->g.np);
     return 0;
 }

@@ -14,22 +14,26 @@ namespace c3d {
 
 template <typename R, int C, int PART, int W = 32>
 __global__ void __launch_bounds__(XMAXT) kb_xA(const StepArgs<R> *__restrict__ A, const BMap *__restrict__ map) {
+    pdl_enter();
     const BMap m = map[blockIdx.x];
     b_xA<R, C, PART, W>(A[m.ch], Blk{m.x, m.y, m.gx});
 }
 template <typename R, int C, int W = 32>
 __global__ void __launch_bounds__(XMAXT) kb_xB(const StepArgs<R> *__restrict__ A, const BMap *__restrict__ map) {
+    pdl_enter();
     const BMap m = map[blockIdx.x];
     b_xB<R, C, W>(A[m.ch], Blk{m.x, m.y, m.gx});
 }
 template <typename R, int C, bool X4, int W = 32>
 __global__ void __launch_bounds__(XMAXT) kb_xC(const StepArgs<R> *__restrict__ A, const BMap *__restrict__ map) {
+    pdl_enter();
     const BMap m = map[blockIdx.x];
     const StepArgs<R> &a = A[m.ch];
     b_xC<R, C, 0, X4, W>(a, a.exz, a.eyz, Blk{m.x, m.y, m.gx});
 }
 template <typename R, int C, bool X4, int W = 32>
 __global__ void __launch_bounds__(XMAXT) kb_xD(const StepArgs<R> *__restrict__ A, const BMap *__restrict__ map) {
+    pdl_enter();
     const BMap m = map[blockIdx.x];
     const StepArgs<R> &a = A[m.ch];
     b_xD<R, C, X4, W>(a, a.exz, a.wsq, Blk{m.x, m.y, m.gx});

@@ -71,7 +71,7 @@ static bool launch_xc_bulk(c3d_channel *ch, StepArgs<R> &a, int xw, const R *p0,
     const int nrows = g.n2m * g.n3m;
     const int grid = persistent_grid((const void *)fn, xw * 32, smem, nblk(nrows, xw), ch->device);
     if (grid <= 0) return false;
-    fn<<<grid, xw * 32, smem, ch->stream>>>(a, p0, p1);
+    klaunch(ch, ch->stream, fn, grid, xw * 32, smem, a, p0, p1);
     return true;
 }
 
@@ -99,11 +99,11 @@ static int launch_x_c(c3d_channel *ch, StepArgs<R> &a, int which, const R *p0, c
                 cudaFuncSetAttribute(k_xAs<R, C, 3>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)s3);
                 const bool cc = par_on(ch);   // the pieces as concurrent branches (knob 15)
                 if (cc && (rc = par_fork(ch))) return rc;
-                k_xAs<R, C, 1><<<grid, nt, s1, cc ? ch->par[0] : st>>>(a);
+                klaunch(ch, cc ? ch->par[0] : st, k_xAs<R, C, 1>, grid, nt, s1, a);
                 mark(ch, nl, "xA_u", N * (16 + 2 * Rb));
-                k_xAs<R, C, 2><<<grid, nt, s2, cc ? ch->par[1] : st>>>(a);
+                klaunch(ch, cc ? ch->par[1] : st, k_xAs<R, C, 2>, grid, nt, s2, a);
                 mark(ch, nl, "xA_v", N * (24 + 3 * Rb));
-                k_xAs<R, C, 3><<<grid, nt, s3, st>>>(a);
+                klaunch(ch, st, k_xAs<R, C, 3>, grid, nt, s3, a);
                 mark(ch, nl, "xA_w", N * (8 + 2 * Rb));
                 if (cc && (rc = par_join(ch))) return rc;
                 break;
@@ -114,22 +114,22 @@ static int launch_x_c(c3d_channel *ch, StepArgs<R> &a, int which, const R *p0, c
                 cudaFuncSetAttribute(k_xA<R, C, 3>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sb);
                 const bool cc = par_on(ch);
                 if (cc && (rc = par_fork(ch))) return rc;
-                k_xA<R, C, 1><<<grid, nt, sb, cc ? ch->par[0] : st>>>(a);
+                klaunch(ch, cc ? ch->par[0] : st, k_xA<R, C, 1>, grid, nt, sb, a);
                 mark(ch, nl, "xA_u", N * (16 + 2 * Rb));   // u, P; R1, HH1
-                k_xA<R, C, 2><<<grid, nt, sb, cc ? ch->par[1] : st>>>(a);
+                klaunch(ch, cc ? ch->par[1] : st, k_xA<R, C, 2>, grid, nt, sb, a);
                 mark(ch, nl, "xA_v", N * (24 + 3 * Rb));   // v, P, u; R2, HH2, E_xy
-                k_xA<R, C, 3><<<grid, nt, sb, st>>>(a);
+                klaunch(ch, st, k_xA<R, C, 3>, grid, nt, sb, a);
                 mark(ch, nl, "xA_w", N * (8 + 2 * Rb));    // w; R3, WW1
                 if (cc && (rc = par_join(ch))) return rc;
                 break;
             }
             cudaFuncSetAttribute(k_xA<R, C, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sb);
-            k_xA<R, C, 0><<<grid, nt, sb, st>>>(a);
+            klaunch(ch, st, k_xA<R, C, 0>, grid, nt, sb, a);
             mark(ch, nl, "xA", N * (32 + 7 * Rb));
             break;
         case 1:
             cudaFuncSetAttribute(k_xB<R, C>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sb);
-            k_xB<R, C><<<grid, nt, sb, st>>>(a);
+            klaunch(ch, st, k_xB<R, C>, grid, nt, sb, a);
             mark(ch, nl, "xB", N * 18 * Rb);
             break;
         case 2: {
@@ -146,22 +146,22 @@ static int launch_x_c(c3d_channel *ch, StepArgs<R> &a, int which, const R *p0, c
             }
             // register row FFT (all 32 lanes hold a chunk: N1M = 32 C, C even): no shared memory
             if (!done && C % 2 == 0 && ch->tune.fxp == 3 && ch->g.n1m == 32 * C) {
-                k_xC<R, C, 0, (C % 2 == 0)><<<grid, nt, sb, st>>>(a, p0, p1);
+                klaunch(ch, st, k_xC<R, C, 0, (C % 2 == 0)>, grid, nt, sb, a, p0, p1);
                 done = true;
             }
             if (!done) {
                 cudaFuncSetAttribute(k_xC<R, C, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fb);
-                k_xC<R, C, 0><<<grid, nt, fb, st>>>(a, p0, p1);
+                klaunch(ch, st, k_xC<R, C, 0>, grid, nt, fb, a, p0, p1);
             }
             mark(ch, nl, "xC", N * (16 + 4 * Rb));
             break;
         }
         case 3:
             if (C % 2 == 0 && ch->tune.fxp == 3 && ch->g.n1m == 32 * C) {
-                k_xD<R, C, (C % 2 == 0)><<<grid, nt, sb, st>>>(a, p0, p1);
+                klaunch(ch, st, k_xD<R, C, (C % 2 == 0)>, grid, nt, sb, a, p0, p1);
             } else {
                 cudaFuncSetAttribute(k_xD<R, C>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fb);
-                k_xD<R, C><<<grid, nt, fb, st>>>(a, p0, p1);
+                klaunch(ch, st, k_xD<R, C>, grid, nt, fb, a, p0, p1);
             }
             mark(ch, nl, "xD", N * 5 * Rb);
             break;
@@ -169,7 +169,7 @@ static int launch_x_c(c3d_channel *ch, StepArgs<R> &a, int which, const R *p0, c
             const double b = 22.0, r = -2.0 / (b + sqrt(b * b - 4.0));
             Cyc<double> c22 = {r, -r, (int)ceil(log(1e-17) / log(fabs(r)))};
             cudaFuncSetAttribute(k_diag_x<R, C>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sb);
-            k_diag_x<R, C><<<grid, TPB, sb, st>>>(a, (double *)p0, c22);
+            klaunch(ch, st, k_diag_x<R, C>, grid, TPB, sb, a, (double *)p0, c22);
             mark(ch, nl, "diag_x", N * 48);
             break;
         }
@@ -195,13 +195,13 @@ static int launch_x_seg(c3d_channel *ch, StepArgs<R> &a, int which, const R *p0,
     cudaStream_t st = ch->stream;
     if (which == 2) {
         cudaFuncSetAttribute(k_xC<R, C, 0, false, W>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fb);
-        k_xC<R, C, 0, false, W><<<grid, nt, fb, st>>>(a, p0, p1);
+        klaunch(ch, st, k_xC<R, C, 0, false, W>, grid, nt, fb, a, p0, p1);
         mark(ch, nl, "xC", N * (16 + 4 * Rb));
         return 0;
     }
     if (which == 3) {
         cudaFuncSetAttribute(k_xD<R, C, false, W>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fb);
-        k_xD<R, C, false, W><<<grid, nt, fb, st>>>(a, p0, p1);
+        klaunch(ch, st, k_xD<R, C, false, W>, grid, nt, fb, a, p0, p1);
         mark(ch, nl, "xD", N * 5 * Rb);
         return 0;
     }
@@ -209,15 +209,15 @@ static int launch_x_seg(c3d_channel *ch, StepArgs<R> &a, int which, const R *p0,
         const bool cc = par_on(ch);   // the pieces as concurrent branches (knob 15)
         int rc;
         if (cc && (rc = par_fork(ch))) return rc;
-        k_xA<R, C, 1, W><<<grid, nt, 0, cc ? ch->par[0] : st>>>(a);
+        klaunch(ch, cc ? ch->par[0] : st, k_xA<R, C, 1, W>, grid, nt, 0, a);
         mark(ch, nl, "xA_u", N * (16 + 2 * Rb));
-        k_xA<R, C, 2, W><<<grid, nt, 0, cc ? ch->par[1] : st>>>(a);
+        klaunch(ch, cc ? ch->par[1] : st, k_xA<R, C, 2, W>, grid, nt, 0, a);
         mark(ch, nl, "xA_v", N * (24 + 3 * Rb));
-        k_xA<R, C, 3, W><<<grid, nt, 0, st>>>(a);
+        klaunch(ch, st, k_xA<R, C, 3, W>, grid, nt, 0, a);
         mark(ch, nl, "xA_w", N * (8 + 2 * Rb));
         if (cc && (rc = par_join(ch))) return rc;
     } else {
-        k_xB<R, C, W><<<grid, nt, 0, st>>>(a);
+        klaunch(ch, st, k_xB<R, C, W>, grid, nt, 0, a);
         mark(ch, nl, "xB", N * 18 * Rb);
     }
     return 0;

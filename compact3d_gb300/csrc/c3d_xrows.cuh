@@ -384,6 +384,7 @@ __device__ __forceinline__ void b_xA(const StepArgs<R> &a, const Blk blk) {
 // bound by the FP64 pipe, which a few warps fill: two blocks.
 template <typename R, int C, int PART, int W = 32>
 __global__ void __launch_bounds__(XMAXT, sizeof(R) == 8 ? 2 : 3) k_xA(StepArgs<R> a) {
+    pdl_enter();
     b_xA<R, C, PART, W>(a, Blk{blockIdx.x, blockIdx.y, gridDim.x});
 }
 
@@ -403,6 +404,7 @@ __host__ __device__ inline size_t xa_stage_bytes(int part, int n1m) {
 
 template <typename R, int C, int PART>
 __global__ void __launch_bounds__(XMAXT) k_xAs(StepArgs<R> a) {
+    pdl_enter();
     typedef typename SType<R>::S S;
     static_assert(sizeof(S) == 8, "state rows are 8-byte values");
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -558,6 +560,7 @@ __device__ __forceinline__ void b_xB(const StepArgs<R> &a, const Blk blk) {
 }
 template <typename R, int C, int W = 32>
 __global__ void __launch_bounds__(XMAXT) k_xB(StepArgs<R> a) {
+    pdl_enter();
     b_xB<R, C, W>(a, Blk{blockIdx.x, blockIdx.y, gridDim.x});
 }
 
@@ -743,6 +746,7 @@ __device__ __forceinline__ void b_xC(const StepArgs<R> &a, const R *d0, const R 
 }
 template <typename R, int C, int NS, bool X4 = false, int W = 32>
 __global__ void __launch_bounds__(XMAXT) k_xC(StepArgs<R> a, const R *d0, const R *d1) {
+    pdl_enter();
     b_xC<R, C, NS, X4, W>(a, d0, d1, Blk{blockIdx.x, blockIdx.y, gridDim.x});
 }
 
@@ -873,6 +877,7 @@ __device__ __forceinline__ void b_xD(const StepArgs<R> &a, const R *d0, const R 
 }
 template <typename R, int C, bool X4 = false, int W = 32>
 __global__ void __launch_bounds__(XMAXT) k_xD(StepArgs<R> a, const R *d0, const R *d2) {
+    pdl_enter();
     b_xD<R, C, X4, W>(a, d0, d2, Blk{blockIdx.x, blockIdx.y, gridDim.x});
 }
 
@@ -885,6 +890,7 @@ __global__ void __launch_bounds__(XMAXT) k_xD(StepArgs<R> a, const R *d0, const 
 // ---------------------------------------------------------------------------------
 template <typename R, int C>
 __global__ void __launch_bounds__(TPB) k_diag_x(StepArgs<R> a, double *divx, Cyc<double> c22) {
+    pdl_enter();
     typedef typename SType<R>::S S;
     typedef St<R> ST;
     extern __shared__ __align__(16) unsigned char smem_raw[];

@@ -259,6 +259,7 @@ __device__ __forceinline__ void b_zA(const StepArgs<R> &a, const Blk blk) {
 }
 template <typename R, int L, int PART, int MODE>
 __global__ void __launch_bounds__(MODE == 1 ? zjt<R, L>() : TPB) k_zA(StepArgs<R> a) {
+    pdl_enter();
     b_zA<R, L, PART, MODE>(a, Blk{blockIdx.x, blockIdx.y, gridDim.x});
 }
 
@@ -315,6 +316,7 @@ __device__ __forceinline__ void b_zB(const StepArgs<R> &a, const Blk blk) {
 }
 template <typename R, int L, int MODE>
 __global__ void __launch_bounds__(MODE == 1 ? zjt<R, L>() : TPB) k_zB(StepArgs<R> a) {
+    pdl_enter();
     b_zB<R, L, MODE>(a, Blk{blockIdx.x, blockIdx.y, gridDim.x});
 }
 
@@ -354,6 +356,7 @@ __device__ __forceinline__ void b_zC(const StepArgs<R> &a, R *d0, R *d1, R *d2, 
 }
 template <typename R, int L, int MODE>
 __global__ void __launch_bounds__(MODE == 1 ? zjt<R, L>() : TPB) k_zC(StepArgs<R> a, R *d0, R *d1, R *d2) {
+    pdl_enter();
     b_zC<R, L, MODE>(a, d0, d1, d2, Blk{blockIdx.x, blockIdx.y, gridDim.x});
 }
 
@@ -384,6 +387,7 @@ __device__ __forceinline__ void b_zD(const StepArgs<R> &a, const R *d2, const Bl
 }
 template <typename R, int L, int MODE>
 __global__ void __launch_bounds__(MODE == 1 ? zjt<R, L>() : TPB) k_zD(StepArgs<R> a, const R *d2) {
+    pdl_enter();
     b_zD<R, L, MODE>(a, d2, Blk{blockIdx.x, blockIdx.y, gridDim.x});
 }
 
@@ -456,6 +460,7 @@ __device__ __forceinline__ void b_zE(const StepArgs<R> &a, const R *d0, const R 
 }
 template <typename R, int L, int MODE>
 __global__ void __launch_bounds__(MODE == 1 ? zjt<R, L>() : TPB) k_zE(StepArgs<R> a, const R *d0, const R *d1, const R *d2, int updp) {
+    pdl_enter();
     b_zE<R, L, MODE>(a, d0, d1, d2, updp, Blk{blockIdx.x, blockIdx.y, gridDim.x});
 }
 
@@ -476,6 +481,7 @@ struct WalkDiagZ {
 template <typename R, int L, int MODE>
 __global__ void __launch_bounds__(MODE == 1 ? zjt<double, L>() : TPB) k_diag_z(StepArgs<R> a, const double *divx,
                                                                                Cyc<double> c22) {
+    pdl_enter();
     const Geo g = a.g;
     ZCo c;
     unsigned long long m = 0;
@@ -509,28 +515,33 @@ static int launch_zpass_l(c3d_channel *ch, StepArgs<R> &a, int which, R *d0, R *
 // ---------------------------------------------------------------------------------
 template <typename R, int PART, int L, int MODE>
 __global__ void __launch_bounds__(MODE == 1 ? zjt<R, L>() : TPB) kb_zA(const StepArgs<R> *__restrict__ A, const BMap *__restrict__ map) {
+    pdl_enter();
     const BMap m = map[blockIdx.x];
     b_zA<R, L, PART, MODE>(A[m.ch], Blk{m.x, m.y, m.gx});
 }
 template <typename R, int L, int MODE>
 __global__ void __launch_bounds__(MODE == 1 ? zjt<R, L>() : TPB) kb_zB(const StepArgs<R> *__restrict__ A, const BMap *__restrict__ map) {
+    pdl_enter();
     const BMap m = map[blockIdx.x];
     b_zB<R, L, MODE, true>(A[m.ch], Blk{m.x, m.y, m.gx});
 }
 template <typename R, int L, int MODE>
 __global__ void __launch_bounds__(MODE == 1 ? zjt<R, L>() : TPB) kb_zC(const StepArgs<R> *__restrict__ A, const BMap *__restrict__ map) {
+    pdl_enter();
     const BMap m = map[blockIdx.x];
     const StepArgs<R> &a = A[m.ch];
     b_zC<R, L, MODE>(a, a.exz, a.eyz, a.wsq, Blk{m.x, m.y, m.gx});
 }
 template <typename R, int L, int MODE>
 __global__ void __launch_bounds__(MODE == 1 ? zjt<R, L>() : TPB) kb_zD(const StepArgs<R> *__restrict__ A, const BMap *__restrict__ map) {
+    pdl_enter();
     const BMap m = map[blockIdx.x];
     const StepArgs<R> &a = A[m.ch];
     b_zD<R, L, MODE>(a, a.wsq, Blk{m.x, m.y, m.gx});
 }
 template <typename R, int L, int MODE>
 __global__ void __launch_bounds__(MODE == 1 ? zjt<R, L>() : TPB) kb_zE(const StepArgs<R> *__restrict__ A, const BMap *__restrict__ map) {
+    pdl_enter();
     const BMap m = map[blockIdx.x];
     const StepArgs<R> &a = A[m.ch];
     b_zE<R, L, MODE>(a, a.exz, a.eyz, a.wsq, 1, Blk{m.x, m.y, m.gx});
@@ -598,13 +609,13 @@ static int launch_diag_z(c3d_channel *ch, StepArgs<R> &a, const double *divx, in
     const long long ncol = (long long)g.n2m * g.n1m;
     auto go = [&](auto *fn, int L, int cols) {
         const int nt = cols * (g.n3m / L);
-        fn<<<nblk(ncol, cols), nt, 2 * (size_t)nt * sizeof(double), ch->stream>>>(a, divx, c22);
+        klaunch(ch, ch->stream, fn, nblk(ncol, cols), nt, 2 * (size_t)nt * sizeof(double), a, divx, c22);
     };
     switch (zjoin_len<double>(g.n3m)) {
         case 8: go(k_diag_z<R, 8, 1>, 8, zjoin_cols<double, 8>(g.n3m, ncol)); break;
         case 12: go(k_diag_z<R, 12, 1>, 12, zjoin_cols<double, 12>(g.n3m, ncol)); break;
         case 16: go(k_diag_z<R, 16, 1>, 16, zjoin_cols<double, 16>(g.n3m, ncol)); break;
-        default: k_diag_z<R, ZL, 0><<<nblk(ncol * (g.n3m / ZL)), TPB, 0, ch->stream>>>(a, divx, c22);
+        default: klaunch(ch, ch->stream, k_diag_z<R, ZL, 0>, nblk(ncol * (g.n3m / ZL)), TPB, 0, a, divx, c22);
     }
     mark(ch, nl, "diag_z", (double)ncol * g.n3m * 16);
     return 0;
@@ -656,23 +667,23 @@ static int launch_zpass_l(c3d_channel *ch, StepArgs<R> &a, int which, R *d0, R *
                 const bool cc = par_on(ch);
                 int rc;
                 if (cc && (rc = par_fork(ch))) return rc;
-                k_zA<R, L, 1, MODE><<<nb, TB, zs2, cc ? ch->par[0] : st>>>(a);
+                klaunch(ch, cc ? ch->par[0] : st, k_zA<R, L, 1, MODE>, nb, TB, zs2, a);
                 mark(ch, nl, "zA_u", N * (8 + 4 * Rb));    // u; WW1, R1 -> R1, E_xz
-                k_zA<R, L, 2, MODE><<<nb, TB, zsm, cc ? ch->par[1] : st>>>(a);
+                klaunch(ch, cc ? ch->par[1] : st, k_zA<R, L, 2, MODE>, nb, TB, zsm, a);
                 mark(ch, nl, "zA_wp", N * (16 + 3 * Rb));  // w, P; R3 -> R3, WW3^2
-                k_zA<R, L, 3, MODE><<<nbv, TB, zs2, st>>>(a);
+                klaunch(ch, st, k_zA<R, L, 3, MODE>, nbv, TB, zs2, a);
                 mark(ch, nl, "zA_v", N * (16 + 3 * Rb));   // v, w; R2 -> R2, E_yz
                 if (cc && (rc = par_join(ch))) return rc;
             } else {
-                k_zA<R, L, 0, MODE><<<nb, TB, zsm, st>>>(a);
+                klaunch(ch, st, k_zA<R, L, 0, MODE>, nb, TB, zsm, a);
                 mark(ch, nl, "zA", N * (32 + 10 * Rb));
             }
             break;
-        case 1: k_zB<R, L, MODE><<<nb, TB, zsm, st>>>(a); mark(ch, nl, "zB", N * 8 * Rb); break;
-        case 2: k_zC<R, L, MODE><<<nb, TB, zsm, st>>>(a, d0, d1, d2); mark(ch, nl, "zC", N * 6 * Rb); break;
-        case 3: k_zD<R, L, MODE><<<nb, TB, zs1, st>>>(a, d2); mark(ch, nl, "zD", N * (8 + 2 * Rb)); break;
+        case 1: klaunch(ch, st, k_zB<R, L, MODE>, nb, TB, zsm, a); mark(ch, nl, "zB", N * 8 * Rb); break;
+        case 2: klaunch(ch, st, k_zC<R, L, MODE>, nb, TB, zsm, a, d0, d1, d2); mark(ch, nl, "zC", N * 6 * Rb); break;
+        case 3: klaunch(ch, st, k_zD<R, L, MODE>, nb, TB, zs1, a, d2); mark(ch, nl, "zD", N * (8 + 2 * Rb)); break;
         case 4:   // the mixed form reads delta1 - DT dDP/dx from one field (xD), FP64 both
-            k_zE<R, L, MODE><<<nb, TB, zs1, st>>>(a, d0, d1, d2, flag);
+            klaunch(ch, st, k_zE<R, L, MODE>, nb, TB, zs1, a, d0, d1, d2, flag);
             mark(ch, nl, "zE", N * (64 + (sizeof(R) == 4 ? 4 : 5) * Rb));
             break;
         default: return C3D_EINVAL;
