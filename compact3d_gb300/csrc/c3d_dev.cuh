@@ -217,6 +217,31 @@ __device__ __forceinline__ void xsolve_full(R (&x)[C], int lane, const Cyc<R> &c
 // |x| < 2^-56 by its exponent (an integer test: FP64 instructions are what bounds the FP64 form).
 __device__ __forceinline__ bool negligible(double x) { return (__double2hiint(x) & 0x7ff00000) < (1023 - 56) << 20; }
 
+// Decaying roots r of 1 + OP r + r^2 for the compact operators (1, OP, 1), known at compile
+// time, so that the FP64 solves' powers of r are constants.  OP = 0: the root is the caller's
+// (the Crank-Nicolson factors').
+template <int OP> struct Root { static constexpr double r = 0.0; };
+template <> struct Root<6> { static constexpr double r = -0.171572875253809902396622551580603842860; };    // -3 + sqrt(8)
+template <> struct Root<10> { static constexpr double r = -0.101020514433643803605431850588217216068; };   // -5 + sqrt(24)
+template <> struct Root<22> { static constexpr double r = -0.04554884989667773086060434398395732094; };    // -11 + sqrt(120)
+__host__ __device__ constexpr double cpow(double x, int n) {
+    double p = 1.0;
+    for (int i = 0; i < n; ++i) p *= x;
+    return p;
+}
+__host__ __device__ constexpr bool cnegligible(double x) { return (x < 0 ? -x : x) < 1.0 / 72057594037927936.0; }   // 2^-56
+// Points after which r^n is negligible, at most C.
+template <int OP, int C>
+__host__ __device__ constexpr int croot_len() {
+    if (OP == 0) return C;
+    int n = 1;
+    while (n < C && !cnegligible(cpow(Root<OP>::r, n))) ++n;
+    return n;
+}
+// The root of a z solve's operator: the constant in FP64, the argument in FP32.
+template <int OP> __device__ __forceinline__ double zroot(double) { return Root<OP>::r; }
+template <int OP> __device__ __forceinline__ float zroot(float r) { return r; }
+
 // What enters each lane's chunk in the FP64 recurrences of one direction: e = the chunk's own
 // sum, m = r^C.  The sums of the lanes before it (DIR -1) or after it (DIR +1) are added over
 // a ring of P lanes by doubling, each level covering twice the lanes, and the levels stop
@@ -238,27 +263,48 @@ __device__ __forceinline__ double ring_carry(double e, double m, int lane, int P
     return shfl_idx(e, DIR < 0 ? (lane == 0 ? P - 1 : lane - 1) : (lane + 1 >= P ? 0 : lane + 1), W);
 }
 
+// The same with a compile-time root: the levels and their factors are constants.
+template <int W, int DIR, int OP, int C, int B = 0>
+__device__ __forceinline__ double ring_carry_op(double e, int lane, int P, int off = 1) {
+    constexpr double m = cpow(Root<OP>::r, C << B);
+    if constexpr (!cnegligible(m) && B < 6) {
+        int src = DIR < 0 ? lane - off : lane + off;
+        if (DIR < 0 && src < 0) src += P;
+        if (DIR > 0 && src >= P) src -= P;
+        e = e + m * shfl_idx(e, src, W);
+        off *= 2;
+        if (off >= P) off -= P;
+        return ring_carry_op<W, DIR, OP, C, B + 1>(e, lane, P, off);
+    } else {
+        return shfl_idx(e, DIR < 0 ? (lane == 0 ? P - 1 : lane - 1) : (lane + 1 >= P ? 0 : lane + 1), W);
+    }
+}
+
 // FP64 solve on lane chunks without the scale s (B(F(d)); callers fold s into their
 // constants): two sweeps of C multiply-adds each way and the ring carries.  Against scans
 // over all lanes with per-lane multipliers and a closure it executes about half the FP64
 // instructions, and the FP64 pipe bounds the FP64 x passes (192 x 128 x 144 points: xA's
 // pieces 409, 312, 222 -> 264, 240, 152 us, xB 529 -> 353, xC 337 -> 303, xD 279 -> 244).
-template <int W, int C>
+// With a compile-time root a chunk's sum takes only its last points that reach the next chunk.
+template <int W, int OP, int C>
 __device__ __forceinline__ void xsolve_ring(double (&x)[C], int lane, int P, const Cyc<double> &c) {
-    const double r = c.r, m = rpow<C>(r);
-    double y = x[0];
+    constexpr int T = croot_len<OP, C>();
+    const double r = OP ? Root<OP>::r : c.r, m = OP ? 0.0 : rpow<C>(r);
+    double y = x[C - T];
 #pragma unroll
-    for (int t = 1; t < C; ++t) y = x[t] + r * y;
-    y = ring_carry<W, -1>(y, m, lane, P);
+    for (int t = C - T + 1; t < C; ++t) y = x[t] + r * y;
+    if constexpr (OP != 0) y = ring_carry_op<W, -1, OP, C>(y, lane, P);
+    else y = ring_carry<W, -1>(y, m, lane, P);
 #pragma unroll
     for (int t = 0; t < C; ++t) {
         y = x[t] + r * y;
         x[t] = y;
     }
-    double z = x[C - 1];
+    double z = x[T - 1];
 #pragma unroll
-    for (int t = C - 2; t >= 0; --t) z = x[t] + r * z;
-    z = ring_carry<W, +1>(z, m, lane, P);
+    for (int t = T - 2; t >= 0; --t) z = x[t] + r * z;
+    if constexpr (OP != 0) z = ring_carry_op<W, +1, OP, C>(z, lane, P);
+    else z = ring_carry<W, +1>(z, m, lane, P);
 #pragma unroll
     for (int t = C - 1; t >= 0; --t) {
         z = x[t] + r * z;
@@ -334,11 +380,11 @@ __device__ __forceinline__ void xsolve_general(R (&x)[C], int lane, int P, const
 // every segment of the warp calling together); in place, returns s*B(F(x)).  FP64 takes the
 // ring form; otherwise P = W takes the constant-multiplier form above and P < W (idle lanes)
 // the general one.
-template <int W = 32, typename R, int C>
+template <int W = 32, int OP = 0, typename R, int C>
 __device__ __forceinline__ void xsolve(R (&x)[C], int lane, int P, const Cyc<R> &c) {
     static_assert(W == 4 || W == 8 || W == 16 || W == 32, "row segments of 4, 8, 16 or 32 lanes");
     if constexpr (std::is_same<R, double>::value) {
-        xsolve_ring<W>(x, lane, P, c);
+        xsolve_ring<W, OP>(x, lane, P, c);
 #pragma unroll
         for (int t = 0; t < C; ++t) x[t] *= c.s;
         return;
@@ -351,9 +397,9 @@ __device__ __forceinline__ void xsolve(R (&x)[C], int lane, int P, const Cyc<R> 
 
 // The same with the FP64 scale left to the caller: xfold(f, c) is the factor f of a
 // right-hand side with the operator's scale folded in (FP64) or f itself.
-template <int W = 32, typename R, int C>
+template <int W = 32, int OP = 0, typename R, int C>
 __device__ __forceinline__ void xsolve_f(R (&x)[C], int lane, int P, const Cyc<R> &c) {
-    if constexpr (std::is_same<R, double>::value) xsolve_ring<W>(x, lane, P, c);
+    if constexpr (std::is_same<R, double>::value) xsolve_ring<W, OP>(x, lane, P, c);
     else xsolve<W>(x, lane, P, c);
 }
 __device__ __forceinline__ double xfold(double f, const Cyc<double> &c) { return f * c.s; }

@@ -58,6 +58,7 @@ struct StepArgs {
     double *scal;                       // device scalars (see SCAL_*)
     double *part;                       // per-row partial sums for the bulk-flow forcing
     Cyc<R> c6x, c10x, c22x, c6z, c10z, c22z, cnx, cnz;
+    R kx[2], kz[2];                     // FP64: the CN factors as partial fractions (cn_factors)
     const double *ycn;                  // CN wall-normal factors: 3 comps x (A, RBET, GAM) x (n2+1)
     const double *prb, *pgam;           // Poisson factor tables [j][mode], FP64
     const float2 *prbdf, *pgamdf;       // the same as double-float pairs (mixed form)

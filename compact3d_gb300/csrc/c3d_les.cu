@@ -1183,7 +1183,7 @@ __global__ void __launch_bounds__(TPB) k_les_x1(StepArgs<R> a, LesArgs<R> l) {
             R pv = sprev(nv[C - 1], lane, P);
 #pragma unroll
             for (int t = 0; t < C; ++t) d[t] = four * (nv[t] + (t == 0 ? pv : nv[t - 1]));
-            xsolve(d, lane, P, a.c6x);
+            xsolve<32, 6>(d, lane, P, a.c6x);
             srow_store(l.nux + o, d, sbR, lane, P);
         }
         {
@@ -1192,14 +1192,14 @@ __global__ void __launch_bounds__(TPB) k_les_x1(StepArgs<R> a, LesArgs<R> l) {
             S nx = snext(uc[0], lane, P);
 #pragma unroll
             for (int t = 0; t < C; ++t) d[t] = f24 * ST::d(t == C - 1 ? nx : uc[t + 1], uc[t]);
-            xsolve(d, lane, P, a.c22x);
+            xsolve<32, 22>(d, lane, P, a.c22x);
 #pragma unroll
             for (int t = 0; t < C; ++t) d[t] = nv[t] * d[t];
             R pv = sprev(d[C - 1], lane, P);
             R e[C];
 #pragma unroll
             for (int t = 0; t < C; ++t) e[t] = f24 * (d[t] - (t == 0 ? pv : d[t - 1]));
-            xsolve(e, lane, P, a.c22x);
+            xsolve<32, 22>(e, lane, P, a.c22x);
             R h[C];
             srow_load(h, a.hh[0] + o, sbR, lane, P);
 #pragma unroll
@@ -1212,7 +1212,7 @@ __global__ void __launch_bounds__(TPB) k_les_x1(StepArgs<R> a, LesArgs<R> l) {
             S pv = sprev(vc[C - 1], lane, P);
 #pragma unroll
             for (int t = 0; t < C; ++t) d[t] = f24 * ST::d(vc[t], t == 0 ? pv : vc[t - 1]);
-            xsolve(d, lane, P, a.c22x);
+            xsolve<32, 22>(d, lane, P, a.c22x);
             srow_store(l.dvdx + o, d, sbR, lane, P);
         }
         {
@@ -1221,7 +1221,7 @@ __global__ void __launch_bounds__(TPB) k_les_x1(StepArgs<R> a, LesArgs<R> l) {
             S pv = sprev(wc[C - 1], lane, P);
 #pragma unroll
             for (int t = 0; t < C; ++t) d[t] = f24 * ST::d(wc[t], t == 0 ? pv : wc[t - 1]);
-            xsolve(d, lane, P, a.c22x);
+            xsolve<32, 22>(d, lane, P, a.c22x);
             srow_store(l.dwdx + o, d, sbR, lane, P);
         }
     }
@@ -1269,7 +1269,7 @@ __global__ void __launch_bounds__(MODE == 1 ? zjt<R, L>() : TPB) k_les_z1(StepAr
     const int n = g.n3m, s = g.n1m, j = c.j, k0 = c.k0;
     const long long o = fidx(g, c.i, j, 0);
     R out[5][L];
-    const R rr[5] = {a.c6z.r, a.c6z.r, a.c22z.r, a.c22z.r, a.c22z.r};
+    const R r6 = zroot<6>(a.c6z.r), r22 = zroot<22>(a.c22z.r), rr[5] = {r6, r6, r22, r22, r22};
     const R ss[5] = {a.c6z.s, a.c6z.s, a.c22z.s, a.c22z.s, a.c22z.s};
     WalkLesZ1<R> f{l.nu + o, l.nux + o, a.u + o, a.v + o, a.w + o, n, s, zrhs<MODE>((R)4.0), zrhs<MODE>(a.f24z), j >= 2};
     zsolve<R, L, WM<R>::M6, 5, MODE>(out, c, n, rr, ss, f);
@@ -1331,7 +1331,7 @@ __global__ void __launch_bounds__(MODE == 1 ? zjt<R, L>() : TPB) k_les_z2(StepAr
     const long long o = fidx(g, i, j, 0), om = fidx(g, i, j - 1, 0), op = fidx(g, i, j + 1, 0);
     const bool hv = j >= 2;
     R out[3][L];
-    const R rr[3] = {a.c22z.r, a.c22z.r, a.c22z.r}, ss[3] = {a.c22z.s, a.c22z.s, a.c22z.s};
+    const R r22 = zroot<22>(a.c22z.r), rr[3] = {r22, r22, r22}, ss[3] = {a.c22z.s, a.c22z.s, a.c22z.s};
     WalkLesZ2<R> f{l.t13 + o, l.nuwz + o, l.nuz + o, l.nuz + om, l.dvdz + o, a.w + o, a.w + om,
                    n, s, zrhs<MODE>(a.f24z), a.m.rh[j], a.m.hdy[j], a.m.hdy[j - 1], hv};
     zsolve<R, L, WM<R>::M22, 3, MODE>(out, c, n, rr, ss, f);
@@ -1405,7 +1405,7 @@ __global__ void __launch_bounds__(TPB) k_les_x2(StepArgs<R> a, LesArgs<R> l) {
             R nx = snext(tc[0], lane, P);
 #pragma unroll
             for (int t = 0; t < C; ++t) d[t] = f24 * ((t == C - 1 ? nx : tc[t + 1]) - tc[t]);
-            xsolve(d, lane, P, a.c22x);
+            xsolve<32, 22>(d, lane, P, a.c22x);
             R h[C];
             srow_load(h, a.hh[2] + o, sbR, lane, P);
 #pragma unroll
@@ -1432,7 +1432,7 @@ __global__ void __launch_bounds__(TPB) k_les_x2(StepArgs<R> a, LesArgs<R> l) {
             R nx = snext(tau[0], lane, P);
 #pragma unroll
             for (int t = 0; t < C; ++t) d[t] = f24 * ((t == C - 1 ? nx : tau[t + 1]) - tau[t]);
-            xsolve(d, lane, P, a.c22x);
+            xsolve<32, 22>(d, lane, P, a.c22x);
             S vc[C], vm[C], vp[C];
             srow_load(vc, a.v + o, sbS, lane, P);
             srow_load(vm, a.v + om, sbS, lane, P);

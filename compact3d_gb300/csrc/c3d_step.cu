@@ -18,7 +18,7 @@
 #include <string.h>
 #include <type_traits>
 #include <vector>
-#include "c3d_kern.cuh"
+#include "c3d_zcols.cuh"
 
 namespace c3d {
 
@@ -467,6 +467,22 @@ struct FromDF { __device__ double operator()(float2 x) const { return St<float>:
 // ---------------------------------------------------------------------------------
 // Host-side drivers
 // ---------------------------------------------------------------------------------
+// FP64: the Crank-Nicolson factors (1,10,1)/(A,B,A) of x and z as (1 + k z/(1 + (B/A) z + z^2))/A
+// with k = 10 - B/A, which takes one multiply-add a point in place of the right-hand side's
+// stencil: kx[0] = 1/(A_x A_z) goes into xB's DT, kx[1] and kz[1] = k times the solve's scale.
+// k is about -144 q DX^2 with q = DT/(2 RE), some 1e-3 in a channel's step; past 1/2 (the two
+// terms would cancel to a digit) and on lines that zC does not join, kx[0] = kz[0] = 0 and both
+// passes take the stencil.
+static void cn_factors(StepArgs<double> &a, int n3m, double api, double aci, double apk, double ack) {
+    const double kx = -a.cnx.r * (10.0 - aci / api), kz = -a.cnz.r * (10.0 - ack / apk);
+    if (!(api > 0.5 && apk > 0.5 && fabs(kx) <= 0.5 && fabs(kz) <= 0.5) || !zjoin_len<double>(n3m)) return;
+    a.kx[0] = 1.0 / (api * apk);
+    a.kz[0] = 1.0;
+    a.kx[1] = kx;
+    a.kz[1] = kz;
+}
+static void cn_factors(StepArgs<float> &, int, double, double, double, double) {}
+
 template <typename R>
 static StepArgs<R> make_args(c3d_channel *ch, double dt) {
     typedef typename SType<R>::S S;
@@ -526,6 +542,7 @@ static StepArgs<R> make_args(c3d_channel *ch, double dt) {
     const double ack = 10.0 - dt / 2.0 * (1. / RE) * 12.0 * ch->g.dx3q * (-2.0);
     a.cnx = mk(api, aci, f32);
     a.cnz = mk(apk, ack, f32);
+    cn_factors(a, ch->g.n3m, api, aci, apk, ack);
     return a;
 }
 

@@ -59,15 +59,20 @@ __device__ __forceinline__ void xrow(T (&v)[C], const T *p, T *sb, int lane, int
     else srow_load(v, p, sb, lane, P);
 }
 
-// One row (j, k) of the u (PART 1), v (PART 2, faces J >= 2) or w (PART 3) piece of xA.
+}  // namespace c3d
+#include "c3d_x64.cuh"
+namespace c3d {
+
+// One row (j, k) of the u (PART 1), v (PART 2, faces J >= 2) or w (PART 3) piece of xA in
+// the mixed form.
 template <typename R, int C, int PART, bool STG, int W = 32>
-__device__ __forceinline__ void xa_piece(const StepArgs<R> &a, int j, long long o, long long om, long long op,
+__device__ __forceinline__ void xa_piece32(const StepArgs<R> &a, int j, long long o, long long om, long long op,
                                          const typename SType<R>::S *st, typename SType<R>::S *sbS, R *sbR, int lane,
                                          int P) {
     typedef typename SType<R>::S S;
     typedef St<R> ST;
     const int n = a.g.n1m;
-    const R RE1 = a.re1, f12 = xfold(a.f12x, a.c10x), f24 = xfold(a.f24x, a.c22x), four = xfold((R)4.0, a.c6x);
+    const R RE1 = a.re1, f12 = a.f12x, f24 = a.f24x, four = (R)4.0;
     const R presg = (R)a.scal[SCAL_PRESG];
     if (PART == 2 && j >= 2) {
         // The v piece on its own, ordered so that few rows are live at once: the y
@@ -108,7 +113,7 @@ __device__ __forceinline__ void xa_piece(const StepArgs<R> &a, int j, long long 
             S l = (t == 0) ? pv : vc[t - 1], rr = (t == C - 1) ? nx : vc[t + 1];
             d[t] = f12 * ST::d2(l, vc[t], rr);
         }
-        xsolve_f<W>(d, lane, P, a.c10x);
+        xsolve_f<W, 10>(d, lane, P, a.c10x);
 #pragma unroll
         for (int t = 0; t < C; ++t) acc[t] = acc[t] + RE1 * d[t];
         srow_store(a.r[1] + o, acc, sbR, lane, P);
@@ -117,7 +122,7 @@ __device__ __forceinline__ void xa_piece(const StepArgs<R> &a, int j, long long 
             S l = (t == 0) ? pv : vc[t - 1];
             d[t] = four * (ST::hi(l) + ST::hi(vc[t]));
         }
-        xsolve_f<W>(d, lane, P, a.c6x);
+        xsolve_f<W, 6>(d, lane, P, a.c6x);
         {   // u at the y faces
             S uc[C], um[C];
             xrow<STG>(uc, xa_src<STG, PART>(a, XA_UC, o, om, op, st, n), sbS, lane, P);
@@ -150,7 +155,7 @@ __device__ __forceinline__ void xa_piece(const StepArgs<R> &a, int j, long long 
             S l = (t == 0) ? pv : uc[t - 1], rr = (t == C - 1) ? nx : uc[t + 1];
             d[t] = f12 * ST::d2(l, uc[t], rr);
         }
-        xsolve_f<W>(d, lane, P, a.c10x);
+        xsolve_f<W, 10>(d, lane, P, a.c10x);
 #pragma unroll
         for (int t = 0; t < C; ++t) acc[t] = acc[t] + RE1 * d[t];
 #pragma unroll
@@ -158,7 +163,7 @@ __device__ __forceinline__ void xa_piece(const StepArgs<R> &a, int j, long long 
             S rr = (t == C - 1) ? nx : uc[t + 1];
             d[t] = four * (ST::hi(uc[t]) + ST::hi(rr));
         }
-        xsolve_f<W>(d, lane, P, a.c6x);
+        xsolve_f<W, 6>(d, lane, P, a.c6x);
         R sq[C];
 #pragma unroll
         for (int t = 0; t < C; ++t) sq[t] = d[t] * d[t];
@@ -168,7 +173,7 @@ __device__ __forceinline__ void xa_piece(const StepArgs<R> &a, int j, long long 
             R l = (t == 0) ? ps : sq[t - 1];
             d[t] = f24 * (sq[t] - l);
         }
-        xsolve_f<W>(d, lane, P, a.c22x);
+        xsolve_f<W, 22>(d, lane, P, a.c22x);
         srow_store(a.hh[0] + o, d, sbR, lane, P);
         {
             S pc[C];
@@ -180,7 +185,7 @@ __device__ __forceinline__ void xa_piece(const StepArgs<R> &a, int j, long long 
                 d[t] = f24 * ST::d(pc[t], l);
             }
         }
-        xsolve_f<W>(d, lane, P, a.c22x);
+        xsolve_f<W, 22>(d, lane, P, a.c22x);
 #pragma unroll
         for (int t = 0; t < C; ++t) acc[t] = acc[t] - d[t] - presg;
         srow_store(a.r[0] + o, acc, sbR, lane, P);
@@ -206,7 +211,7 @@ __device__ __forceinline__ void xa_piece(const StepArgs<R> &a, int j, long long 
             S l = (t == 0) ? pv : wc[t - 1], rr = (t == C - 1) ? nx : wc[t + 1];
             d[t] = f12 * ST::d2(l, wc[t], rr);
         }
-        xsolve_f<W>(d, lane, P, a.c10x);
+        xsolve_f<W, 10>(d, lane, P, a.c10x);
 #pragma unroll
         for (int t = 0; t < C; ++t) acc[t] = acc[t] + RE1 * d[t];
         srow_store(a.r[2] + o, acc, sbR, lane, P);
@@ -215,12 +220,20 @@ __device__ __forceinline__ void xa_piece(const StepArgs<R> &a, int j, long long 
             S l = (t == 0) ? pv : wc[t - 1];
             d[t] = four * (ST::hi(l) + ST::hi(wc[t]));
         }
-        xsolve_f<W>(d, lane, P, a.c6x);
+        xsolve_f<W, 6>(d, lane, P, a.c6x);
         srow_store(a.ww1 + o, d, sbR, lane, P);
     }
 }
 
-// PART 0 computes the u, v and w pieces in one kernel; PART 1, 2, 3 compute one of them
+template <typename R, int C, int PART, bool STG, int W = 32>
+__device__ __forceinline__ void xa_piece(const StepArgs<R> &a, int j, long long o, long long om, long long op,
+                                         const typename SType<R>::S *st, typename SType<R>::S *sbS, R *sbR, int lane,
+                                         int P) {
+    if constexpr (sizeof(R) == 8) xa64<C, PART, W>(a, j, o, om, op, sbR, lane, P);
+    else xa_piece32<R, C, PART, STG, W>(a, j, o, om, op, st, sbS, sbR, lane, P);
+}
+
+// PART 0 computes the u, v and w pieces in one kernel (FP64: one after another); PART 1, 2, 3 compute one of them
 // (the split form has fewer registers per thread; PART 2 reads the two u rows of the
 // y-face interpolant again).  A row is held by a segment of W lanes (W = 32: a warp); with
 // W < 32 the 32/W rows of a warp must share J (N3M a multiple of 32/W) so that the warp
@@ -237,7 +250,7 @@ __device__ __forceinline__ void b_xA(const StepArgs<R> &a, const Blk blk) {
     S *sbS = reinterpret_cast<S *>(smem_raw + wid * stage_bytes(g.n1m, C));
     R *sbR = reinterpret_cast<R *>(sbS);
     const int nrows = g.n2m * g.n3m;
-    const R RE1 = a.re1, f12 = xfold(a.f12x, a.c10x), f24 = xfold(a.f24x, a.c22x), four = xfold((R)4.0, a.c6x);
+    const R RE1 = a.re1, f12 = a.f12x, f24 = a.f24x, four = (R)4.0;
     const R presg = (R)a.scal[SCAL_PRESG];
     for (int row = blk.x * rpb + wid; row < nrows; row += blk.gx * rpb) {
         const int j = 1 + row / g.n3m, k = row % g.n3m;
@@ -255,9 +268,14 @@ __device__ __forceinline__ void b_xA(const StepArgs<R> &a, const Blk blk) {
         R uy[C];
         if (PART >= 1) {
             xa_piece<R, C, PART, false, W>(a, j, o, om, op, nullptr, sbS, sbR, lane, P);
+        } else if constexpr (sizeof(R) == 8) {
+            xa_piece<R, C, 1, false, W>(a, j, o, om, op, nullptr, sbS, sbR, lane, P);
+            xa_piece<R, C, 2, false, W>(a, j, o, om, op, nullptr, sbS, sbR, lane, P);
+            xa_piece<R, C, 3, false, W>(a, j, o, om, op, nullptr, sbS, sbR, lane, P);
+            continue;
         }
         // ---- u: R1 = visc_y + visc_x/RE - dP/dx - PRESG ; HH1 = d(uu)/dx ----
-        if (PART == 0) {
+        if (PART == 0 && sizeof(R) == 4) {
             S uc[C], um[C], up[C];
             srow_load(uc, a.u + o, sbS, lane, P);
             srow_load(um, a.u + om, sbS, lane, P);
@@ -270,7 +288,7 @@ __device__ __forceinline__ void b_xA(const StepArgs<R> &a, const Blk blk) {
                 S l = (t == 0) ? pv : uc[t - 1], rr = (t == C - 1) ? nx : uc[t + 1];
                 d[t] = f12 * ST::d2(l, uc[t], rr);
             }
-            xsolve_f<W>(d, lane, P, a.c10x);
+            xsolve_f<W, 10>(d, lane, P, a.c10x);
 #pragma unroll
             for (int t = 0; t < C; ++t) acc[t] = RE1 * ST::yvisc(HPj, HCj, HMj, Z0, up[t], uc[t], um[t]) + RE1 * d[t];
             {
@@ -282,7 +300,7 @@ __device__ __forceinline__ void b_xA(const StepArgs<R> &a, const Blk blk) {
                     S l = (t == 0) ? pp : pc[t - 1];
                     d[t] = f24 * ST::d(pc[t], l);
                 }
-                xsolve_f<W>(d, lane, P, a.c22x);
+                xsolve_f<W, 22>(d, lane, P, a.c22x);
 #pragma unroll
                 for (int t = 0; t < C; ++t) acc[t] = acc[t] - d[t] - presg;
                 srow_store(a.r[0] + o, acc, sbR, lane, P);
@@ -292,7 +310,7 @@ __device__ __forceinline__ void b_xA(const StepArgs<R> &a, const Blk blk) {
                 S rr = (t == C - 1) ? nx : uc[t + 1];
                 d[t] = four * (ST::hi(uc[t]) + ST::hi(rr));
             }
-            xsolve_f<W>(d, lane, P, a.c6x);
+            xsolve_f<W, 6>(d, lane, P, a.c6x);
             R sq[C];
 #pragma unroll
             for (int t = 0; t < C; ++t) sq[t] = d[t] * d[t];
@@ -302,7 +320,7 @@ __device__ __forceinline__ void b_xA(const StepArgs<R> &a, const Blk blk) {
                 R l = (t == 0) ? ps : sq[t - 1];
                 d[t] = f24 * (sq[t] - l);
             }
-            xsolve_f<W>(d, lane, P, a.c22x);
+            xsolve_f<W, 22>(d, lane, P, a.c22x);
             srow_store(a.hh[0] + o, d, sbR, lane, P);
             if (PART == 0 && j >= 2) {
                 const R Hj1 = a.m.rh[j], a1 = a.m.hdy[j], a2 = a.m.hdy[j - 1];
@@ -311,7 +329,7 @@ __device__ __forceinline__ void b_xA(const StepArgs<R> &a, const Blk blk) {
             }
         }
         // ---- v (faces J=2..N2M): R2, HH2 = d(vv)/dy, E_xy = VV1 * UY ----
-        if (PART == 0 && j >= 2) {
+        if (PART == 0 && sizeof(R) == 4 && j >= 2) {
             S vc[C], vm[C], vp[C];
             srow_load(vc, a.v + o, sbS, lane, P);
             srow_load(vm, a.v + om, sbS, lane, P);
@@ -323,7 +341,7 @@ __device__ __forceinline__ void b_xA(const StepArgs<R> &a, const Blk blk) {
                 S l = (t == 0) ? pv : vc[t - 1], rr = (t == C - 1) ? nx : vc[t + 1];
                 d[t] = f12 * ST::d2(l, vc[t], rr);
             }
-            xsolve_f<W>(d, lane, P, a.c10x);
+            xsolve_f<W, 10>(d, lane, P, a.c10x);
             const R DYPj = a.m.dyp[j], DYCj = a.m.dyc[j], DYMj = a.m.dym[j], Z0 = a.m.dyz[j];
             const R Hj = a.m.h[j], Hj1 = a.m.rh[j];
             {
@@ -345,13 +363,13 @@ __device__ __forceinline__ void b_xA(const StepArgs<R> &a, const Blk blk) {
                 S l = (t == 0) ? pv : vc[t - 1];
                 d[t] = four * (ST::hi(l) + ST::hi(vc[t]));
             }
-            xsolve_f<W>(d, lane, P, a.c6x);
+            xsolve_f<W, 6>(d, lane, P, a.c6x);
 #pragma unroll
             for (int t = 0; t < C; ++t) d[t] = d[t] * uy[t];
             srow_store(a.exy + o, d, sbR, lane, P);
         }
         // ---- w: R3 = visc_y + visc_x/RE ; WW1 = w at x faces ----
-        if (PART == 0) {
+        if (PART == 0 && sizeof(R) == 4) {
             S wc[C], wm[C], wp[C];
             srow_load(wc, a.w + o, sbS, lane, P);
             srow_load(wm, a.w + om, sbS, lane, P);
@@ -363,7 +381,7 @@ __device__ __forceinline__ void b_xA(const StepArgs<R> &a, const Blk blk) {
                 S l = (t == 0) ? pv : wc[t - 1], rr = (t == C - 1) ? nx : wc[t + 1];
                 d[t] = f12 * ST::d2(l, wc[t], rr);
             }
-            xsolve_f<W>(d, lane, P, a.c10x);
+            xsolve_f<W, 10>(d, lane, P, a.c10x);
             const R HPj = a.m.hp[j], HCj = a.m.hc[j], HMj = a.m.hm[j], Z0 = a.m.hz[j];
 #pragma unroll
             for (int t = 0; t < C; ++t) acc[t] = RE1 * ST::yvisc(HPj, HCj, HMj, Z0, wp[t], wc[t], wm[t]) + RE1 * d[t];
@@ -373,7 +391,7 @@ __device__ __forceinline__ void b_xA(const StepArgs<R> &a, const Blk blk) {
                 S l = (t == 0) ? pv : wc[t - 1];
                 d[t] = four * (ST::hi(l) + ST::hi(wc[t]));
             }
-            xsolve_f<W>(d, lane, P, a.c6x);
+            xsolve_f<W, 6>(d, lane, P, a.c6x);
             srow_store(a.ww1 + o, d, sbR, lane, P);
         }
     }
@@ -458,19 +476,31 @@ __global__ void __launch_bounds__(XMAXT) k_xAs(StepArgs<R> a) {
 template <typename R, int C, int W = 32>
 __device__ __forceinline__ void ab2_cnx(const StepArgs<R> &a, int c, long long o, const R (&hc)[C], R *sb,
                                         int lane, int P, R dt) {
-    const R dts = xfold(dt, a.cnx);
+    // FP64: (1,10,1)/(A,B,A) = (1 + (10 - B/A) z / (1 + B/A z + z^2)) / A with the factors kx,
+    // unless B/A is so far from 10 that the two terms would cancel (cn_factors)
+    const bool pf = sizeof(R) == 8 && a.kx[0] != R(0);
+    const R dts = pf ? dt * a.kx[0] : xfold(dt, a.cnx);
     R rr[C], ho[C], d[C];
     srow_load(rr, a.r[c] + o, sb, lane, P);
     srow_load(ho, a.ho[c] + o, sb, lane, P);
 #pragma unroll
     for (int t = 0; t < C; ++t) rr[t] = (rr[t] - (R)1.5 * hc[t] + (R)0.5 * ho[t]) * dts;
-    R pv = sprev<W>(rr[C - 1], lane, P), nx = snext<W>(rr[0], lane, P);
+    if (pf) {
 #pragma unroll
-    for (int t = 0; t < C; ++t) {
-        R l = (t == 0) ? pv : rr[t - 1], r2 = (t == C - 1) ? nx : rr[t + 1];
-        d[t] = (l + (R)10.0 * rr[t]) + r2;
+        for (int t = 0; t < C; ++t) d[t] = rr[t];
+    } else {
+        R pv = sprev<W>(rr[C - 1], lane, P), nx = snext<W>(rr[0], lane, P);
+#pragma unroll
+        for (int t = 0; t < C; ++t) {
+            R l = (t == 0) ? pv : rr[t - 1], r2 = (t == C - 1) ? nx : rr[t + 1];
+            d[t] = (l + (R)10.0 * rr[t]) + r2;
+        }
     }
     xsolve_f<W>(d, lane, P, a.cnx);
+    if (pf) {
+#pragma unroll
+        for (int t = 0; t < C; ++t) d[t] = rr[t] + a.kx[1] * d[t];
+    }
     srow_store(a.r[c] + o, d, sb, lane, P);
 }
 
@@ -483,7 +513,8 @@ __device__ __forceinline__ void b_xB(const StepArgs<R> &a, const Blk blk) {
     const int P = g.n1m / C;
     R *sb = reinterpret_cast<R *>(smem_raw + wid * stage_bytes(g.n1m, C));
     const int nrows = g.n2m * g.n3m;
-    const R f = xfold(a.f24x, a.c22x);
+    // FP64: plain differences into the solves, their factor in the sum after them
+    const R f = sizeof(R) == 8 ? R(1) : a.f24x, fo = sizeof(R) == 8 ? xfold(a.f24x, a.c22x) : R(1);
     const R dt = (R)a.dt;
     for (int row = blk.x * rpb + wid; row < nrows; row += blk.gx * rpb) {
         const int j = 1 + row / g.n3m, k = row % g.n3m;
@@ -523,9 +554,9 @@ __device__ __forceinline__ void b_xB(const StepArgs<R> &a, const Blk blk) {
                 R rr = (t == C - 1) ? nx : e[t + 1];
                 d[t] = f * (rr - e[t]);
             }
-            xsolve_f<W>(d, lane, P, a.c22x);
+            xsolve_f<W, 22>(d, lane, P, a.c22x);
 #pragma unroll
-            for (int t = 0; t < C; ++t) h2[t] = h2[t] + d[t];                 // d(uv)/dx
+            for (int t = 0; t < C; ++t) h2[t] = h2[t] + (sizeof(R) == 8 ? fo * d[t] : d[t]);                 // d(uv)/dx
             srow_store(a.hh[1] + o, h2, sb, lane, P);
             ab2_cnx<R, C, W>(a, 1, o, h2, sb, lane, P, dt);
         }
@@ -539,9 +570,9 @@ __device__ __forceinline__ void b_xB(const StepArgs<R> &a, const Blk blk) {
                 d[t] = f * (rr - e[t]);
             }
         }
-        xsolve_f<W>(d, lane, P, a.c22x);
+        xsolve_f<W, 22>(d, lane, P, a.c22x);
 #pragma unroll
-        for (int t = 0; t < C; ++t) h3[t] = h3[t] + d[t];
+        for (int t = 0; t < C; ++t) h3[t] = h3[t] + (sizeof(R) == 8 ? fo * d[t] : d[t]);
         if (j >= 2) srow_load(e, a.eyz + o, sb, lane, P);
         else {
 #pragma unroll
@@ -595,9 +626,19 @@ __device__ __forceinline__ void xc_row(const StepArgs<R> &a, int j, int k, const
     S *sbS = reinterpret_cast<S *>(sbuf);
     R *sbR = reinterpret_cast<R *>(sbuf);
     R *rbuf = reinterpret_cast<R *>(bufa);
-    const R rdt = a.rdt, f24 = xfold(a.f24x, a.c22x);
+    const R rdt = a.rdt, f24 = a.f24x;
     R d[C], base[C];
-    {
+    if constexpr (sizeof(R) == 8) {   // differences of u + delta; the factor enters below
+        R uc[C];
+        xrow<SH>(uc, u, sbS, lane, P);
+        xrow<SH>(d, d0, sbR, lane, P);
+#pragma unroll
+        for (int t = 0; t < C; ++t) uc[t] = uc[t] + d[t];
+        const R nu = snext<W>(uc[0], lane, P);
+#pragma unroll
+        for (int t = 0; t < C; ++t) d[t] = (t == C - 1 ? nu : uc[t + 1]) - uc[t];
+        xsolve_ring<W, 22>(d, lane, P, a.c22x);
+    } else {
         S uc[C];
         R dd[C];
         xrow<SH>(uc, u, sbS, lane, P);
@@ -610,7 +651,7 @@ __device__ __forceinline__ void xc_row(const StepArgs<R> &a, int j, int k, const
             R rd = (t == C - 1) ? nd : dd[t + 1];
             d[t] = f24 * Sten<R>::dd(ru, rd, uc[t], dd[t]);
         }
-        xsolve_f<W>(d, lane, P, a.c22x);
+        xsolve_f<W, 22>(d, lane, P, a.c22x);
     }
     {
         const bool up = (j + 1 <= g.n2m), lo = (j >= 2);
@@ -624,14 +665,15 @@ __device__ __forceinline__ void xc_row(const StepArgs<R> &a, int j, int k, const
         for (int t = 0; t < C; ++t) {
             // (FJUP*UH2(J+1) - FJUM*UH2(J))/DY(J), UH2 = V + delta2, UH2 = 0 on the walls
             R dv = Sten<R>::dd(up ? vpv[t] : zs, up ? dpv[t] : R(0), lo ? vcv[t] : zs, lo ? dcv[t] : R(0));
-            base[t] = dv * ry;
+            if constexpr (sizeof(R) == 8) d[t] = (rdt * xfold(f24, a.c22x)) * d[t] + dv * ry;
+            else base[t] = dv * ry;
         }
     }
     {
         R zc[C];
         xrow<SH>(zc, zr, sbR, lane, P);
 #pragma unroll
-        for (int t = 0; t < C; ++t) d[t] = (base[t] + d[t] * rdt) + zc[t];
+        for (int t = 0; t < C; ++t) d[t] = sizeof(R) == 8 ? d[t] + zc[t] : (base[t] + d[t] * rdt) + zc[t];
     }
     const C2 *twx;
     if constexpr (sizeof(R) == 8) twx = reinterpret_cast<const C2 *>(a.twx64);
@@ -771,7 +813,8 @@ __device__ __forceinline__ void b_xD(const StepArgs<R> &a, const R *d0, const R 
     const C2 *twx;
     if constexpr (sizeof(R) == 8) twx = reinterpret_cast<const C2 *>(a.twx64);
     else twx = reinterpret_cast<const C2 *>(a.twx32);
-    const R scale = a.xscale, f24 = xfold(a.f24x, a.c22x);
+    // FP64: g1 is the solve's sum without its factor, which zE's DT carries
+    const R scale = a.xscale, f24 = sizeof(R) == 8 ? R(1) : a.f24x;
     for (int row = blk.x * rpb + wid; row < nrows; row += blk.gx * rpb) {
         const int j = 1 + row / g.n3m, k = row % g.n3m;
         const long long o = fidx(g, 0, j, k);
@@ -817,7 +860,7 @@ __device__ __forceinline__ void b_xD(const StepArgs<R> &a, const R *d0, const R 
             R l = (t == 0) ? pv : dpv[t - 1];
             d[t] = f24 * (dpv[t] - l);
         }
-        xsolve_f<W>(d, lane, P, a.c22x);
+        xsolve_f<W, 22>(d, lane, P, a.c22x);
         // bulk-flow partial sums below: sum_i delta * DY(J)/DX3/DX1 for u and w
         R q1[C], q3[C];
         srow_load(q1, d0 + o, sbR, lane, P);
@@ -919,7 +962,7 @@ __global__ void __launch_bounds__(TPB) k_diag_x(StepArgs<R> a, double *divx, Cyc
         const double nx = snext(uc[0], lane, P);
 #pragma unroll
         for (int t = 0; t < C; ++t) d[t] = ((t == C - 1) ? nx : uc[t + 1]) - uc[t];
-        xsolve_f<32>(d, lane, P, c22);
+        xsolve_f<32, 22>(d, lane, P, c22);
         const double rdy = 1.0 / g.dy[j], h2 = 0.5 * rdy;
 #pragma unroll
         for (int t = 0; t < C; ++t) {

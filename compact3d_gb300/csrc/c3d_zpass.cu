@@ -112,6 +112,18 @@ struct WalkCN {
     }
 };
 
+// zC by partial fractions (FP64): x itself
+template <typename R>
+struct WalkX3 {
+    const R *X[3]; int n, s; int k;
+    __device__ void start(int k0) { k = k0; }
+    __device__ void next(R (&d)[3]) {
+#pragma unroll
+        for (int c = 0; c < 3; ++c) d[c] = X[c][k * s];
+        ++k;
+    }
+};
+
 // zD: f24*((W+ + D+) - (W + D))
 template <typename R>
 struct WalkDivZ {
@@ -180,11 +192,12 @@ __device__ __forceinline__ void b_zA(const StepArgs<R> &a, const Blk blk) {
     const R kv = RE1 * zfold<MODE>(a.f12z, a.c10z.s), ki = zfold<MODE>((R)4.0, a.c6z.s), kp = zfold<MODE>(a.f24z, a.c22z.s);
     if (PART == 0 || PART == 1) {   // u: R1 += (1/RE) d2u/dz2 ; E_xz = UU3 * WW1
         R out[2][L];
-        const R rr[2] = {a.c10z.r, a.c6z.r}, ss[2] = {a.c10z.s, a.c6z.s};
+        const R rr[2] = {zroot<10>(a.c10z.r), zroot<6>(a.c6z.r)}, ss[2] = {a.c10z.s, a.c6z.s};
         WalkVisBack<R> f{a.u + o, n, s, f12, four};
         zsolve<R, L, M6, 2, MODE, NH>(out, c, n, rr, ss, f);
         R *Rp = a.r[0] + o, *E = a.exz + o;
         const R *Wx = a.ww1 + o;
+        const R kw = ki * ((R)4.0 * a.c6x.s);   // FP64: WW1 comes without its factor
         if (c.act) {
 #pragma unroll
             for (int b = 0; b < L; b += B) {
@@ -195,17 +208,18 @@ __device__ __forceinline__ void b_zA(const StepArgs<R> &a, const Blk blk) {
                 for (int t = 0; t < B; ++t) {
                     const int kk = (k0 + b + t) * s;
                     Rp[kk] = rv[t] + kv * out[0][b + t];
-                    E[kk] = MODE == 1 ? out[1][b + t] * (ki * wv[t]) : out[1][b + t] * wv[t];
+                    E[kk] = sizeof(R) == 8 ? out[1][b + t] * (kw * wv[t])
+                            : MODE == 1    ? out[1][b + t] * (ki * wv[t]) : out[1][b + t] * wv[t];
                 }
             }
         }
     }
     if (PART == 0 || PART == 2) {   // w, P: R3 += (1/RE) d2w/dz2 - dP/dz - PRESG3 ; WW3^2
         R out[3][L];
-        const R rr[3] = {a.c10z.r, a.c6z.r, a.c22z.r}, ss[3] = {a.c10z.s, a.c6z.s, a.c22z.s};
+        const R rr[3] = {zroot<10>(a.c10z.r), zroot<6>(a.c6z.r), zroot<22>(a.c22z.r)}, ss[3] = {a.c10z.s, a.c6z.s, a.c22z.s};
         WalkWP<R> f{a.w + o, a.p + o, n, s, f12, four, f24};
         zsolve<R, L, M6, 3, MODE>(out, c, n, rr, ss, f);
-        const R presg3 = (R)a.scal[SCAL_PRESG3];
+        const R presg3 = sizeof(R) == 8 ? R(0) : (R)a.scal[SCAL_PRESG3];   // FP64: in xA's sum
         R *Rp = a.r[2] + o, *Q = a.wsq + o;
         if (c.act) {
 #pragma unroll
@@ -216,7 +230,8 @@ __device__ __forceinline__ void b_zA(const StepArgs<R> &a, const Blk blk) {
                 for (int t = 0; t < B; ++t) {
                     const int kk = (k0 + b + t) * s;
                     if constexpr (MODE == 1) {
-                        Rp[kk] = rv[t] + kv * out[0][b + t] - kp * out[2][b + t] - presg3;
+                        const R rn = rv[t] + kv * out[0][b + t] - kp * out[2][b + t];
+                        Rp[kk] = sizeof(R) == 8 ? rn : rn - presg3;
                         const R ww3 = ki * out[1][b + t];
                         Q[kk] = ww3 * ww3;
                     } else {
@@ -230,7 +245,7 @@ __device__ __forceinline__ void b_zA(const StepArgs<R> &a, const Blk blk) {
     if (PART == 0 || PART == 3) {   // v: R2 += (1/RE) d2v/dz2 ; E_yz = VV3 * (w at y face J)
         if (MODE == 0 && j < 2) return;
         R out[2][L];
-        const R rr[2] = {a.c10z.r, a.c6z.r}, ss[2] = {a.c10z.s, a.c6z.s};
+        const R rr[2] = {zroot<10>(a.c10z.r), zroot<6>(a.c6z.r)}, ss[2] = {a.c10z.s, a.c6z.s};
         WalkVisBack<R> f{a.v + o, n, s, f12, four};
         zsolve<R, L, M6, 2, MODE, NH>(out, c, n, rr, ss, f);
         const R Hj1 = a.m.rh[j], a1 = a.m.hdy[j], a2 = a.m.hdy[j - 1];
@@ -286,7 +301,7 @@ __device__ __forceinline__ void b_zB(const StepArgs<R> &a, const Blk blk) {
     }
     R out[3][L];
     const R sc = a.c22z.s, s1 = RND ? R(1) : sc;
-    const R rr[3] = {a.c22z.r, a.c22z.r, a.c22z.r}, ss[3] = {s1, s1, s1};
+    const R r22 = zroot<22>(a.c22z.r), rr[3] = {r22, r22, r22}, ss[3] = {s1, s1, s1};
     WalkZB<R> f{a.exz + o, a.wsq + o, a.eyz + o, n, s, zrhs<MODE>(a.f24z)};
     f.v = (j >= 2);
     zsolve<R, L, WM<R>::M22, 3, MODE>(out, c, n, rr, ss, f);
@@ -339,12 +354,36 @@ __device__ __forceinline__ void b_zC(const StepArgs<R> &a, R *d0, R *d1, R *d2, 
     }
     R out[3][L];
     const R rr[3] = {a.cnz.r, a.cnz.r, a.cnz.r}, ss[3] = {a.cnz.s, a.cnz.s, a.cnz.s};
+    R *D0 = d0 + o, *D1 = d1 + o, *D2 = d2 + o;
+    const R ks = zfold<MODE>(R(1), a.cnz.s);
+    if constexpr (sizeof(R) == 8 && MODE == 1) {
+        if (a.kz[0] != R(0)) {   // partial fractions, as in xB (which applied their common factor)
+            WalkX3<R> f{{a.r[0] + o, a.r[1] + o, a.r[2] + o}, n, s, 0};
+            zsolve<R, L, WM<R>::MCN, 3, MODE>(out, c, n, rr, ss, f);
+            if (!c.act) return;
+            constexpr int B = ztb<L>() / 2;
+            const R kz = a.kz[1];
+#pragma unroll
+            for (int b = 0; b < L; b += B) {
+                R x0[B], x1[B], x2[B];
+                zload(x0, f.X[0], k0 + b, s);
+                zload(x1, f.X[1], k0 + b, s);
+                zload(x2, f.X[2], k0 + b, s);
+#pragma unroll
+                for (int t = 0; t < B; ++t) {
+                    const int kk = (k0 + b + t) * s;
+                    D0[kk] = x0[t] + kz * out[0][b + t];
+                    D1[kk] = x1[t] + kz * out[1][b + t];
+                    D2[kk] = x2[t] + kz * out[2][b + t];
+                }
+            }
+            return;
+        }
+    }
     WalkCN<R> f;
     f.X[0] = a.r[0] + o; f.X[1] = a.r[1] + o; f.X[2] = a.r[2] + o;
     f.n = n; f.s = s;
     zsolve<R, L, WM<R>::MCN, 3, MODE>(out, c, n, rr, ss, f);
-    R *D0 = d0 + o, *D1 = d1 + o, *D2 = d2 + o;
-    const R ks = zfold<MODE>(R(1), a.cnz.s);
     if (!c.act) return;
 #pragma unroll
     for (int t = 0; t < L; ++t) {
@@ -376,7 +415,7 @@ __device__ __forceinline__ void b_zD(const StepArgs<R> &a, const R *d2, const Bl
         pf_cols(d2 + o0, sb * sizeof(R), 32 * (int)sizeof(R), k0, WM<R>::M22 + 1, L, n, lane);
     }
     R out[1][L];
-    const R rr[1] = {a.c22z.r}, ss[1] = {a.c22z.s};
+    const R rr[1] = {zroot<22>(a.c22z.r)}, ss[1] = {a.c22z.s};
     WalkDivZ<R> f{a.w + o, d2 + o, n, s, zrhs<MODE>(a.f24z)};
     zsolve<R, L, WM<R>::M22, 1, MODE>(out, c, n, rr, ss, f);
     const R rdt = a.rdt * zfold<MODE>(a.f24z, a.c22z.s);
@@ -419,13 +458,14 @@ __device__ __forceinline__ void b_zE(const StepArgs<R> &a, const R *d0, const R 
         pf_cols(a.g1 + o0, sb * sizeof(R), 32 * (int)sizeof(R), k0, 0, L, n, lane);
     }
     R out[1][L];
-    const R rr[1] = {a.c22z.r}, ss[1] = {a.c22z.s};
+    const R rr[1] = {zroot<22>(a.c22z.r)}, ss[1] = {a.c22z.s};
     WalkGradZ<R> f{DP, n, s, zrhs<MODE>(a.f24z)};
     zsolve<R, L, WM<R>::M22, 1, MODE>(out, c, n, rr, ss, f);
     S *W = a.w + o, *U = a.u + o, *V = a.v + o, *Pp = a.p + o;
     const R *D0 = d0 + o, *D1 = d1 + o, *D2 = d2 + o, *G1 = a.g1 + o;
     const R *DPm = a.dp + fidx(g, i, j - 1, 0);
     const R rHj = a.m.rh[j], dtg = dt * zfold<MODE>(a.f24z, a.c22z.s), dth = dt * rHj;
+    const R dtx = dt * xfold(a.f24x, a.c22x);   // FP64: g1 without its factor (xD)
     if (!c.act) return;
     constexpr int B = ztb<L>() / 2;   // nine fields are live
 #pragma unroll
@@ -449,7 +489,7 @@ __device__ __forceinline__ void b_zE(const StepArgs<R> &a, const R *d0, const R 
             const int kk = (k0 + b + t) * s;
             W[kk] = Sten<R>::upd(wv[t], d2v[t], dtg * out[0][b + t], dtdm3);
             if constexpr (sizeof(R) == 4) U[kk] = ST::add(uv[t], gv[t] - dtdm);   // G1: delta1 - DT dDP/dx (xD)
-            else U[kk] = Sten<R>::upd(uv[t], d0v[t], dt * gv[t], dtdm);
+            else U[kk] = Sten<R>::upd(uv[t], d0v[t], dtx * gv[t], dtdm);
             if (j >= 2) {
                 const R dpy = MODE == 1 ? dth * (pc[t] - pm[t]) : dt * (pc[t] - pm[t]) * rHj;
                 V[kk] = Sten<R>::upd(vv[t], d1v[t], dpy, R(0));
