@@ -89,24 +89,26 @@ static int launch_x_c(c3d_channel *ch, StepArgs<R> &a, int which, const R *p0, c
     const size_t fb = (stage_bytes(ch->g.n1m, C) + 2 * (size_t)(M + 1) * sizeof(C2)) * xw;
     switch (which) {
         case 0:
-            if (ch->tune.xsplit && ch->tune.xstage && ch->g.n1m % 2 == 0) {
-                // the pieces with their rows staged by bulk copies (rows of 16-byte multiples)
-                const size_t s1 = xa_stage_bytes(1, ch->g.n1m) * xw, s2 = xa_stage_bytes(2, ch->g.n1m) * xw,
-                             s3 = xa_stage_bytes(3, ch->g.n1m) * xw;
-                if (s2 > 227 * 1024) { set_error("xA stage exceeds shared memory"); return C3D_EINVAL; }
-                cudaFuncSetAttribute(k_xAs<R, C, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)s1);
-                cudaFuncSetAttribute(k_xAs<R, C, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)s2);
-                cudaFuncSetAttribute(k_xAs<R, C, 3>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)s3);
-                const bool cc = par_on(ch);   // the pieces as concurrent branches (knob 15)
-                if (cc && (rc = par_fork(ch))) return rc;
-                klaunch(ch, cc ? ch->par[0] : st, k_xAs<R, C, 1>, grid, nt, s1, a);
-                mark(ch, nl, "xA_u", N * (16 + 2 * Rb));
-                klaunch(ch, cc ? ch->par[1] : st, k_xAs<R, C, 2>, grid, nt, s2, a);
-                mark(ch, nl, "xA_v", N * (24 + 3 * Rb));
-                klaunch(ch, st, k_xAs<R, C, 3>, grid, nt, s3, a);
-                mark(ch, nl, "xA_w", N * (8 + 2 * Rb));
-                if (cc && (rc = par_join(ch))) return rc;
-                break;
+            // FP64 reads its rows from global memory in every schedule: its pipe is 84% busy, DRAM 7%
+            if constexpr (sizeof(R) == 4) {
+                if (ch->tune.xsplit && ch->tune.xstage && ch->g.n1m % 2 == 0) {
+                    // the pieces with their rows staged by bulk copies (rows of 16-byte multiples)
+                    const size_t s1 = xa_stage_bytes(1, ch->g.n1m) * xw, s2 = xa_stage_bytes(2, ch->g.n1m) * xw,
+                                 s3 = xa_stage_bytes(3, ch->g.n1m) * xw;
+                    cudaFuncSetAttribute(k_xAs<R, C, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)s1);
+                    cudaFuncSetAttribute(k_xAs<R, C, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)s2);
+                    cudaFuncSetAttribute(k_xAs<R, C, 3>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)s3);
+                    const bool cc = par_on(ch);   // the pieces as concurrent branches (knob 15)
+                    if (cc && (rc = par_fork(ch))) return rc;
+                    klaunch(ch, cc ? ch->par[0] : st, k_xAs<R, C, 1>, grid, nt, s1, a);
+                    mark(ch, nl, "xA_u", N * (16 + 2 * Rb));
+                    klaunch(ch, cc ? ch->par[1] : st, k_xAs<R, C, 2>, grid, nt, s2, a);
+                    mark(ch, nl, "xA_v", N * (24 + 3 * Rb));
+                    klaunch(ch, st, k_xAs<R, C, 3>, grid, nt, s3, a);
+                    mark(ch, nl, "xA_w", N * (8 + 2 * Rb));
+                    if (cc && (rc = par_join(ch))) return rc;
+                    break;
+                }
             }
             if (ch->tune.xsplit) {   // the u, v and w pieces as three kernels
                 cudaFuncSetAttribute(k_xA<R, C, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sb);
@@ -179,17 +181,22 @@ static int launch_x_c(c3d_channel *ch, StepArgs<R> &a, int which, const R *p0, c
 }
 
 
-// xA's pieces (unless staged), xB, and xC and xD (with the shared-memory row FFT and no
-// bulk-copy ring) with a row per segment of W lanes (schedule knob x_row_lanes).  Returns
-// 0 when launched, 1 when the schedule runs the pass on whole warps, or an error code.
+// xA (its pieces; FP64 in one kernel too) unless staged, xB, and xC and xD (with the
+// shared-memory row FFT and no bulk-copy ring) with a row per segment of W lanes (schedule
+// knob x_row_lanes; FP64 by N1M).  Returns 0 when launched, 1 when the schedule runs the pass
+// on whole warps, or an error code.
 template <typename R, int C, int W>
 static int launch_x_seg(c3d_channel *ch, StepArgs<R> &a, int which, const R *p0, const R *p1, int *nl) {
     typedef typename Cx<R>::T C2;
     const Tune &t = ch->tune;
-    if (which == 0 && (!t.xsplit || t.xstage)) return 1;
+    if (which == 0 && sizeof(R) == 4 && (!t.xsplit || t.xstage)) return 1;
     if ((which == 2 || which == 3) && (t.fxp == 3 || t.xbulk)) return 1;
-    const int nrows = ch->g.n2m * ch->g.n3m, rpb = t.xw * 32 / W;
-    const int grid = nblk(nrows, rpb), nt = t.xw * 32;
+    const int nrows = ch->g.n2m * ch->g.n3m;
+    // FP64: blocks of one warp while there are fewer than 16 warps per SM (152), so that the
+    // last wave is short (96 x 48 x 64 points, dynamic LES: 650 -> 640 us a step)
+    const int xw = sizeof(R) == 8 ? std::max(1, std::min(t.xw, (nrows / (32 / W)) / (152 * 8))) : t.xw;
+    const int rpb = xw * 32 / W;
+    const int grid = nblk(nrows, rpb), nt = xw * 32;
     const double N = (double)ch->g.n1m * ch->g.n2m * ch->g.n3m, Rb = sizeof(R);
     const size_t fb = (stage_bytes(ch->g.n1m, C) + 2 * (size_t)(ch->g.n1m / 2 + 1) * sizeof(C2)) * rpb;
     cudaStream_t st = ch->stream;
@@ -204,6 +211,13 @@ static int launch_x_seg(c3d_channel *ch, StepArgs<R> &a, int which, const R *p0,
         klaunch(ch, st, k_xD<R, C, false, W>, grid, nt, fb, a, p0, p1);
         mark(ch, nl, "xD", N * 5 * Rb);
         return 0;
+    }
+    if constexpr (sizeof(R) == 8) {
+        if (which == 0 && !t.xsplit) {
+            klaunch(ch, st, k_xA<R, C, 0, W>, grid, nt, 0, a);
+            mark(ch, nl, "xA", N * (32 + 7 * Rb));
+            return 0;
+        }
     }
     if (which == 0) {
         const bool cc = par_on(ch);   // the pieces as concurrent branches (knob 15)
@@ -225,7 +239,35 @@ static int launch_x_seg(c3d_channel *ch, StepArgs<R> &a, int which, const R *p0,
 
 template <typename R>
 int launch_xpass(c3d_channel *ch, StepArgs<R> &a, int which, const R *p0, const R *p1, int *nl) {
-    if (which >= 0 && which <= 3 && ch->tune.xlanes) {
+    const Tune &t = ch->tune;
+    if (which == 0 && t.xsplit && t.xstage && ch->g.n1m % 2 == 0 && xa_stage_bytes(2, ch->g.n1m) * t.xw > 227 * 1024) {
+        set_error("xA stage exceeds shared memory");
+        return C3D_EINVAL;
+    }
+    if constexpr (sizeof(R) == 8) {
+        // FP64, whatever the schedule's row lanes: segments that have no idle lanes and more
+        // points per lane than a warp would (the carries of a solve cost 2 instructions per
+        // level and lane whatever the chunk, and the FP64 pipe issues idle lanes too: the
+        // shared-memory row FFT of 64 points has 8 butterflies a stage).  Step times with a
+        // warp, 16 and 8 lanes a row: 32 x 24 x 48 points 144, 142, 150 us, 64^3 316, 271,
+        // 266, 96 x 48 x 64 LES 672, 640, 646, 128 x 96 x 128 1230, 1126, 1172,
+        // 192 x 128 x 144 2448, 2348, 2347; 256 x 96 x 128 with 16: 2069 against 2057.
+        int r = 1;
+        if (which >= 0 && which <= 3) switch (ch->g.n1m) {
+            case 16: r = launch_x_seg<R, 2, 8>(ch, a, which, p0, p1, nl); break;
+            case 24: r = launch_x_seg<R, 3, 8>(ch, a, which, p0, p1, nl); break;
+            case 32: r = launch_x_seg<R, 2, 16>(ch, a, which, p0, p1, nl); break;
+            case 48: r = launch_x_seg<R, 3, 16>(ch, a, which, p0, p1, nl); break;
+            case 64: r = launch_x_seg<R, 8, 8>(ch, a, which, p0, p1, nl); break;
+            case 72: r = launch_x_seg<R, 9, 8>(ch, a, which, p0, p1, nl); break;
+            case 96: r = launch_x_seg<R, 6, 16>(ch, a, which, p0, p1, nl); break;
+            case 128: r = launch_x_seg<R, 8, 16>(ch, a, which, p0, p1, nl); break;
+            case 192: r = launch_x_seg<R, 12, 16>(ch, a, which, p0, p1, nl); break;
+            default: break;
+        }
+        if (r <= 0) return r;
+    } else
+    if (which >= 0 && which <= 3 && t.xlanes) {
         int r = 1;
         switch (ch->g.n1m) {   // the shapes x_segment_lanes accepts
             case 48: r = launch_x_seg<R, 6, 8>(ch, a, which, p0, p1, nl); break;

@@ -395,7 +395,8 @@ int c3d_checkpoint_read(c3d_channel *ch, const char *path, int *ntime, double *t
  *       mixed form, N1M a multiple of 4)
  *   [12] the u, v and w pieces of the explicit x pass (with [10] = 1) read their rows
  *       from global memory (0), or stage every row of a warp's (J, K) in shared memory
- *       by one bulk copy per row before computing (1; N1M even)
+ *       by one bulk copy per row before computing (1; N1M even; FP64 reads them from
+ *       global memory either way)
  *   [13] the wall-normal Crank-Nicolson factor (TDMAI): one thread per column with
  *       register batches of planes (0), or blocks of 32 or 64 columns whose planes
  *       are staged in shared memory by bulk copies so that each value is read and
@@ -407,6 +408,7 @@ int c3d_checkpoint_read(c3d_channel *ch, const char *path, int *ntime, double *t
  *       96 (8 lanes) or 128 (16 lanes) with N3M a multiple of 32 / lanes, so that each
  *       lane holds 6 to 12 points and the cross-lane scans of the line solves take 3
  *       or 4 steps instead of 5
+ *       (FP64 takes its segment by N1M, whatever this is)
  *   [15] the u, v and w pieces of the explicit x pass ([10] = 1), then those of the
  *       explicit z pass ([9] = 1), as three concurrent branches on three streams (1)
  *       or one after another (0); they write disjoint fields.  The per-kernel profile
