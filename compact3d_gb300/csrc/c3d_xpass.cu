@@ -93,18 +93,17 @@ static int launch_x_c(c3d_channel *ch, StepArgs<R> &a, int which, const R *p0, c
             if constexpr (sizeof(R) == 4) {
                 if (ch->tune.xsplit && ch->tune.xstage && ch->g.n1m % 2 == 0) {
                     // the pieces with their rows staged by bulk copies (rows of 16-byte multiples)
-                    const size_t s1 = xa_stage_bytes(1, ch->g.n1m) * xw, s2 = xa_stage_bytes(2, ch->g.n1m) * xw,
-                                 s3 = xa_stage_bytes(3, ch->g.n1m) * xw;
+                    const size_t s1 = xa_stage_bytes(ch->g.n1m) * xw;
                     cudaFuncSetAttribute(k_xAs<R, C, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)s1);
-                    cudaFuncSetAttribute(k_xAs<R, C, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)s2);
-                    cudaFuncSetAttribute(k_xAs<R, C, 3>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)s3);
+                    cudaFuncSetAttribute(k_xAs<R, C, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)s1);
+                    cudaFuncSetAttribute(k_xAs<R, C, 3>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)s1);
                     const bool cc = par_on(ch);   // the pieces as concurrent branches (knob 15)
                     if (cc && (rc = par_fork(ch))) return rc;
                     klaunch(ch, cc ? ch->par[0] : st, k_xAs<R, C, 1>, grid, nt, s1, a);
                     mark(ch, nl, "xA_u", N * (16 + 2 * Rb));
-                    klaunch(ch, cc ? ch->par[1] : st, k_xAs<R, C, 2>, grid, nt, s2, a);
+                    klaunch(ch, cc ? ch->par[1] : st, k_xAs<R, C, 2>, grid, nt, s1, a);
                     mark(ch, nl, "xA_v", N * (24 + 3 * Rb));
-                    klaunch(ch, st, k_xAs<R, C, 3>, grid, nt, s3, a);
+                    klaunch(ch, st, k_xAs<R, C, 3>, grid, nt, s1, a);
                     mark(ch, nl, "xA_w", N * (8 + 2 * Rb));
                     if (cc && (rc = par_join(ch))) return rc;
                     break;
@@ -240,7 +239,9 @@ static int launch_x_seg(c3d_channel *ch, StepArgs<R> &a, int which, const R *p0,
 template <typename R>
 int launch_xpass(c3d_channel *ch, StepArgs<R> &a, int which, const R *p0, const R *p1, int *nl) {
     const Tune &t = ch->tune;
-    if (which == 0 && t.xsplit && t.xstage && ch->g.n1m % 2 == 0 && xa_stage_bytes(2, ch->g.n1m) * t.xw > 227 * 1024) {
+    // rows that seven slots a warp (the v piece's rows) would not hold
+    if (which == 0 && t.xsplit && t.xstage && ch->g.n1m % 2 == 0 &&
+        (16 + 7 * (size_t)ch->g.n1m * 8) * t.xw > 227 * 1024) {
         set_error("xA stage exceeds shared memory");
         return C3D_EINVAL;
     }

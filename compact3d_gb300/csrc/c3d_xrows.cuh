@@ -17,13 +17,13 @@ namespace c3d {
 // xA
 // ---------------------------------------------------------------------------------
 // Rows of u, v, w and P at J-1, J, J+1 that the xA pieces read, and their slots in the
-// warp's shared-memory stage when the rows are staged by bulk copies.
+// warp's shared-memory stage when the rows are staged by bulk copies: three, refilled with
+// the rows that are read later (k_xAs).
 enum XaRow { XA_UM, XA_UC, XA_UP, XA_PM, XA_PC, XA_VM, XA_VC, XA_VP, XA_WM, XA_WC, XA_WP };
 template <int PART>
 __host__ __device__ constexpr int xa_slot(int r) {
-    return PART == 1 ? (r == XA_UM ? 0 : r == XA_UC ? 1 : r == XA_UP ? 2 : 3)
-         : PART == 2 ? (r == XA_VM ? 0 : r == XA_VC ? 1 : r == XA_VP ? 2 : r == XA_PM ? 3 : r == XA_PC ? 4
-                        : r == XA_UM ? 5 : 6)
+    return PART == 1 ? (r == XA_UM || r == XA_PC ? 0 : r == XA_UC ? 1 : 2)
+         : PART == 2 ? (r == XA_VM || r == XA_PM || r == XA_UM ? 0 : r == XA_VC ? 1 : 2)
                      : (r == XA_WM ? 0 : r == XA_WC ? 1 : 2);
 }
 // The row r of (j, k): in global memory at offsets o (J), om (J-1), op (J+1), or slot
@@ -67,11 +67,38 @@ namespace c3d {
 // the mixed form.
 template <typename R, int C, int PART, bool STG, int W = 32>
 __device__ __forceinline__ void xa_piece32(const StepArgs<R> &a, int j, long long o, long long om, long long op,
-                                         const typename SType<R>::S *st, typename SType<R>::S *sbS, R *sbR, int lane,
-                                         int P) {
+                                         typename SType<R>::S *st, typename SType<R>::S *sbS, R *sbR, int lane, int P,
+                                         uint64_t *bar) {
     typedef typename SType<R>::S S;
     typedef St<R> ST;
     const int n = a.g.n1m;
+    // staged rows: bulk copies of the rows r0 (and r1) into their slots, whose last readers are
+    // done, and the wait for them
+    auto refill = [&](int r0, int r1) {
+        if constexpr (STG) {
+            __syncwarp();
+            if (lane == 0) {
+                const uint32_t rb = (uint32_t)n * (uint32_t)sizeof(S);
+                fence_async_smem();
+                mbar_expect_tx(bar, (r1 == r0 ? 1u : 2u) * rb);
+                bulk_g2s(st + (size_t)xa_slot<PART>(r0) * n, xa_src<false, PART>(a, r0, o, om, op, st, n), rb, bar);
+                if (r1 != r0)
+                    bulk_g2s(st + (size_t)xa_slot<PART>(r1) * n, xa_src<false, PART>(a, r1, o, om, op, st, n), rb, bar);
+            }
+            __syncwarp();
+        }
+    };
+    auto ready = [&](uint32_t parity) {
+        if constexpr (STG) {
+            if (!mbar_wait(bar, parity)) {
+                if (lane == 0) a.scal[SCAL_PIPEERR] = 1.0;
+                mbar_wait(bar, parity);   // the copies in flight target this warp's stage
+                return false;
+            }
+        }
+        return true;
+    };
+    if (!ready(0)) return;
     const R RE1 = a.re1, f12 = a.f12x, f24 = a.f24x, four = (R)4.0;
     const R presg = (R)a.scal[SCAL_PRESG];
     if (PART == 2 && j >= 2) {
@@ -92,8 +119,10 @@ __device__ __forceinline__ void xa_piece32(const StepArgs<R> &a, int j, long lon
                 acc[t] = RE1 * ST::yvisc(DYPj, DYCj, DYMj, Z0, vp[t], vc[t], vm[t]);
                 hh[t] = Hj1 * Sten<R>::vv(vp[t], vc[t], vm[t]);
             }
+            refill(XA_PM, XA_PC);
             srow_store(a.hh[1] + o, hh, sbR, lane, P);
         }
+        if (!ready(1)) return;
         {
             S pc[C], pm[C];
             xrow<STG>(pc, xa_src<STG, PART>(a, XA_PC, o, om, op, st, n), sbS, lane, P);
@@ -104,6 +133,7 @@ __device__ __forceinline__ void xa_piece32(const StepArgs<R> &a, int j, long lon
                 acc[t] = -pg + acc[t];
             }
         }
+        refill(XA_UM, XA_UC);
         S vc[C];
         xrow<STG>(vc, xa_src<STG, PART>(a, XA_VC, o, om, op, st, n), sbS, lane, P);
         R d[C];
@@ -123,6 +153,7 @@ __device__ __forceinline__ void xa_piece32(const StepArgs<R> &a, int j, long lon
             d[t] = four * (ST::hi(l) + ST::hi(vc[t]));
         }
         xsolve_f<W, 6>(d, lane, P, a.c6x);
+        if (!ready(0)) return;
         {   // u at the y faces
             S uc[C], um[C];
             xrow<STG>(uc, xa_src<STG, PART>(a, XA_UC, o, om, op, st, n), sbS, lane, P);
@@ -146,6 +177,7 @@ __device__ __forceinline__ void xa_piece32(const StepArgs<R> &a, int j, long lon
 #pragma unroll
             for (int t = 0; t < C; ++t) acc[t] = RE1 * ST::yvisc(HPj, HCj, HMj, Z0, up[t], uc0[t], um[t]);
         }
+        refill(XA_PC, XA_PC);
         S uc[C];
         xrow<STG>(uc, xa_src<STG, PART>(a, XA_UC, o, om, op, st, n), sbS, lane, P);
         R d[C];
@@ -175,6 +207,7 @@ __device__ __forceinline__ void xa_piece32(const StepArgs<R> &a, int j, long lon
         }
         xsolve_f<W, 22>(d, lane, P, a.c22x);
         srow_store(a.hh[0] + o, d, sbR, lane, P);
+        if (!ready(1)) return;
         {
             S pc[C];
             xrow<STG>(pc, xa_src<STG, PART>(a, XA_PC, o, om, op, st, n), sbS, lane, P);
@@ -227,10 +260,10 @@ __device__ __forceinline__ void xa_piece32(const StepArgs<R> &a, int j, long lon
 
 template <typename R, int C, int PART, bool STG, int W = 32>
 __device__ __forceinline__ void xa_piece(const StepArgs<R> &a, int j, long long o, long long om, long long op,
-                                         const typename SType<R>::S *st, typename SType<R>::S *sbS, R *sbR, int lane,
-                                         int P) {
+                                         typename SType<R>::S *st, typename SType<R>::S *sbS, R *sbR, int lane, int P,
+                                         uint64_t *bar = nullptr) {
     if constexpr (sizeof(R) == 8) xa64<C, PART, W>(a, j, o, om, op, sbR, lane, P);
-    else xa_piece32<R, C, PART, STG, W>(a, j, o, om, op, st, sbS, sbR, lane, P);
+    else xa_piece32<R, C, PART, STG, W>(a, j, o, om, op, st, sbS, sbR, lane, P, bar);
 }
 
 // PART 0 computes the u, v and w pieces in one kernel (FP64: one after another); PART 1, 2, 3 compute one of them
@@ -406,22 +439,22 @@ __global__ void __launch_bounds__(XMAXT, sizeof(R) == 8 ? 2 : 3) k_xA(StepArgs<R
     b_xA<R, C, PART, W>(a, Blk{blockIdx.x, blockIdx.y, gridDim.x});
 }
 
-// The u, v or w piece of xA with the rows it reads staged in shared memory: lane 0 of
-// each warp issues one bulk copy per row (cp.async.bulk, completion counted on one
-// mbarrier by bytes), so every row of the warp's (j, k) is in flight at once instead of
-// one dependent group after another; the piece then reads the rows from shared memory.
-// One row per warp.  Rows staged: u at J-1, J, J+1 and P at J (PART 1); v at J-1, J, J+1,
-// P at J-1, J and u at J-1, J (PART 2); w at J-1, J, J+1 (PART 3).  A wait that runs out
-// (about a second) sets SCAL_PIPEERR, waits once more for the warp's copies in flight and
-// returns.
-template <int PART> struct XaStage { static constexpr int rows = PART == 1 ? 4 : PART == 2 ? 7 : 3; };
-
-__host__ __device__ inline size_t xa_stage_bytes(int part, int n1m) {
-    return 16 + (size_t)(part == 1 ? 4 : part == 2 ? 7 : 3) * (size_t)n1m * 8;
-}
+// The u, v or w piece of xA with the rows it reads staged in shared memory (mixed form): lane
+// 0 of each warp issues one bulk copy per row (cp.async.bulk, completion counted on one
+// mbarrier by bytes), so the rows of the warp's (j, k) are in flight at once instead of one
+// dependent group after another; the piece then reads the rows from shared memory.  One row
+// per warp, three slots: u (PART 1), v (PART 2) or w (PART 3) at J-1, J, J+1 first; the slots
+// of J-1 and J+1 then take P (PARTs 1, 2) and u at J-1, J (PART 2) while the warp computes.
+// A warp spends most of its time on its own dependent instructions, so the time follows the
+// warps an SM holds: three slots instead of every row's and at most 80 registers give 24
+// instead of 10 to 20 (384 x 256 x 384 points, mixed, u, v, w: 217, 325, 156 -> 204, 276, 156 us).  A wait
+// that runs out (about a second) sets SCAL_PIPEERR, waits once more for the warp's copies in
+// flight and returns.
+constexpr int XA_SLOTS = 3;
+__host__ __device__ inline size_t xa_stage_bytes(int n1m) { return 16 + XA_SLOTS * (size_t)n1m * 8; }
 
 template <typename R, int C, int PART>
-__global__ void __launch_bounds__(XMAXT) k_xAs(StepArgs<R> a) {
+__global__ void __launch_bounds__(XMAXT, 3) k_xAs(StepArgs<R> a) {
     pdl_enter();
     typedef typename SType<R>::S S;
     static_assert(sizeof(S) == 8, "state rows are 8-byte values");
@@ -429,8 +462,7 @@ __global__ void __launch_bounds__(XMAXT) k_xAs(StepArgs<R> a) {
     const Geo g = a.g;
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     const int P = g.n1m / C;
-    constexpr int NR = XaStage<PART>::rows;
-    unsigned char *wb = smem_raw + wid * xa_stage_bytes(PART, g.n1m);
+    unsigned char *wb = smem_raw + wid * xa_stage_bytes(g.n1m);
     uint64_t *bar = reinterpret_cast<uint64_t *>(wb);
     S *st = reinterpret_cast<S *>(wb + 16);
     const int row = blockIdx.x * (int)(blockDim.x >> 5) + wid;
@@ -441,33 +473,23 @@ __global__ void __launch_bounds__(XMAXT) k_xAs(StepArgs<R> a) {
     const int n = g.n1m;
     const uint32_t rb = (uint32_t)n * (uint32_t)sizeof(S);
     if (lane == 0) {
-        const S *src[NR];
-        if constexpr (PART == 1) {
-            src[xa_slot<1>(XA_UM)] = a.u + om; src[xa_slot<1>(XA_UC)] = a.u + o; src[xa_slot<1>(XA_UP)] = a.u + op;
-            src[xa_slot<1>(XA_PC)] = a.p + o;
-        }
-        if constexpr (PART == 2) {
-            src[xa_slot<2>(XA_VM)] = a.v + om; src[xa_slot<2>(XA_VC)] = a.v + o; src[xa_slot<2>(XA_VP)] = a.v + op;
-            src[xa_slot<2>(XA_PM)] = a.p + om; src[xa_slot<2>(XA_PC)] = a.p + o;
-            src[xa_slot<2>(XA_UM)] = a.u + om; src[xa_slot<2>(XA_UC)] = a.u + o;
-        }
-        if constexpr (PART == 3) {
-            src[xa_slot<3>(XA_WM)] = a.w + om; src[xa_slot<3>(XA_WC)] = a.w + o; src[xa_slot<3>(XA_WP)] = a.w + op;
-        }
+        constexpr int R0 = PART == 1 ? XA_UM : PART == 2 ? XA_VM : XA_WM;   // the rows J-1, J, J+1 follow each other
         mbar_init(bar, 1);
         mbar_init_fence();
         fence_async_smem();
-        mbar_expect_tx(bar, NR * rb);
+        mbar_expect_tx(bar, XA_SLOTS * rb);
 #pragma unroll
-        for (int q = 0; q < NR; ++q) bulk_g2s(st + (size_t)q * n, src[q], rb, bar);
+        for (int q = 0; q < XA_SLOTS; ++q)
+            bulk_g2s(st + (size_t)q * n, xa_src<false, PART>(a, R0 + q, o, om, op, st, n), rb, bar);
+    }
+    if (PART <= 2) pf_row(a.p + o, (int)rb, lane, 32);   // what the slots take next
+    if (PART == 2) {
+        pf_row(a.p + om, (int)rb, lane, 32);
+        pf_row(a.u + om, (int)rb, lane, 32);
+        pf_row(a.u + o, (int)rb, lane, 32);
     }
     __syncwarp();
-    if (!mbar_wait(bar, 0)) {
-        if (lane == 0) a.scal[SCAL_PIPEERR] = 1.0;
-        mbar_wait(bar, 0);   // the copies in flight target this warp's stage
-        return;
-    }
-    xa_piece<R, C, PART, true>(a, j, o, om, op, st, nullptr, nullptr, lane, P);
+    xa_piece<R, C, PART, true>(a, j, o, om, op, st, nullptr, nullptr, lane, P, bar);
 }
 
 // ---------------------------------------------------------------------------------
