@@ -51,7 +51,9 @@ __global__ void k_bcond(Geo g, typename SType<R>::S *u, typename SType<R>::S *v,
 // Wall-normal CN factor (TDMAI, compact3d.f:8630-8659), one thread per (i, k), in place.
 // The factors (A, 1/BET, GAM per J) are in the working precision; the j loops load UY
 // planes ahead so that the sequential chain does not wait on memory.
-constexpr int UY = 32;   // planes per batch (8: 0.273 ms, 16: 0.265, 32: 0.252 on channel384)
+// Planes per batch: FP32 32 (384 x 256 x 384 points: 8: 273 us, 16: 265, 32: 252), FP64 16, whose
+// batch of 32 leaves half the threads (in blocks of 128: 256 x 96 x 128 points 82 -> 74 us).
+template <typename R> constexpr int ycn_batch() { return sizeof(R) == 8 ? 16 : 32; }
 template <typename R>
 __device__ __forceinline__ void b_ycn(const StepArgs<R> &a, const R *ycn, const Blk blk) {
     const Geo g = a.g;
@@ -64,6 +66,7 @@ __device__ __forceinline__ void b_ycn(const StepArgs<R> &a, const R *ycn, const 
     const R *A = ycn + (c * 3 + 0) * m, *RB = ycn + (c * 3 + 1) * m, *GM = ycn + (c * 3 + 2) * m;
     R *X = a.r[c] + col;
     const long long s = g.np;
+    constexpr int UY = ycn_batch<R>();
     R xp = R(0);
     for (int j0 = js; j0 <= g.n2m; j0 += UY) {
         R q[UY];
@@ -105,17 +108,17 @@ __global__ void __launch_bounds__(TPB) k_ycn(StepArgs<R> a, const R *ycn) {
 }
 
 // The wall-normal CN factor with the columns staged in shared memory: a block owns TX
-// consecutive columns (i, k) of one component over all planes; its first warp fetches each
-// plane's TX-value row segment by a bulk copy (cp.async.bulk) into the block's tile, in
-// YCH chunks of planes each completing on its own mbarrier, so the forward sweep starts on
-// the first chunk while the others arrive; the forward sweep writes the tile in place,
-// the backward sweep reads it and stores each result once.  Every value crosses DRAM once
-// in each direction.  A wait that runs out sets SCAL_PIPEERR and returns after waiting
-// (bounded) for the block's copies in flight.
+// consecutive columns (i, k) of one component over all planes, one thread a column; the
+// block copies its part of every plane into its tile in 16-byte pieces (cp.async), in YCH
+// groups of planes, so the forward sweep starts on the first group while the others arrive;
+// the forward sweep writes the tile in place, the backward sweep reads it and stores each
+// result once.  Every value crosses DRAM once in each direction (the register form: twice).
+// Bulk copies, one per plane, were slower (384 x 256 x 384 points, mixed: 32 columns 278 -> 234
+// us, 64 columns 266 -> 215): 128 to 256 bytes are too little for one.
 constexpr int YCH = 8;
 template <typename R>
 __host__ __device__ inline size_t ycn_tile_bytes(int tx, int n2m) {
-    // barriers, coefficients (rounded up to 16 bytes: the tile's rows are bulk-copy targets), tile
+    // coefficients (rounded up to 16 bytes), tile
     return 64 + (((3 * (size_t)n2m * sizeof(R)) + 15) & ~(size_t)15) + (size_t)n2m * tx * sizeof(R);
 }
 
@@ -125,45 +128,32 @@ __device__ __forceinline__ void b_ycnt(const StepArgs<R> &a, const R *ycn, const
     const Geo g = a.g;
     const int np = g.np, ntile = (np + TX - 1) / TX;
     const int c = (int)blk.x / ntile, q = (int)blk.x % ntile;
-    const int col0 = q * TX, ncol = min(TX, np - col0);
+    const int col0 = q * TX, ncol = min(TX, np - col0);   // a multiple of 16 (N3M is)
     const int js = (c == 1) ? 2 : 1, nj = g.n2m - js + 1;
     const int m = g.n2 + 1;
     const R *A = ycn + (c * 3 + 0) * m, *RBt = ycn + (c * 3 + 1) * m, *GM = ycn + (c * 3 + 2) * m;
     R *X = a.r[c] + col0;
-    uint64_t *bar = reinterpret_cast<uint64_t *>(smem_raw);
-    R *sA = reinterpret_cast<R *>(smem_raw + 64), *sR = sA + nj, *sG = sR + nj;
-    R *T = reinterpret_cast<R *>(smem_raw + 64 + (((3 * (size_t)nj * sizeof(R)) + 15) & ~(size_t)15));
+    R *sA = reinterpret_cast<R *>(smem_raw), *sR = sA + nj, *sG = sR + nj;
+    R *T = reinterpret_cast<R *>(smem_raw + (((3 * (size_t)nj * sizeof(R)) + 15) & ~(size_t)15));
     const int t = threadIdx.x;
     const int cpl = (nj + YCH - 1) / YCH;
-    const uint32_t rowb = (uint32_t)ncol * (uint32_t)sizeof(R);
-    if (t == 0) {
-        for (int b = 0; b < YCH; ++b) mbar_init(bar + b, 1);
-        mbar_init_fence();
-        fence_async_smem();
-        for (int b = 0; b < YCH; ++b) {
-            const int p0 = b * cpl, p1 = min(nj, p0 + cpl);
-            if (p1 > p0) mbar_expect_tx(bar + b, (uint32_t)(p1 - p0) * rowb);
-        }
+    constexpr int V = 16 / (int)sizeof(R), PP = TX / V, PR = TX / PP;   // pieces a plane, planes a block's copy
+    const int pc = (t % PP) * V, pr = t / PP;
+#pragma unroll
+    for (int b = 0; b < YCH; ++b) {
+        const int p1 = min(nj, (b + 1) * cpl);
+        if (pc < ncol)
+            for (int p = b * cpl + pr; p < p1; p += PR) cp_async16(T + (size_t)p * TX + pc, X + (long long)(js + p) * np + pc);
+        cp_async_commit();
     }
-    for (int p = t; p < nj; p += blockDim.x) {
+    for (int p = t; p < nj; p += TX) {
         sA[p] = A[js + p];
         sR[p] = RBt[js + p];
         sG[p] = GM[js + p];
     }
-    __syncthreads();   // barriers set up before any copy can complete; coefficients staged
-    if (t < 32)
-        for (int p = t; p < nj; p += 32) bulk_g2s(T + (size_t)p * TX, X + (long long)(js + p) * np, rowb, bar + p / cpl);
-    if (t >= ncol) return;   // no copy targets this thread's column; the block stays until the others end
     R xp = R(0);
-    for (int b = 0; b < YCH; ++b) {
+    auto group = [&](int b) {   // the forward sweep of the planes of group b
         const int p0 = b * cpl, p1 = min(nj, p0 + cpl);
-        if (p1 <= p0) break;
-        if (!mbar_wait(bar + b, 0)) {
-            a.scal[SCAL_PIPEERR] = 1.0;
-            for (int b2 = b; b2 < YCH; ++b2)
-                if (b2 * cpl < nj) mbar_wait(bar + b2, 0);   // the copies in flight target this tile
-            return;
-        }
         // eight planes read ahead of the recurrence, so the shared-memory latency is not on
         // its dependent chain
         int p = p0;
@@ -185,7 +175,18 @@ __device__ __forceinline__ void b_ycnt(const StepArgs<R> &a, const R *ycn, const
             xp = (p == 0) ? v * sR[p] : (v - sA[p] * xp) * sR[p];
             T[(size_t)p * TX + t] = xp;
         }
-    }
+    };
+    static_assert(YCH == 8, "a wait per group");
+    const bool act = t < ncol;
+    cp_async_wait<7>(); __syncthreads(); if (act) group(0);
+    cp_async_wait<6>(); __syncthreads(); if (act) group(1);
+    cp_async_wait<5>(); __syncthreads(); if (act) group(2);
+    cp_async_wait<4>(); __syncthreads(); if (act) group(3);
+    cp_async_wait<3>(); __syncthreads(); if (act) group(4);
+    cp_async_wait<2>(); __syncthreads(); if (act) group(5);
+    cp_async_wait<1>(); __syncthreads(); if (act) group(6);
+    cp_async_wait<0>(); __syncthreads(); if (act) group(7);
+    if (!act) return;
     X[(long long)(js + nj - 1) * np + t] = xp;
     int p = nj - 2;
     for (; p >= 7; p -= 8) {
@@ -212,12 +213,16 @@ __global__ void __launch_bounds__(64) k_ycnt(StepArgs<R> a, const R *ycn) {
 }
 
 // Launches the wall-normal CN factor in the form the schedule names (0: one thread per
-// column with register batches; 32 or 64: the shared-memory tiles of that many columns,
-// when the tile fits).
+// column with register batches, but on FP32 grids of 2^25 points and more the tiles of 64,
+// whose single pass over memory then pays for the shared memory's reconfiguration (384 x 256
+// x 384 points: 252 -> 215 us, step 3258 -> 3229; 256 x 192 x 256: 92 -> 82, step 1863 -> 1868;
+// the results are the same bits); 32 or 64: the shared-memory tiles of that many columns;
+// tiles where they fit).
 template <typename R>
 static void launch_ycn(c3d_channel *ch, StepArgs<R> &a, int *nl) {
     const R *ycn = sizeof(R) == 8 ? (const R *)ch->ycn : (const R *)ch->ycn32;
-    const int tx = ch->tune.ycn;
+    const bool big = sizeof(R) == 4 && (long long)ch->g.np * ch->g.n2m >= 1LL << 25;
+    const int tx = ch->tune.ycn ? ch->tune.ycn : big ? 64 : 0;
     const size_t sm = ycn_tile_bytes<R>(tx == 0 ? 32 : tx, ch->g.n2m);
     if ((tx == 32 || tx == 64) && sm <= 227 * 1024) {
         const int nb = 3 * ((ch->g.np + tx - 1) / tx);
@@ -232,7 +237,8 @@ static void launch_ycn(c3d_channel *ch, StepArgs<R> &a, int *nl) {
             klaunch(ch, ch->stream, k_ycnt<R, 64>, nb, 64, sm, a, ycn);
         }
     } else {
-        klaunch(ch, ch->stream, k_ycn<R>, nblk(3LL * ch->g.np), TPB, 0, a, ycn);
+        const int nt = sizeof(R) == 8 ? 128 : TPB;
+        klaunch(ch, ch->stream, k_ycn<R>, nblk(3LL * ch->g.np, nt), nt, 0, a, ycn);
     }
     mark(ch, nl, "ycn", (double)ch->g.n1m * ch->g.n2m * ch->g.n3m * 6 * sizeof(R));
 }
