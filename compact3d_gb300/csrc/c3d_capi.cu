@@ -688,7 +688,10 @@ int c3d_create(const c3d_grid *gr, c3d_channel **out) {
     ch->fz.tw32 = ch->tw32 + nx;
     ch->dt_cached = -1.0;
     ch->cur = 0;
-    ch->pdl = 1;
+    // not with SGSSD, whose coefficients take 130 us on a side stream beside the step's kernels:
+    // with the attribute the two streams hold each other up (128 x 64 x 128 points, mixed: 824 to
+    // 1046 us a step, without it 664)
+    ch->pdl = ch->files != 3;
     cudaError_t e = cudaDeviceSynchronize();
     if (e != cudaSuccess) {
         set_error(std::string("create: ") + cudaGetErrorString(e));
@@ -2023,10 +2026,11 @@ static int batch_capture(c3d_batch *b, const double *dt, int par) {
         c3d_channel *c = b->ch[i];
         cudaStreamWaitEvent(c->stream, b->fork, 0);
         int keep = c->prof_on;
+        const int pdl = c->pdl;
         c->prof_on = 0;
         c->pdl = 0;   // plain dependences between the graph's nodes
         rc = launch_step(c, dt[i], &nl);
-        c->pdl = 1;
+        c->pdl = pdl;
         c->prof_on = keep;
         cudaEventRecord(b->join[i], c->stream);
         cudaStreamWaitEvent(b->stream, b->join[i], 0);
