@@ -251,7 +251,7 @@ template <int OP> __device__ __forceinline__ float zroot(float r) { return r; }
 template <int W, int DIR>
 __device__ __forceinline__ double ring_carry(double e, double m, int lane, int P) {
     int off = 1;
-    for (int b = 0; b < 12 && !negligible(m); ++b) {
+    for (int b = 0; b < 40 && !negligible(m); ++b) {
         int src = DIR < 0 ? lane - off : lane + off;
         if (DIR < 0 && src < 0) src += P;
         if (DIR > 0 && src >= P) src -= P;

@@ -37,6 +37,14 @@ struct MetR {
 };
 constexpr int NMETR = 13;
 
+// The Crank-Nicolson solve along z where its root r reaches past the warm-ups and the joined
+// segments (k_zCfar): m points a side (at most N3M), 1/(1 - r^N3M) of a whole line, s/(1 - r^2);
+// m = 0 within their reach.
+struct CnFar {
+    double r, c, y0;
+    int m;
+};
+
 // Everything one step's kernels need, passed by value.  R is the working precision of
 // the intermediates (double for the FP64 form, float for the mixed form).
 template <typename R>
@@ -59,6 +67,7 @@ struct StepArgs {
     double *part;                       // per-row partial sums for the bulk-flow forcing
     Cyc<R> c6x, c10x, c22x, c6z, c10z, c22z, cnx, cnz;
     R kx[2], kz[2];                     // FP64: the CN factors as partial fractions (cn_factors)
+    CnFar zfar;                         // the z factor where its root reaches past the warm-ups
     const double *ycn;                  // CN wall-normal factors: 3 comps x (A, RBET, GAM) x (n2+1)
     const double *prb, *pgam;           // Poisson factor tables [j][mode], FP64
     const float2 *prbdf, *pgamdf;       // the same as double-float pairs (mixed form)
@@ -320,6 +329,7 @@ int batch_plan(c3d_channel *ch, const BatchSched &s, std::vector<BKern> &out);
 size_t batch_args_size(const c3d_channel *ch);
 void batch_args(c3d_channel *ch, double dt, void *dst);
 int launch_poisson_tables(c3d_channel *ch);
+c3d::CnFar cn_far(const c3d_channel *ch, double dt);
 // what: 0 U component, 1 P, 2 HH component, 3 SGSVIS (to host), 4 operand (to device),
 // 5 operator result (to host)
 // ENERGY's plane statistics of the current state into out (N2M x 29, device), with

@@ -489,6 +489,47 @@ static void cn_factors(StepArgs<double> &a, int n3m, double api, double aci, dou
 }
 static void cn_factors(StepArgs<float> &, int, double, double, double, double) {}
 
+// Crank-Nicolson coefficients of one direction, A = 1 - 12 q, B = 10 + 24 q with q = DT DX^2/(2 RE)
+// (GETUH1-3, compact3d.f:8280-8282, 8314-8316).
+static void cn_coef(const Geo &g, double dxq, double dt, double &A, double &B) {
+    A = 1.0 - dt / 2.0 * (1. / g.re) * 12.0 * dxq * (1.0);
+    B = 10.0 - dt / 2.0 * (1. / g.re) * 12.0 * dxq * (-2.0);
+}
+
+// Root r, |r| < 1, and scale s of tridiag(A, B, A), B > 2 |A|: 1/tridiag = s / ((1 - r S)(1 - r S^-1)).
+// For A <= 0 (q >= 1/12) -2 / (B/A + sqrt(..)) is the growing root, and A = 0 has none: the form
+// without B/A has the decaying one for either sign.
+static void pade_root(double A, double B, double &r, double &s) {
+    if (A > 0.0) {
+        const double beta = B / A;
+        r = -2.0 / (beta + sqrt(beta * beta - 4.0));
+        s = -r / A;
+    } else {
+        const double d = B + sqrt((B - 2.0 * A) * (B + 2.0 * A));
+        r = -2.0 * A / d;
+        s = 2.0 / d;
+    }
+}
+// Points after which |r|^m is below tol.
+static int root_reach(double r, double tol) {
+    const double m = ceil(log(tol) / log(fabs(r)));
+    return m < 1e9 ? (int)m : 1000000000;
+}
+
+CnFar cn_far(const c3d_channel *ch, double dt) {
+    const bool f32 = ch->precision != C3D_FP64;
+    const int n = ch->g.n3m;
+    CnFar f = {0.0, 0.0, 0.0, 0};
+    double A, B, s;
+    cn_coef(ch->g, ch->g.dx3q, dt, A, B);
+    pade_root(A, B, f.r, s);
+    if (root_reach(f.r, f32 ? 3e-8 : 1e-17) <= (f32 ? WM<float>::MCN : WM<double>::MCN)) return f;
+    f.m = std::min(root_reach(f.r, 1e-17), n);
+    f.y0 = f.m == n ? 1.0 / (1.0 - pow(f.r, n)) : 1.0;
+    f.c = s / ((1.0 - f.r) * (1.0 + f.r));
+    return f;
+}
+
 template <typename R>
 static StepArgs<R> make_args(c3d_channel *ch, double dt) {
     typedef typename SType<R>::S S;
@@ -529,26 +570,23 @@ static StepArgs<R> make_args(c3d_channel *ch, double dt) {
     a.xscale = (R)(1.0 / ((double)ch->g.n1m * (double)ch->g.n3m));
     auto mk = [&](double A, double B, bool fp32) {
         Cyc<R> c;
-        double beta = B / A;
-        double r = -2.0 / (beta + sqrt(beta * beta - 4.0));
+        double r, s;
+        pade_root(A, B, r, s);
         c.r = (R)r;
-        c.s = (R)(-r / A);
-        double tol = fp32 ? 3e-8 : 1e-17;
-        c.m = (int)ceil(log(tol) / log(fabs(r)));
+        c.s = (R)s;
+        c.m = root_reach(r, fp32 ? 3e-8 : 1e-17);
         return c;
     };
     const bool f32 = sizeof(R) == 4;
     a.c6x = mk(1.0, 6.0, f32); a.c10x = mk(1.0, 10.0, f32); a.c22x = mk(1.0, 22.0, f32);
     a.c6z = a.c6x; a.c10z = a.c10x; a.c22z = a.c22x;
-    const double RE = ch->g.re;
-    // CN x and z factors of GETUH1-3 (compact3d.f:8280-8282, 8314-8316)
-    const double api = 1.0 - dt / 2.0 * (1. / RE) * 12.0 * ch->g.dx1q * (1.0);
-    const double aci = 10.0 - dt / 2.0 * (1. / RE) * 12.0 * ch->g.dx1q * (-2.0);
-    const double apk = 1.0 - dt / 2.0 * (1. / RE) * 12.0 * ch->g.dx3q * (1.0);
-    const double ack = 10.0 - dt / 2.0 * (1. / RE) * 12.0 * ch->g.dx3q * (-2.0);
+    double api, aci, apk, ack;
+    cn_coef(ch->g, ch->g.dx1q, dt, api, aci);
+    cn_coef(ch->g, ch->g.dx3q, dt, apk, ack);
     a.cnx = mk(api, aci, f32);
     a.cnz = mk(apk, ack, f32);
     cn_factors(a, ch->g.n3m, api, aci, apk, ack);
+    a.zfar = cn_far(ch, dt);
     return a;
 }
 

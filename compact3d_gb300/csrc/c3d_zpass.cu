@@ -399,6 +399,68 @@ __global__ void __launch_bounds__(MODE == 1 ? zjt<R, L>() : TPB) k_zC(StepArgs<R
     b_zC<R, L, MODE>(a, d0, d1, d2, Blk{blockIdx.x, blockIdx.y, gridDim.x});
 }
 
+// zC where the root reaches past the warm-ups (a.zfar.m > 0: q = DT DX3^2 / (2 RE) above about
+// 1/5; the channels' own DT keep it some 1e-3): s B(F(d)) as s/(1 - r^2) times the sum of r^|m|
+// over both sides, each side from up to a whole line of points before the segment, closed over
+// the line by 1/(1 - r^N).  In FP64 whatever the form: the gain 1/(1 - r)^2 grows with q.
+template <typename R>
+__device__ __forceinline__ void b_zCfar(const StepArgs<R> &a, R *d0, R *d1, R *d2, const Blk blk) {
+    constexpr int L = ZL;
+    const Geo g = a.g;
+    ZCo c;
+    if (!zcoords<L, 0>(blk, g, 1, c)) return;
+    const CnFar f = a.zfar;
+    const int n = g.n3m, s = g.n1m;
+    const long long o = fidx(g, c.i, c.j, 0);
+#pragma unroll 1
+    for (int q = 0; q < 3; ++q) {
+        const R *X = (q == 0 ? a.r[0] : q == 1 ? a.r[1] : a.r[2]) + o;
+        R *D = (q == 0 ? d0 : q == 1 ? d1 : d2) + o;
+        // right-hand sides from position k on, upwards (DIR 1) or downwards: xa, xb the values at
+        // the position before and at k
+        int k = wrapi(c.k0 - f.m, n);
+        double xa = X[zprev(k, n) * s], xb = X[k * s];
+        auto up = [&]() {
+            k = znext(k, n);
+            const double xc = X[k * s], d = (xa + 10.0 * xb) + xc;
+            xa = xb;
+            xb = xc;
+            return d;
+        };
+        auto down = [&]() {
+            k = zprev(k, n);
+            const double xc = X[k * s], d = (xa + 10.0 * xb) + xc;
+            xa = xb;
+            xb = xc;
+            return d;
+        };
+        double y = 0.0, out[L];
+        for (int t = 0; t < f.m; ++t) y = up() + f.r * y;
+        y *= f.y0;
+#pragma unroll
+        for (int t = 0; t < L; ++t) {
+            y = up() + f.r * y;
+            out[t] = y;
+        }
+        k = wrapi(c.k0 + L - 1 + f.m, n);
+        xa = X[znext(k, n) * s];
+        xb = X[k * s];
+        y = 0.0;
+        for (int t = 0; t < f.m; ++t) y = down() + f.r * y;
+        y *= f.y0;
+#pragma unroll
+        for (int t = L - 1; t >= 0; --t) {
+            D[(c.k0 + t) * s] = (R)(f.c * (out[t] + f.r * y));
+            y = down() + f.r * y;
+        }
+    }
+}
+template <typename R>
+__global__ void __launch_bounds__(TPB) k_zCfar(StepArgs<R> a, R *d0, R *d1, R *d2) {
+    pdl_enter();
+    b_zCfar<R>(a, d0, d1, d2, Blk{blockIdx.x, blockIdx.y, gridDim.x});
+}
+
 // z part of RHSDP: rdpz = compact d(UH3)/dz / DT with UH3 = W + delta3
 template <typename R, int L, int MODE>
 __device__ __forceinline__ void b_zD(const StepArgs<R> &a, const R *d2, const Blk blk) {
@@ -572,6 +634,13 @@ __global__ void __launch_bounds__(MODE == 1 ? zjt<R, L>() : TPB) kb_zC(const Ste
     const StepArgs<R> &a = A[m.ch];
     b_zC<R, L, MODE>(a, a.exz, a.eyz, a.wsq, Blk{m.x, m.y, m.gx});
 }
+template <typename R>
+__global__ void __launch_bounds__(TPB) kb_zCfar(const StepArgs<R> *__restrict__ A, const BMap *__restrict__ map) {
+    pdl_enter();
+    const BMap m = map[blockIdx.x];
+    const StepArgs<R> &a = A[m.ch];
+    b_zCfar<R>(a, a.exz, a.eyz, a.wsq, Blk{m.x, m.y, m.gx});
+}
 template <typename R, int L, int MODE>
 __global__ void __launch_bounds__(MODE == 1 ? zjt<R, L>() : TPB) kb_zD(const StepArgs<R> *__restrict__ A, const BMap *__restrict__ map) {
     pdl_enter();
@@ -622,6 +691,10 @@ int zpass_bkern(const c3d_channel *ch, int which, int L, std::vector<BKern> &out
     if (ch->g.n3m % ZL != 0) return C3D_EINVAL;
     if (L != 8 && L != 32) L = 16;
     if (ch->g.n3m % L != 0) L = 16;
+    if (which == 2 && cn_far(ch, ch->dt_cached).m > 0) {   // DT of the step that is captured
+        out.push_back({(const void *)kb_zCfar<R>, TPB, 0, (unsigned)nblk((long long)ch->g.n2m * (ch->g.n3m / ZL) * ch->g.n1m)});
+        return 0;
+    }
     if constexpr (sizeof(R) == 8) {   // joined segments, as for one channel
         switch (zjoin_len<R>(ch->g.n3m)) {
             case 8: return zbk<R, 8, 1>(ch, which, out);
@@ -664,6 +737,12 @@ static int launch_diag_z(c3d_channel *ch, StepArgs<R> &a, const double *divx, in
 template <typename R>
 int launch_zpass(c3d_channel *ch, StepArgs<R> &a, int which, R *d0, R *d1, R *d2, int flag, int *nl) {
     if (which == 5) return launch_diag_z<R>(ch, a, (const double *)d0, nl);
+    if (which == 2 && a.zfar.m > 0) {
+        const Geo &g = ch->g;
+        klaunch(ch, ch->stream, k_zCfar<R>, nblk((long long)g.n2m * (g.n3m / ZL) * g.n1m), TPB, 0, a, d0, d1, d2);
+        mark(ch, nl, "zC", (double)g.n1m * g.n2m * g.n3m * 6 * sizeof(R));
+        return 0;
+    }
     const int zl = ch->tune.zl[which];
     // FP64 always joins its segments: the FP64 pipe (2 lanes per clock and SM) bounds these
     // passes, and with M = 23 warm-up points a segment of 16 evaluates 62 right-hand sides

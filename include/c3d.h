@@ -121,7 +121,9 @@ int c3d_set_device(int device);
  * c3d_step      one call of GETUP(U,P,HH,SS,NTIME,PRESG,PRESG3,SGSVIS)
  *               (compact3d.f:879-960): BCOND, RHS1-3 with AB2, GETUH1-3
  *               (Crank-Nicolson ADI), RHSDP, GETDP (FFT Poisson), UPCALC.
- *               dt is COMMON /TSTEP/ DT; presg/presg3 are in-out.
+ *               dt is COMMON /TSTEP/ DT, any positive value (past DT DX3^2 / (2 RE) of
+ *               about 1/5 the z solve of GETUH takes its slower form of long reach);
+ *               presg/presg3 are in-out.
  * c3d_diagnose  DIVCHECK + CFL + CHKMF + WALLSS on the current device state.
  * c3d_getup     drop-in for a driver that keeps the fields on the host:
  *               upload, step, download in one call.
