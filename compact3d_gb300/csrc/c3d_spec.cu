@@ -297,6 +297,15 @@ constexpr int TWZ_MAX = 16;   // widest z-FFT tile the autotuner tries
 
 constexpr size_t SMEM_MAX = 227 * 1024;
 
+// The widest z-FFT tile, from `want` kx columns down, whose two buffers fit in shared memory
+// (N3M lines of C2 values: FP64 lines of more than 900 points narrow a tile of 8, FP32 of 1800).
+template <typename C2>
+static int fftz_tile(int n3m, int want) {
+    int tw = want;
+    while (tw > 1 && 2 * (size_t)n3m * tw * sizeof(C2) > SMEM_MAX) tw /= 2;
+    return tw;
+}
+
 template <typename R>
 void set_spec_smem(c3d_channel *ch) {
     typedef typename Cx<R>::T C2;
@@ -335,8 +344,8 @@ static bool launch_fftz4(c3d_channel *ch, StepArgs<R> &a) {
 
 // ---------------------------------------------------------------------------------
 // Batch form: the z FFTs of the channels with the same N3M in one launch (the four-step
-// warp form when N3M = 32 N1, tiles of 8 kx columns in shared memory otherwise) and the
-// Poisson solves of every channel in one launch.
+// warp form when N3M = 32 N1, tiles of 8 kx columns in shared memory otherwise, of fewer where
+// a long line's would not fit) and the Poisson solves of every channel in one launch.
 // ---------------------------------------------------------------------------------
 constexpr int TW_BATCH = 8;
 
@@ -346,11 +355,11 @@ __global__ void __launch_bounds__(FZW * 32) kb_fftz4(const StepArgs<R> *__restri
     const BMap m = map[blockIdx.x];
     b_fftz4<R, N1, SIGN>(A[m.ch], Blk{m.x, m.y, m.gx});
 }
-template <typename R, int SIGN>
+template <typename R, int SIGN, int TW>
 __global__ void __launch_bounds__(TPB) kb_fftz(const StepArgs<R> *__restrict__ A, const BMap *__restrict__ map) {
     pdl_enter();
     const BMap m = map[blockIdx.x];
-    b_fftz<R>(A[m.ch], SIGN, TW_BATCH, Blk{m.x, m.y, m.gx});
+    b_fftz<R>(A[m.ch], SIGN, TW, Blk{m.x, m.y, m.gx});
 }
 __global__ void __launch_bounds__(TPB) kb_poisson64(const StepArgs<double> *__restrict__ A, const BMap *__restrict__ map) {
     pdl_enter();
@@ -377,6 +386,16 @@ static const void *fftz4_batch_fn(int n1) {
     }
 }
 
+template <typename R, int SIGN>
+static const void *fftz_batch_fn(int tw) {
+    switch (tw) {
+        case 1: return (const void *)kb_fftz<R, SIGN, 1>;
+        case 2: return (const void *)kb_fftz<R, SIGN, 2>;
+        case 4: return (const void *)kb_fftz<R, SIGN, 4>;
+        default: return (const void *)kb_fftz<R, SIGN, TW_BATCH>;
+    }
+}
+
 template <typename R>
 int spec_bkern(const c3d_channel *ch, int which, std::vector<BKern> &out) {
     typedef typename Cx<R>::T C2;
@@ -394,9 +413,10 @@ int spec_bkern(const c3d_channel *ch, int which, std::vector<BKern> &out) {
         out.push_back({f4, FZW * 32, sm4, (unsigned)(g.n2m * ((g.n1h + TWW - 1) / TWW))});
         return 0;
     }
-    const size_t smz = 2 * (size_t)g.n3m * TW_BATCH * sizeof(C2);
-    const void *fn = which == 0 ? (const void *)kb_fftz<R, -1> : (const void *)kb_fftz<R, +1>;
-    out.push_back({fn, TPB, smz, (unsigned)(g.n2m * ((g.n1h + TW_BATCH - 1) / TW_BATCH))});
+    const int tw = fftz_tile<C2>(g.n3m, TW_BATCH);
+    const size_t smz = 2 * (size_t)g.n3m * tw * sizeof(C2);
+    const void *fn = which == 0 ? fftz_batch_fn<R, -1>(tw) : fftz_batch_fn<R, +1>(tw);
+    out.push_back({fn, TPB, smz, (unsigned)(g.n2m * ((g.n1h + tw - 1) / tw))});
     return 0;
 }
 template int spec_bkern<double>(const c3d_channel *, int, std::vector<BKern> &);
@@ -413,8 +433,7 @@ int launch_spec(c3d_channel *ch, StepArgs<R> &a, int which, int *nl) {
             return 0;
         }
     }
-    int tw = ch->tune.twz == 0 ? 8 : ch->tune.twz;
-    while (tw > 1 && 2 * (size_t)ch->g.n3m * tw * sizeof(C2) > SMEM_MAX) tw /= 2;   // long FP64 lines
+    const int tw = fftz_tile<C2>(ch->g.n3m, ch->tune.twz == 0 ? 8 : ch->tune.twz);
     const int ntile = (ch->g.n1h + tw - 1) / tw;
     const size_t smz = 2 * (size_t)ch->g.n3m * tw * sizeof(C2);
     switch (which) {
