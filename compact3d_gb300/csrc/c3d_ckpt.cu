@@ -15,7 +15,7 @@ struct CkF64 {
     __device__ static void put(double *a, long long q, double x) { a[q] = x; }
 };
 struct CkDF {
-    __device__ static double get(const float2 *a, long long q) { return St<float>::dbl(a[q]); }
+    __device__ static double get(const float2 *a, long long q) { return St<float>::value(a[q]); }
     __device__ static void put(float2 *a, long long q, double x) { a[q] = St<float>::from_double(x); }
 };
 struct CkF32 {

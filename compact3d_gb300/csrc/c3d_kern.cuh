@@ -26,7 +26,9 @@ template <typename R> struct St;
 
 // float -> double in integer arithmetic: the conversion instruction runs at the FP64 rate (2
 // lanes per clock and SM).  Exact for normal numbers, zeros, infinities and NaN; magnitudes
-// below 2^-126 (which a low part reaches only where its value is below 2^-102) become zero.
+// below 2^-126 become zero, an error below 2^-126 per part (a low part lies anywhere below
+// 2^-25 of its value): for terms of sums and maxima and for the models; values that leave the
+// library as they are convert by St::value.
 __device__ __forceinline__ double f2d(float x) {
     const unsigned b = __float_as_uint(x), e = b & 0x7f800000u;
     unsigned hi = ((b & 0x7fffffffu) >> 3) + 0x38000000u, lo = b << 29;
@@ -67,6 +69,7 @@ template <> struct St<float> {
         return make_float2(h, l);
     }
     static __device__ __forceinline__ double dbl(float2 a) { return f2d(a.x) + f2d(a.y); }
+    static __device__ __forceinline__ double value(float2 a) { return (double)a.x + (double)a.y; }
     static __device__ __forceinline__ float2 scale(float2 a, float s) { return make_float2(a.x * s, a.y * s); }
     static __host__ __device__ __forceinline__ float2 from_double(double a) {
         float h = (float)a;

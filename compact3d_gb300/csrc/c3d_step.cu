@@ -468,7 +468,7 @@ struct ToF32 { __device__ float operator()(double x) const { return (float)x; } 
 struct ToDF { __device__ float2 operator()(double x) const { return St<float>::from_double(x); } };
 struct FromF64 { __device__ double operator()(double x) const { return x; } };
 struct FromF32 { __device__ double operator()(float x) const { return (double)x; } };
-struct FromDF { __device__ double operator()(float2 x) const { return St<float>::dbl(x); } };
+struct FromDF { __device__ double operator()(float2 x) const { return St<float>::value(x); } };
 
 // ---------------------------------------------------------------------------------
 // Host-side drivers
