@@ -668,6 +668,7 @@ int c3d_create(const c3d_grid *gr, c3d_channel **out) {
     if (rc) return fail(rc);
     // FFT plans and twiddles: [x: N1M/2][z: N3M][x post-processing: N1M/2+1]
     ch->tune = Tune{{16, 16, 16, 16, 16}, 4, 8, 0, 0, 0, 0, 0, 0, 0, 0, 0};
+    ch->tune.ycn = ycn_default(ch);
     ch->fx = make_plan(g.n1m / 2, 0);
     ch->fz = make_plan(g.n3m, 0);
     if (ch->fx.nst < 0 || ch->fz.nst < 0) { set_error("FFT plan index arithmetic"); return fail(C3D_EINVAL); }

@@ -329,6 +329,7 @@ int batch_plan(c3d_channel *ch, const BatchSched &s, std::vector<BKern> &out);
 size_t batch_args_size(const c3d_channel *ch);
 void batch_args(c3d_channel *ch, double dt, void *dst);
 int launch_poisson_tables(c3d_channel *ch);
+int ycn_default(const c3d_channel *ch);
 c3d::CnFar cn_far(const c3d_channel *ch, double dt);
 // what: 0 U component, 1 P, 2 HH component, 3 SGSVIS (to host), 4 operand (to device),
 // 5 operator result (to host)

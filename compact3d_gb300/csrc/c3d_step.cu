@@ -213,16 +213,24 @@ __global__ void __launch_bounds__(64) k_ycnt(StepArgs<R> a, const R *ycn) {
 }
 
 // Launches the wall-normal CN factor in the form the schedule names (0: one thread per
-// column with register batches, but on FP32 grids of 2^25 points and more the tiles of 64,
-// whose single pass over memory then pays for the shared memory's reconfiguration (384 x 256
-// x 384 points: 252 -> 215 us, step 3258 -> 3229; 256 x 192 x 256: 92 -> 82, step 1863 -> 1868;
-// the results are the same bits); 32 or 64: the shared-memory tiles of that many columns;
-// tiles where they fit).
+// column with register batches; 32 or 64: the shared-memory tiles of that many columns,
+// where they fit).  All forms give the same bits.
+// The form a new channel's schedule names: on mixed grids of 2^25 points and more, whose
+// component (134 MB) exceeds L2 (129 MB), the tiles of 64, which read and write memory once.
+// Steps with the register form and with the tiles, us: 384 x 256 x 384 points 3610, 3567;
+// 384 x 172 x 512, just past the line, 3285, 3272.  Below it the tiles gain no more than that
+// (256 x 255 x 512 3252, 3225; 256 x 192 x 256 1272, 1260) and lose on the refined form, whose
+// other kernels wait for the shared memory's reconfiguration (256 x 192 x 256 1863, 1868), so
+// those grids start with the register form and leave the choice to the tuner.
+int ycn_default(const c3d_channel *ch) {
+    const bool big = ch->precision == C3D_MIXED && (long long)ch->g.np * ch->g.n2m >= 1LL << 25;
+    return big && ycn_tile_bytes<float>(64, ch->g.n2m) <= 227 * 1024 ? 64 : 0;
+}
+
 template <typename R>
 static void launch_ycn(c3d_channel *ch, StepArgs<R> &a, int *nl) {
     const R *ycn = sizeof(R) == 8 ? (const R *)ch->ycn : (const R *)ch->ycn32;
-    const bool big = sizeof(R) == 4 && (long long)ch->g.np * ch->g.n2m >= 1LL << 25;
-    const int tx = ch->tune.ycn ? ch->tune.ycn : big ? 64 : 0;
+    const int tx = ch->tune.ycn;
     const size_t sm = ycn_tile_bytes<R>(tx == 0 ? 32 : tx, ch->g.n2m);
     if ((tx == 32 || tx == 64) && sm <= 227 * 1024) {
         const int nb = 3 * ((ch->g.np + tx - 1) / tx);

@@ -400,10 +400,10 @@ int c3d_checkpoint_read(c3d_channel *ch, const char *path, int *ntime, double *t
  *       by one bulk copy per row before computing (1; N1M even; FP64 reads them from
  *       global memory either way)
  *   [13] the wall-normal Crank-Nicolson factor (TDMAI): one thread per column with
- *       register batches of planes (0; mixed grids of 2^25 points and more: as 64), or
- *       blocks of 32 or 64 columns whose planes
- *       are staged in shared memory by asynchronous copies so that each value is read and
- *       written once (falls back to 0 when the tile exceeds shared memory)
+ *       register batches of planes (0), or blocks of 32 or 64 columns whose planes are
+ *       staged in shared memory by asynchronous copies so that each value is read and
+ *       written once (falls back to 0 when the tile exceeds shared memory); mixed grids of
+ *       2^25 points and more start with 64, all others with 0
  *   [14] lanes per row of the explicit x pieces read from global memory, of the
  *       x pass of the remaining terms, and of the pressure x passes with the
  *       shared-memory row FFT ([7] != 3) and no bulk-copy ring ([11] = 0): 0 (a warp
