@@ -1744,8 +1744,12 @@ int c3d_autotune(c3d_channel *ch, int *sched) {
              : q == 10 ? t.xsplit : q == 11 ? t.xbulk : q == 12 ? t.xstage : q == 13 ? t.ycn : q == 14 ? t.xlanes
              : t.conc;
     };
+    // FP64 joins its z segments, takes its row lanes by N1M and reads xA's rows from global
+    // memory whatever these knobs say: they keep their values, and no equal kernels are timed
+    auto unread = [&](int q) { return ch->precision == C3D_FP64 && (q <= 4 || q == 12 || q == 14); };
     Tune best = ch->tune;
     for (const Group &gp : groups) {
+        if (unread(gp.knob)) continue;
         double bcost = 1e300;
         int bval = knob(best, gp.knob);
         for (int v : gp.cand) {
