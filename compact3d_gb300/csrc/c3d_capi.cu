@@ -1745,8 +1745,9 @@ int c3d_autotune(c3d_channel *ch, int *sched) {
              : t.conc;
     };
     // FP64 joins its z segments, takes its row lanes by N1M and reads xA's rows from global
-    // memory whatever these knobs say: they keep their values, and no equal kernels are timed
-    auto unread = [&](int q) { return ch->precision == C3D_FP64 && (q <= 4 || q == 12 || q == 14); };
+    // memory and has no bulk-copy ring, whatever these knobs say: they keep their values, and no
+    // equal kernels are timed
+    auto unread = [&](int q) { return ch->precision == C3D_FP64 && (q <= 4 || q == 11 || q == 12 || q == 14); };
     Tune best = ch->tune;
     for (const Group &gp : groups) {
         if (unread(gp.knob)) continue;

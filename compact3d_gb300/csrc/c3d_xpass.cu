@@ -189,7 +189,7 @@ static int launch_x_seg(c3d_channel *ch, StepArgs<R> &a, int which, const R *p0,
     typedef typename Cx<R>::T C2;
     const Tune &t = ch->tune;
     if (which == 0 && sizeof(R) == 4 && (!t.xsplit || t.xstage)) return 1;
-    if ((which == 2 || which == 3) && (t.fxp == 3 || t.xbulk)) return 1;
+    if ((which == 2 || which == 3) && (t.fxp == 3 || (sizeof(R) == 4 && t.xbulk))) return 1;   // FP64 has no ring
     const int nrows = ch->g.n2m * ch->g.n3m;
     // FP64: blocks of one warp while there are fewer than 16 warps per SM (152), so that the
     // last wave is short (96 x 48 x 64 points, dynamic LES: 650 -> 640 us a step)

@@ -411,7 +411,7 @@ int c3d_checkpoint_read(c3d_channel *ch, const char *path, int *ntime, double *t
  *       96 (8 lanes) or 128 (16 lanes) with N3M a multiple of 32 / lanes, so that each
  *       lane holds 6 to 12 points and the cross-lane scans of the line solves take 3
  *       or 4 steps instead of 5
- *       (FP64 takes its segment by N1M, whatever this is)
+ *       (FP64 takes its segment by N1M, whatever this and [11] are)
  *   [15] the u, v and w pieces of the explicit x pass ([10] = 1), then those of the
  *       explicit z pass ([9] = 1), as three concurrent branches on three streams (1)
  *       or one after another (0); they write disjoint fields.  The per-kernel profile
