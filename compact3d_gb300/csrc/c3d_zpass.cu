@@ -278,12 +278,11 @@ __global__ void __launch_bounds__(MODE == 1 ? zjt<R, L>() : TPB) k_zA(StepArgs<R
     b_zA<R, L, PART, MODE>(a, Blk{blockIdx.x, blockIdx.y, gridDim.x});
 }
 
-// H += s z per position.  BAT: the rounding that ensembles have always had, so that their
-// results stay the same bits: one rounding (a fused multiply-add) at a segment's first
-// position for H1, two at the others.
-template <typename R, int L, int MODE, bool BAT = false>
+// H += k z with one rounding at every position, written out: left to the compiler, which
+// multiply-adds it fuses differs between the instances, and with it the bits of a channel alone
+// and in an ensemble.
+template <typename R, int L, int MODE>
 __device__ __forceinline__ void b_zB(const StepArgs<R> &a, const Blk blk) {
-    constexpr bool RND = BAT && sizeof(R) == 4 && MODE == 0;
     const Geo g = a.g;
     ZCo c;
     if (!zcoords<L, MODE>(blk, g, 1, c)) return;
@@ -300,13 +299,12 @@ __device__ __forceinline__ void b_zB(const StepArgs<R> &a, const Blk blk) {
         pf_cols(a.hh[1] + o0, sb * sizeof(R), 32 * (int)sizeof(R), k0, 0, L, n, lane);
     }
     R out[3][L];
-    const R sc = a.c22z.s, s1 = RND ? R(1) : sc;
-    const R r22 = zroot<22>(a.c22z.r), rr[3] = {r22, r22, r22}, ss[3] = {s1, s1, s1};
+    const R r22 = zroot<22>(a.c22z.r), rr[3] = {r22, r22, r22}, ss[3] = {R(1), R(1), R(1)};
     WalkZB<R> f{a.exz + o, a.wsq + o, a.eyz + o, n, s, zrhs<MODE>(a.f24z)};
     f.v = (j >= 2);
     zsolve<R, L, WM<R>::M22, 3, MODE>(out, c, n, rr, ss, f);
     R *H1 = a.hh[0] + o, *H2 = a.hh[1] + o, *H3 = a.hh[2] + o;
-    const R ks = zfold<MODE>(a.f24z, a.c22z.s);
+    const R ks = MODE == 1 ? zfold<MODE>(a.f24z, a.c22z.s) : a.c22z.s;
     if (!c.act) return;
     constexpr int B = ztb<L>();
 #pragma unroll
@@ -317,15 +315,9 @@ __device__ __forceinline__ void b_zB(const StepArgs<R> &a, const Blk blk) {
 #pragma unroll
         for (int t = 0; t < B; ++t) {
             const int kk = (k0 + b + t) * s;
-            if constexpr (RND) {
-                H1[kk] = b + t == 0 ? __fmaf_rn(sc, out[0][0], h1[0]) : __fadd_rn(h1[t], __fmul_rn(sc, out[0][b + t]));
-                H3[kk] = __fmul_rn(sc, out[1][b + t]);
-                if (j >= 2) H2[kk] = __fadd_rn(h2[t], __fmul_rn(sc, out[2][b + t]));
-            } else {
-                H1[kk] = h1[t] + ks * out[0][b + t];          // d(uw)/dz
-                H3[kk] = ks * out[1][b + t];                  // d(ww)/dz
-                if (j >= 2) H2[kk] = h2[t] + ks * out[2][b + t];   // d(vw)/dz
-            }
+            H1[kk] = fma(ks, out[0][b + t], h1[t]);               // d(uw)/dz
+            H3[kk] = ks * out[1][b + t];                          // d(ww)/dz
+            if (j >= 2) H2[kk] = fma(ks, out[2][b + t], h2[t]);   // d(vw)/dz
         }
     }
 }
@@ -625,7 +617,7 @@ template <typename R, int L, int MODE>
 __global__ void __launch_bounds__(MODE == 1 ? zjt<R, L>() : TPB) kb_zB(const StepArgs<R> *__restrict__ A, const BMap *__restrict__ map) {
     pdl_enter();
     const BMap m = map[blockIdx.x];
-    b_zB<R, L, MODE, true>(A[m.ch], Blk{m.x, m.y, m.gx});
+    b_zB<R, L, MODE>(A[m.ch], Blk{m.x, m.y, m.gx});
 }
 template <typename R, int L, int MODE>
 __global__ void __launch_bounds__(MODE == 1 ? zjt<R, L>() : TPB) kb_zC(const StepArgs<R> *__restrict__ A, const BMap *__restrict__ map) {
