@@ -131,7 +131,6 @@ __device__ __forceinline__ dfl shfl_idx(dfl v, int s, int w = 32) {
 
 // 1 - x rounds to 1 (so that y / (1 - x) is y exactly) for |x| below half an ulp of 1.
 __device__ __forceinline__ bool below_half_ulp(float x) { return fabsf(x) < 0x1p-25f; }
-__device__ __forceinline__ bool below_half_ulp(double x) { return fabs(x) < 0x1p-54; }
 template <typename R>
 __device__ __forceinline__ bool below_half_ulp(R) { return false; }
 
@@ -502,42 +501,6 @@ __device__ __forceinline__ void zseg(R (&out)[L], int k0, int n, const Cyc<R> &c
     }
 }
 
-// The same with the warm-up length M a compile-time constant, so that every loop unrolls
-// and the loads of D can be issued ahead of the recurrence.
-template <typename R, int L, int M, typename F>
-__device__ __forceinline__ void zsegm(R (&out)[L], int k0, int n, const Cyc<R> &c, F D) {
-    const R r = c.r;
-    R y = R(0);
-    int kk = wrapi(k0 - M, n);
-#pragma unroll
-    for (int q = 0; q < M; ++q) {
-        y = D(kk) + r * y;
-        kk = (kk + 1 == n) ? 0 : kk + 1;
-    }
-    R ys[L];
-#pragma unroll
-    for (int t = 0; t < L; ++t) {
-        y = D(kk) + r * y;
-        ys[t] = y;
-        kk = (kk + 1 == n) ? 0 : kk + 1;
-    }
-    R acc = R(0), pw = R(1);
-#pragma unroll
-    for (int q = 0; q < M; ++q) {
-        y = D(kk) + r * y;
-        acc = acc + pw * y;
-        pw *= r;
-        kk = (kk + 1 == n) ? 0 : kk + 1;
-    }
-    R z = acc;
-    const R s = c.s;
-#pragma unroll
-    for (int t = L - 1; t >= 0; --t) {
-        z = ys[t] + r * z;
-        out[t] = s * z;
-    }
-}
-
 // Several cyclic solves along one column in a single sweep.  The functor f walks the
 // column once, in order, from position k0 - M (wrapped): f.start(k) positions it and
 // f.next(d) returns the NR right-hand sides at the current position and advances, so it
@@ -671,10 +634,10 @@ __device__ __forceinline__ void zjoin(R (&out)[NR][L], int k0, const R (&r)[NR],
 }
 
 // Warm-up lengths M = ceil(log(tol)/log|r|) of the Pade operators (1,6,1), (1,10,1),
-// (1,22,1) and the Crank-Nicolson operators (b/a > 10, so M <= M10): tol = 1e-17 in FP64,
-// 3e-8 in FP32.
+// (1,22,1) and the Crank-Nicolson operators (b/a > 10 while DT DX^2 / (2 RE) < 1/12, so MCN is
+// the length of (1,10,1)): tol = 1e-17 in FP64, 3e-8 in FP32.
 template <typename R> struct WM;
-template <> struct WM<double> { static constexpr int M6 = 23, M10 = 18, M22 = 13, MCN = 18; };
-template <> struct WM<float> { static constexpr int M6 = 10, M10 = 8, M22 = 6, MCN = 8; };
+template <> struct WM<double> { static constexpr int M6 = 23, M22 = 13, MCN = 18; };
+template <> struct WM<float> { static constexpr int M6 = 10, M22 = 6, MCN = 8; };
 
 }  // namespace c3d

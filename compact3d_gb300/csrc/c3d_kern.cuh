@@ -234,55 +234,6 @@ __device__ __forceinline__ void drow_store(T *__restrict__ g, const T (&v)[C], i
     }
 }
 
-#ifndef C3D_STAGED_ROWS
-#define C3D_STAGED_ROWS 0
-#endif
-
-template <typename T, int C>
-__device__ __forceinline__ void srow_load(T (&v)[C], const T *__restrict__ g, T *sb, int lane, int P) {
-    if (!C3D_STAGED_ROWS) {
-        (void)sb;
-        drow_load(v, g, lane, P);
-        return;
-    }
-    const int n = P * C;
-#pragma unroll
-    for (int t = 0; t < C; ++t) {
-        int e = lane + 32 * t;
-        if (e < n) sb[e + e / C] = ldro(g + e);
-    }
-    __syncwarp();
-    if (lane < P) {
-#pragma unroll
-        for (int t = 0; t < C; ++t) v[t] = sb[lane * (C + 1) + t];
-    } else {
-#pragma unroll
-        for (int t = 0; t < C; ++t) v[t] = T();
-    }
-    __syncwarp();
-}
-
-template <typename T, int C>
-__device__ __forceinline__ void srow_store(T *__restrict__ g, const T (&v)[C], T *sb, int lane, int P) {
-    if (!C3D_STAGED_ROWS) {
-        (void)sb;
-        drow_store(g, v, lane, P);
-        return;
-    }
-    const int n = P * C;
-    if (lane < P) {
-#pragma unroll
-        for (int t = 0; t < C; ++t) sb[lane * (C + 1) + t] = v[t];
-    }
-    __syncwarp();
-#pragma unroll
-    for (int t = 0; t < C; ++t) {
-        int e = lane + 32 * t;
-        if (e < n) g[e] = sb[e + e / C];
-    }
-    __syncwarp();
-}
-
 // Lane-chunk row load from a 16-byte aligned shared-memory row (a bulk-copy stage).
 template <typename T, int C>
 __device__ __forceinline__ void crow_load(T (&v)[C], const T *s, int lane, int P) {
@@ -374,12 +325,6 @@ __device__ __forceinline__ bool mbar_wait(uint64_t *b, uint32_t parity, unsigned
     while (!mbar_try_wait(b, parity))
         if (gtimer_ns() - t0 > limit_ns) return false;
     return true;
-}
-
-// Bytes of the per-warp staging buffer for rows of n1m points (none when rows move directly:
-// reserved shared memory would only shrink the L1 cache).
-__host__ __device__ inline size_t stage_bytes(int n1m, int C) {
-    return C3D_STAGED_ROWS ? (size_t)(n1m + n1m / C + 2) * 8 : 0;
 }
 
 // ---------------------------------------------------------------------------------

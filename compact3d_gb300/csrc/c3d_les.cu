@@ -1170,25 +1170,23 @@ __global__ void __launch_bounds__(TPB) k_les_x1(StepArgs<R> a, LesArgs<R> l) {
     const Geo g = a.g;
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     const int P = g.n1m / C;
-    S *sbS = reinterpret_cast<S *>(smem_raw + wid * stage_bytes(g.n1m, C));
-    R *sbR = reinterpret_cast<R *>(sbS);
     const int nrows = g.n2m * g.n3m;
     const R f24 = a.f24x, four = (R)4.0, two = (R)2.0;
     for (int row = blockIdx.x * (TPB / 32) + wid; row < nrows; row += gridDim.x * (TPB / 32)) {
         const int j = 1 + row / g.n3m, k = row % g.n3m;
         const long long o = fidx(g, 0, j, k);
         R nv[C], d[C];
-        srow_load(nv, l.nu + o, sbR, lane, P);
+        drow_load(nv, l.nu + o, lane, P);
         {
             R pv = sprev(nv[C - 1], lane, P);
 #pragma unroll
             for (int t = 0; t < C; ++t) d[t] = four * (nv[t] + (t == 0 ? pv : nv[t - 1]));
             xsolve<32, 6>(d, lane, P, a.c6x);
-            srow_store(l.nux + o, d, sbR, lane, P);
+            drow_store(l.nux + o, d, lane, P);
         }
         {
             S uc[C];
-            srow_load(uc, a.u + o, sbS, lane, P);
+            drow_load(uc, a.u + o, lane, P);
             S nx = snext(uc[0], lane, P);
 #pragma unroll
             for (int t = 0; t < C; ++t) d[t] = f24 * ST::d(t == C - 1 ? nx : uc[t + 1], uc[t]);
@@ -1201,28 +1199,28 @@ __global__ void __launch_bounds__(TPB) k_les_x1(StepArgs<R> a, LesArgs<R> l) {
             for (int t = 0; t < C; ++t) e[t] = f24 * (d[t] - (t == 0 ? pv : d[t - 1]));
             xsolve<32, 22>(e, lane, P, a.c22x);
             R h[C];
-            srow_load(h, a.hh[0] + o, sbR, lane, P);
+            drow_load(h, a.hh[0] + o, lane, P);
 #pragma unroll
             for (int t = 0; t < C; ++t) h[t] = h[t] - two * e[t];
-            srow_store(a.hh[0] + o, h, sbR, lane, P);
+            drow_store(a.hh[0] + o, h, lane, P);
         }
         if (j >= 2) {
             S vc[C];
-            srow_load(vc, a.v + o, sbS, lane, P);
+            drow_load(vc, a.v + o, lane, P);
             S pv = sprev(vc[C - 1], lane, P);
 #pragma unroll
             for (int t = 0; t < C; ++t) d[t] = f24 * ST::d(vc[t], t == 0 ? pv : vc[t - 1]);
             xsolve<32, 22>(d, lane, P, a.c22x);
-            srow_store(l.dvdx + o, d, sbR, lane, P);
+            drow_store(l.dvdx + o, d, lane, P);
         }
         {
             S wc[C];
-            srow_load(wc, a.w + o, sbS, lane, P);
+            drow_load(wc, a.w + o, lane, P);
             S pv = sprev(wc[C - 1], lane, P);
 #pragma unroll
             for (int t = 0; t < C; ++t) d[t] = f24 * ST::d(wc[t], t == 0 ? pv : wc[t - 1]);
             xsolve<32, 22>(d, lane, P, a.c22x);
-            srow_store(l.dwdx + o, d, sbR, lane, P);
+            drow_store(l.dwdx + o, d, lane, P);
         }
     }
 }
@@ -1390,8 +1388,6 @@ __global__ void __launch_bounds__(TPB) k_les_x2(StepArgs<R> a, LesArgs<R> l) {
     const Geo g = a.g;
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     const int P = g.n1m / C;
-    S *sbS = reinterpret_cast<S *>(smem_raw + wid * stage_bytes(g.n1m, C));
-    R *sbR = reinterpret_cast<R *>(sbS);
     const int nrows = g.n2m * g.n3m;
     const R f24 = a.f24x, half = (R)0.5, two = (R)2.0;
     for (int row = blockIdx.x * (TPB / 32) + wid; row < nrows; row += gridDim.x * (TPB / 32)) {
@@ -1401,25 +1397,25 @@ __global__ void __launch_bounds__(TPB) k_les_x2(StepArgs<R> a, LesArgs<R> l) {
         R d[C];
         {   // HH3 -= Dx(tau13)
             R tc[C];
-            srow_load(tc, l.t13 + o, sbR, lane, P);
+            drow_load(tc, l.t13 + o, lane, P);
             R nx = snext(tc[0], lane, P);
 #pragma unroll
             for (int t = 0; t < C; ++t) d[t] = f24 * ((t == C - 1 ? nx : tc[t + 1]) - tc[t]);
             xsolve<32, 22>(d, lane, P, a.c22x);
             R h[C];
-            srow_load(h, a.hh[2] + o, sbR, lane, P);
+            drow_load(h, a.hh[2] + o, lane, P);
 #pragma unroll
             for (int t = 0; t < C; ++t) h[t] = h[t] - d[t];
-            srow_store(a.hh[2] + o, h, sbR, lane, P);
+            drow_store(a.hh[2] + o, h, lane, P);
         }
         S uc[C], um[C];
-        srow_load(uc, a.u + o, sbS, lane, P);
-        srow_load(um, a.u + om, sbS, lane, P);
+        drow_load(uc, a.u + o, lane, P);
+        drow_load(um, a.u + om, lane, P);
         R nxc[C], nxm[C], dvc[C];
-        srow_load(nxc, l.nux + o, sbR, lane, P);
+        drow_load(nxc, l.nux + o, lane, P);
         if (j >= 2) {
-            srow_load(nxm, l.nux + om, sbR, lane, P);
-            srow_load(dvc, l.dvdx + o, sbR, lane, P);
+            drow_load(nxm, l.nux + om, lane, P);
+            drow_load(dvc, l.dvdx + o, lane, P);
         } else {
 #pragma unroll
             for (int t = 0; t < C; ++t) { nxm[t] = R(0); dvc[t] = R(0); }
@@ -1434,41 +1430,41 @@ __global__ void __launch_bounds__(TPB) k_les_x2(StepArgs<R> a, LesArgs<R> l) {
             for (int t = 0; t < C; ++t) d[t] = f24 * ((t == C - 1 ? nx : tau[t + 1]) - tau[t]);
             xsolve<32, 22>(d, lane, P, a.c22x);
             S vc[C], vm[C], vp[C];
-            srow_load(vc, a.v + o, sbS, lane, P);
-            srow_load(vm, a.v + om, sbS, lane, P);
-            srow_load(vp, a.v + op, sbS, lane, P);
+            drow_load(vc, a.v + o, lane, P);
+            drow_load(vm, a.v + om, lane, P);
+            drow_load(vp, a.v + op, lane, P);
             R nc[C], nm[C], h[C];
-            srow_load(nc, l.nu + o, sbR, lane, P);
-            srow_load(nm, l.nu + om, sbR, lane, P);
-            srow_load(h, a.hh[1] + o, sbR, lane, P);
+            drow_load(nc, l.nu + o, lane, P);
+            drow_load(nm, l.nu + om, lane, P);
+            drow_load(h, a.hh[1] + o, lane, P);
             const R rdy = a.m.rdy[j], rdym = a.m.rdy[j - 1];
 #pragma unroll
             for (int t = 0; t < C; ++t) {
                 const R vis22 = rh * (nc[t] * (rdy * ST::d(vp[t], vc[t])) - nm[t] * (rdym * ST::d(vc[t], vm[t])));
                 h[t] = h[t] - d[t] - two * vis22;
             }
-            srow_store(a.hh[1] + o, h, sbR, lane, P);
+            drow_store(a.hh[1] + o, h, lane, P);
         }
         {   // HH1 -= d/dy(nu_xy (du/dy + dv/dx))
             S up[C];
-            srow_load(up, a.u + op, sbS, lane, P);
+            drow_load(up, a.u + op, lane, P);
             R nxp[C], dvp[C], nw[C];
             if (fjup) {
-                srow_load(nxp, l.nux + op, sbR, lane, P);
-                srow_load(dvp, l.dvdx + op, sbR, lane, P);
+                drow_load(nxp, l.nux + op, lane, P);
+                drow_load(dvp, l.dvdx + op, lane, P);
             } else {
 #pragma unroll
                 for (int t = 0; t < C; ++t) { nxp[t] = R(0); dvp[t] = R(0); }
             }
             // wall viscosity (x average of the ghost plane) where the face is a wall
-            if (!fjup || !fjum) srow_load(nw, l.nu + (fjup ? fidx(g, 0, 0, k) : fidx(g, 0, g.n2, k)), sbR, lane, P);
+            if (!fjup || !fjum) drow_load(nw, l.nu + (fjup ? fidx(g, 0, 0, k) : fidx(g, 0, g.n2, k)), lane, P);
             R pw = sprev((!fjup || !fjum) ? nw[C - 1] : R(0), lane, P);
             const R rh = a.m.rh[j], rhp = a.m.rh[j + 1], hd = a.m.hdy[j], hdm = a.m.hdy[j - 1], hdp = a.m.hdy[j + 1];
             const R f2 = (R)(1.0 - l.ifwall * (fjup ? 0.0 : 1.0) * (g.aly - 1.0));
             const R f1 = (R)(1.0 - l.ifwall * (fjum ? 0.0 : 1.0));
             const R rdy = a.m.rdy[j];
             R h[C];
-            srow_load(h, a.hh[0] + o, sbR, lane, P);
+            drow_load(h, a.hh[0] + o, lane, P);
 #pragma unroll
             for (int t = 0; t < C; ++t) {
                 const R wv = (!fjup || !fjum) ? half * (nw[t] + (t == 0 ? pw : nw[t - 1])) : R(0);
@@ -1478,13 +1474,13 @@ __global__ void __launch_bounds__(TPB) k_les_x2(StepArgs<R> a, LesArgs<R> l) {
                 const R uu11 = rh * ST::d(uc[t], um[t]);
                 h[t] = h[t] - rdy * ((f2 * sj2) * (uu22 + dvp[t]) - (f1 * sj1) * (uu11 + dvc[t]));
             }
-            srow_store(a.hh[0] + o, h, sbR, lane, P);
+            drow_store(a.hh[0] + o, h, lane, P);
         }
         if (l.ifwall && (!fjum || !fjup)) {   // wall-stress terms (IFWALL)
             const double rdy1 = 1.0 / g.dy[1], rdyt = 1.0 / g.dy[g.n2m];
             R r0[C], r2[C];
-            srow_load(r0, a.r[0] + o, sbR, lane, P);
-            srow_load(r2, a.r[2] + o, sbR, lane, P);
+            drow_load(r0, a.r[0] + o, lane, P);
+            drow_load(r2, a.r[2] + o, lane, P);
             if (lane < P) {
 #pragma unroll
                 for (int t = 0; t < C; ++t) {
@@ -1497,8 +1493,8 @@ __global__ void __launch_bounds__(TPB) k_les_x2(StepArgs<R> a, LesArgs<R> l) {
                     r2[t] = r2[t] + (R)b3;
                 }
             }
-            srow_store(a.r[0] + o, r0, sbR, lane, P);
-            srow_store(a.r[2] + o, r2, sbR, lane, P);
+            drow_store(a.r[0] + o, r0, lane, P);
+            drow_store(a.r[2] + o, r2, lane, P);
         }
     }
 }
@@ -1509,16 +1505,13 @@ __global__ void __launch_bounds__(TPB) k_les_x2(StepArgs<R> a, LesArgs<R> l) {
 // ---------------------------------------------------------------------------------
 template <typename R, int C>
 static void launch_les_x(c3d_channel *ch, StepArgs<R> &a, LesArgs<R> &l, int which, int *nl) {
-    const size_t sb = (TPB / 32) * stage_bytes(ch->g.n1m, C);
     const int grid = nblk((long long)ch->g.n2m * ch->g.n3m, TPB / 32);
     const double N = (double)ch->g.n1m * ch->g.n2m * ch->g.n3m, Rb = sizeof(R);
     if (which == 0) {
-        cudaFuncSetAttribute(k_les_x1<R, C>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sb);
-        klaunch(ch, ch->stream, k_les_x1<R, C>, grid, TPB, sb, a, l);
+        klaunch(ch, ch->stream, k_les_x1<R, C>, grid, TPB, 0, a, l);
         mark(ch, nl, "les_x1", N * (24 + 6 * Rb));
     } else {
-        cudaFuncSetAttribute(k_les_x2<R, C>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sb);
-        klaunch(ch, ch->stream, k_les_x2<R, C>, grid, TPB, sb, a, l);
+        klaunch(ch, ch->stream, k_les_x2<R, C>, grid, TPB, 0, a, l);
         mark(ch, nl, "les_x2", N * (16 + 14 * Rb));
     }
 }

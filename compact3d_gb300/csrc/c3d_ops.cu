@@ -24,10 +24,7 @@ __global__ void __launch_bounds__(TPB) k_op_x(StepArgs<R> a, int op, const R *in
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     const int P = g.n1m / C;
     const int M = g.n1m / 2;
-    const size_t sbytes = stage_bytes(g.n1m, C), fbytes = 2 * (size_t)(M + 1) * sizeof(C2);
-    unsigned char *wb = smem_raw + wid * (sbytes + fbytes);
-    R *sb = reinterpret_cast<R *>(wb);
-    C2 *bufa = reinterpret_cast<C2 *>(wb + sbytes);
+    C2 *bufa = reinterpret_cast<C2 *>(smem_raw) + wid * 2 * (M + 1);
     C2 *bufb = bufa + (M + 1);
     R *rbuf = reinterpret_cast<R *>(bufa);
     const C2 *twx;
@@ -58,11 +55,11 @@ __global__ void __launch_bounds__(TPB) k_op_x(StepArgs<R> a, int op, const R *in
 #pragma unroll
             for (int t = 0; t < C; ++t) v[t] = lane < P ? rz[lane * C + t] * scale : R(0);
             __syncwarp();
-            srow_store(out + o, v, sb, lane, P);
+            drow_store(out + o, v, lane, P);
             continue;
         }
         R f[C], d[C];
-        srow_load(f, in + o, sb, lane, P);
+        drow_load(f, in + o, lane, P);
         const R pv = sprev(f[C - 1], lane, P), nx = snext(f[0], lane, P);
         if (op == C3D_OP_POISSON) {   // real row -> spectrum (R2C)
             if (lane < P) {
@@ -93,7 +90,7 @@ __global__ void __launch_bounds__(TPB) k_op_x(StepArgs<R> a, int op, const R *in
             else d[t] = (R)4.0 * (f[t] + r);
         }
         xsolve(d, lane, P, *cy);
-        srow_store(out + o, d, sb, lane, P);
+        drow_store(out + o, d, lane, P);
     }
 }
 
@@ -146,7 +143,7 @@ template <typename R, int C>
 static void launch_op_x(c3d_channel *ch, StepArgs<R> &a, int op, const R *in, R *out) {
     typedef typename Cx<R>::T C2;
     const int M = ch->g.n1m / 2;
-    const size_t fb = (stage_bytes(ch->g.n1m, C) + 2 * (size_t)(M + 1) * sizeof(C2)) * (TPB / 32);
+    const size_t fb = 2 * (size_t)(M + 1) * sizeof(C2) * (TPB / 32);
     cudaFuncSetAttribute(k_op_x<R, C>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fb);
     k_op_x<R, C><<<nblk((long long)ch->g.n2m * ch->g.n3m, TPB / 32), TPB, fb, ch->stream>>>(a, op, in, out);
 }

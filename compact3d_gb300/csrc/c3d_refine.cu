@@ -62,11 +62,7 @@ __global__ void __launch_bounds__(TPB) k_ir_x(StepArgs<float> a, RefArgs r) {
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     const int P = g.n1m / C;
     const int M = g.n1m / 2;
-    const size_t sbytes = stage_bytes(g.n1m, C), fbytes = 2 * (size_t)(M + 1) * sizeof(C2);
-    unsigned char *wb = smem_raw + wid * (sbytes + fbytes);
-    float2 *sbS = reinterpret_cast<float2 *>(wb);
-    float *sbR = reinterpret_cast<float *>(wb);
-    C2 *bufa = reinterpret_cast<C2 *>(wb + sbytes);
+    C2 *bufa = reinterpret_cast<C2 *>(smem_raw) + wid * 2 * (M + 1);
     C2 *bufb = bufa + (M + 1);
     float *rbuf = reinterpret_cast<float *>(bufa);
     const C2 *twx = reinterpret_cast<const C2 *>(a.twx32);
@@ -77,7 +73,7 @@ __global__ void __launch_bounds__(TPB) k_ir_x(StepArgs<float> a, RefArgs r) {
         dfl d[C];
         {
             float2 uc[C];
-            srow_load(uc, a.u + o, sbS, lane, P);
+            drow_load(uc, a.u + o, lane, P);
             const float2 nu = snext(uc[0], lane, P);
 #pragma unroll
             for (int t = 0; t < C; ++t) d[t] = r.f24x * (sdf(t == C - 1 ? nu : uc[t + 1]) - sdf(uc[t]));
@@ -88,10 +84,10 @@ __global__ void __launch_bounds__(TPB) k_ir_x(StepArgs<float> a, RefArgs r) {
             const bool up = (j + 1 <= g.n2m), lo = (j >= 2);
             float2 vp[C], vc[C];
             float zh[C], zl[C];
-            if (up) srow_load(vp, a.v + op, sbS, lane, P);
-            if (lo) srow_load(vc, a.v + o, sbS, lane, P);
-            srow_load(zh, r.rzh + o, sbR, lane, P);
-            srow_load(zl, r.rzl + o, sbR, lane, P);
+            if (up) drow_load(vp, a.v + op, lane, P);
+            if (lo) drow_load(vc, a.v + o, lane, P);
+            drow_load(zh, r.rzh + o, lane, P);
+            drow_load(zl, r.rzl + o, lane, P);
             const dfl ry = r.rdy[j];
 #pragma unroll
             for (int t = 0; t < C; ++t) {
@@ -130,10 +126,7 @@ __global__ void __launch_bounds__(TPB) k_ir_d(StepArgs<float> a) {
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     const int P = g.n1m / C;
     const int M = g.n1m / 2;
-    const size_t sbytes = stage_bytes(g.n1m, C), fbytes = 2 * (size_t)(M + 1) * sizeof(C2);
-    unsigned char *wb = smem_raw + wid * (sbytes + fbytes);
-    float *sbR = reinterpret_cast<float *>(wb);
-    C2 *bufa = reinterpret_cast<C2 *>(wb + sbytes);
+    C2 *bufa = reinterpret_cast<C2 *>(smem_raw) + wid * 2 * (M + 1);
     C2 *bufb = bufa + (M + 1);
     const C2 *twx = reinterpret_cast<const C2 *>(a.twx32);
     const float scale = a.xscale, f24 = a.f24x;
@@ -160,12 +153,12 @@ __global__ void __launch_bounds__(TPB) k_ir_d(StepArgs<float> a) {
 #pragma unroll
         for (int t = 0; t < C; ++t) dpv[t] = lane < P ? rz[lane * C + t] * scale : 0.f;
         __syncwarp();
-        srow_store(a.dp + o, dpv, sbR, lane, P);
+        drow_store(a.dp + o, dpv, lane, P);
         const float pv = sprev(dpv[C - 1], lane, P);
 #pragma unroll
         for (int t = 0; t < C; ++t) d[t] = f24 * (dpv[t] - (t == 0 ? pv : dpv[t - 1]));
         xsolve(d, lane, P, a.c22x);
-        srow_store(a.g1 + o, d, sbR, lane, P);
+        drow_store(a.g1 + o, d, lane, P);
     }
 }
 
@@ -224,7 +217,7 @@ __global__ void __launch_bounds__(TPB) k_ir_e(StepArgs<float> a, int updp) {
 template <int C>
 static void launch_ir_x(c3d_channel *ch, StepArgs<float> &a, RefArgs &r, int which) {
     const int M = ch->g.n1m / 2;
-    const size_t fb = (stage_bytes(ch->g.n1m, C) + 2 * (size_t)(M + 1) * sizeof(float2)) * (TPB / 32);
+    const size_t fb = 2 * (size_t)(M + 1) * sizeof(float2) * (TPB / 32);
     const int grid = nblk((long long)ch->g.n2m * ch->g.n3m, TPB / 32);
     if (which == 0) {
         cudaFuncSetAttribute(k_ir_x<C>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fb);

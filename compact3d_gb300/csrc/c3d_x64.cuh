@@ -12,11 +12,11 @@ namespace c3d {
 // J >= 2) or w (PART 3) piece; rows as in xa_piece.
 template <int C, int PART, int W = 32>
 __device__ __forceinline__ void xa64(const StepArgs<double> &a, int j, long long o, long long om, long long op,
-                                     double *sb, int lane, int P) {
+                                     int lane, int P) {
     typedef double D;
     const D RE1 = a.re1, k10 = RE1 * a.f12x * a.c10x.s;
     auto row = [&](D (&v)[C], int r) {
-        srow_load(v, xa_src<false, PART>(a, r, o, om, op, (const D *)nullptr, 0), sb, lane, P);
+        drow_load(v, xa_src<false, PART>(a, r, o, om, op, (const D *)nullptr, 0), lane, P);
     };
     if constexpr (PART == 2) {
         if (j < 2) return;
@@ -33,7 +33,7 @@ __device__ __forceinline__ void xa64(const StepArgs<double> &a, int j, long long
                 const D v2 = vp[t] + vc[t], v1 = vc[t] + vm[t];
                 hh[t] = rq * (v2 * v2 - v1 * v1);
             }
-            srow_store(a.hh[1] + o, hh, sb, lane, P);
+            drow_store(a.hh[1] + o, hh, lane, P);
         }
         {
             D pc[C], pm[C];
@@ -51,7 +51,7 @@ __device__ __forceinline__ void xa64(const StepArgs<double> &a, int j, long long
         xsolve_ring<W, 10>(d, lane, P, a.c10x);
 #pragma unroll
         for (int t = 0; t < C; ++t) acc[t] = acc[t] + k10 * d[t];
-        srow_store(a.r[1] + o, acc, sb, lane, P);
+        drow_store(a.r[1] + o, acc, lane, P);
 #pragma unroll
         for (int t = 0; t < C; ++t) d[t] = (t == 0 ? pv : vc[t - 1]) + vc[t];
         xsolve_ring<W, 6>(d, lane, P, a.c6x);
@@ -63,7 +63,7 @@ __device__ __forceinline__ void xa64(const StepArgs<double> &a, int j, long long
 #pragma unroll
             for (int t = 0; t < C; ++t) d[t] = d[t] * (a1 * um[t] + a2 * uc[t]);
         }
-        srow_store(a.exy + o, d, sb, lane, P);
+        drow_store(a.exy + o, d, lane, P);
     } else {
         // u: the y stencil, the x terms (HH1 stored), -dP/dx; w: the y stencil, the x terms
         constexpr int XC = PART == 1 ? XA_UC : XA_WC, XM = PART == 1 ? XA_UM : XA_WM, XP = PART == 1 ? XA_UP : XA_WP;
@@ -88,11 +88,11 @@ __device__ __forceinline__ void xa64(const StepArgs<double> &a, int j, long long
 #pragma unroll
         for (int t = 0; t < C; ++t) acc[t] = acc[t] + k10 * d[t];
         if constexpr (PART == 3) {
-            srow_store(a.r[2] + o, acc, sb, lane, P);
+            drow_store(a.r[2] + o, acc, lane, P);
 #pragma unroll
             for (int t = 0; t < C; ++t) d[t] = (t == 0 ? pv : xc[t - 1]) + xc[t];
             xsolve_ring<W, 6>(d, lane, P, a.c6x);
-            srow_store(a.ww1 + o, d, sb, lane, P);
+            drow_store(a.ww1 + o, d, lane, P);
         } else {
             const D kp = a.f24x * a.c22x.s, k6 = 4.0 * a.c6x.s, kq = kp * k6 * k6;
 #pragma unroll
@@ -106,7 +106,7 @@ __device__ __forceinline__ void xa64(const StepArgs<double> &a, int j, long long
             xsolve_ring<W, 22>(d, lane, P, a.c22x);
 #pragma unroll
             for (int t = 0; t < C; ++t) d[t] = kq * d[t];
-            srow_store(a.hh[0] + o, d, sb, lane, P);
+            drow_store(a.hh[0] + o, d, lane, P);
             row(xc, XA_PC);
             const D pp = sprev<W>(xc[C - 1], lane, P);
 #pragma unroll
@@ -114,7 +114,7 @@ __device__ __forceinline__ void xa64(const StepArgs<double> &a, int j, long long
             xsolve_ring<W, 22>(d, lane, P, a.c22x);
 #pragma unroll
             for (int t = 0; t < C; ++t) acc[t] = acc[t] - kp * d[t];
-            srow_store(a.r[0] + o, acc, sb, lane, P);
+            drow_store(a.r[0] + o, acc, lane, P);
         }
     }
 }

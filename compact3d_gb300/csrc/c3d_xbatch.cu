@@ -44,22 +44,21 @@ static int xbk(const c3d_channel *ch, int which, int xw, std::vector<BKern> &out
     typedef typename Cx<R>::T C2;
     const int nrows = ch->g.n2m * ch->g.n3m;
     const unsigned nb = (unsigned)nblk(nrows, xw), nt = xw * 32;
-    const size_t sb = stage_bytes(ch->g.n1m, C) * xw;
-    const size_t fb = (stage_bytes(ch->g.n1m, C) + 2 * (size_t)(ch->g.n1m / 2 + 1) * sizeof(C2)) * xw;
+    const size_t fb = 2 * (size_t)(ch->g.n1m / 2 + 1) * sizeof(C2) * xw;
     const bool x4 = (C % 2 == 0) && ch->g.n1m == 32 * C;   // register row FFT (see launch_x_c)
     switch (which) {
         case 0:
-            out.push_back({(const void *)kb_xA<R, C, 1>, nt, sb, nb, 1, 0});
-            out.push_back({(const void *)kb_xA<R, C, 2>, nt, sb, nb, 1, 1});
-            out.push_back({(const void *)kb_xA<R, C, 3>, nt, sb, nb, 1, 2});
+            out.push_back({(const void *)kb_xA<R, C, 1>, nt, 0, nb, 1, 0});
+            out.push_back({(const void *)kb_xA<R, C, 2>, nt, 0, nb, 1, 1});
+            out.push_back({(const void *)kb_xA<R, C, 3>, nt, 0, nb, 1, 2});
             return 0;
-        case 1: out.push_back({(const void *)kb_xB<R, C>, nt, sb, nb}); return 0;
+        case 1: out.push_back({(const void *)kb_xB<R, C>, nt, 0, nb}); return 0;
         case 2:
-            if (x4) out.push_back({(const void *)kb_xC<R, C, (C % 2 == 0)>, nt, sb, nb});
+            if (x4) out.push_back({(const void *)kb_xC<R, C, (C % 2 == 0)>, nt, 0, nb});
             else out.push_back({(const void *)kb_xC<R, C, false>, nt, fb, nb});
             return 0;
         case 3:
-            if (x4) out.push_back({(const void *)kb_xD<R, C, (C % 2 == 0)>, nt, sb, nb});
+            if (x4) out.push_back({(const void *)kb_xD<R, C, (C % 2 == 0)>, nt, 0, nb});
             else out.push_back({(const void *)kb_xD<R, C, false>, nt, fb, nb});
             return 0;
         default: return C3D_EINVAL;
@@ -77,8 +76,8 @@ static int xbk_seg(const c3d_channel *ch, int which, int xw, std::vector<BKern> 
     typedef typename Cx<R>::T C2;
     const int nrows = ch->g.n2m * ch->g.n3m, rpb = xw * 32 / W;
     const unsigned nb = (unsigned)nblk(nrows, rpb), nt = xw * 32;
-    // xC and xD: a stage and the two FFT buffers per row segment
-    const size_t fb = (stage_bytes(ch->g.n1m, C) + 2 * (size_t)(ch->g.n1m / 2 + 1) * sizeof(C2)) * rpb;
+    // xC and xD: the two FFT buffers per row segment
+    const size_t fb = 2 * (size_t)(ch->g.n1m / 2 + 1) * sizeof(C2) * rpb;
     switch (which) {
         case 0:
             out.push_back({(const void *)kb_xA<R, C, 1, W>, nt, 0, nb, 1, 0});

@@ -84,15 +84,15 @@ static int launch_x_c(c3d_channel *ch, StepArgs<R> &a, int which, const R *p0, c
     const int grid = nblk(nrows, xw), nt = xw * 32;
     cudaStream_t st = ch->stream;
     const double N = (double)ch->g.n1m * ch->g.n2m * ch->g.n3m, Rb = sizeof(R);
-    const size_t sb = stage_bytes(ch->g.n1m, C) * xw;
     const int M = ch->g.n1m / 2;
-    const size_t fb = (stage_bytes(ch->g.n1m, C) + 2 * (size_t)(M + 1) * sizeof(C2)) * xw;
+    const size_t fb = 2 * (size_t)(M + 1) * sizeof(C2) * xw;
     switch (which) {
         case 0:
             // FP64 reads its rows from global memory in every schedule: its pipe is 84% busy, DRAM 7%
             if constexpr (sizeof(R) == 4) {
                 if (ch->tune.xsplit && ch->tune.xstage && ch->g.n1m % 2 == 0) {
-                    // the pieces with their rows staged by bulk copies (rows of 16-byte multiples)
+                    // the pieces with their rows staged by bulk copies (rows of 16-byte multiples;
+                    // eight warps of N1M = 384 take 74 KB)
                     const size_t s1 = xa_stage_bytes(ch->g.n1m) * xw;
                     cudaFuncSetAttribute(k_xAs<R, C, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)s1);
                     cudaFuncSetAttribute(k_xAs<R, C, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)s1);
@@ -110,27 +110,22 @@ static int launch_x_c(c3d_channel *ch, StepArgs<R> &a, int which, const R *p0, c
                 }
             }
             if (ch->tune.xsplit) {   // the u, v and w pieces as three kernels
-                cudaFuncSetAttribute(k_xA<R, C, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sb);
-                cudaFuncSetAttribute(k_xA<R, C, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sb);
-                cudaFuncSetAttribute(k_xA<R, C, 3>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sb);
                 const bool cc = par_on(ch);
                 if (cc && (rc = par_fork(ch))) return rc;
-                klaunch(ch, cc ? ch->par[0] : st, k_xA<R, C, 1>, grid, nt, sb, a);
+                klaunch(ch, cc ? ch->par[0] : st, k_xA<R, C, 1>, grid, nt, 0, a);
                 mark(ch, nl, "xA_u", N * (16 + 2 * Rb));   // u, P; R1, HH1
-                klaunch(ch, cc ? ch->par[1] : st, k_xA<R, C, 2>, grid, nt, sb, a);
+                klaunch(ch, cc ? ch->par[1] : st, k_xA<R, C, 2>, grid, nt, 0, a);
                 mark(ch, nl, "xA_v", N * (24 + 3 * Rb));   // v, P, u; R2, HH2, E_xy
-                klaunch(ch, st, k_xA<R, C, 3>, grid, nt, sb, a);
+                klaunch(ch, st, k_xA<R, C, 3>, grid, nt, 0, a);
                 mark(ch, nl, "xA_w", N * (8 + 2 * Rb));    // w; R3, WW1
                 if (cc && (rc = par_join(ch))) return rc;
                 break;
             }
-            cudaFuncSetAttribute(k_xA<R, C, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sb);
-            klaunch(ch, st, k_xA<R, C, 0>, grid, nt, sb, a);
+            klaunch(ch, st, k_xA<R, C, 0>, grid, nt, 0, a);
             mark(ch, nl, "xA", N * (32 + 7 * Rb));
             break;
         case 1:
-            cudaFuncSetAttribute(k_xB<R, C>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sb);
-            klaunch(ch, st, k_xB<R, C>, grid, nt, sb, a);
+            klaunch(ch, st, k_xB<R, C>, grid, nt, 0, a);
             mark(ch, nl, "xB", N * 18 * Rb);
             break;
         case 2: {
@@ -147,7 +142,7 @@ static int launch_x_c(c3d_channel *ch, StepArgs<R> &a, int which, const R *p0, c
             }
             // register row FFT (all 32 lanes hold a chunk: N1M = 32 C, C even): no shared memory
             if (!done && C % 2 == 0 && ch->tune.fxp == 3 && ch->g.n1m == 32 * C) {
-                klaunch(ch, st, k_xC<R, C, 0, (C % 2 == 0)>, grid, nt, sb, a, p0, p1);
+                klaunch(ch, st, k_xC<R, C, 0, (C % 2 == 0)>, grid, nt, 0, a, p0, p1);
                 done = true;
             }
             if (!done) {
@@ -159,7 +154,7 @@ static int launch_x_c(c3d_channel *ch, StepArgs<R> &a, int which, const R *p0, c
         }
         case 3:
             if (C % 2 == 0 && ch->tune.fxp == 3 && ch->g.n1m == 32 * C) {
-                klaunch(ch, st, k_xD<R, C, (C % 2 == 0)>, grid, nt, sb, a, p0, p1);
+                klaunch(ch, st, k_xD<R, C, (C % 2 == 0)>, grid, nt, 0, a, p0, p1);
             } else {
                 cudaFuncSetAttribute(k_xD<R, C>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fb);
                 klaunch(ch, st, k_xD<R, C>, grid, nt, fb, a, p0, p1);
@@ -169,8 +164,7 @@ static int launch_x_c(c3d_channel *ch, StepArgs<R> &a, int which, const R *p0, c
         case 4: {
             const double b = 22.0, r = -2.0 / (b + sqrt(b * b - 4.0));
             Cyc<double> c22 = {r, -r, (int)ceil(log(1e-17) / log(fabs(r)))};
-            cudaFuncSetAttribute(k_diag_x<R, C>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sb);
-            klaunch(ch, st, k_diag_x<R, C>, grid, TPB, sb, a, (double *)p0, c22);
+            klaunch(ch, st, k_diag_x<R, C>, grid, TPB, 0, a, (double *)p0, c22);
             mark(ch, nl, "diag_x", N * 48);
             break;
         }
@@ -197,7 +191,7 @@ static int launch_x_seg(c3d_channel *ch, StepArgs<R> &a, int which, const R *p0,
     const int rpb = xw * 32 / W;
     const int grid = nblk(nrows, rpb), nt = xw * 32;
     const double N = (double)ch->g.n1m * ch->g.n2m * ch->g.n3m, Rb = sizeof(R);
-    const size_t fb = (stage_bytes(ch->g.n1m, C) + 2 * (size_t)(ch->g.n1m / 2 + 1) * sizeof(C2)) * rpb;
+    const size_t fb = 2 * (size_t)(ch->g.n1m / 2 + 1) * sizeof(C2) * rpb;
     cudaStream_t st = ch->stream;
     if (which == 2) {
         cudaFuncSetAttribute(k_xC<R, C, 0, false, W>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fb);
@@ -239,12 +233,6 @@ static int launch_x_seg(c3d_channel *ch, StepArgs<R> &a, int which, const R *p0,
 template <typename R>
 int launch_xpass(c3d_channel *ch, StepArgs<R> &a, int which, const R *p0, const R *p1, int *nl) {
     const Tune &t = ch->tune;
-    // rows that seven slots a warp (the v piece's rows) would not hold
-    if (which == 0 && t.xsplit && t.xstage && ch->g.n1m % 2 == 0 &&
-        (16 + 7 * (size_t)ch->g.n1m * 8) * t.xw > 227 * 1024) {
-        set_error("xA stage exceeds shared memory");
-        return C3D_EINVAL;
-    }
     if constexpr (sizeof(R) == 8) {
         // FP64, whatever the schedule's row lanes: segments that have no idle lanes and more
         // points per lane than a warp would (the carries of a solve cost 2 instructions per

@@ -54,9 +54,9 @@ __device__ __forceinline__ const typename SType<R>::S *xa_src(const StepArgs<R> 
 // Row operand of an x pass: a global row (read through the read-only path) or a row
 // already staged in shared memory by bulk copies.
 template <bool STG, typename T, int C>
-__device__ __forceinline__ void xrow(T (&v)[C], const T *p, T *sb, int lane, int P) {
+__device__ __forceinline__ void xrow(T (&v)[C], const T *p, int lane, int P) {
     if constexpr (STG) crow_load(v, p, lane, P);
-    else srow_load(v, p, sb, lane, P);
+    else drow_load(v, p, lane, P);
 }
 
 }  // namespace c3d
@@ -67,7 +67,7 @@ namespace c3d {
 // the mixed form.
 template <typename R, int C, int PART, bool STG, int W = 32>
 __device__ __forceinline__ void xa_piece32(const StepArgs<R> &a, int j, long long o, long long om, long long op,
-                                         typename SType<R>::S *st, typename SType<R>::S *sbS, R *sbR, int lane, int P,
+                                         typename SType<R>::S *st, int lane, int P,
                                          uint64_t *bar) {
     typedef typename SType<R>::S S;
     typedef St<R> ST;
@@ -110,9 +110,9 @@ __device__ __forceinline__ void xa_piece32(const StepArgs<R> &a, int j, long lon
         R acc[C];
         {
             S vc[C], vm[C], vp[C];
-            xrow<STG>(vc, xa_src<STG, PART>(a, XA_VC, o, om, op, st, n), sbS, lane, P);
-            xrow<STG>(vm, xa_src<STG, PART>(a, XA_VM, o, om, op, st, n), sbS, lane, P);
-            xrow<STG>(vp, xa_src<STG, PART>(a, XA_VP, o, om, op, st, n), sbS, lane, P);
+            xrow<STG>(vc, xa_src<STG, PART>(a, XA_VC, o, om, op, st, n), lane, P);
+            xrow<STG>(vm, xa_src<STG, PART>(a, XA_VM, o, om, op, st, n), lane, P);
+            xrow<STG>(vp, xa_src<STG, PART>(a, XA_VP, o, om, op, st, n), lane, P);
             R hh[C];
 #pragma unroll
             for (int t = 0; t < C; ++t) {
@@ -120,13 +120,13 @@ __device__ __forceinline__ void xa_piece32(const StepArgs<R> &a, int j, long lon
                 hh[t] = Hj1 * Sten<R>::vv(vp[t], vc[t], vm[t]);
             }
             refill(XA_PM, XA_PC);
-            srow_store(a.hh[1] + o, hh, sbR, lane, P);
+            drow_store(a.hh[1] + o, hh, lane, P);
         }
         if (!ready(1)) return;
         {
             S pc[C], pm[C];
-            xrow<STG>(pc, xa_src<STG, PART>(a, XA_PC, o, om, op, st, n), sbS, lane, P);
-            xrow<STG>(pm, xa_src<STG, PART>(a, XA_PM, o, om, op, st, n), sbS, lane, P);
+            xrow<STG>(pc, xa_src<STG, PART>(a, XA_PC, o, om, op, st, n), lane, P);
+            xrow<STG>(pm, xa_src<STG, PART>(a, XA_PM, o, om, op, st, n), lane, P);
 #pragma unroll
             for (int t = 0; t < C; ++t) {
                 R pg = ST::d(pc[t], pm[t]) * Hj1;
@@ -135,7 +135,7 @@ __device__ __forceinline__ void xa_piece32(const StepArgs<R> &a, int j, long lon
         }
         refill(XA_UM, XA_UC);
         S vc[C];
-        xrow<STG>(vc, xa_src<STG, PART>(a, XA_VC, o, om, op, st, n), sbS, lane, P);
+        xrow<STG>(vc, xa_src<STG, PART>(a, XA_VC, o, om, op, st, n), lane, P);
         R d[C];
         S pv = sprev<W>(vc[C - 1], lane, P), nx = snext<W>(vc[0], lane, P);
 #pragma unroll
@@ -146,7 +146,7 @@ __device__ __forceinline__ void xa_piece32(const StepArgs<R> &a, int j, long lon
         xsolve_f<W, 10>(d, lane, P, a.c10x);
 #pragma unroll
         for (int t = 0; t < C; ++t) acc[t] = acc[t] + RE1 * d[t];
-        srow_store(a.r[1] + o, acc, sbR, lane, P);
+        drow_store(a.r[1] + o, acc, lane, P);
 #pragma unroll
         for (int t = 0; t < C; ++t) {
             S l = (t == 0) ? pv : vc[t - 1];
@@ -156,13 +156,13 @@ __device__ __forceinline__ void xa_piece32(const StepArgs<R> &a, int j, long lon
         if (!ready(0)) return;
         {   // u at the y faces
             S uc[C], um[C];
-            xrow<STG>(uc, xa_src<STG, PART>(a, XA_UC, o, om, op, st, n), sbS, lane, P);
-            xrow<STG>(um, xa_src<STG, PART>(a, XA_UM, o, om, op, st, n), sbS, lane, P);
+            xrow<STG>(uc, xa_src<STG, PART>(a, XA_UC, o, om, op, st, n), lane, P);
+            xrow<STG>(um, xa_src<STG, PART>(a, XA_UM, o, om, op, st, n), lane, P);
             const R a1 = a.m.hdy[j], a2 = a.m.hdy[j - 1];
 #pragma unroll
             for (int t = 0; t < C; ++t) d[t] = d[t] * (Hj1 * (a1 * ST::hi(um[t]) + a2 * ST::hi(uc[t])));
         }
-        srow_store(a.exy + o, d, sbR, lane, P);
+        drow_store(a.exy + o, d, lane, P);
     }
     if (PART == 1) {
         // The u piece on its own, ordered so that few rows are live at once: the y
@@ -171,15 +171,15 @@ __device__ __forceinline__ void xa_piece32(const StepArgs<R> &a, int j, long lon
         R acc[C];
         {
             S um[C], up[C], uc0[C];
-            xrow<STG>(uc0, xa_src<STG, PART>(a, XA_UC, o, om, op, st, n), sbS, lane, P);
-            xrow<STG>(um, xa_src<STG, PART>(a, XA_UM, o, om, op, st, n), sbS, lane, P);
-            xrow<STG>(up, xa_src<STG, PART>(a, XA_UP, o, om, op, st, n), sbS, lane, P);
+            xrow<STG>(uc0, xa_src<STG, PART>(a, XA_UC, o, om, op, st, n), lane, P);
+            xrow<STG>(um, xa_src<STG, PART>(a, XA_UM, o, om, op, st, n), lane, P);
+            xrow<STG>(up, xa_src<STG, PART>(a, XA_UP, o, om, op, st, n), lane, P);
 #pragma unroll
             for (int t = 0; t < C; ++t) acc[t] = RE1 * ST::yvisc(HPj, HCj, HMj, Z0, up[t], uc0[t], um[t]);
         }
         refill(XA_PC, XA_PC);
         S uc[C];
-        xrow<STG>(uc, xa_src<STG, PART>(a, XA_UC, o, om, op, st, n), sbS, lane, P);
+        xrow<STG>(uc, xa_src<STG, PART>(a, XA_UC, o, om, op, st, n), lane, P);
         R d[C];
         S pv = sprev<W>(uc[C - 1], lane, P), nx = snext<W>(uc[0], lane, P);
 #pragma unroll
@@ -206,11 +206,11 @@ __device__ __forceinline__ void xa_piece32(const StepArgs<R> &a, int j, long lon
             d[t] = f24 * (sq[t] - l);
         }
         xsolve_f<W, 22>(d, lane, P, a.c22x);
-        srow_store(a.hh[0] + o, d, sbR, lane, P);
+        drow_store(a.hh[0] + o, d, lane, P);
         if (!ready(1)) return;
         {
             S pc[C];
-            xrow<STG>(pc, xa_src<STG, PART>(a, XA_PC, o, om, op, st, n), sbS, lane, P);
+            xrow<STG>(pc, xa_src<STG, PART>(a, XA_PC, o, om, op, st, n), lane, P);
             S pp = sprev<W>(pc[C - 1], lane, P);
 #pragma unroll
             for (int t = 0; t < C; ++t) {
@@ -221,7 +221,7 @@ __device__ __forceinline__ void xa_piece32(const StepArgs<R> &a, int j, long lon
         xsolve_f<W, 22>(d, lane, P, a.c22x);
 #pragma unroll
         for (int t = 0; t < C; ++t) acc[t] = acc[t] - d[t] - presg;
-        srow_store(a.r[0] + o, acc, sbR, lane, P);
+        drow_store(a.r[0] + o, acc, lane, P);
     }
     if (PART == 3) {
         // The w piece on its own: the y stencil first, then the x terms.
@@ -229,14 +229,14 @@ __device__ __forceinline__ void xa_piece32(const StepArgs<R> &a, int j, long lon
         R acc[C];
         {
             S wm[C], wp[C], wc0[C];
-            xrow<STG>(wc0, xa_src<STG, PART>(a, XA_WC, o, om, op, st, n), sbS, lane, P);
-            xrow<STG>(wm, xa_src<STG, PART>(a, XA_WM, o, om, op, st, n), sbS, lane, P);
-            xrow<STG>(wp, xa_src<STG, PART>(a, XA_WP, o, om, op, st, n), sbS, lane, P);
+            xrow<STG>(wc0, xa_src<STG, PART>(a, XA_WC, o, om, op, st, n), lane, P);
+            xrow<STG>(wm, xa_src<STG, PART>(a, XA_WM, o, om, op, st, n), lane, P);
+            xrow<STG>(wp, xa_src<STG, PART>(a, XA_WP, o, om, op, st, n), lane, P);
 #pragma unroll
             for (int t = 0; t < C; ++t) acc[t] = RE1 * ST::yvisc(HPj, HCj, HMj, Z0, wp[t], wc0[t], wm[t]);
         }
         S wc[C];
-        xrow<STG>(wc, xa_src<STG, PART>(a, XA_WC, o, om, op, st, n), sbS, lane, P);
+        xrow<STG>(wc, xa_src<STG, PART>(a, XA_WC, o, om, op, st, n), lane, P);
         R d[C];
         S pv = sprev<W>(wc[C - 1], lane, P), nx = snext<W>(wc[0], lane, P);
 #pragma unroll
@@ -247,23 +247,23 @@ __device__ __forceinline__ void xa_piece32(const StepArgs<R> &a, int j, long lon
         xsolve_f<W, 10>(d, lane, P, a.c10x);
 #pragma unroll
         for (int t = 0; t < C; ++t) acc[t] = acc[t] + RE1 * d[t];
-        srow_store(a.r[2] + o, acc, sbR, lane, P);
+        drow_store(a.r[2] + o, acc, lane, P);
 #pragma unroll
         for (int t = 0; t < C; ++t) {
             S l = (t == 0) ? pv : wc[t - 1];
             d[t] = four * (ST::hi(l) + ST::hi(wc[t]));
         }
         xsolve_f<W, 6>(d, lane, P, a.c6x);
-        srow_store(a.ww1 + o, d, sbR, lane, P);
+        drow_store(a.ww1 + o, d, lane, P);
     }
 }
 
 template <typename R, int C, int PART, bool STG, int W = 32>
 __device__ __forceinline__ void xa_piece(const StepArgs<R> &a, int j, long long o, long long om, long long op,
-                                         typename SType<R>::S *st, typename SType<R>::S *sbS, R *sbR, int lane, int P,
+                                         typename SType<R>::S *st, int lane, int P,
                                          uint64_t *bar = nullptr) {
-    if constexpr (sizeof(R) == 8) xa64<C, PART, W>(a, j, o, om, op, sbR, lane, P);
-    else xa_piece32<R, C, PART, STG, W>(a, j, o, om, op, st, sbS, sbR, lane, P, bar);
+    if constexpr (sizeof(R) == 8) xa64<C, PART, W>(a, j, o, om, op, lane, P);
+    else xa_piece32<R, C, PART, STG, W>(a, j, o, om, op, st, lane, P, bar);
 }
 
 // PART 0 computes the u, v and w pieces in one kernel (FP64: one after another); PART 1, 2, 3 compute one of them
@@ -275,13 +275,9 @@ template <typename R, int C, int PART, int W = 32>
 __device__ __forceinline__ void b_xA(const StepArgs<R> &a, const Blk blk) {
     typedef typename SType<R>::S S;
     typedef St<R> ST;
-    static_assert(W == 32 || !C3D_STAGED_ROWS, "rows staged per warp need one row per warp");
-    extern __shared__ __align__(16) unsigned char smem_raw[];
     const Geo g = a.g;
     const int lane = threadIdx.x & (W - 1), wid = threadIdx.x / W, rpb = (int)blockDim.x / W;
     const int P = g.n1m / C;
-    S *sbS = reinterpret_cast<S *>(smem_raw + wid * stage_bytes(g.n1m, C));
-    R *sbR = reinterpret_cast<R *>(sbS);
     const int nrows = g.n2m * g.n3m;
     const R RE1 = a.re1, f12 = a.f12x, f24 = a.f24x, four = (R)4.0;
     const R presg = (R)a.scal[SCAL_PRESG];
@@ -300,19 +296,19 @@ __device__ __forceinline__ void b_xA(const StepArgs<R> &a, const Blk blk) {
         }
         R uy[C];
         if (PART >= 1) {
-            xa_piece<R, C, PART, false, W>(a, j, o, om, op, nullptr, sbS, sbR, lane, P);
+            xa_piece<R, C, PART, false, W>(a, j, o, om, op, nullptr, lane, P);
         } else if constexpr (sizeof(R) == 8) {
-            xa_piece<R, C, 1, false, W>(a, j, o, om, op, nullptr, sbS, sbR, lane, P);
-            xa_piece<R, C, 2, false, W>(a, j, o, om, op, nullptr, sbS, sbR, lane, P);
-            xa_piece<R, C, 3, false, W>(a, j, o, om, op, nullptr, sbS, sbR, lane, P);
+            xa_piece<R, C, 1, false, W>(a, j, o, om, op, nullptr, lane, P);
+            xa_piece<R, C, 2, false, W>(a, j, o, om, op, nullptr, lane, P);
+            xa_piece<R, C, 3, false, W>(a, j, o, om, op, nullptr, lane, P);
             continue;
         }
         // ---- u: R1 = visc_y + visc_x/RE - dP/dx - PRESG ; HH1 = d(uu)/dx ----
         if (PART == 0 && sizeof(R) == 4) {
             S uc[C], um[C], up[C];
-            srow_load(uc, a.u + o, sbS, lane, P);
-            srow_load(um, a.u + om, sbS, lane, P);
-            srow_load(up, a.u + op, sbS, lane, P);
+            drow_load(uc, a.u + o, lane, P);
+            drow_load(um, a.u + om, lane, P);
+            drow_load(up, a.u + op, lane, P);
             const R HPj = a.m.hp[j], HCj = a.m.hc[j], HMj = a.m.hm[j], Z0 = a.m.hz[j];
             R acc[C], d[C];
             S pv = sprev<W>(uc[C - 1], lane, P), nx = snext<W>(uc[0], lane, P);
@@ -326,7 +322,7 @@ __device__ __forceinline__ void b_xA(const StepArgs<R> &a, const Blk blk) {
             for (int t = 0; t < C; ++t) acc[t] = RE1 * ST::yvisc(HPj, HCj, HMj, Z0, up[t], uc[t], um[t]) + RE1 * d[t];
             {
                 S pc[C];
-                srow_load(pc, a.p + o, sbS, lane, P);
+                drow_load(pc, a.p + o, lane, P);
                 S pp = sprev<W>(pc[C - 1], lane, P);
 #pragma unroll
                 for (int t = 0; t < C; ++t) {
@@ -336,7 +332,7 @@ __device__ __forceinline__ void b_xA(const StepArgs<R> &a, const Blk blk) {
                 xsolve_f<W, 22>(d, lane, P, a.c22x);
 #pragma unroll
                 for (int t = 0; t < C; ++t) acc[t] = acc[t] - d[t] - presg;
-                srow_store(a.r[0] + o, acc, sbR, lane, P);
+                drow_store(a.r[0] + o, acc, lane, P);
             }
 #pragma unroll
             for (int t = 0; t < C; ++t) {
@@ -354,7 +350,7 @@ __device__ __forceinline__ void b_xA(const StepArgs<R> &a, const Blk blk) {
                 d[t] = f24 * (sq[t] - l);
             }
             xsolve_f<W, 22>(d, lane, P, a.c22x);
-            srow_store(a.hh[0] + o, d, sbR, lane, P);
+            drow_store(a.hh[0] + o, d, lane, P);
             if (PART == 0 && j >= 2) {
                 const R Hj1 = a.m.rh[j], a1 = a.m.hdy[j], a2 = a.m.hdy[j - 1];
 #pragma unroll
@@ -364,9 +360,9 @@ __device__ __forceinline__ void b_xA(const StepArgs<R> &a, const Blk blk) {
         // ---- v (faces J=2..N2M): R2, HH2 = d(vv)/dy, E_xy = VV1 * UY ----
         if (PART == 0 && sizeof(R) == 4 && j >= 2) {
             S vc[C], vm[C], vp[C];
-            srow_load(vc, a.v + o, sbS, lane, P);
-            srow_load(vm, a.v + om, sbS, lane, P);
-            srow_load(vp, a.v + op, sbS, lane, P);
+            drow_load(vc, a.v + o, lane, P);
+            drow_load(vm, a.v + om, lane, P);
+            drow_load(vp, a.v + op, lane, P);
             R d[C], acc[C], hh[C];
             S pv = sprev<W>(vc[C - 1], lane, P), nx = snext<W>(vc[0], lane, P);
 #pragma unroll
@@ -379,8 +375,8 @@ __device__ __forceinline__ void b_xA(const StepArgs<R> &a, const Blk blk) {
             const R Hj = a.m.h[j], Hj1 = a.m.rh[j];
             {
                 S pc[C], pm[C];
-                srow_load(pc, a.p + o, sbS, lane, P);
-                srow_load(pm, a.p + om, sbS, lane, P);
+                drow_load(pc, a.p + o, lane, P);
+                drow_load(pm, a.p + om, lane, P);
 #pragma unroll
                 for (int t = 0; t < C; ++t) {
                     R visc = RE1 * ST::yvisc(DYPj, DYCj, DYMj, Z0, vp[t], vc[t], vm[t]);
@@ -389,8 +385,8 @@ __device__ __forceinline__ void b_xA(const StepArgs<R> &a, const Blk blk) {
                     hh[t] = Hj1 * Sten<R>::vv(vp[t], vc[t], vm[t]);
                 }
             }
-            srow_store(a.r[1] + o, acc, sbR, lane, P);
-            srow_store(a.hh[1] + o, hh, sbR, lane, P);
+            drow_store(a.r[1] + o, acc, lane, P);
+            drow_store(a.hh[1] + o, hh, lane, P);
 #pragma unroll
             for (int t = 0; t < C; ++t) {
                 S l = (t == 0) ? pv : vc[t - 1];
@@ -399,14 +395,14 @@ __device__ __forceinline__ void b_xA(const StepArgs<R> &a, const Blk blk) {
             xsolve_f<W, 6>(d, lane, P, a.c6x);
 #pragma unroll
             for (int t = 0; t < C; ++t) d[t] = d[t] * uy[t];
-            srow_store(a.exy + o, d, sbR, lane, P);
+            drow_store(a.exy + o, d, lane, P);
         }
         // ---- w: R3 = visc_y + visc_x/RE ; WW1 = w at x faces ----
         if (PART == 0 && sizeof(R) == 4) {
             S wc[C], wm[C], wp[C];
-            srow_load(wc, a.w + o, sbS, lane, P);
-            srow_load(wm, a.w + om, sbS, lane, P);
-            srow_load(wp, a.w + op, sbS, lane, P);
+            drow_load(wc, a.w + o, lane, P);
+            drow_load(wm, a.w + om, lane, P);
+            drow_load(wp, a.w + op, lane, P);
             R d[C], acc[C];
             S pv = sprev<W>(wc[C - 1], lane, P), nx = snext<W>(wc[0], lane, P);
 #pragma unroll
@@ -418,14 +414,14 @@ __device__ __forceinline__ void b_xA(const StepArgs<R> &a, const Blk blk) {
             const R HPj = a.m.hp[j], HCj = a.m.hc[j], HMj = a.m.hm[j], Z0 = a.m.hz[j];
 #pragma unroll
             for (int t = 0; t < C; ++t) acc[t] = RE1 * ST::yvisc(HPj, HCj, HMj, Z0, wp[t], wc[t], wm[t]) + RE1 * d[t];
-            srow_store(a.r[2] + o, acc, sbR, lane, P);
+            drow_store(a.r[2] + o, acc, lane, P);
 #pragma unroll
             for (int t = 0; t < C; ++t) {
                 S l = (t == 0) ? pv : wc[t - 1];
                 d[t] = four * (ST::hi(l) + ST::hi(wc[t]));
             }
             xsolve_f<W, 6>(d, lane, P, a.c6x);
-            srow_store(a.ww1 + o, d, sbR, lane, P);
+            drow_store(a.ww1 + o, d, lane, P);
         }
     }
 }
@@ -489,22 +485,21 @@ __global__ void __launch_bounds__(XMAXT, 3) k_xAs(StepArgs<R> a) {
         pf_row(a.u + o, (int)rb, lane, 32);
     }
     __syncwarp();
-    xa_piece<R, C, PART, true>(a, j, o, om, op, st, nullptr, nullptr, lane, P, bar);
+    xa_piece<R, C, PART, true>(a, j, o, om, op, st, lane, P, bar);
 }
 
 // ---------------------------------------------------------------------------------
 // xB: remaining convective terms, AB2, x factor of Crank-Nicolson
 // ---------------------------------------------------------------------------------
 template <typename R, int C, int W = 32>
-__device__ __forceinline__ void ab2_cnx(const StepArgs<R> &a, int c, long long o, const R (&hc)[C], R *sb,
-                                        int lane, int P, R dt) {
+__device__ __forceinline__ void ab2_cnx(const StepArgs<R> &a, int c, long long o, const R (&hc)[C], int lane, int P, R dt) {
     // FP64: (1,10,1)/(A,B,A) = (1 + (10 - B/A) z / (1 + B/A z + z^2)) / A with the factors kx,
     // unless B/A is so far from 10 that the two terms would cancel (cn_factors)
     const bool pf = sizeof(R) == 8 && a.kx[0] != R(0);
     const R dts = pf ? dt * a.kx[0] : xfold(dt, a.cnx);
     R rr[C], ho[C], d[C];
-    srow_load(rr, a.r[c] + o, sb, lane, P);
-    srow_load(ho, a.ho[c] + o, sb, lane, P);
+    drow_load(rr, a.r[c] + o, lane, P);
+    drow_load(ho, a.ho[c] + o, lane, P);
 #pragma unroll
     for (int t = 0; t < C; ++t) rr[t] = (rr[t] - (R)1.5 * hc[t] + (R)0.5 * ho[t]) * dts;
     if (pf) {
@@ -523,17 +518,14 @@ __device__ __forceinline__ void ab2_cnx(const StepArgs<R> &a, int c, long long o
 #pragma unroll
         for (int t = 0; t < C; ++t) d[t] = rr[t] + a.kx[1] * d[t];
     }
-    srow_store(a.r[c] + o, d, sb, lane, P);
+    drow_store(a.r[c] + o, d, lane, P);
 }
 
 template <typename R, int C, int W = 32>
 __device__ __forceinline__ void b_xB(const StepArgs<R> &a, const Blk blk) {
-    static_assert(W == 32 || !C3D_STAGED_ROWS, "rows staged per warp need one row per warp");
-    extern __shared__ __align__(16) unsigned char smem_raw[];
     const Geo g = a.g;
     const int lane = threadIdx.x & (W - 1), wid = threadIdx.x / W, rpb = (int)blockDim.x / W;
     const int P = g.n1m / C;
-    R *sb = reinterpret_cast<R *>(smem_raw + wid * stage_bytes(g.n1m, C));
     const int nrows = g.n2m * g.n3m;
     // FP64: plain differences into the solves, their factor in the sum after them
     const R f = sizeof(R) == 8 ? R(1) : a.f24x, fo = sizeof(R) == 8 ? xfold(a.f24x, a.c22x) : R(1);
@@ -550,26 +542,26 @@ __device__ __forceinline__ void b_xB(const StepArgs<R> &a, const Blk blk) {
         }
         const R rdy = a.m.rdy[j];
         R h1[C], h3[C], e[C], ep[C], d[C];
-        srow_load(h1, a.hh[0] + o, sb, lane, P);
-        srow_load(h3, a.hh[2] + o, sb, lane, P);
+        drow_load(h1, a.hh[0] + o, lane, P);
+        drow_load(h3, a.hh[2] + o, lane, P);
         // E_xy at faces j and j+1 (zero on the walls)
-        if (j >= 2) srow_load(e, a.exy + o, sb, lane, P);
+        if (j >= 2) drow_load(e, a.exy + o, lane, P);
         else {
 #pragma unroll
             for (int t = 0; t < C; ++t) e[t] = R(0);
         }
-        if (j + 1 <= g.n2m) srow_load(ep, a.exy + op, sb, lane, P);
+        if (j + 1 <= g.n2m) drow_load(ep, a.exy + op, lane, P);
         else {
 #pragma unroll
             for (int t = 0; t < C; ++t) ep[t] = R(0);
         }
 #pragma unroll
         for (int t = 0; t < C; ++t) h1[t] = h1[t] + rdy * (ep[t] - e[t]);   // d(uv)/dy
-        srow_store(a.hh[0] + o, h1, sb, lane, P);
-        ab2_cnx<R, C, W>(a, 0, o, h1, sb, lane, P, dt);
+        drow_store(a.hh[0] + o, h1, lane, P);
+        ab2_cnx<R, C, W>(a, 0, o, h1, lane, P, dt);
         if (j >= 2) {
             R h2[C];
-            srow_load(h2, a.hh[1] + o, sb, lane, P);
+            drow_load(h2, a.hh[1] + o, lane, P);
             R nx = snext<W>(e[0], lane, P);
 #pragma unroll
             for (int t = 0; t < C; ++t) {
@@ -579,11 +571,11 @@ __device__ __forceinline__ void b_xB(const StepArgs<R> &a, const Blk blk) {
             xsolve_f<W, 22>(d, lane, P, a.c22x);
 #pragma unroll
             for (int t = 0; t < C; ++t) h2[t] = h2[t] + (sizeof(R) == 8 ? fo * d[t] : d[t]);                 // d(uv)/dx
-            srow_store(a.hh[1] + o, h2, sb, lane, P);
-            ab2_cnx<R, C, W>(a, 1, o, h2, sb, lane, P, dt);
+            drow_store(a.hh[1] + o, h2, lane, P);
+            ab2_cnx<R, C, W>(a, 1, o, h2, lane, P, dt);
         }
         // d(uw)/dx from E_xz, d(wv)/dy from E_yz at faces j, j+1
-        srow_load(e, a.exz + o, sb, lane, P);
+        drow_load(e, a.exz + o, lane, P);
         {
             R nx = snext<W>(e[0], lane, P);
 #pragma unroll
@@ -595,20 +587,20 @@ __device__ __forceinline__ void b_xB(const StepArgs<R> &a, const Blk blk) {
         xsolve_f<W, 22>(d, lane, P, a.c22x);
 #pragma unroll
         for (int t = 0; t < C; ++t) h3[t] = h3[t] + (sizeof(R) == 8 ? fo * d[t] : d[t]);
-        if (j >= 2) srow_load(e, a.eyz + o, sb, lane, P);
+        if (j >= 2) drow_load(e, a.eyz + o, lane, P);
         else {
 #pragma unroll
             for (int t = 0; t < C; ++t) e[t] = R(0);
         }
-        if (j + 1 <= g.n2m) srow_load(ep, a.eyz + op, sb, lane, P);
+        if (j + 1 <= g.n2m) drow_load(ep, a.eyz + op, lane, P);
         else {
 #pragma unroll
             for (int t = 0; t < C; ++t) ep[t] = R(0);
         }
 #pragma unroll
         for (int t = 0; t < C; ++t) h3[t] = h3[t] + rdy * (ep[t] - e[t]);
-        srow_store(a.hh[2] + o, h3, sb, lane, P);
-        ab2_cnx<R, C, W>(a, 2, o, h3, sb, lane, P, dt);
+        drow_store(a.hh[2] + o, h3, lane, P);
+        ab2_cnx<R, C, W>(a, 2, o, h3, lane, P, dt);
     }
 }
 template <typename R, int C, int W = 32>
@@ -638,22 +630,20 @@ template <bool SH, typename R, int C, bool X4 = false, int W = 32>
 __device__ __forceinline__ void xc_row(const StepArgs<R> &a, int j, int k, const typename SType<R>::S *u,
                                        const R *d0, const typename SType<R>::S *vc, const R *dc,
                                        const typename SType<R>::S *vp, const R *dp, const R *zr,
-                                       unsigned char *sbuf, typename Cx<R>::T *bufa, typename Cx<R>::T *bufb,
+                                       typename Cx<R>::T *bufa, typename Cx<R>::T *bufb,
                                        int lane) {
     typedef typename SType<R>::S S;
     typedef typename Cx<R>::T C2;
     static_assert(W == 32 || !X4, "the register row FFT spans a warp");
     const Geo &g = a.g;
     const int P = g.n1m / C, M = g.n1m / 2;
-    S *sbS = reinterpret_cast<S *>(sbuf);
-    R *sbR = reinterpret_cast<R *>(sbuf);
     R *rbuf = reinterpret_cast<R *>(bufa);
     const R rdt = a.rdt, f24 = a.f24x;
     R d[C], base[C];
     if constexpr (sizeof(R) == 8) {   // differences of u + delta; the factor enters below
         R uc[C];
-        xrow<SH>(uc, u, sbS, lane, P);
-        xrow<SH>(d, d0, sbR, lane, P);
+        xrow<SH>(uc, u, lane, P);
+        xrow<SH>(d, d0, lane, P);
 #pragma unroll
         for (int t = 0; t < C; ++t) uc[t] = uc[t] + d[t];
         const R nu = snext<W>(uc[0], lane, P);
@@ -663,8 +653,8 @@ __device__ __forceinline__ void xc_row(const StepArgs<R> &a, int j, int k, const
     } else {
         S uc[C];
         R dd[C];
-        xrow<SH>(uc, u, sbS, lane, P);
-        xrow<SH>(dd, d0, sbR, lane, P);
+        xrow<SH>(uc, u, lane, P);
+        xrow<SH>(dd, d0, lane, P);
         S nu = snext<W>(uc[0], lane, P);
         R nd = snext<W>(dd[0], lane, P);
 #pragma unroll
@@ -679,8 +669,8 @@ __device__ __forceinline__ void xc_row(const StepArgs<R> &a, int j, int k, const
         const bool up = (j + 1 <= g.n2m), lo = (j >= 2);
         S vpv[C], vcv[C];
         R dpv[C], dcv[C];
-        if (up) { xrow<SH>(vpv, vp, sbS, lane, P); xrow<SH>(dpv, dp, sbR, lane, P); }
-        if (lo) { xrow<SH>(vcv, vc, sbS, lane, P); xrow<SH>(dcv, dc, sbR, lane, P); }
+        if (up) { xrow<SH>(vpv, vp, lane, P); xrow<SH>(dpv, dp, lane, P); }
+        if (lo) { xrow<SH>(vcv, vc, lane, P); xrow<SH>(dcv, dc, lane, P); }
         const R ry = a.m.rdy[j] * rdt;   // 1/(DY(J) DT)
         const S zs = S();
 #pragma unroll
@@ -693,7 +683,7 @@ __device__ __forceinline__ void xc_row(const StepArgs<R> &a, int j, int k, const
     }
     {
         R zc[C];
-        xrow<SH>(zc, zr, sbR, lane, P);
+        xrow<SH>(zc, zr, lane, P);
 #pragma unroll
         for (int t = 0; t < C; ++t) d[t] = sizeof(R) == 8 ? d[t] + zc[t] : (base[t] + d[t] * rdt) + zc[t];
     }
@@ -743,9 +733,7 @@ __device__ __forceinline__ void b_xC(const StepArgs<R> &a, const R *d0, const R 
     const int nrows = g.n2m * g.n3m;
     const size_t fbytes = 2 * (size_t)(M + 1) * sizeof(C2);
     if constexpr (NS == 0) {
-        const size_t sbytes = stage_bytes(g.n1m, C);
-        unsigned char *wb = smem_raw + wid * (sbytes + fbytes);
-        C2 *bufa = reinterpret_cast<C2 *>(wb + sbytes);
+        C2 *bufa = reinterpret_cast<C2 *>(smem_raw + wid * fbytes);
         for (int row = blk.x * wpb + wid; row < nrows; row += blk.gx * wpb) {
             const int j = 1 + row / g.n3m, k = row % g.n3m;
             const long long o = fidx(g, 0, j, k), op = fidx(g, 0, j + 1, k);
@@ -755,7 +743,7 @@ __device__ __forceinline__ void b_xC(const StepArgs<R> &a, const R *d0, const R 
                 if (j >= 2) { pf_row(a.v + o, rs_, lane, W); pf_row(d1 + o, rr_, lane, W); }
                 if (j + 1 <= g.n2m) { pf_row(a.v + op, rs_, lane, W); pf_row(d1 + op, rr_, lane, W); }
             }
-            xc_row<false, R, C, X4, W>(a, j, k, a.u + o, d0 + o, a.v + o, d1 + o, a.v + op, d1 + op, a.rdpz + o, wb,
+            xc_row<false, R, C, X4, W>(a, j, k, a.u + o, d0 + o, a.v + o, d1 + o, a.v + op, d1 + op, a.rdpz + o,
                                     bufa, bufa + (M + 1), lane);
         }
     } else {
@@ -804,7 +792,7 @@ __device__ __forceinline__ void b_xC(const StepArgs<R> &a, const R *d0, const R 
             xc_row<true, R, C, X4>(a, j, k, reinterpret_cast<const S *>(st + L.u), reinterpret_cast<const R *>(st + L.d0),
                                reinterpret_cast<const S *>(st + L.vc), reinterpret_cast<const R *>(st + L.dc),
                                reinterpret_cast<const S *>(st + L.vp), reinterpret_cast<const R *>(st + L.dp),
-                               reinterpret_cast<const R *>(st + L.z), nullptr, bufa, bufa + (M + 1), lane);
+                               reinterpret_cast<const R *>(st + L.z), bufa, bufa + (M + 1), lane);
         }
     }
 }
@@ -826,10 +814,7 @@ __device__ __forceinline__ void b_xD(const StepArgs<R> &a, const R *d0, const R 
     const int lane = threadIdx.x & (W - 1), wid = threadIdx.x / W, rpb = (int)blockDim.x / W;
     const int P = g.n1m / C;
     const int M = g.n1m / 2;
-    const size_t sbytes = stage_bytes(g.n1m, C), fbytes = 2 * (size_t)(M + 1) * sizeof(C2);
-    unsigned char *wb = smem_raw + wid * (sbytes + fbytes);
-    R *sbR = reinterpret_cast<R *>(wb);
-    C2 *bufa = reinterpret_cast<C2 *>(wb + sbytes);
+    C2 *bufa = reinterpret_cast<C2 *>(smem_raw) + wid * 2 * (M + 1);
     C2 *bufb = bufa + (M + 1);
     const int nrows = g.n2m * g.n3m;
     const C2 *twx;
@@ -874,7 +859,7 @@ __device__ __forceinline__ void b_xD(const StepArgs<R> &a, const R *d0, const R 
             }
             __syncwarp();
         }
-        srow_store(a.dp + o, dpv, sbR, lane, P);
+        drow_store(a.dp + o, dpv, lane, P);
         R d[C];
         R pv = sprev<W>(dpv[C - 1], lane, P);
 #pragma unroll
@@ -885,7 +870,7 @@ __device__ __forceinline__ void b_xD(const StepArgs<R> &a, const R *d0, const R 
         xsolve_f<W, 22>(d, lane, P, a.c22x);
         // bulk-flow partial sums below: sum_i delta * DY(J)/DX3/DX1 for u and w
         R q1[C], q3[C];
-        srow_load(q1, d0 + o, sbR, lane, P);
+        drow_load(q1, d0 + o, lane, P);
         if constexpr (sizeof(R) == 4) {
             // mixed form: the u update's increment delta1 - DT dDP/dx, formed here in the
             // order UPCALC's update forms it in FP32 (zE then adds it, less dm, to U and
@@ -894,8 +879,8 @@ __device__ __forceinline__ void b_xD(const StepArgs<R> &a, const R *d0, const R 
 #pragma unroll
             for (int t = 0; t < C; ++t) d[t] = q1[t] - dt * d[t];
         }
-        srow_store(a.g1 + o, d, sbR, lane, P);
-        srow_load(q3, d2 + o, sbR, lane, P);
+        drow_store(a.g1 + o, d, lane, P);
+        drow_load(q3, d2 + o, lane, P);
         if constexpr (sizeof(R) == 8) {
             R l1 = R(0), l3 = R(0);
 #pragma unroll
@@ -962,8 +947,6 @@ __global__ void __launch_bounds__(TPB) k_diag_x(StepArgs<R> a, double *divx, Cyc
     const Geo g = a.g;
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     const int P = g.n1m / C;
-    S *sbS = reinterpret_cast<S *>(smem_raw + wid * stage_bytes(g.n1m, C));
-    double *sbD = reinterpret_cast<double *>(sbS);
     const int nrows = g.n2m * g.n3m;
     unsigned long long cmax = 0;
     bool bad = false;
@@ -973,11 +956,11 @@ __global__ void __launch_bounds__(TPB) k_diag_x(StepArgs<R> a, double *divx, Cyc
         const int kp = (k + 1 == g.n3m) ? 0 : k + 1;
         const long long o = fidx(g, 0, j, k), op = fidx(g, 0, j + 1, k), okp = fidx(g, 0, j, kp);
         S su[C], sv[C], svp[C], sw[C], swk[C];
-        srow_load(su, a.u + o, sbS, lane, P);
-        srow_load(sv, a.v + o, sbS, lane, P);
-        srow_load(svp, a.v + op, sbS, lane, P);
-        srow_load(sw, a.w + o, sbS, lane, P);
-        srow_load(swk, a.w + okp, sbS, lane, P);
+        drow_load(su, a.u + o, lane, P);
+        drow_load(sv, a.v + o, lane, P);
+        drow_load(svp, a.v + op, lane, P);
+        drow_load(sw, a.w + o, lane, P);
+        drow_load(swk, a.w + okp, lane, P);
         double uc[C], d[C];
 #pragma unroll
         for (int t = 0; t < C; ++t) uc[t] = ST::dbl(su[t]);
@@ -998,7 +981,7 @@ __global__ void __launch_bounds__(TPB) k_diag_x(StepArgs<R> a, double *divx, Cyc
                 if (cf <= INF_BITS && cf > cmax) cmax = cf;   // not a NaN
             }
         }
-        srow_store(divx + o, d, sbD, lane, P);
+        drow_store(divx + o, d, lane, P);
     }
     warp_max_to(&a.scal[SCAL_CFL], cmax, bad, &a.scal[SCAL_NONFIN]);
 }
