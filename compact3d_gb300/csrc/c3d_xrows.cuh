@@ -785,6 +785,9 @@ __device__ __forceinline__ void b_xC(const StepArgs<R> &a, const R *d0, const R 
             if (lane == 0 && nrow < nrows) issue(nrow, (it + NS - 1) % NS);
             if (!mbar_wait(bar + s, (uint32_t)(it / NS) & 1u)) {
                 if (lane == 0) a.scal[SCAL_PIPEERR] = 1.0;
+                // the copies in flight, of this row and the NS - 1 after it, target this warp's stages
+                for (int q = 0; q < NS && row + q * nw < nrows; ++q)
+                    mbar_wait(bar + (it + q) % NS, (uint32_t)((it + q) / NS) & 1u);
                 return;
             }
             const int j = 1 + row / g.n3m, k = row % g.n3m;
