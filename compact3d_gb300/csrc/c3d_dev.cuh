@@ -247,10 +247,12 @@ template <int OP> __device__ __forceinline__ float zroot(float r) { return r; }
 // where the next factor r^(C 2^b) is below the rounding unit: after one or two for the
 // compact operators and chunks of 4 points or more (a scan over 32 lanes has five).  A level
 // that runs round the ring adds the next period of the periodic sum, so there is no closure.
-template <int W, int DIR>
+// LV levels at most: 12 reach 4096 chunks; more, or a bound that a launch could change, cost
+// xB 4% (192 x 128 x 144 points, 291 -> 304 us), so CN roots past that take their own instance.
+template <int W, int DIR, int LV>
 __device__ __forceinline__ double ring_carry(double e, double m, int lane, int P) {
     int off = 1;
-    for (int b = 0; b < 40 && !negligible(m); ++b) {
+    for (int b = 0; b < LV && !negligible(m); ++b) {
         int src = DIR < 0 ? lane - off : lane + off;
         if (DIR < 0 && src < 0) src += P;
         if (DIR > 0 && src >= P) src -= P;
@@ -285,7 +287,7 @@ __device__ __forceinline__ double ring_carry_op(double e, int lane, int P, int o
 // instructions, and the FP64 pipe bounds the FP64 x passes (192 x 128 x 144 points: xA's
 // pieces 409, 312, 222 -> 264, 240, 152 us, xB 529 -> 353, xC 337 -> 303, xD 279 -> 244).
 // With a compile-time root a chunk's sum takes only its last points that reach the next chunk.
-template <int W, int OP, int C>
+template <int W, int OP, int LV = 12, int C>
 __device__ __forceinline__ void xsolve_ring(double (&x)[C], int lane, int P, const Cyc<double> &c) {
     constexpr int T = croot_len<OP, C>();
     const double r = OP ? Root<OP>::r : c.r, m = OP ? 0.0 : rpow<C>(r);
@@ -293,7 +295,7 @@ __device__ __forceinline__ void xsolve_ring(double (&x)[C], int lane, int P, con
 #pragma unroll
     for (int t = C - T + 1; t < C; ++t) y = x[t] + r * y;
     if constexpr (OP != 0) y = ring_carry_op<W, -1, OP, C>(y, lane, P);
-    else y = ring_carry<W, -1>(y, m, lane, P);
+    else y = ring_carry<W, -1, LV>(y, m, lane, P);
 #pragma unroll
     for (int t = 0; t < C; ++t) {
         y = x[t] + r * y;
@@ -303,7 +305,7 @@ __device__ __forceinline__ void xsolve_ring(double (&x)[C], int lane, int P, con
 #pragma unroll
     for (int t = T - 2; t >= 0; --t) z = x[t] + r * z;
     if constexpr (OP != 0) z = ring_carry_op<W, +1, OP, C>(z, lane, P);
-    else z = ring_carry<W, +1>(z, m, lane, P);
+    else z = ring_carry<W, +1, LV>(z, m, lane, P);
 #pragma unroll
     for (int t = C - 1; t >= 0; --t) {
         z = x[t] + r * z;
@@ -396,9 +398,9 @@ __device__ __forceinline__ void xsolve(R (&x)[C], int lane, int P, const Cyc<R> 
 
 // The same with the FP64 scale left to the caller: xfold(f, c) is the factor f of a
 // right-hand side with the operator's scale folded in (FP64) or f itself.
-template <int W = 32, int OP = 0, typename R, int C>
+template <int W = 32, int OP = 0, int LV = 12, typename R, int C>
 __device__ __forceinline__ void xsolve_f(R (&x)[C], int lane, int P, const Cyc<R> &c) {
-    if constexpr (std::is_same<R, double>::value) xsolve_ring<W, OP>(x, lane, P, c);
+    if constexpr (std::is_same<R, double>::value) xsolve_ring<W, OP, LV>(x, lane, P, c);
     else xsolve<W>(x, lane, P, c);
 }
 __device__ __forceinline__ double xfold(double f, const Cyc<double> &c) { return f * c.s; }

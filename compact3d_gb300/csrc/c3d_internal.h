@@ -2,6 +2,7 @@
 #pragma once
 #include <cuda_runtime.h>
 #include <string>
+#include <cmath>
 #include <vector>
 #include "../../include/c3d.h"
 #include "c3d_dev.cuh"
@@ -331,6 +332,10 @@ void batch_args(c3d_channel *ch, double dt, void *dst);
 int launch_poisson_tables(c3d_channel *ch);
 int ycn_default(const c3d_channel *ch);
 c3d::CnFar cn_far(const c3d_channel *ch, double dt);
+// The Crank-Nicolson root along x, and whether FP64's ring of chunks of C points needs more than
+// 12 levels for it: r^(C 2^12) at or above 2^-56 (q = DT DX1^2 / (2 RE) of 1e4 and more).
+double cn_x_root(const c3d_channel *ch, double dt);
+inline bool cn_x_far(double r, int C) { return std::pow(std::fabs(r), C * 4096.0) >= 0x1p-56; }
 // what: 0 U component, 1 P, 2 HH component, 3 SGSVIS (to host), 4 operand (to device),
 // 5 operator result (to host)
 // ENERGY's plane statistics of the current state into out (N2M x 29, device), with

@@ -524,6 +524,13 @@ static int root_reach(double r, double tol) {
     return m < 1e9 ? (int)m : 1000000000;
 }
 
+double cn_x_root(const c3d_channel *ch, double dt) {
+    double A, B, r, s;
+    cn_coef(ch->g, ch->g.dx1q, dt, A, B);
+    pade_root(A, B, r, s);
+    return r;
+}
+
 CnFar cn_far(const c3d_channel *ch, double dt) {
     const bool f32 = ch->precision != C3D_FP64;
     const int n = ch->g.n3m;

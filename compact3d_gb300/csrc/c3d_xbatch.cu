@@ -18,11 +18,11 @@ __global__ void __launch_bounds__(XMAXT) kb_xA(const StepArgs<R> *__restrict__ A
     const BMap m = map[blockIdx.x];
     b_xA<R, C, PART, W>(A[m.ch], Blk{m.x, m.y, m.gx});
 }
-template <typename R, int C, int W = 32>
+template <typename R, int C, int W = 32, bool FAR = false>
 __global__ void __launch_bounds__(XMAXT) kb_xB(const StepArgs<R> *__restrict__ A, const BMap *__restrict__ map) {
     pdl_enter();
     const BMap m = map[blockIdx.x];
-    b_xB<R, C, W>(A[m.ch], Blk{m.x, m.y, m.gx});
+    b_xB<R, C, W, FAR>(A[m.ch], Blk{m.x, m.y, m.gx});
 }
 template <typename R, int C, bool X4, int W = 32>
 __global__ void __launch_bounds__(XMAXT) kb_xC(const StepArgs<R> *__restrict__ A, const BMap *__restrict__ map) {
@@ -39,6 +39,13 @@ __global__ void __launch_bounds__(XMAXT) kb_xD(const StepArgs<R> *__restrict__ A
     b_xD<R, C, X4, W>(a, a.exz, a.wsq, Blk{m.x, m.y, m.gx});
 }
 
+// xB's kernel for the DT of the step that is captured.
+template <typename R, int C, int W>
+static const void *xb_fn(const c3d_channel *ch) {
+    if (sizeof(R) == 8 && cn_x_far(cn_x_root(ch, ch->dt_cached), C)) return (const void *)kb_xB<R, C, W, sizeof(R) == 8>;
+    return (const void *)kb_xB<R, C, W>;
+}
+
 template <typename R, int C>
 static int xbk(const c3d_channel *ch, int which, int xw, std::vector<BKern> &out) {
     typedef typename Cx<R>::T C2;
@@ -52,7 +59,7 @@ static int xbk(const c3d_channel *ch, int which, int xw, std::vector<BKern> &out
             out.push_back({(const void *)kb_xA<R, C, 2>, nt, 0, nb, 1, 1});
             out.push_back({(const void *)kb_xA<R, C, 3>, nt, 0, nb, 1, 2});
             return 0;
-        case 1: out.push_back({(const void *)kb_xB<R, C>, nt, 0, nb}); return 0;
+        case 1: out.push_back({xb_fn<R, C, 32>(ch), nt, 0, nb}); return 0;
         case 2:
             if (x4) out.push_back({(const void *)kb_xC<R, C, (C % 2 == 0)>, nt, 0, nb});
             else out.push_back({(const void *)kb_xC<R, C, false>, nt, fb, nb});
@@ -84,7 +91,7 @@ static int xbk_seg(const c3d_channel *ch, int which, int xw, std::vector<BKern> 
             out.push_back({(const void *)kb_xA<R, C, 2, W>, nt, 0, nb, 1, 1});
             out.push_back({(const void *)kb_xA<R, C, 3, W>, nt, 0, nb, 1, 2});
             return 0;
-        case 1: out.push_back({(const void *)kb_xB<R, C, W>, nt, 0, nb}); return 0;
+        case 1: out.push_back({xb_fn<R, C, W>(ch), nt, 0, nb}); return 0;
         case 2: out.push_back({(const void *)kb_xC<R, C, false, W>, nt, fb, nb}); return 0;
         case 3: out.push_back({(const void *)kb_xD<R, C, false, W>, nt, fb, nb}); return 0;
         default: return C3D_EINVAL;

@@ -125,7 +125,8 @@ static int launch_x_c(c3d_channel *ch, StepArgs<R> &a, int which, const R *p0, c
             mark(ch, nl, "xA", N * (32 + 7 * Rb));
             break;
         case 1:
-            klaunch(ch, st, k_xB<R, C>, grid, nt, 0, a);
+            if (sizeof(R) == 8 && cn_x_far(a.cnx.r, C)) klaunch(ch, st, k_xB<R, C, 32, sizeof(R) == 8>, grid, nt, 0, a);
+            else klaunch(ch, st, k_xB<R, C>, grid, nt, 0, a);
             mark(ch, nl, "xB", N * 18 * Rb);
             break;
         case 2: {
@@ -224,7 +225,8 @@ static int launch_x_seg(c3d_channel *ch, StepArgs<R> &a, int which, const R *p0,
         mark(ch, nl, "xA_w", N * (8 + 2 * Rb));
         if (cc && (rc = par_join(ch))) return rc;
     } else {
-        klaunch(ch, st, k_xB<R, C, W>, grid, nt, 0, a);
+        if (sizeof(R) == 8 && cn_x_far(a.cnx.r, C)) klaunch(ch, st, k_xB<R, C, W, sizeof(R) == 8>, grid, nt, 0, a);
+        else klaunch(ch, st, k_xB<R, C, W>, grid, nt, 0, a);
         mark(ch, nl, "xB", N * 18 * Rb);
     }
     return 0;

@@ -491,7 +491,7 @@ __global__ void __launch_bounds__(XMAXT, 3) k_xAs(StepArgs<R> a) {
 // ---------------------------------------------------------------------------------
 // xB: remaining convective terms, AB2, x factor of Crank-Nicolson
 // ---------------------------------------------------------------------------------
-template <typename R, int C, int W = 32>
+template <typename R, int C, int W, bool FAR>
 __device__ __forceinline__ void ab2_cnx(const StepArgs<R> &a, int c, long long o, const R (&hc)[C], int lane, int P, R dt) {
     // FP64: (1,10,1)/(A,B,A) = (1 + (10 - B/A) z / (1 + B/A z + z^2)) / A with the factors kx,
     // unless B/A is so far from 10 that the two terms would cancel (cn_factors)
@@ -513,7 +513,7 @@ __device__ __forceinline__ void ab2_cnx(const StepArgs<R> &a, int c, long long o
             d[t] = (l + (R)10.0 * rr[t]) + r2;
         }
     }
-    xsolve_f<W>(d, lane, P, a.cnx);
+    xsolve_f<W, 0, FAR ? 64 : 12>(d, lane, P, a.cnx);
     if (pf) {
 #pragma unroll
         for (int t = 0; t < C; ++t) d[t] = rr[t] + a.kx[1] * d[t];
@@ -521,7 +521,8 @@ __device__ __forceinline__ void ab2_cnx(const StepArgs<R> &a, int c, long long o
     drow_store(a.r[c] + o, d, lane, P);
 }
 
-template <typename R, int C, int W = 32>
+// FAR: FP64 with a CN root past 12 levels of the ring (cn_x_far).
+template <typename R, int C, int W = 32, bool FAR = false>
 __device__ __forceinline__ void b_xB(const StepArgs<R> &a, const Blk blk) {
     const Geo g = a.g;
     const int lane = threadIdx.x & (W - 1), wid = threadIdx.x / W, rpb = (int)blockDim.x / W;
@@ -558,7 +559,7 @@ __device__ __forceinline__ void b_xB(const StepArgs<R> &a, const Blk blk) {
 #pragma unroll
         for (int t = 0; t < C; ++t) h1[t] = h1[t] + rdy * (ep[t] - e[t]);   // d(uv)/dy
         drow_store(a.hh[0] + o, h1, lane, P);
-        ab2_cnx<R, C, W>(a, 0, o, h1, lane, P, dt);
+        ab2_cnx<R, C, W, FAR>(a, 0, o, h1, lane, P, dt);
         if (j >= 2) {
             R h2[C];
             drow_load(h2, a.hh[1] + o, lane, P);
@@ -572,7 +573,7 @@ __device__ __forceinline__ void b_xB(const StepArgs<R> &a, const Blk blk) {
 #pragma unroll
             for (int t = 0; t < C; ++t) h2[t] = h2[t] + (sizeof(R) == 8 ? fo * d[t] : d[t]);                 // d(uv)/dx
             drow_store(a.hh[1] + o, h2, lane, P);
-            ab2_cnx<R, C, W>(a, 1, o, h2, lane, P, dt);
+            ab2_cnx<R, C, W, FAR>(a, 1, o, h2, lane, P, dt);
         }
         // d(uw)/dx from E_xz, d(wv)/dy from E_yz at faces j, j+1
         drow_load(e, a.exz + o, lane, P);
@@ -600,13 +601,13 @@ __device__ __forceinline__ void b_xB(const StepArgs<R> &a, const Blk blk) {
 #pragma unroll
         for (int t = 0; t < C; ++t) h3[t] = h3[t] + rdy * (ep[t] - e[t]);
         drow_store(a.hh[2] + o, h3, lane, P);
-        ab2_cnx<R, C, W>(a, 2, o, h3, lane, P, dt);
+        ab2_cnx<R, C, W, FAR>(a, 2, o, h3, lane, P, dt);
     }
 }
-template <typename R, int C, int W = 32>
+template <typename R, int C, int W = 32, bool FAR = false>
 __global__ void __launch_bounds__(XMAXT) k_xB(StepArgs<R> a) {
     pdl_enter();
-    b_xB<R, C, W>(a, Blk{blockIdx.x, blockIdx.y, gridDim.x});
+    b_xB<R, C, W, FAR>(a, Blk{blockIdx.x, blockIdx.y, gridDim.x});
 }
 
 // ---------------------------------------------------------------------------------

@@ -53,6 +53,35 @@ def test_step_past_the_sign_change(oracle_mod, prec, n1m, n3m, q3):
     check(g, got, (U, P), prec, dt)
 
 
+# roots within 1e-3 of 1 in x (1, 3 and 4 points a lane: segments, whole warps with and without
+# idle lanes), which the ring's usual levels do not reach round
+@pytest.mark.gpu
+@pytest.mark.parametrize("n1m,batch", [(18, False), (24, False), (48, False), (108, False), (48, True)])
+def test_roots_near_one(oracle_mod, n1m, batch):
+    from compact3d_gb300 import build, lib
+    build.build()
+    q = 1e6
+    g, dt = grid(n1m, 16, q * (32 / n1m) ** 2, C3D_FP64)
+    orc = oracle_mod.Oracle(g)
+    U, P, HH = ic.perturbed_laminar(g)
+    orc.project(U)
+    ch = lib.Batch([g]) if batch else lib.Channel(g)
+    one = ch.channels[0] if batch else ch
+    one.upload(U, P, HH)
+    orc.getup(U, P, HH, 1, dt, 0.0, 0.0)
+    if batch:
+        ch.step(1, [dt], [0.0], [0.0])
+    else:
+        ch.step(1, dt, 0.0, 0.0)
+    Ug = one.download()[0]
+    ch.close()
+    # the explicit terms' rounding, 12 q a term, which the solve passes on in its lowest modes
+    tol = 100 * q * np.finfo(float).eps
+    i, k = slice(1, g.n1m + 1), slice(1, g.n3m + 1)
+    a, b = (f[i, 1:g.n2m + 1, k] for f in (Ug, U))
+    assert np.linalg.norm(a - b) < tol * np.linalg.norm(b)
+
+
 @pytest.mark.gpu
 @pytest.mark.parametrize("prec", [C3D_FP64, C3D_MIXED])
 def test_batch_past_the_sign_change(oracle_mod, prec):
