@@ -690,8 +690,8 @@ int c3d_create(const c3d_grid *gr, c3d_channel **out) {
     ch->dt_cached = -1.0;
     ch->cur = 0;
     // not with SGSSD, whose coefficients take 130 us on a side stream beside the step's kernels:
-    // with the attribute the two streams hold each other up (128 x 64 x 128 points, mixed: 824 to
-    // 1046 us a step, without it 664)
+    // measured slower with the attribute (128 x 64 x 128 points, mixed: 824 to 1046 us a step,
+    // without it 664); the cause is not known.  The wall models' side streams keep it
     ch->pdl = ch->files != 3;
     cudaError_t e = cudaDeviceSynchronize();
     if (e != cudaSuccess) {

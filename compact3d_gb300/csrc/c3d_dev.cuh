@@ -13,12 +13,15 @@
 //   tridiag(a, b, a) = (-a/r) (1 - r S)(1 - r S^-1)      (S = cyclic shift)
 // so x = s * B(F(d)) with s = -r/a, F: y_i = d_i + r y_{i-1} and B: z_i = y_i + r z_{i+1},
 // both cyclic.  The kernels evaluate these two first-order recurrences:
-//   * along x (contiguous rows): one warp per row (or, for rows of 48-128 points, a
-//     segment of 8 or 16 lanes per row), every lane owns C consecutive points, and the
-//     cyclic carries between lanes come from shuffle scans of affine maps;
-//   * along z (strided columns): one thread per (column, segment of L points); the cyclic
-//     start values come from a warm-up of M points, M chosen so |r|^M is below the
-//     working precision's rounding unit.
+//   * along x (contiguous rows): one warp per row (or, for short rows, a segment of 8 or 16
+//     lanes per row), every lane owns C consecutive points, and the cyclic carries between
+//     lanes come from shuffle scans of affine maps (FP32 and double-float: xsolve_full,
+//     xsolve_general) or from doubling round the ring of lanes until the next power of r^C
+//     is below rounding (FP64: xsolve_ring);
+//   * along z (strided columns): one thread per (column, segment of L points).  FP32 and
+//     double-float start each recurrence M points early (zsweep), M chosen so |r|^M is below
+//     the working precision's rounding unit; FP64, and FP32 where the schedule says so, joins
+//     the segments of a line through shared memory (zjoin), which reach as far.
 // The result equals the reference's bordered-LU solution to rounding.
 #pragma once
 #include <cuda_runtime.h>
@@ -244,8 +247,9 @@ template <int OP> __device__ __forceinline__ float zroot(float r) { return r; }
 // What enters each lane's chunk in the FP64 recurrences of one direction: e = the chunk's own
 // sum, m = r^C.  The sums of the lanes before it (DIR -1) or after it (DIR +1) are added over
 // a ring of P lanes by doubling, each level covering twice the lanes, and the levels stop
-// where the next factor r^(C 2^b) is below the rounding unit: after one or two for the
-// compact operators and chunks of 4 points or more (a scan over 32 lanes has five).  A level
+// where the next factor r^(C 2^b) is below the rounding unit: for the compact operators after
+// three at most with chunks of 4 points or more (r^16 is 2^-41 for (1,6,1), 2^-53 for (1,10,1),
+// 2^-71 for (1,22,1)), two with chunks of 8 (a scan over 32 lanes has five).  A level
 // that runs round the ring adds the next period of the periodic sum, so there is no closure.
 // LV levels at most: 12 reach 4096 chunks; more, or a bound that a launch could change, cost
 // xB 4% (192 x 128 x 144 points, 291 -> 304 us), so CN roots past that take their own instance.

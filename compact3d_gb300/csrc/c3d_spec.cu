@@ -134,7 +134,8 @@ __global__ void __launch_bounds__(FZW * 32) k_fftz4(StepArgs<R> a) {
 // while the other computes), positions are 32-bit, and the tables' planes up to UPF further on
 // are requested from DRAM into L2.  Against a thread per mode with guarded batches (55 to 78
 // instructions a plane): 64^3 points, FP64, 31 -> 18 us, 192 x 128 x 144 67 -> 37, mixed
-// 128 x 96 x 128 27 -> 23, 256 x 192 x 256 111 -> 109.
+// 128 x 96 x 128 27 -> 23, 256 x 192 x 256 111 -> 109; 384 x 256 x 384 points, with modes
+// enough for every SM, is slower: 132 -> 151.
 constexpr int UJ = 8, UPF = 32;
 
 // The warp's 16 modes of a table's rows (`row` points at the calling thread's own value) at UJ

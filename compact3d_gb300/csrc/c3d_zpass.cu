@@ -1,6 +1,7 @@
-// c3d_zpass.cu -- z-column passes of the step: one thread per (i, segment of ZL points,
+// c3d_zpass.cu -- z-column passes of the step: one thread per (i, segment of L points,
 // plane j); consecutive threads take consecutive i, so every access is coalesced.  The
-// cyclic compact solves use the warm-up recurrences of zseg (c3d_dev.cuh).
+// cyclic compact solves run with warm-ups (zsweep: FP32) or with the segments of a line
+// joined in the block (zjoin: FP64, and FP32 under schedule 0).
 //   zA  RHS1/2/3 pieces along z (compact3d.f:6160-6185, 6337-6433, 6957-7060, 7474-7705)
 //   zB  d(uw)/dz, d(vw)/dz, d(ww)/dz (1,22,1)
 //   zC  z factor of Crank-Nicolson (CTDMA3I in GETUH1-3)
